@@ -593,22 +593,30 @@ int Ctx::step_ctx(StepCtx &S) {
   S.plan = DevPlan{plan[0].n, plan[0].dst, plan[0].src};
   const double *const *g = (const double *const *)stepgeo;
   S.GRD_x = g[0], S.GRD_x_pl = g[1], S.cg = g[2], S.cg_pl = g[3], S.rdgz = g[4], S.afact = g[5], S.bfact = g[6];
+  rc0 = build_fast_tables();
+  if (rc0) return rc0;
+  S.nb = fast.nb, S.ns = fast.ns, S.bsrc = fast.bsrc, S.seam = fast.seam_list, S.ring = fast.ring;
   struct B {
     double **p;
     const char *name;
     size_t n;
   } bl[] = {{&S.flx, "st_flx", n3 * 6}, {&S.flx_pl, "st_flxp", n3p}, {&S.xc, "st_xc", n3 * 9},
-            {&S.xc_pl, "st_xcp", n3p * 3}, {&S.ch, "st_ch", n3 * 6}, {&S.ch_pl, "st_chp", n3p},
-            {&S.cm, "st_cm", n3 * 6}, {&S.cm_pl, "st_cmp", n3p}, {&S.zero, "st_zero", n3},
-            {&S.zero_pl, "st_zerop", n3p}, {&S.q, "st_q", n3}, {&S.q_pl, "st_qp", n3p},
-            {&S.grad, "st_grad", n3 * 3}, {&S.grad_pl, "st_gradp", n3p * 3}, {&S.qa, "st_qa", n3 * 6},
-            {&S.qa_pl, "st_qap", n3p}, {&S.qout, "st_qout", n3 * 2}, {&S.qout_pl, "st_qoutp", n3p * 2},
-            {&S.qin_pl, "st_qinp", n3p * 4}};
+            {&S.xc_pl, "st_xcp", n3p * 3}, {&S.fv, "st_work", n3 * 3 * kPlainGroup}, {&S.ch_pl, "st_chp", n3p},
+            {&S.cm_pl, "st_cmp", n3p}, {&S.zero, "st_zero", n3},
+            {&S.zero_pl, "st_zerop", n3p}, {&S.q_pl, "st_qp", n3p},
+            {&S.grad_pl, "st_gradp", n3p * 3},
+            {&S.qa_pl, "st_qap", n3p}, {&S.qout_pl, "st_qoutp", n3p * 2},
+            {&S.qin_pl, "st_qinp", n3p * 4},
+            {&S.bb, "st_bb", (size_t)kPlainGroup * sz.kall * fast.nb * 5}};
   bool fresh_zero = bufs.find("st_zero") == bufs.end();
   for (auto &b : bl) {
     *b.p = (double *)buf(b.name, b.n * sizeof(double));
     if (!*b.p) return set_error(std::string("cudaMalloc ") + b.name), ICA_ERR_NOMEM;
   }
+  // the adjoint's fields of one tracer share the face values' memory: 24 fields
+  static_assert(3 * kPlainGroup == 24, "ch 6, cm 6, q 1, grad 3, qa 6, qout 2");
+  S.ch = S.fv, S.cm = S.fv + 6 * n3, S.q = S.fv + 12 * n3, S.grad = S.fv + 13 * n3, S.qa = S.fv + 16 * n3;
+  S.qout = S.fv + 22 * n3;
   if (fresh_zero) {
     cudaMemsetAsync(S.zero, 0, n3 * sizeof(double), stream);
     cudaMemsetAsync(S.zero_pl, 0, n3p * sizeof(double), stream);
@@ -663,7 +671,7 @@ int ica_advect_step_dev(ica_ctx *c, int ntr, double dt, double *rhog, double *rh
   if (rc) return rc;
   rc = step_plain(S, ntr, dt, rhog, rhog_pl, rhogq, rhogq_pl, vx, vx_pl, vy, vy_pl, vz, vz_pl, w, w_pl, c->stream,
                   c->launches);
-  if (rc) return set_error("ica_advect_step: kall above 128"), rc;
+  if (rc) return rc;
   return c->check_launch("ica_advect_step");
 }
 
@@ -828,7 +836,7 @@ int ica_adjoint_record(ica_ctx *c, int ntr, double dt, int nsteps, int every, do
     if (s % every == 0) copy_state(c, state_at(c, ck + (size_t)(s / every) * sd, ntr), rhog, rhog_pl, rhogq, rhogq_pl, ntr);
     rc = step_plain(S, ntr, dt, rhog, rhog_pl, rhogq, rhogq_pl, vx, vx_pl, vy, vy_pl, vz, vz_pl, w, w_pl, c->stream,
                     c->launches);
-    if (rc) return set_error("ica_adjoint_record: kall above 128"), rc;
+    if (rc) return rc;
   }
   c->tape = AdjTape{true, ntr, nsteps, every, dt};
   return c->check_launch("ica_adjoint_record");
@@ -867,7 +875,7 @@ int ica_adjoint_sweep(ica_ctx *c, const double *vx, const double *vx_pl, const d
       copy_state(c, st[u], st[u - 1].r, st[u - 1].rp, st[u - 1].q, st[u - 1].qp, T.ntr);
       rc = step_plain(S, T.ntr, T.dt, st[u].r, st[u].rp, st[u].q, st[u].qp, vx, vx_pl, vy, vy_pl, vz, vz_pl, w, w_pl,
                       c->stream, c->launches);
-      if (rc) return set_error("ica_adjoint_sweep: kall above 128"), rc;
+      if (rc) return rc;
     }
     for (int u = L - 1; u >= 0; --u) {
       rc = step_adjoint(S, A, T.ntr, T.dt, st[u].r, st[u].rp, st[u].q, st[u].qp, vx, vx_pl, vy, vy_pl, vz, vz_pl, w,

@@ -1,7 +1,8 @@
-// The composed tracer step, plain FP64 path: the reference kernels chained with
-// the pieces the reference leaves out (Courant numbers, gradient, remap,
-// rhogq update, vertical flux), one kernel each, tracer by tracer.  This is
-// the "plain per-tracer" GPU path; the batched path is fast_kernels.cu.
+// The composed tracer step, plain FP64 path: the reference kernels' operations
+// with the pieces the reference leaves out (Courant numbers, gradient, remap,
+// rhogq update, vertical flux), fused into three launches per group of tracers
+// (below).  The one-kernel-per-piece forms that come first serve the adjoint's
+// recompute.  The FP32 / FP64 batched path is fast_kernels.cu.
 //
 // The composition (horizontal sub-step, then vertical sub-step, then the halo
 // fill of the state) and every formula match the CPU oracle's definition of
@@ -131,26 +132,6 @@ __global__ void k_remap_pl(int kall, const double *q_pl, const double *grad_pl, 
   qa_pl[off + v] = cc * vu + (1.0 - cc) * vs;
 }
 
-// rhogq -= sum_m flx_h(m) q_a(m) at interior cells (all levels); pole centres
-__global__ void k_update_h(Dims D, const double *flx, const double *qa, double *Q) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, G = D.gall_1d;
-  const int i = c % G + 1, j = c / G + 1;
-  if (i < D.gmin || i > D.gmax || j < D.gmin || j > D.gmax) return;
-  const size_t off = (size_t)kl * D.gall + c, fs = (size_t)D.lall * D.kall * D.gall;
-  double s = flx[off] * qa[off];
-  for (int m = 1; m < 6; ++m) s = s + flx[m * fs + off] * qa[m * fs + off];
-  Q[off] = Q[off] - s;
-}
-__global__ void k_update_h_pl(int kall, const double *flx_pl, const double *qa_pl, double *Qp) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kLallPl * kall) return;
-  const size_t off = (size_t)t * kGallPl;
-  double s = flx_pl[off + 1] * qa_pl[off + 1];
-  for (int v = 3; v <= 6; ++v) s = s + flx_pl[off + v - 1] * qa_pl[off + v - 1];
-  Qp[off] = Qp[off] - s;
-}
 // rhog -= sum_m flx_h(m)
 __global__ void k_update_rho(Dims D, const double *flx, double *rho) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -172,99 +153,553 @@ __global__ void k_update_rho_pl(int kall, const double *flx_pl, double *rho_pl) 
   rho_pl[off] = rho_pl[off] - s;
 }
 
-// Thuburn vertical bounds of level k (0-based) of one column, region form (:107-142)
-struct VCol {
-  const double *q, *ck1, *ck2;
+// ---------------------------------------------------------------------------
+// The step itself: the tracers go through in groups of up to kPlainGroup, three launches a group.
+//
+//   k_plain_cells  one thread per interior cell, a tile's levels and tracers streamed through: the
+//                  gradient, Qout and the 4-point bounds of the cell's six faces from q in shared
+//                  memory, and the limited value of each of its outflow faces (the faces whose
+//                  upwind cell it is), which needs nothing but what the thread then holds.  Gradient
+//                  and Qout go to memory at region-boundary cells and pole centres only (bb), the
+//                  values halo cells stand for.
+//   k_plain_seam   the limited value of the faces with a halo cell on one side, per region as the
+//                  reference computes them (each side in its own index frame), from bb.
+//   k_plain_column rhogq after the horizontal sub-step, formed level by level from the six face
+//                  values, and the vertical sub-step of the column as it streams by, in place.
+//
+// A face value travels once through memory (24 bytes written and read per update); gradient,
+// remap value, Courant number, mask and Qout never do.  Against one launch per piece and tracer
+// (14 launches a tracer, a column's levels in local memory): 9.90 -> 5.27 ms for glevel 7, kall 61,
+// 5 tracers, 1.59 -> 0.49 ms for glevel 5, kall 42, 8 tracers.  Every value is the result of the
+// reference's operation sequence; where the reference blends two sides by a mask of 0 or 1
+// (c a + (1 - c) b), the chosen side is taken, which is the same number.
+constexpr int kTileCells = 256;  // threads of k_plain_cells: one per cell of a TX x (256 / TX) tile
+constexpr int kPair = 2;         // tracers a thread of k_plain_cells / k_plain_column takes at once
+
+struct PlainArgs {
+  Dims D;
+  int nt, nb, ns;                    // tracers of the group; boundary entries, seam faces
+  double dt;
+  double *Q, *Qp;                    // the group's rhogq
+  const double *rho, *rhop, *w, *wp, *flx, *flxp, *xc, *xcp;
+  const double *GRD_x, *GRD_xp, *cg, *cgp, *rdgz, *afact, *bfact;
+  const int *bsrc, *seam, *ring;     // boundary entry of a point, seam face codes, pole ring's entries
+  double *fv;                        // (nt, 3, lall, kall, gall): limited values of faces AI, AIJ, AJ of their owner
+  double *bb;                        // (nt, kall, nb, 5): gradient x/y/z, Qout min / max
+  __device__ size_t n3() const { return (size_t)D.lall * D.kall * D.gall; }
+  __device__ size_t n3p() const { return (size_t)kLallPl * D.kall * kGallPl; }
+  __device__ double *bval(int t, int k, int b) const { return bb + (((size_t)t * D.kall + k) * nb + b) * 5; }
+  __device__ bool inner(int i, int j) const { return i >= D.gmin && i <= D.gmax && j >= D.gmin && j <= D.gmax; }
 };
-__device__ __forceinline__ void vqout(const double *q, const double *ck1, const double *ck2, int k, double &inflagL,
-                                      double &Qmin, double &Qmax) {
-  const double BIG = DBL_MAX, EPS = DBL_EPSILON;
-  inflagL = 0.5 - sgn(0.5, ck1[k]);
-  const double inflagU = 0.5 + sgn(0.5, ck1[k + 1]);
-  const double qk = q[k], qm = q[k - 1], qp = q[k + 1];
-  const double minL = ((qm < qk) ? qm : qk) + (1.0 - inflagL) * BIG;
-  const double minU = ((qp < qk) ? qp : qk) + (1.0 - inflagU) * BIG;
-  const double maxL = ((qm > qk) ? qm : qk) - (1.0 - inflagL) * BIG;
-  const double maxU = ((qp > qk) ? qp : qk) - (1.0 - inflagU) * BIG;
-  double qnmin = (minU < minL) ? minU : minL;
-  qnmin = (qk < qnmin) ? qk : qnmin;
-  double qnmax = (maxU > maxL) ? maxU : maxL;
-  qnmax = (qk > qnmax) ? qk : qnmax;
-  const double c1 = ck1[k], c2 = ck2[k];
-  const double Cin = inflagL * c1 + inflagU * c2;
-  const double Cout = (1.0 - inflagL) * c1 + (1.0 - inflagU) * c2;
-  const double CQmin = inflagL * c1 * minL + inflagU * c2 * minU;
-  const double CQmax = inflagL * c1 * maxL + inflagU * c2 * maxU;
-  const double zerosw = 0.5 - sgn(0.5, fabs(Cout) - EPS);
-  const double dv = 0.0;
-  Qmin = ((qk - qnmax) + qnmax * (Cin + Cout - dv) - CQmax) / (Cout + zerosw) * (1.0 - zerosw) + qk * zerosw;
-  Qmax = ((qk - qnmin) + qnmin * (Cin + Cout - dv) - CQmin) / (Cout + zerosw) * (1.0 - zerosw) + qk * zerosw;
+
+__device__ __forceinline__ double mn(double a, double b) { return (b < a) ? b : a; }
+__device__ __forceinline__ double mx(double a, double b) { return (b > a) ? b : a; }
+__device__ __forceinline__ double mn4(double a, double b, double c, double d) { return mn(mn(mn(a, b), c), d); }
+__device__ __forceinline__ double mx4(double a, double b, double c, double d) { return mx(mx(mx(a, b), c), d); }
+// cmask of a Courant number: true where it is 1 (the face's neighbour is its upwind cell)
+__device__ __forceinline__ bool upmask(double ch) { return 0.5 - sgn(0.5, ch - DBL_EPSILON) != 0.0; }
+
+// pole centre (p, k) of tracer t: gradient and Qout (mod_src_tracer.f90:307-367) into bb
+__device__ __forceinline__ void pole_centre(const PlainArgs &P, int t, int p, int k) {
+  const double BIG = DBL_MAX;
+  const size_t off = ((size_t)p * P.D.kall + k) * kGallPl;
+  double q[kGallPl];
+  for (int v = 0; v < kGallPl; ++v) q[v] = P.Qp[t * P.n3p() + off + v] / P.rhop[off + v];
+  double *o = P.bval(t, k, P.nb - 2 + p);
+  for (int x = 0; x < 3; ++x) {
+    const double *cx = P.cgp + ((size_t)p * 3 + x) * 6;
+    double s = cx[0] * q[0];
+    for (int v = 1; v < 6; ++v) s = s + cx[v] * q[v];
+    o[x] = s;
+  }
+  double qnmin = q[0], qnmax = q[0], Cin = 0, Cout = 0, CQmax = 0, CQmin = 0;
+  for (int v = 1; v <= 5; ++v) {
+    const int vp = (v == 5) ? 1 : v + 1, vm = (v == 1) ? 5 : v - 1;
+    const double ch = P.flxp[off + v] / P.rhop[off];
+    const double c = upmask(ch) ? 1.0 : 0.0;
+    const double qmin = c * mn4(q[0], q[v], q[vm], q[vp]) + (1.0 - c) * BIG;
+    const double qmax = c * mx4(q[0], q[v], q[vm], q[vp]) + (1.0 - c) * (-BIG);
+    qnmin = mn(qnmin, qmin), qnmax = mx(qnmax, qmax);
+    const double chm = c * ch;
+    Cin = Cin + chm;
+    Cout = Cout - chm + ch;
+    CQmin = CQmin + chm * qmin;
+    CQmax = CQmax + chm * qmax;
+  }
+  const double zsw = 0.5 - sgn(0.5, fabs(Cout) - DBL_EPSILON), dn = 0.0;
+  o[3] = (q[0] - CQmax - qnmax * (1.0 - Cin - Cout + dn)) / (Cout + zsw) * (1.0 - zsw) + q[0] * zsw;
+  o[4] = (q[0] - CQmin - qnmin * (1.0 - Cin - Cout + dn)) / (Cout + zsw) * (1.0 - zsw) + q[0] * zsw;
 }
 
-// vertical sub-step of one column (interior columns and the two pole centres)
-template <int KMAX>
-__global__ void k_vertical(Dims D, int ntr, double dt, double *rho, double *Q, const double *w, double *rho_pl,
-                           double *Qp, const double *w_pl, const double *rdgz, const double *afact,
-                           const double *bfact) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ncol = D.lall * D.gall;
-  double *R, *QQ;
+template <int TX>
+struct CellSmem {
+  static constexpr int TY = kTileCells / TX, WW = TX + 2, NW = WW * (TY + 2);  // window: the tile and one ring
+  static constexpr int OW = TX + 1, NO = OW * (TY + 1);                        // owners of the tile's faces
+  double cg[21][kTileCells];
+  double disp[9][NO];              // [face * 3 + x][owner]: xc - x(upwind cell), read by the upwind cell's thread
+  double rho[NW];
+  double q[2][kPair][NW];
+};
+
+// grid: blocks 0 .. ntile*nlb-1 (level block fastest: a tile's gradient coefficients come from L2
+// after the first), then the pole centres
+template <int TX>
+__global__ void __launch_bounds__(kTileCells, 2) k_plain_cells(PlainArgs P, int ntx, int nty, int nlb, int lpb) {
+  using S = CellSmem<TX>;
+  extern __shared__ __align__(16) unsigned char raw[];
+  S &s = *reinterpret_cast<S *>(raw);
+  const Dims &D = P.D;
+  const int G = D.gall_1d, tid = threadIdx.x;
+  const int nmain = ntx * nty * D.lall * nlb;
+  if ((int)blockIdx.x >= nmain) {
+    const int u = ((int)blockIdx.x - nmain) * kTileCells + tid;
+    if (u < P.nt * kLallPl * D.kall) pole_centre(P, u / (kLallPl * D.kall), u / D.kall % kLallPl, u % D.kall);
+    return;
+  }
+  const int lb = (int)blockIdx.x % nlb, tile = (int)blockIdx.x / nlb;
+  const int l = tile / (ntx * nty), tr = tile % (ntx * nty);
+  const int i0 = D.gmin + (tr % ntx) * TX, j0 = D.gmin + (tr / ntx) * S::TY;  // first cell, 1-based
+  const int x = tid % TX, y = tid / TX, i = i0 + x, j = j0 + y;
+  const bool act = i <= D.gmax && j <= D.gmax;
+  const int c = act ? (j - 1) * G + (i - 1) : 0;
+  const bool sing = D.have_sgp[l] != 0 && i == D.gmin && j == D.gmin;
+  const int bs = act ? P.bsrc[(size_t)l * D.gall + c] : -1;
+  const size_t n3 = P.n3(), gw = (size_t)D.lall * D.gall;
+#pragma unroll
+  for (int n = 0; n < 21; ++n) s.cg[n][tid] = act ? P.cg[((size_t)l * 21 + n) * D.gall + c] : 0.0;
+  // this thread's window slots and their cells (-1: none)
+  constexpr int NSLOT = (S::NW + kTileCells - 1) / kTileCells;
+  int wc[NSLOT];
+#pragma unroll
+  for (int r = 0; r < NSLOT; ++r) {
+    const int e = tid + r * kTileCells, wi = i0 - 1 + e % S::WW, wj = j0 - 1 + e / S::WW;  // >= 1
+    wc[r] = (e < S::NW && wi <= G && wj <= G) ? (wj - 1) * G + (wi - 1) : -1;
+  }
+  const int ew = (y + 1) * S::WW + x + 1;
+  const int wn[7] = {ew, ew + 1, ew + S::WW + 1, ew + S::WW, ew - 1, ew - S::WW - 1, ew - S::WW};
+  // face m (1..6): its owner's slot, owner cell and other cell
+  const int ow = (y + 1) * S::OW + x + 1;
+  const int os[7] = {0, ow, ow, ow, ow - 1, ow - S::OW - 1, ow - S::OW};
+  const int oc[7] = {0, c, c, c, c - 1, c - G - 1, c - G};
+  unsigned both = 0;  // bit m: the cell across face m is interior too (not a seam face)
+  if (act) {
+    constexpr int DX[7] = {0, 1, 1, 0, -1, -1, 0}, DY[7] = {0, 0, 1, 1, 0, -1, -1};
+#pragma unroll
+    for (int m = 1; m <= 6; ++m) both |= P.inner(i + DX[m], j + DY[m]) ? 1u << m : 0u;
+  }
+  const int kfirst = D.kmin - 1, kend = D.kmax;  // physical levels, 0-based
+  const int k0 = kfirst + lb * lpb, k1 = min(k0 + lpb, kend);
+  const double BIG = DBL_MAX;
+  for (int k = k0; k < k1; ++k) {
+    const size_t off = ((size_t)l * D.kall + k) * D.gall;
+    double Qw[NSLOT][kPair], rw[NSLOT];
+    auto load = [&](int t0) {
+#pragma unroll
+      for (int r = 0; r < NSLOT; ++r)
+        if (wc[r] >= 0) {
+#pragma unroll
+          for (int h = 0; h < kPair; ++h) Qw[r][h] = P.Q[(size_t)min(t0 + h, P.nt - 1) * n3 + off + wc[r]];
+        }
+    };
+    load(0);
+    __syncthreads();  // the previous level's shared data is read
+#pragma unroll
+    for (int r = 0; r < NSLOT; ++r) {
+      rw[r] = 1.0;
+      if (wc[r] >= 0) s.rho[tid + r * kTileCells] = rw[r] = P.rho[off + wc[r]];
+    }
+    __syncthreads();
+    // ---- tracer-independent: Courant numbers, upwind sides, outflow sums, displacements
+    double chm[7] = {}, omc = 0.0, den = 1.0, zsw = 1.0;
+    unsigned in = 0, out = 0;
+    if (act) {
+      const double rc = s.rho[ew];
+      double ch[7];
+#pragma unroll
+      for (int m = 1; m <= 6; ++m) {
+        ch[m] = P.flx[(size_t)(m - 1) * n3 + off + c] / rc;
+        chm[m] = mn(ch[m], 0.0);
+        // the owner's mask: 1 takes the owner's neighbour as the upwind cell
+        const bool cm = (m <= 3) ? upmask(ch[m]) : upmask(P.flx[(size_t)(m - 4) * n3 + off + oc[m]] / s.rho[wn[m]]);
+        if (cm == (m <= 3)) in |= 1u << m;
+        else if ((both >> m) & 1u) out |= 1u << m;
+      }
+      const double Cin = chm[1] + chm[2] + chm[3] + chm[4] + chm[5] + chm[6];
+      const double Cout =
+          ch[1] - chm[1] + ch[2] - chm[2] + ch[3] - chm[3] + ch[4] - chm[4] + ch[5] - chm[5] + ch[6] - chm[6];
+      const double dv = 0.0;
+      zsw = 0.5 - sgn(0.5, fabs(Cout) - DBL_EPSILON);
+      den = Cout + zsw;
+      omc = 1.0 - Cin - Cout + dv;
+#pragma unroll
+      for (int m = 1; m <= 6; ++m)
+        if ((out >> m) & 1u) {
+          const int a = (m - 1) % 3;
+#pragma unroll
+          for (int d = 0; d < 3; ++d)
+            s.disp[a * 3 + d][os[m]] = P.xc[((size_t)d * 3 + a) * n3 + off + oc[m]] - P.GRD_x[d * gw + (size_t)l * D.gall + c];
+        }
+    }
+    // ---- the tracers, two at a time; q of a pair alternates between two buffers
+    for (int t0 = 0, b = 0; t0 < P.nt; t0 += kPair, b ^= 1) {
+#pragma unroll
+      for (int r = 0; r < NSLOT; ++r)
+        if (wc[r] >= 0) {
+#pragma unroll
+          for (int h = 0; h < kPair; ++h) s.q[b][h][tid + r * kTileCells] = Qw[r][h] / rw[r];
+        }
+      if (t0 + kPair < P.nt) load(t0 + kPair);
+      __syncthreads();
+      if (!act) continue;
+      double n[kPair][7], g[kPair][3];
+#pragma unroll
+      for (int h = 0; h < kPair; ++h)
+#pragma unroll
+        for (int m = 0; m < 7; ++m) n[h][m] = s.q[b][h][wn[m]];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const double c0 = s.cg[d * 7][tid];
+#pragma unroll
+        for (int h = 0; h < kPair; ++h) g[h][d] = c0 * n[h][0];
+#pragma unroll
+        for (int m = 1; m < 7; ++m) {
+          const double cm = s.cg[d * 7 + m][tid];
+#pragma unroll
+          for (int h = 0; h < kPair; ++h) g[h][d] = g[h][d] + cm * n[h][m];
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < kPair; ++h) {
+        const double c0 = n[h][0], n1 = n[h][1], n2 = n[h][2], n3v = n[h][3], n4 = n[h][4], n5 = n[h][5], n6 = n[h][6];
+        // 4-point bounds of the six faces (mod_src_tracer.f90:152-214), the owner's q first
+        const double b5 = sing ? c0 : n6, c5 = sing ? n1 : c0;  // face 5 of a singular corner: the shifted stencil
+        double lo[7], hi[7];
+        lo[1] = mn4(c0, n6, n1, n2), hi[1] = mx4(c0, n6, n1, n2);
+        lo[2] = mn4(c0, n1, n2, n3v), hi[2] = mx4(c0, n1, n2, n3v);
+        lo[3] = mn4(c0, n2, n3v, n4), hi[3] = mx4(c0, n2, n3v, n4);
+        lo[4] = mn4(n4, n5, c0, n3v), hi[4] = mx4(n4, n5, c0, n3v);
+        lo[5] = mn4(n5, b5, c5, n4), hi[5] = mx4(n5, b5, c5, n4);
+        lo[6] = mn4(n6, n1, c0, n5), hi[6] = mx4(n6, n1, c0, n5);
+        // Qout (:219-282, d = 0)
+        double qnmin = c0, qnmax = c0, CQmin = 0.0, CQmax = 0.0;
+#pragma unroll
+        for (int m = 1; m <= 6; ++m) {
+          const bool f = (in >> m) & 1u;
+          const double qmin = f ? lo[m] : BIG, qmax = f ? hi[m] : -BIG;
+          qnmin = mn(qnmin, qmin), qnmax = mx(qnmax, qmax);
+          CQmin = (m == 1) ? chm[1] * qmin : CQmin + chm[m] * qmin;
+          CQmax = (m == 1) ? chm[1] * qmax : CQmax + chm[m] * qmax;
+        }
+        const double Qmin = (c0 - CQmax - qnmax * omc) / den * (1.0 - zsw) + c0 * zsw;
+        const double Qmax = (c0 - CQmin - qnmin * omc) / den * (1.0 - zsw) + c0 * zsw;
+        const int t = min(t0 + h, P.nt - 1);  // an odd group's last pair writes its tracer twice, the same values
+        double *fv = P.fv + (size_t)t * 3 * n3 + off;
+#pragma unroll
+        for (int m = 1; m <= 6; ++m)
+          if ((out >> m) & 1u) {
+            const int a = (m - 1) % 3;
+            double v = c0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) v = v + g[h][d] * s.disp[a * 3 + d][os[m]];
+            v = mn(mx(v, lo[m]), hi[m]);
+            fv[(size_t)a * n3 + oc[m]] = mx(mn(v, Qmax), Qmin);
+          }
+        if (bs >= 0) {
+          double *o = P.bval(t, k, bs);
+          o[0] = g[h][0], o[1] = g[h][1], o[2] = g[h][2], o[3] = Qmin, o[4] = Qmax;
+        }
+      }
+    }
+  }
+}
+
+// faces with a halo cell on one side: one thread per (seam face, level, tracer)
+__global__ void k_plain_seam(PlainArgs P) {
+  const Dims &D = P.D;
+  const int K = D.kmax - D.kmin + 1;
+  const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= (long long)P.ns * K * P.nt) return;
+  const int e = (int)(u % P.ns), k = D.kmin - 1 + (int)(u / P.ns % K), t = (int)(u / P.ns / K);
+  const int code = P.seam[e], G = D.gall_1d;
+  const int a = code % 3, o = code / 3 % D.gall, l = code / 3 / D.gall;
+  const int i = o % G + 1, j = o / G + 1;
+  const int nb = o + (a == 0 ? 1 : (a == 1 ? G + 1 : G));
+  const bool inO = P.inner(i, j), inN = P.inner(a < 2 ? i + 1 : i, a > 0 ? j + 1 : j);
+  if (!inO && !inN) return;  // no interior cell reads it
+  const size_t n3 = P.n3(), off = ((size_t)l * D.kall + k) * D.gall, gw = (size_t)D.lall * D.gall;
+  const double *Q = P.Q + (size_t)t * n3 + off, *rho = P.rho + off;
+  auto q = [&](int p) { return Q[p] / rho[p]; };
+  // the face's 4 points, owner first (mod_src_tracer.f90:152-214)
+  int p1, p2, p3;
+  if (a == 0) {
+    p1 = max(o - G, 0), p2 = o + 1, p3 = o + G + 1;
+  } else if (a == 1) {
+    const bool sing = D.have_sgp[l] != 0 && i == D.gmin - 1 && j == D.gmin - 1;
+    p1 = sing ? o + G + 1 : o + 1, p2 = sing ? o + G + 2 : o + G + 1, p3 = o + G;
+  } else {
+    p1 = o + G + 1, p2 = o + G, p3 = max(o - 1, 0);
+  }
+  const double q0 = q(o), q1 = q(p1), q2 = q(p2), q3 = q(p3);
+  const double lo = mn4(q0, q1, q2, q3), hi = mx4(q0, q1, q2, q3);
+  const int up = upmask(P.flx[(size_t)a * n3 + off + o] / rho[o]) ? nb : o;
+  const double qu = q(up);
+  const int b = P.bsrc[(size_t)l * D.gall + up];
+  // a halo point no list fills has no gradient, and Qout = q
+  const double *bv = b >= 0 ? P.bval(t, k, b) : nullptr;
+  double v = qu;
+  for (int d = 0; d < 3; ++d)
+    v = v + (bv ? bv[d] : 0.0) * (P.xc[((size_t)d * 3 + a) * n3 + off + o] - P.GRD_x[d * gw + (size_t)l * D.gall + up]);
+  v = mn(mx(v, lo), hi);
+  v = mx(mn(v, bv ? bv[4] : qu), bv ? bv[3] : qu);
+  P.fv[((size_t)t * 3 + a) * n3 + off + o] = v;
+}
+
+// Vertical limiter (dyn_vert_adv_limiter/src/mod_src_tracer.f90:107-186, d = 0): the
+// tracer-independent part of a level and one tracer's Qout.
+struct VPar {
+  double infl, bl, bu, a1, a2, icm, den, zsw;
+};
+__device__ __forceinline__ VPar vpar(double c1, double c2, double c1u) {
+  VPar v;
+  v.infl = 0.5 - sgn(0.5, c1);
+  const double infu = 0.5 + sgn(0.5, c1u), dv = 0.0;
+  v.bl = (1.0 - v.infl) * DBL_MAX, v.bu = (1.0 - infu) * DBL_MAX;
+  v.a1 = v.infl * c1, v.a2 = infu * c2;
+  const double Cin = v.a1 + v.a2, Cout = (1.0 - v.infl) * c1 + (1.0 - infu) * c2;
+  v.zsw = 0.5 - sgn(0.5, fabs(Cout) - DBL_EPSILON);
+  v.den = Cout + v.zsw;
+  v.icm = Cin + Cout - dv;
+  return v;
+}
+__device__ __forceinline__ void vqout(const VPar &v, double qm, double qk, double qp, double &Qmin, double &Qmax) {
+  const double minL = mn(qk, qm) + v.bl, minU = mn(qk, qp) + v.bu;
+  const double maxL = mx(qk, qm) - v.bl, maxU = mx(qk, qp) - v.bu;
+  const double qnmin = mn(mn(minL, minU), qk), qnmax = mx(mx(maxL, maxU), qk);
+  const double CQmin = v.a1 * minL + v.a2 * minU, CQmax = v.a1 * maxL + v.a2 * maxU;
+  Qmin = ((qk - qnmax) + qnmax * v.icm - CQmax) / v.den * (1.0 - v.zsw) + qk * v.zsw;
+  Qmax = ((qk - qnmin) + qnmin * v.icm - CQmin) / v.den * (1.0 - v.zsw) + qk * v.zsw;
+}
+__device__ __forceinline__ double vclamp(double infl, double h, double mnL, double mxL, double mnU, double mxU) {
+  const double a1 = (h < mxL) ? h : mxL, b1 = (mnL > a1) ? mnL : a1;
+  const double a2 = (h < mxU) ? h : mxU, b2 = (mnU > a2) ? mnU : a2;
+  return infl * b1 + (1.0 - infl) * b2;
+}
+
+constexpr int kColThreads = 128;
+
+// the two sub-steps of one pole column (p, tracer t): a thread per level, every stage level-parallel
+__device__ __forceinline__ void pole_column(const PlainArgs &P, int p, int t) {
+  __shared__ double sq[kColThreads], sh[kColThreads], s1[kColThreads], s2[kColThreads], smn[kColThreads],
+      smx[kColThreads];
+  const Dims &D = P.D;
+  const int K = D.kall, k = threadIdx.x, kmin = D.kmin - 1, kmax = D.kmax - 1;
+  const size_t off = ((size_t)p * K + k) * kGallPl, n3p = P.n3p();
+  double *Q = P.Qp + (size_t)t * n3p;
+  const bool phys = k >= kmin && k <= kmax;
+  double Qh = 0.0, r = 1.0;
+  if (k < K) {
+    double rs = P.flxp[off + 1];
+    for (int v = 2; v <= 5; ++v) rs = rs + P.flxp[off + v];
+    r = P.rhop[off] - rs;
+  }
+  if (phys) {  // rhogq after the horizontal sub-step: the five ring faces
+    double q[kGallPl], s = 0.0;
+    for (int v = 0; v < kGallPl; ++v) q[v] = Q[off + v] / P.rhop[off + v];
+    const double *bc = P.bval(t, k, P.nb - 2 + p);
+    for (int v = 1; v <= 5; ++v) {
+      const int vp = (v == 5) ? 1 : v + 1, vm = (v == 1) ? 5 : v - 1;
+      const bool c = upmask(P.flxp[off + v] / P.rhop[off]);
+      const int up = c ? v : 0;
+      const double *bv = c ? P.bval(t, k, P.ring[p * kVlink + v - 1]) : bc;
+      double f = q[up];
+      for (int d = 0; d < 3; ++d)
+        f = f + bv[d] * (P.xcp[d * n3p + off + v] - P.GRD_xp[((size_t)d * kLallPl + p) * kGallPl + up]);
+      f = mn(mx(f, mn4(q[0], q[v], q[vm], q[vp])), mx4(q[0], q[v], q[vm], q[vp]));
+      f = mx(mn(f, bv[4]), bv[3]);
+      s = (v == 1) ? P.flxp[off + v] * f : s + P.flxp[off + v] * f;
+    }
+    Qh = Q[off] - s;
+  }
+  if (K == 1) {
+    if (k == 0) Q[off] = Qh;
+    return;
+  }
+  auto W = [&](int kk) { return P.wp[((size_t)p * K + kk) * kGallPl]; };
+  double c1 = 0.0, c2 = 0.0;
+  if (phys || k == K - 1) c1 = -W(k) * P.dt * P.rdgz[k] / r;
+  if (phys) c2 = W(k + 1) * P.dt * P.rdgz[k] / r;
+  if (k < K) s1[k] = c1, s2[k] = c2;
+  if (phys) {
+    const double qk = Qh / r;
+    sq[k] = qk;
+    if (k == kmin) sq[0] = qk;
+    if (k == kmax) sq[K - 1] = qk;
+  }
+  __syncthreads();
+  double h = (k >= kmin && k < K) ? P.afact[k] * sq[k] + P.bfact[k] * sq[k - 1] : 0.0, infl = 0.0;
+  if (phys) {
+    const VPar v = vpar(s1[k], s2[k], s1[k + 1]);
+    infl = v.infl;
+    vqout(v, sq[k - 1], sq[k], sq[k + 1], smn[k], smx[k]);
+  }
+  __syncthreads();
+  if (phys && k > kmin) h = vclamp(infl, h, smn[k - 1], smx[k - 1], smn[k], smx[k]);
+  if (k < K) sh[k] = h;
+  __syncthreads();
+  if (phys) {
+    const double fu = W(k + 1) * sh[k + 1], fl = W(k) * sh[k];
+    const double Qn = Qh - (fu - fl) * P.dt * P.rdgz[k];
+    Q[off] = Qn;
+    if (k == kmin) Q[(size_t)p * K * kGallPl] = Qn;
+    if (k == kmax) Q[((size_t)p * K + K - 1) * kGallPl] = Qn;
+  }
+}
+
+// A column and kPair tracers per thread (tracer pairs of a column block are consecutive blocks and
+// share rhog, rhogw and the fluxes in L2), the next level's inputs loaded while a level is worked on.
+// Level k gives Qout of level k-1 and the limited flux of the face below it, which finish level k-2.
+// The last blocks take the pole columns.
+__global__ void __launch_bounds__(kColThreads) k_plain_column(PlainArgs P, int ncolblk) {
+  const Dims &D = P.D;
+  const int npair = (P.nt + kPair - 1) / kPair;
+  if ((int)blockIdx.x >= ncolblk * npair) {
+    const int u = (int)blockIdx.x - ncolblk * npair;
+    pole_column(P, u % kLallPl, u / kLallPl);
+    return;
+  }
+  const int n = D.gmax - D.gmin + 1, col = (int)blockIdx.x / npair * kColThreads + (int)threadIdx.x;
+  if (col >= D.lall * n * n) return;
+  const int t0 = (int)blockIdx.x % npair * kPair, t1 = min(t0 + 1, P.nt - 1);  // an odd group's last pair: one tracer twice
+  const int l = col / (n * n), G = D.gall_1d, K = D.kall;
+  const int c = (col / n % n + D.gmin - 1) * G + col % n + D.gmin - 1;
+  const size_t n3 = P.n3(), base = (size_t)l * K * D.gall + c;
+  const int g = D.gall;
+  const double *flx = P.flx + base, *rho = P.rho + base, *W = P.w + base;
+  double *Q[kPair] = {P.Q + (size_t)t0 * n3 + base, P.Q + (size_t)t1 * n3 + base};
+  const double *fv[kPair] = {P.fv + (size_t)t0 * 3 * n3 + base, P.fv + (size_t)t1 * 3 * n3 + base};
+  static_assert(kPair == 2, "Q and fv hold a pair");
+  struct In {
+    double Q[kPair], f[kPair][6], flx[6], rho, w;
+  };
+  auto load = [&](int k, bool phys) {
+    In v;
+    const size_t o = (size_t)k * g;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) v.flx[m] = flx[m * n3 + o];
+    v.rho = rho[o], v.w = W[o];
+    if (phys) {
+#pragma unroll
+      for (int h = 0; h < kPair; ++h) {
+        v.Q[h] = Q[h][o];
+        const double *f = fv[h] + o;
+        v.f[h][0] = f[0], v.f[h][1] = f[n3], v.f[h][2] = f[2 * n3];
+        v.f[h][3] = f[-1], v.f[h][4] = (f + n3)[-G - 1], v.f[h][5] = (f + 2 * n3)[-G];
+      }
+    }
+    return v;
+  };
+  auto horiz = [&](const In &v, int h) {  // rhogq after the horizontal sub-step
+    double s = v.flx[0] * v.f[h][0];
+#pragma unroll
+    for (int m = 1; m < 6; ++m) s = s + v.flx[m] * v.f[h][m];
+    return v.Q[h] - s;
+  };
+  auto dens = [&](const In &v) {
+    double s = v.flx[0];
+#pragma unroll
+    for (int m = 1; m < 6; ++m) s = s + v.flx[m];
+    return v.rho - s;
+  };
+  const int kmin = D.kmin - 1, kmax = D.kmax - 1;
+  In nx = load(kmin, true);
+  if (K == 1) {
+#pragma unroll
+    for (int h = 0; h < kPair; ++h) Q[h][0] = horiz(nx, h);
+    return;
+  }
+  double qm[kPair], q[kPair], Qhm[kPair], Qh[kPair], Qmn[kPair], Qmx[kPair], fl[kPair];  // levels k-2 (m), k-1
+  double c1 = 0.0, c2 = 0.0, rp = 1.0, wk = 0.0;  // level k-1: ck1; its density and w
+  for (int k = kmin; k <= kmax + 1; ++k) {
+    const In v = nx;
+    if (k <= kmax) nx = load(k + 1, k < kmax);
+    const double r = dens(v);
+    const double c1n = -v.w * P.dt * P.rdgz[k] / r;
+    if (k == kmin) {
+#pragma unroll
+      for (int h = 0; h < kPair; ++h) {
+        Qh[h] = horiz(v, h), q[h] = Qh[h] / r, qm[h] = q[h], Qhm[h] = 0.0, Qmn[h] = Qmx[h] = fl[h] = 0.0;
+      }
+    } else {
+      c2 = v.w * P.dt * P.rdgz[k - 1] / rp;  // ck2 of level k-1
+      const VPar vp = vpar(c1, c2, c1n);
+      const double af = P.afact[k - 1], bf = P.bfact[k - 1];
+#pragma unroll
+      for (int h = 0; h < kPair; ++h) {
+        double Qn = 0.0, qn = q[h];
+        if (k <= kmax) Qn = horiz(v, h), qn = Qn / r;
+        double lo, hi;
+        vqout(vp, qm[h], q[h], qn, lo, hi);
+        double qh = af * q[h] + bf * qm[h];
+        if (k - 1 > kmin) qh = vclamp(vp.infl, qh, Qmn[h], Qmx[h], lo, hi);
+        const double fu = wk * qh;  // through the face below level k-1
+        if (k - 1 > kmin) {
+          const double z = Qhm[h] - (fu - fl[h]) * P.dt * P.rdgz[k - 2];
+          Q[h][(size_t)(k - 2) * g] = z;
+          if (k - 2 == kmin) Q[h][0] = z;
+        }
+        fl[h] = fu, Qmn[h] = lo, Qmx[h] = hi;
+        Qhm[h] = Qh[h], Qh[h] = Qn, qm[h] = q[h], q[h] = qn;
+      }
+    }
+    c1 = c1n, rp = r, wk = v.w;
+  }
+  // level kmax: the flux through the top face is unlimited
+#pragma unroll
+  for (int h = 0; h < kPair; ++h) {
+    const double qh = P.afact[kmax + 1] * q[h] + P.bfact[kmax + 1] * qm[h];
+    const double z = Qhm[h] - (wk * qh - fl[h]) * P.dt * P.rdgz[kmax];
+    Q[h][(size_t)kmax * g] = z;
+    Q[h][(size_t)(K - 1) * g] = z;
+    if (kmin == kmax) Q[h][0] = z;
+  }
+}
+
+// the density: rhog -= sum_m flx_h(m), then -= d(rhogw)/dz dt, ghost levels copied.  One thread per
+// (cell, level), after every tracer has read the old density; the last threads take the pole centres.
+__global__ void k_plain_rho(Dims D, double dt, const double *flx, const double *flx_pl, const double *w,
+                            const double *w_pl, const double *rdgz, double *rho, double *rho_pl) {
+  const int n = D.gmax - D.gmin + 1, K = D.kall, kmin = D.kmin - 1, kmax = D.kmax - 1, NK = kmax - kmin + 1;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, nc = (long long)D.lall * NK * n * n;
+  double *R, *col;
   const double *W;
-  size_t s, tstride;
-  if (t < ncol) {
-    const int l = t / D.gall, c = t % D.gall, G = D.gall_1d;
-    const int i = c % G + 1, j = c / G + 1;
-    if (i < D.gmin || i > D.gmax || j < D.gmin || j > D.gmax) return;
-    const size_t base = (size_t)l * D.kall * D.gall + c;
-    R = rho + base, QQ = Q + base, W = w + base, s = D.gall;
-    tstride = (size_t)D.lall * D.kall * D.gall;
-  } else if (t < ncol + kLallPl) {
-    const size_t base = (size_t)(t - ncol) * D.kall * kGallPl;
-    R = rho_pl + base, QQ = Qp + base, W = w_pl + base, s = kGallPl;
-    tstride = (size_t)kLallPl * D.kall * kGallPl;
+  double s;
+  size_t lev;
+  int k;
+  if (t < nc) {
+    const int r = (int)(t % (n * n)), c = (r / n + D.gmin - 1) * D.gall_1d + r % n + D.gmin - 1;
+    k = kmin + (int)(t / (n * n) % NK);
+    const size_t n3 = (size_t)D.lall * K * D.gall, cb = (size_t)(t / (n * n) / NK) * K * D.gall + c;
+    lev = D.gall;
+    const size_t o = cb + k * lev;
+    col = rho + cb, R = rho + o, W = w + o;
+    s = flx[o];
+    for (int m = 1; m < 6; ++m) s = s + flx[m * n3 + o];
+  } else if (t < nc + kLallPl * NK) {
+    const int p = (int)(t - nc) / NK;
+    k = kmin + (int)(t - nc) % NK;
+    lev = kGallPl;
+    const size_t cb = (size_t)p * K * kGallPl, o = cb + k * lev;
+    col = rho_pl + cb, R = rho_pl + o, W = w_pl + o;
+    s = flx_pl[o + 1];
+    for (int v = 2; v <= 5; ++v) s = s + flx_pl[o + v];
   } else {
     return;
   }
-  const int K = D.kall, kmin = D.kmin - 1, kmax = D.kmax - 1;  // 0-based
-  double ck1[KMAX], ck2[KMAX], q[KMAX], qh[KMAX];
-  for (int k = 0; k < K; ++k) ck1[k] = ck2[k] = 0.0;
-  for (int k = kmin; k <= kmax; ++k) {
-    const double r = R[k * s];
-    ck1[k] = -W[k * s] * dt * rdgz[k] / r;
-    ck2[k] = W[(k + 1) * s] * dt * rdgz[k] / r;
-  }
-  ck1[K - 1] = -W[(K - 1) * s] * dt * rdgz[K - 1] / R[(K - 1) * s];
-  for (int tr = 0; tr < ntr; ++tr) {
-    double *Qt = QQ + tr * tstride;
-    for (int k = kmin; k <= kmax; ++k) q[k] = Qt[k * s] / R[k * s];
-    q[0] = q[kmin];
-    q[K - 1] = q[kmax];
-    for (int k = kmin; k <= kmax + 1 && k < K; ++k) qh[k] = afact[k] * q[k] + bfact[k] * q[k - 1];
-    // vertical_limiter_thuburn on this column (dyn_vert_adv_limiter/src/mod_src_tracer.f90:107-186)
-    double fl, Qmin_km1, Qmax_km1;
-    vqout(q, ck1, ck2, kmin, fl, Qmin_km1, Qmax_km1);
-    for (int k = kmin + 1; k <= kmax; ++k) {
-      double inflagL, Qmin, Qmax;
-      vqout(q, ck1, ck2, k, inflagL, Qmin, Qmax);
-      const double h = qh[k];
-      const double a1 = (h < Qmax_km1) ? h : Qmax_km1;
-      const double b1 = (Qmin_km1 > a1) ? Qmin_km1 : a1;
-      const double a2 = (h < Qmax) ? h : Qmax;
-      const double b2 = (Qmin > a2) ? Qmin : a2;
-      qh[k] = inflagL * b1 + (1.0 - inflagL) * b2;
-      Qmin_km1 = Qmin;
-      Qmax_km1 = Qmax;
-    }
-    for (int k = kmin; k <= kmax; ++k) {
-      const double fu = W[(k + 1) * s] * qh[k + 1], flo = W[k * s] * qh[k];
-      Qt[k * s] = Qt[k * s] - (fu - flo) * dt * rdgz[k];
-    }
-    Qt[0] = Qt[kmin * s];
-    Qt[(K - 1) * s] = Qt[kmax * s];
-  }
-  for (int k = kmin; k <= kmax; ++k) R[k * s] = R[k * s] - (W[(k + 1) * s] - W[k * s]) * dt * rdgz[k];
-  R[0] = R[kmin * s];
-  R[(K - 1) * s] = R[kmax * s];
+  double r = *R - s;
+  if (K > 1) r = r - (W[lev] - W[0]) * dt * rdgz[k];
+  *R = r;
+  if (k == kmin && k != 0) col[0] = r;
+  if (k == kmax && k != K - 1) col[(size_t)(K - 1) * lev] = r;
 }
 
 // ---------------------------------------------------------------------------
@@ -301,54 +736,66 @@ void launch_remap(const StepCtx &S, cudaStream_t st) {
                                                                    S.GRD_x_pl, S.qa_pl);
 }
 
-void launch_update_h(const StepCtx &S, const double *qa, const double *qa_pl, double *Q, double *Qp, cudaStream_t st) {
-  const Dims &D = S.D;
-  k_update_h<<<slab(D, kSlabThreads), kSlabThreads, 0, st>>>(D, S.flx, qa, Q);
-  k_update_h_pl<<<(unsigned)((kLallPl * D.kall + 255) / 256), 256, 0, st>>>(D.kall, S.flx_pl, qa_pl, Qp);
-}
-
 void launch_update_rho(const StepCtx &S, double *rho, double *rho_pl, cudaStream_t st) {
   const Dims &D = S.D;
   k_update_rho<<<slab(D, kSlabThreads), kSlabThreads, 0, st>>>(D, S.flx, rho);
   k_update_rho_pl<<<(unsigned)((kLallPl * D.kall + 255) / 256), 256, 0, st>>>(D.kall, S.flx_pl, rho_pl);
 }
 
+template <int TX>
+static cudaError_t launch_cells(const PlainArgs &P, cudaStream_t st) {
+  const Dims &D = P.D;
+  using S = CellSmem<TX>;
+  const int n = D.gmax - D.gmin + 1, ntx = (n + TX - 1) / TX, nty = (n + S::TY - 1) / S::TY;
+  const int tiles = ntx * nty * D.lall, NK = D.kmax - D.kmin + 1;
+  // up to 8 levels a block (the gradient coefficients are loaded once per block), fewer while
+  // that leaves less than two waves of the 2 blocks an SM holds
+  int lpb = 8;
+  while (lpb > 1 && (long long)tiles * ((NK + lpb - 1) / lpb) < 2 * 2 * 148) lpb /= 2;
+  const int nlb = (NK + lpb - 1) / lpb;
+  const int npole = (P.nt * kLallPl * D.kall + kTileCells - 1) / kTileCells;
+  cudaError_t e = cudaFuncSetAttribute(k_plain_cells<TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(S));
+  if (e != cudaSuccess) return e;
+  k_plain_cells<TX><<<(unsigned)(tiles * nlb + npole), kTileCells, sizeof(S), st>>>(P, ntx, nty, nlb, lpb);
+  return cudaGetLastError();
+}
+
 int step_plain(StepCtx &S, int ntr, double dt, double *rhog, double *rhog_pl, double *rhogq, double *rhogq_pl,
                const double *vx, const double *vx_pl, const double *vy, const double *vy_pl, const double *vz,
                const double *vz_pl, const double *w, const double *w_pl, cudaStream_t st, long long &launches) {
   const Dims &D = S.D;
+  if (D.kall > kColThreads) return set_error("advect_step: kall above 128"), ICA_ERR_ARG;
   const size_t n3 = n3_of(D), n3p = n3p_of(D);
-  // shared per step
   FluxIn<double> fin{rhog, rhog_pl, vx, vx_pl, vy, vy_pl, vz, vz_pl};
   FluxOut<double> fout{S.flx, S.flx_pl, S.xc, S.xc_pl};
   launch_horizontal_flux<double>(D, fin, fout, S.geo, dt, st);
-  launch_courant(S, rhog, rhog_pl, st);
-  launches += 4;
-  LimIn<double> lin{S.q, S.q_pl, S.zero, S.zero_pl, S.ch, S.ch_pl, S.cm, S.cm_pl};
-  for (int t = 0; t < ntr; ++t) {
-    double *Q = rhogq + t * n3, *Qp = rhogq_pl + t * n3p;
-    launch_divide(S, Q, Qp, rhog, rhog_pl, st);
-    launch_gradient(S, st);
-    launch_remap(S, st);
-    launch_hlim_qout<double>(D, lin, S.qout, S.qout_pl, S.qin_pl, st);
-    launch_gather<double>(D, S.plan.n, S.plan.dst, S.plan.src, D.kall, 2, S.qout, S.qout_pl, st);
-    launch_hlim_apply<double>(D, lin, S.qa, S.qa_pl, S.qout, S.qout_pl, S.qin_pl, st);
-    launch_update_h(S, S.qa, S.qa_pl, Q, Qp, st);
-    launches += 14;
+  launches += 2;
+  const int n = D.gmax - D.gmin + 1, NK = D.kmax - D.kmin + 1;
+  const int ncolblk = (D.lall * n * n + kColThreads - 1) / kColThreads;
+  for (int t0 = 0; t0 < ntr; t0 += kPlainGroup) {
+    PlainArgs P{};
+    P.D = D, P.nt = (ntr - t0 < kPlainGroup) ? ntr - t0 : kPlainGroup, P.nb = S.nb, P.ns = S.ns, P.dt = dt;
+    P.Q = rhogq + t0 * n3, P.Qp = rhogq_pl + t0 * n3p;
+    P.rho = rhog, P.rhop = rhog_pl, P.w = w, P.wp = w_pl;
+    P.flx = S.flx, P.flxp = S.flx_pl, P.xc = S.xc, P.xcp = S.xc_pl;
+    P.GRD_x = S.GRD_x, P.GRD_xp = S.GRD_x_pl, P.cg = S.cg, P.cgp = S.cg_pl;
+    P.rdgz = S.rdgz, P.afact = S.afact, P.bfact = S.bfact;
+    P.bsrc = S.bsrc, P.seam = S.seam, P.ring = S.ring;
+    P.fv = S.fv, P.bb = S.bb;
+    // 32 x 8 tiles need no partial tile in any region 32 or more cells wide (a region is a power of two wide)
+    const cudaError_t e = n >= 32 ? launch_cells<32>(P, st) : launch_cells<16>(P, st);
+    if (e != cudaSuccess) return set_error(std::string("advect_step: ") + cudaGetErrorString(e)), ICA_ERR_CUDA;
+    const long long ns = (long long)P.ns * NK * P.nt;
+    k_plain_seam<<<(unsigned)((ns + 127) / 128), 128, 0, st>>>(P);
+    const int npair = (P.nt + kPair - 1) / kPair;
+    k_plain_column<<<(unsigned)(ncolblk * npair + kLallPl * P.nt), kColThreads, 0, st>>>(P, ncolblk);
+    launches += 3;
   }
-  launch_update_rho(S, rhog, rhog_pl, st);
-  const int ncol = D.lall * D.gall + kLallPl;
-  if (D.kall <= 48)
-    k_vertical<48><<<(ncol + 127) / 128, 128, 0, st>>>(D, ntr, dt, rhog, rhogq, w, rhog_pl, rhogq_pl, w_pl, S.rdgz,
-                                                       S.afact, S.bfact);
-  else if (D.kall <= 128)
-    k_vertical<128><<<(ncol + 127) / 128, 128, 0, st>>>(D, ntr, dt, rhog, rhogq, w, rhog_pl, rhogq_pl, w_pl, S.rdgz,
-                                                        S.afact, S.bfact);
-  else
-    return ICA_ERR_ARG;
+  const long long nr = ((long long)D.lall * n * n + kLallPl) * NK;
+  k_plain_rho<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(D, dt, S.flx, S.flx_pl, w, w_pl, S.rdgz, rhog, rhog_pl);
   launch_gather<double>(D, S.plan.n, S.plan.dst, S.plan.src, D.kall, 1, rhog, rhog_pl, st);
   launch_gather<double>(D, S.plan.n, S.plan.dst, S.plan.src, D.kall, ntr, rhogq, rhogq_pl, st);
-  launches += 5;
+  launches += 3;
   return ICA_OK;
 }
 
