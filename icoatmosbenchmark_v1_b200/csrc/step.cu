@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <type_traits>
 
 #include "step.cuh"
 
@@ -169,12 +170,12 @@ __global__ void k_update_rho_pl(int kall, const double *flx_pl, double *rho_pl) 
 //
 // A face value travels once through memory (24 bytes written and read per update); gradient,
 // remap value, Courant number, mask and Qout never do.  Against one launch per piece and tracer
-// (14 launches a tracer, a column's levels in local memory): 9.90 -> 5.27 ms for glevel 7, kall 61,
-// 5 tracers, 1.59 -> 0.49 ms for glevel 5, kall 42, 8 tracers.  Every value is the result of the
+// (14 launches a tracer, a column's levels in local memory): 9.90 -> 3.61 ms for glevel 7, kall 61,
+// 5 tracers, 1.59 -> 0.35 ms for glevel 5, kall 42, 8 tracers.  Every value is the result of the
 // reference's operation sequence; where the reference blends two sides by a mask of 0 or 1
 // (c a + (1 - c) b), the chosen side is taken, which is the same number.
 constexpr int kTileCells = 256;  // threads of k_plain_cells: one per cell of a TX x (256 / TX) tile
-constexpr int kPair = 2;         // tracers a thread of k_plain_cells / k_plain_column takes at once
+constexpr int kCellBlocks = 2;   // its blocks per SM: 128 registers a thread, which hold one tracer's values
 
 struct PlainArgs {
   Dims D;
@@ -196,8 +197,46 @@ __device__ __forceinline__ double mn(double a, double b) { return (b < a) ? b : 
 __device__ __forceinline__ double mx(double a, double b) { return (b > a) ? b : a; }
 __device__ __forceinline__ double mn4(double a, double b, double c, double d) { return mn(mn(mn(a, b), c), d); }
 __device__ __forceinline__ double mx4(double a, double b, double c, double d) { return mx(mx(mx(a, b), c), d); }
-// cmask of a Courant number: true where it is 1 (the face's neighbour is its upwind cell)
-__device__ __forceinline__ bool upmask(double ch) { return 0.5 - sgn(0.5, ch - DBL_EPSILON) != 0.0; }
+// cmask of the Courant number f / r: true where it is 1 (the face's neighbour is its upwind cell),
+// which is where the rounded quotient is below EPS.  EPS is a power of two, so for an ordinary
+// density that is f < EPS r, without the division.
+__device__ __forceinline__ bool upmask(double f, double r) {
+  if (r >= 0x1p-900) return f < DBL_EPSILON * r;
+  return 0.5 - sgn(0.5, f / r - DBL_EPSILON) != 0.0;
+}
+
+// Several quotients with one divisor, each correctly rounded: y = 1/b is correctly rounded (an
+// IEEE division), q1 = q0 + (a - b q0) y is faithful, and one more such step with its exact
+// residual is a/b correctly rounded (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990).  The residuals are exact while nothing under- or overflows:
+// quotients outside [2^-800, 2^1000) other than those of a zero, and divisors outside
+// [2^-100, 2^101), take the division itself.
+struct Recip {
+  double b, y;
+  bool ok;
+};
+__device__ __forceinline__ bool recip_ok(double b) {
+  return ((unsigned)__double2hiint(b) & 0x7fffffffu) - 0x39b00000u < 0x0c900000u;
+}
+__device__ __forceinline__ Recip recip(double b) { return Recip{b, 1.0 / b, recip_ok(b)}; }
+template <int N>
+__device__ __forceinline__ void quotients(double (&a)[N], const Recip &d) {
+  double q[N];
+  bool ok = d.ok;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const double q0 = a[i] * d.y, q1 = __fma_rn(__fma_rn(-d.b, q0, a[i]), d.y, q0);
+    q[i] = __fma_rn(__fma_rn(-d.b, q1, a[i]), d.y, q1);
+    ok = ok && (((unsigned)__double2hiint(q[i]) & 0x7fffffffu) - 0x0df00000u < 0x70800000u || a[i] == 0.0);
+  }
+  if (ok) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) a[i] = q[i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) a[i] = a[i] / d.b;
+  }
+}
 
 // pole centre (p, k) of tracer t: gradient and Qout (mod_src_tracer.f90:307-367) into bb
 __device__ __forceinline__ void pole_centre(const PlainArgs &P, int t, int p, int k) {
@@ -216,7 +255,7 @@ __device__ __forceinline__ void pole_centre(const PlainArgs &P, int t, int p, in
   for (int v = 1; v <= 5; ++v) {
     const int vp = (v == 5) ? 1 : v + 1, vm = (v == 1) ? 5 : v - 1;
     const double ch = P.flxp[off + v] / P.rhop[off];
-    const double c = upmask(ch) ? 1.0 : 0.0;
+    const double c = upmask(P.flxp[off + v], P.rhop[off]) ? 1.0 : 0.0;
     const double qmin = c * mn4(q[0], q[v], q[vm], q[vp]) + (1.0 - c) * BIG;
     const double qmax = c * mx4(q[0], q[v], q[vm], q[vp]) + (1.0 - c) * (-BIG);
     qnmin = mn(qnmin, qmin), qnmax = mx(qnmax, qmax);
@@ -236,15 +275,20 @@ struct CellSmem {
   static constexpr int TY = kTileCells / TX, WW = TX + 2, NW = WW * (TY + 2);  // window: the tile and one ring
   static constexpr int OW = TX + 1, NO = OW * (TY + 1);                        // owners of the tile's faces
   double cg[21][kTileCells];
-  double disp[9][NO];              // [face * 3 + x][owner]: xc - x(upwind cell), read by the upwind cell's thread
-  double rho[NW];
-  double q[2][kPair][NW];
+  // xc of the face [face * 3 + x][owner]; its upwind cell's thread turns it into xc - x(upwind cell)
+  // and is the one that reads it
+  double disp[9][NO];
+  double rho[NW], y[NW];  // rhog and its reciprocal
+  double q[2][NW];
 };
 
+// Bound by instruction issue (FP64 compare-and-selects of the bounds, then the gradient): 1.62 ms
+// of the 3.61.  One tracer per pass of the loop and two blocks per SM keep every value in
+// registers; two tracers, or three blocks, spill and take 2.5-2.6 ms.
 // grid: blocks 0 .. ntile*nlb-1 (level block fastest: a tile's gradient coefficients come from L2
 // after the first), then the pole centres
 template <int TX>
-__global__ void __launch_bounds__(kTileCells, 2) k_plain_cells(PlainArgs P, int ntx, int nty, int nlb, int lpb) {
+__global__ void __launch_bounds__(kTileCells, kCellBlocks) k_plain_cells(PlainArgs P, int ntx, int nty, int nlb, int lpb) {
   using S = CellSmem<TX>;
   extern __shared__ __align__(16) unsigned char raw[];
   S &s = *reinterpret_cast<S *>(raw);
@@ -260,13 +304,16 @@ __global__ void __launch_bounds__(kTileCells, 2) k_plain_cells(PlainArgs P, int 
   const int l = tile / (ntx * nty), tr = tile % (ntx * nty);
   const int i0 = D.gmin + (tr % ntx) * TX, j0 = D.gmin + (tr / ntx) * S::TY;  // first cell, 1-based
   const int x = tid % TX, y = tid / TX, i = i0 + x, j = j0 + y;
-  const bool act = i <= D.gmax && j <= D.gmax;
-  const int c = act ? (j - 1) * G + (i - 1) : 0;
-  const bool sing = D.have_sgp[l] != 0 && i == D.gmin && j == D.gmin;
+  // regions 32 or more cells wide are whole tiles; in a smaller one a thread without a cell works on
+  // the region's last cell and stores nothing
+  const bool act = TX == 32 || (i <= D.gmax && j <= D.gmax);
+  const int ci = TX == 32 ? i : min(i, D.gmax), cj = TX == 32 ? j : min(j, D.gmax);
+  const int c = (cj - 1) * G + (ci - 1);
+  const bool sing = D.have_sgp[l] != 0 && ci == D.gmin && cj == D.gmin;
   const int bs = act ? P.bsrc[(size_t)l * D.gall + c] : -1;
   const size_t n3 = P.n3(), gw = (size_t)D.lall * D.gall;
 #pragma unroll
-  for (int n = 0; n < 21; ++n) s.cg[n][tid] = act ? P.cg[((size_t)l * 21 + n) * D.gall + c] : 0.0;
+  for (int n = 0; n < 21; ++n) s.cg[n][tid] = P.cg[((size_t)l * 21 + n) * D.gall + c];
   // this thread's window slots and their cells (-1: none)
   constexpr int NSLOT = (S::NW + kTileCells - 1) / kTileCells;
   int wc[NSLOT];
@@ -275,139 +322,192 @@ __global__ void __launch_bounds__(kTileCells, 2) k_plain_cells(PlainArgs P, int 
     const int e = tid + r * kTileCells, wi = i0 - 1 + e % S::WW, wj = j0 - 1 + e / S::WW;  // >= 1
     wc[r] = (e < S::NW && wi <= G && wj <= G) ? (wj - 1) * G + (wi - 1) : -1;
   }
-  const int ew = (y + 1) * S::WW + x + 1;
+  // owner slots of the faces: this cell's, and for the first threads one of the row and column
+  // before the tile
+  const int cx = ci - i0, cy = cj - j0;
+  const int ew = (cy + 1) * S::WW + cx + 1, ow = (cy + 1) * S::OW + cx + 1;
   const int wn[7] = {ew, ew + 1, ew + S::WW + 1, ew + S::WW, ew - 1, ew - S::WW - 1, ew - S::WW};
-  // face m (1..6): its owner's slot, owner cell and other cell
-  const int ow = (y + 1) * S::OW + x + 1;
-  const int os[7] = {0, ow, ow, ow, ow - 1, ow - S::OW - 1, ow - S::OW};
-  const int oc[7] = {0, c, c, c, c - 1, c - G - 1, c - G};
+  int oslot = -1, ocell = 0;
+  if (tid < TX + S::TY + 1) {
+    const int ox = tid <= TX ? tid - 1 : -1, oy = tid <= TX ? -1 : tid - TX - 1;
+    if (i0 + ox <= D.gmax && j0 + oy <= D.gmax)
+      oslot = (oy + 1) * S::OW + ox + 1, ocell = (j0 + oy - 1) * G + (i0 + ox - 1);
+  }
   unsigned both = 0;  // bit m: the cell across face m is interior too (not a seam face)
-  if (act) {
+  {
     constexpr int DX[7] = {0, 1, 1, 0, -1, -1, 0}, DY[7] = {0, 0, 1, 1, 0, -1, -1};
 #pragma unroll
-    for (int m = 1; m <= 6; ++m) both |= P.inner(i + DX[m], j + DY[m]) ? 1u << m : 0u;
+    for (int m = 1; m <= 6; ++m) both |= act && P.inner(ci + DX[m], cj + DY[m]) ? 1u << m : 0u;
   }
+  const double X[3] = {P.GRD_x[(size_t)l * D.gall + c], P.GRD_x[gw + (size_t)l * D.gall + c],
+                       P.GRD_x[2 * gw + (size_t)l * D.gall + c]};
   const int kfirst = D.kmin - 1, kend = D.kmax;  // physical levels, 0-based
   const int k0 = kfirst + lb * lpb, k1 = min(k0 + lpb, kend);
-  const double BIG = DBL_MAX;
   for (int k = k0; k < k1; ++k) {
     const size_t off = ((size_t)l * D.kall + k) * D.gall;
-    double Qw[NSLOT][kPair], rw[NSLOT];
-    auto load = [&](int t0) {
+    double Qw[NSLOT][1];
+    auto load = [&](int t) {
+      const double *Qs = P.Q + (size_t)t * n3 + off;
 #pragma unroll
       for (int r = 0; r < NSLOT; ++r)
-        if (wc[r] >= 0) {
-#pragma unroll
-          for (int h = 0; h < kPair; ++h) Qw[r][h] = P.Q[(size_t)min(t0 + h, P.nt - 1) * n3 + off + wc[r]];
-        }
+        if (wc[r] >= 0) Qw[r][0] = Qs[wc[r]];
     };
+    // ---- every global load of the level's set-up before the first wait
     load(0);
+    double ch[6], fo[3], rv[NSLOT];
+    const double *flx = P.flx + off;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) ch[m] = (flx + m * n3)[c];
+    fo[0] = flx[c - 1], fo[1] = (flx + n3)[c - G - 1], fo[2] = (flx + 2 * n3)[c - G];  // owners of faces 4-6
+#pragma unroll
+    for (int r = 0; r < NSLOT; ++r) rv[r] = wc[r] >= 0 ? P.rho[off + wc[r]] : 1.0;
     __syncthreads();  // the previous level's shared data is read
+    {
+      const double *xc = P.xc + off;
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if (act) s.disp[a * 3 + d][ow] = (xc + (d * 3 + a) * n3)[c];
+          if (oslot >= 0) s.disp[a * 3 + d][oslot] = (xc + (d * 3 + a) * n3)[ocell];
+        }
+    }
+    Recip rw[NSLOT];
 #pragma unroll
     for (int r = 0; r < NSLOT; ++r) {
-      rw[r] = 1.0;
-      if (wc[r] >= 0) s.rho[tid + r * kTileCells] = rw[r] = P.rho[off + wc[r]];
+      rw[r] = recip(rv[r]);
+      if (wc[r] >= 0) s.rho[tid + r * kTileCells] = rv[r], s.y[tid + r * kTileCells] = rw[r].y;
     }
     __syncthreads();
     // ---- tracer-independent: Courant numbers, upwind sides, outflow sums, displacements
-    double chm[7] = {}, omc = 0.0, den = 1.0, zsw = 1.0;
+    double chm[7], omc;
+    Recip den;
     unsigned in = 0, out = 0;
-    if (act) {
+    bool odd = false;  // an inflow Courant number at a face whose mask says outflow (rounding-level fluxes)
+    bool zsw;
+    {
       const double rc = s.rho[ew];
-      double ch[7];
 #pragma unroll
       for (int m = 1; m <= 6; ++m) {
-        ch[m] = P.flx[(size_t)(m - 1) * n3 + off + c] / rc;
-        chm[m] = mn(ch[m], 0.0);
         // the owner's mask: 1 takes the owner's neighbour as the upwind cell
-        const bool cm = (m <= 3) ? upmask(ch[m]) : upmask(P.flx[(size_t)(m - 4) * n3 + off + oc[m]] / s.rho[wn[m]]);
+        const bool cm = (m <= 3) ? upmask(ch[m - 1], rc) : upmask(fo[m - 4], s.rho[wn[m]]);
         if (cm == (m <= 3)) in |= 1u << m;
         else if ((both >> m) & 1u) out |= 1u << m;
       }
+      quotients(ch, Recip{rc, s.y[ew], recip_ok(rc)});
+#pragma unroll
+      for (int m = 1; m <= 6; ++m) {
+        chm[m] = mn(ch[m - 1], 0.0);
+        odd = odd || (!((in >> m) & 1u) && chm[m] != 0.0);
+      }
       const double Cin = chm[1] + chm[2] + chm[3] + chm[4] + chm[5] + chm[6];
-      const double Cout =
-          ch[1] - chm[1] + ch[2] - chm[2] + ch[3] - chm[3] + ch[4] - chm[4] + ch[5] - chm[5] + ch[6] - chm[6];
-      const double dv = 0.0;
-      zsw = 0.5 - sgn(0.5, fabs(Cout) - DBL_EPSILON);
-      den = Cout + zsw;
+      const double Cout = ch[0] - chm[1] + ch[1] - chm[2] + ch[2] - chm[3] + ch[3] - chm[4] + ch[4] - chm[5] + ch[5] -
+                          chm[6];
+      const double dv = 0.0, z = 0.5 - sgn(0.5, fabs(Cout) - DBL_EPSILON);
+      zsw = z != 0.0;
+      den = recip(Cout + z);
       omc = 1.0 - Cin - Cout + dv;
-#pragma unroll
-      for (int m = 1; m <= 6; ++m)
-        if ((out >> m) & 1u) {
-          const int a = (m - 1) % 3;
-#pragma unroll
-          for (int d = 0; d < 3; ++d)
-            s.disp[a * 3 + d][os[m]] = P.xc[((size_t)d * 3 + a) * n3 + off + oc[m]] - P.GRD_x[d * gw + (size_t)l * D.gall + c];
-        }
     }
-    // ---- the tracers, two at a time; q of a pair alternates between two buffers
-    for (int t0 = 0, b = 0; t0 < P.nt; t0 += kPair, b ^= 1) {
+    // Of two opposite faces a and a + 3 a cell usually has one outflow face: sl / st are its owner's
+    // slot and cell (a's own where neither flows out; st < 0 then).  Cells with both go through the
+    // second one again below (again).
+    int sl[3], st[3];
+    unsigned side = 0, again = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const int so = ow - (a == 0 ? 1 : (a == 1 ? S::OW + 1 : S::OW)), sc = c - (a == 0 ? 1 : (a == 1 ? G + 1 : G));
+      const bool o1 = (out >> (a + 1)) & 1u, o2 = (out >> (a + 4)) & 1u;
+      if (!o1 && o2) side |= 1u << a;
+      if (o1 && o2) again |= 1u << a;
+      sl[a] = (!o1 && o2) ? so : ow;
+      st[a] = o1 ? c : (o2 ? sc : -1);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        if (o1 || o2) s.disp[a * 3 + d][sl[a]] -= X[d];
+        if (o1 && o2) s.disp[a * 3 + d][so] -= X[d];
+      }
+    }
+    // ---- the tracers; their q alternates between two buffers
+    for (int t = 0; t < P.nt; ++t) {
+      const int b = t & 1;
 #pragma unroll
       for (int r = 0; r < NSLOT; ++r)
         if (wc[r] >= 0) {
-#pragma unroll
-          for (int h = 0; h < kPair; ++h) s.q[b][h][tid + r * kTileCells] = Qw[r][h] / rw[r];
+          quotients(Qw[r], rw[r]);
+          s.q[b][tid + r * kTileCells] = Qw[r][0];
         }
-      if (t0 + kPair < P.nt) load(t0 + kPair);
+      if (t + 1 < P.nt) load(t + 1);
       __syncthreads();
-      if (!act) continue;
-      double n[kPair][7], g[kPair][3];
-#pragma unroll
-      for (int h = 0; h < kPair; ++h)
-#pragma unroll
-        for (int m = 0; m < 7; ++m) n[h][m] = s.q[b][h][wn[m]];
+      const double c0 = s.q[b][wn[0]], n1 = s.q[b][wn[1]], n2 = s.q[b][wn[2]], n3v = s.q[b][wn[3]], n4 = s.q[b][wn[4]],
+                   n5 = s.q[b][wn[5]], n6 = s.q[b][wn[6]];
+      const double n[7] = {c0, n1, n2, n3v, n4, n5, n6};
+      double g[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const double c0 = s.cg[d * 7][tid];
+        g[d] = s.cg[d * 7][tid] * n[0];
 #pragma unroll
-        for (int h = 0; h < kPair; ++h) g[h][d] = c0 * n[h][0];
-#pragma unroll
-        for (int m = 1; m < 7; ++m) {
-          const double cm = s.cg[d * 7 + m][tid];
-#pragma unroll
-          for (int h = 0; h < kPair; ++h) g[h][d] = g[h][d] + cm * n[h][m];
-        }
+        for (int m = 1; m < 7; ++m) g[d] = g[d] + s.cg[d * 7 + m][tid] * n[m];
       }
+      // 4-point bounds of the six faces (mod_src_tracer.f90:152-214): the cell and three
+      // consecutive neighbours, of which each pair is compared once
+      const double l12 = mn(n1, n2), l34 = mn(n3v, n4), l56 = mn(n5, n6);
+      const double h12 = mx(n1, n2), h34 = mx(n3v, n4), h56 = mx(n5, n6);
+      double lo[7], hi[7];
+      lo[1] = mn(c0, mn(n6, l12)), hi[1] = mx(c0, mx(n6, h12));
+      lo[2] = mn(c0, mn(l12, n3v)), hi[2] = mx(c0, mx(h12, n3v));
+      lo[3] = mn(c0, mn(n2, l34)), hi[3] = mx(c0, mx(n2, h34));
+      lo[4] = mn(c0, mn(l34, n5)), hi[4] = mx(c0, mx(h34, n5));
+      lo[5] = mn(c0, mn(n4, l56)), hi[5] = mx(c0, mx(n4, h56));
+      lo[6] = mn(c0, mn(l56, n1)), hi[6] = mx(c0, mx(h56, n1));
+      if (sing) lo[5] = mn4(n5, c0, n1, n4), hi[5] = mx4(n5, c0, n1, n4);  // the singular point's shifted stencil
+      // Qout (:219-282, d = 0).  An outflow face's +-BIG bound never binds, and its term of CQ is
+      // zero with its Courant number, except at an odd face
+      double qnmin = c0, qnmax = c0, CQmin = chm[1] * lo[1], CQmax = chm[1] * hi[1];
 #pragma unroll
-      for (int h = 0; h < kPair; ++h) {
-        const double c0 = n[h][0], n1 = n[h][1], n2 = n[h][2], n3v = n[h][3], n4 = n[h][4], n5 = n[h][5], n6 = n[h][6];
-        // 4-point bounds of the six faces (mod_src_tracer.f90:152-214), the owner's q first
-        const double b5 = sing ? c0 : n6, c5 = sing ? n1 : c0;  // face 5 of a singular corner: the shifted stencil
-        double lo[7], hi[7];
-        lo[1] = mn4(c0, n6, n1, n2), hi[1] = mx4(c0, n6, n1, n2);
-        lo[2] = mn4(c0, n1, n2, n3v), hi[2] = mx4(c0, n1, n2, n3v);
-        lo[3] = mn4(c0, n2, n3v, n4), hi[3] = mx4(c0, n2, n3v, n4);
-        lo[4] = mn4(n4, n5, c0, n3v), hi[4] = mx4(n4, n5, c0, n3v);
-        lo[5] = mn4(n5, b5, c5, n4), hi[5] = mx4(n5, b5, c5, n4);
-        lo[6] = mn4(n6, n1, c0, n5), hi[6] = mx4(n6, n1, c0, n5);
-        // Qout (:219-282, d = 0)
-        double qnmin = c0, qnmax = c0, CQmin = 0.0, CQmax = 0.0;
+      for (int m = 1; m <= 6; ++m) {
+        const bool f = (in >> m) & 1u;
+        qnmin = (f && lo[m] < qnmin) ? lo[m] : qnmin;
+        qnmax = (f && hi[m] > qnmax) ? hi[m] : qnmax;
+        if (m > 1) CQmin = CQmin + chm[m] * lo[m], CQmax = CQmax + chm[m] * hi[m];
+      }
+      if (odd) {
 #pragma unroll
         for (int m = 1; m <= 6; ++m) {
           const bool f = (in >> m) & 1u;
-          const double qmin = f ? lo[m] : BIG, qmax = f ? hi[m] : -BIG;
-          qnmin = mn(qnmin, qmin), qnmax = mx(qnmax, qmax);
-          CQmin = (m == 1) ? chm[1] * qmin : CQmin + chm[m] * qmin;
-          CQmax = (m == 1) ? chm[1] * qmax : CQmax + chm[m] * qmax;
+          const double tmin = chm[m] * (f ? lo[m] : DBL_MAX), tmax = chm[m] * (f ? hi[m] : -DBL_MAX);
+          CQmin = (m == 1) ? tmin : CQmin + tmin;
+          CQmax = (m == 1) ? tmax : CQmax + tmax;
         }
-        const double Qmin = (c0 - CQmax - qnmax * omc) / den * (1.0 - zsw) + c0 * zsw;
-        const double Qmax = (c0 - CQmin - qnmin * omc) / den * (1.0 - zsw) + c0 * zsw;
-        const int t = min(t0 + h, P.nt - 1);  // an odd group's last pair writes its tracer twice, the same values
-        double *fv = P.fv + (size_t)t * 3 * n3 + off;
+      }
+      double Qo[2] = {c0 - CQmax - qnmax * omc, c0 - CQmin - qnmin * omc};
+      quotients(Qo, den);
+      const double Qmin = zsw ? c0 : Qo[0], Qmax = zsw ? c0 : Qo[1];
+      double *fv = P.fv + (size_t)t * 3 * n3 + off;
 #pragma unroll
-        for (int m = 1; m <= 6; ++m)
-          if ((out >> m) & 1u) {
-            const int a = (m - 1) % 3;
+      for (int a = 0; a < 3; ++a) {
+        const bool f = (side >> a) & 1u;
+        double v = c0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v = v + g[d] * s.disp[a * 3 + d][sl[a]];
+        v = mn(mx(v, f ? lo[a + 4] : lo[a + 1]), f ? hi[a + 4] : hi[a + 1]);
+        v = mx(mn(v, Qmax), Qmin);
+        if (st[a] >= 0) (fv + a * n3)[st[a]] = v;
+      }
+      if (again) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if ((again >> a) & 1u) {
+            const int so = a == 0 ? 1 : (a == 1 ? S::OW + 1 : S::OW), sc = a == 0 ? 1 : (a == 1 ? G + 1 : G);
             double v = c0;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) v = v + g[h][d] * s.disp[a * 3 + d][os[m]];
-            v = mn(mx(v, lo[m]), hi[m]);
-            fv[(size_t)a * n3 + oc[m]] = mx(mn(v, Qmax), Qmin);
+            for (int d = 0; d < 3; ++d) v = v + g[d] * s.disp[a * 3 + d][ow - so];
+            v = mn(mx(v, lo[a + 4]), hi[a + 4]);
+            (fv + a * n3)[c - sc] = mx(mn(v, Qmax), Qmin);
           }
-        if (bs >= 0) {
-          double *o = P.bval(t, k, bs);
-          o[0] = g[h][0], o[1] = g[h][1], o[2] = g[h][2], o[3] = Qmin, o[4] = Qmax;
-        }
+      }
+      if (bs >= 0) {
+        double *o = P.bval(t, k, bs);
+        o[0] = g[0], o[1] = g[1], o[2] = g[2], o[3] = Qmin, o[4] = Qmax;
       }
     }
   }
@@ -441,7 +541,7 @@ __global__ void k_plain_seam(PlainArgs P) {
   }
   const double q0 = q(o), q1 = q(p1), q2 = q(p2), q3 = q(p3);
   const double lo = mn4(q0, q1, q2, q3), hi = mx4(q0, q1, q2, q3);
-  const int up = upmask(P.flx[(size_t)a * n3 + off + o] / rho[o]) ? nb : o;
+  const int up = upmask(P.flx[(size_t)a * n3 + off + o], rho[o]) ? nb : o;
   const double qu = q(up);
   const int b = P.bsrc[(size_t)l * D.gall + up];
   // a halo point no list fills has no gradient, and Qout = q
@@ -457,7 +557,8 @@ __global__ void k_plain_seam(PlainArgs P) {
 // Vertical limiter (dyn_vert_adv_limiter/src/mod_src_tracer.f90:107-186, d = 0): the
 // tracer-independent part of a level and one tracer's Qout.
 struct VPar {
-  double infl, bl, bu, a1, a2, icm, den, zsw;
+  double infl, bl, bu, a1, a2, icm, zsw;
+  Recip den;
 };
 __device__ __forceinline__ VPar vpar(double c1, double c2, double c1u) {
   VPar v;
@@ -467,7 +568,7 @@ __device__ __forceinline__ VPar vpar(double c1, double c2, double c1u) {
   v.a1 = v.infl * c1, v.a2 = infu * c2;
   const double Cin = v.a1 + v.a2, Cout = (1.0 - v.infl) * c1 + (1.0 - infu) * c2;
   v.zsw = 0.5 - sgn(0.5, fabs(Cout) - DBL_EPSILON);
-  v.den = Cout + v.zsw;
+  v.den = recip(Cout + v.zsw);
   v.icm = Cin + Cout - dv;
   return v;
 }
@@ -476,8 +577,10 @@ __device__ __forceinline__ void vqout(const VPar &v, double qm, double qk, doubl
   const double maxL = mx(qk, qm) - v.bl, maxU = mx(qk, qp) - v.bu;
   const double qnmin = mn(mn(minL, minU), qk), qnmax = mx(mx(maxL, maxU), qk);
   const double CQmin = v.a1 * minL + v.a2 * minU, CQmax = v.a1 * maxL + v.a2 * maxU;
-  Qmin = ((qk - qnmax) + qnmax * v.icm - CQmax) / v.den * (1.0 - v.zsw) + qk * v.zsw;
-  Qmax = ((qk - qnmin) + qnmin * v.icm - CQmin) / v.den * (1.0 - v.zsw) + qk * v.zsw;
+  double o[2] = {(qk - qnmax) + qnmax * v.icm - CQmax, (qk - qnmin) + qnmin * v.icm - CQmin};
+  quotients(o, v.den);
+  Qmin = o[0] * (1.0 - v.zsw) + qk * v.zsw;
+  Qmax = o[1] * (1.0 - v.zsw) + qk * v.zsw;
 }
 __device__ __forceinline__ double vclamp(double infl, double h, double mnL, double mxL, double mnU, double mxU) {
   const double a1 = (h < mxL) ? h : mxL, b1 = (mnL > a1) ? mnL : a1;
@@ -508,7 +611,7 @@ __device__ __forceinline__ void pole_column(const PlainArgs &P, int p, int t) {
     const double *bc = P.bval(t, k, P.nb - 2 + p);
     for (int v = 1; v <= 5; ++v) {
       const int vp = (v == 5) ? 1 : v + 1, vm = (v == 1) ? 5 : v - 1;
-      const bool c = upmask(P.flxp[off + v] / P.rhop[off]);
+      const bool c = upmask(P.flxp[off + v], P.rhop[off]);
       const int up = c ? v : 0;
       const double *bv = c ? P.bval(t, k, P.ring[p * kVlink + v - 1]) : bc;
       double f = q[up];
@@ -555,48 +658,44 @@ __device__ __forceinline__ void pole_column(const PlainArgs &P, int p, int t) {
   }
 }
 
-// A column and kPair tracers per thread (tracer pairs of a column block are consecutive blocks and
-// share rhog, rhogw and the fluxes in L2), the next level's inputs loaded while a level is worked on.
-// Level k gives Qout of level k-1 and the limited flux of the face below it, which finish level k-2.
-// The last blocks take the pole columns.
-__global__ void __launch_bounds__(kColThreads) k_plain_column(PlainArgs P, int ncolblk) {
+// One column per thread and two tracers (an odd group's last one alone): the two share the column's
+// density, w and limiter parameters and fill each other's latencies (5 tracers at glevel 7, kall 61:
+// 0.92 ms, one tracer per thread 0.97 ms at 4 blocks per SM).  A column block's tracer pairs are
+// consecutive blocks and share rhog, rhogw and the fluxes in L2; the next level's inputs are loaded
+// while a level is worked on.
+// Level k gives Qout of level k-1 and the limited flux of the face below it, which finish level k-2;
+// levels alternate between two slots, so nothing is copied from level to level.
+template <int NT>
+__device__ __forceinline__ void column(const PlainArgs &P, int t0, int l, int col) {
   const Dims &D = P.D;
-  const int npair = (P.nt + kPair - 1) / kPair;
-  if ((int)blockIdx.x >= ncolblk * npair) {
-    const int u = (int)blockIdx.x - ncolblk * npair;
-    pole_column(P, u % kLallPl, u / kLallPl);
-    return;
-  }
-  const int n = D.gmax - D.gmin + 1, col = (int)blockIdx.x / npair * kColThreads + (int)threadIdx.x;
-  if (col >= D.lall * n * n) return;
-  const int t0 = (int)blockIdx.x % npair * kPair, t1 = min(t0 + 1, P.nt - 1);  // an odd group's last pair: one tracer twice
-  const int l = col / (n * n), G = D.gall_1d, K = D.kall;
-  const int c = (col / n % n + D.gmin - 1) * G + col % n + D.gmin - 1;
-  const size_t n3 = P.n3(), base = (size_t)l * K * D.gall + c;
-  const int g = D.gall;
+  const int n = D.gmax - D.gmin + 1;
+  if (col >= n * n) return;
+  const int G = D.gall_1d, K = D.kall;
+  const unsigned g = (unsigned)D.gall, c = (unsigned)((col / n + D.gmin - 1) * G + col % n + D.gmin - 1);
+  const size_t n3 = P.n3(), base = (size_t)l * K * D.gall;
+  // addresses: a base that is the same for the whole block, and a 32-bit offset within the region
   const double *flx = P.flx + base, *rho = P.rho + base, *W = P.w + base;
-  double *Q[kPair] = {P.Q + (size_t)t0 * n3 + base, P.Q + (size_t)t1 * n3 + base};
-  const double *fv[kPair] = {P.fv + (size_t)t0 * 3 * n3 + base, P.fv + (size_t)t1 * 3 * n3 + base};
-  static_assert(kPair == 2, "Q and fv hold a pair");
-  struct In {
-    double Q[kPair], f[kPair][6], flx[6], rho, w;
-  };
-  auto load = [&](int k, bool phys) {
-    In v;
-    const size_t o = (size_t)k * g;
+  double *Q[NT];
+  const double *fv[NT];
 #pragma unroll
-    for (int m = 0; m < 6; ++m) v.flx[m] = flx[m * n3 + o];
+  for (int h = 0; h < NT; ++h) Q[h] = P.Q + (size_t)(t0 + h) * n3 + base, fv[h] = P.fv + (size_t)(t0 + h) * 3 * n3 + base;
+  struct In {
+    double Q[NT], f[NT][6], flx[6], rho, w;
+  };
+  auto load = [&](In &v, int k, bool phys) {
+    const unsigned o = (unsigned)k * g + c;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) v.flx[m] = (flx + m * n3)[o];
     v.rho = rho[o], v.w = W[o];
     if (phys) {
+      const unsigned o4 = o - 1, o5 = o - G - 1, o6 = o - G;
 #pragma unroll
-      for (int h = 0; h < kPair; ++h) {
+      for (int h = 0; h < NT; ++h) {
         v.Q[h] = Q[h][o];
-        const double *f = fv[h] + o;
-        v.f[h][0] = f[0], v.f[h][1] = f[n3], v.f[h][2] = f[2 * n3];
-        v.f[h][3] = f[-1], v.f[h][4] = (f + n3)[-G - 1], v.f[h][5] = (f + 2 * n3)[-G];
+        v.f[h][0] = fv[h][o], v.f[h][1] = (fv[h] + n3)[o], v.f[h][2] = (fv[h] + 2 * n3)[o];
+        v.f[h][3] = fv[h][o4], v.f[h][4] = (fv[h] + n3)[o5], v.f[h][5] = (fv[h] + 2 * n3)[o6];
       }
     }
-    return v;
   };
   auto horiz = [&](const In &v, int h) {  // rhogq after the horizontal sub-step
     double s = v.flx[0] * v.f[h][0];
@@ -604,64 +703,104 @@ __global__ void __launch_bounds__(kColThreads) k_plain_column(PlainArgs P, int n
     for (int m = 1; m < 6; ++m) s = s + v.flx[m] * v.f[h][m];
     return v.Q[h] - s;
   };
-  auto dens = [&](const In &v) {
-    double s = v.flx[0];
-#pragma unroll
-    for (int m = 1; m < 6; ++m) s = s + v.flx[m];
-    return v.rho - s;
-  };
   const int kmin = D.kmin - 1, kmax = D.kmax - 1;
-  In nx = load(kmin, true);
+  In A, B;
+  load(A, kmin, true);
   if (K == 1) {
+    double x[NT];
 #pragma unroll
-    for (int h = 0; h < kPair; ++h) Q[h][0] = horiz(nx, h);
+    for (int h = 0; h < NT; ++h) x[h] = horiz(A, h);
+#pragma unroll
+    for (int h = 0; h < NT; ++h) Q[h][c] = x[h];
     return;
   }
-  double qm[kPair], q[kPair], Qhm[kPair], Qh[kPair], Qmn[kPair], Qmx[kPair], fl[kPair];  // levels k-2 (m), k-1
-  double c1 = 0.0, c2 = 0.0, rp = 1.0, wk = 0.0;  // level k-1: ck1; its density and w
-  for (int k = kmin; k <= kmax + 1; ++k) {
-    const In v = nx;
-    if (k <= kmax) nx = load(k + 1, k < kmax);
-    const double r = dens(v);
-    const double c1n = -v.w * P.dt * P.rdgz[k] / r;
+  // slot s of a window: the level being worked on (before: level k-2); slot 1 - s: level k-1
+  double q[NT][2], Qh[NT][2], Qmn[NT], Qmx[NT], fl[NT];
+  double c1 = 0.0, wk = 0.0;  // ck1 and w of level k-1
+  Recip rp{1.0, 1.0, true};   // its density
+  auto level = [&](const In &v, int k, auto slot) {
+    constexpr int S = decltype(slot)::value, Z = 1 - S;
+    double r = v.flx[0];
+#pragma unroll
+    for (int m = 1; m < 6; ++m) r = r + v.flx[m];
+    const Recip rr = recip(v.rho - r);
+    double x[1 + NT] = {-v.w * P.dt * P.rdgz[k]}, Qn[NT] = {};  // ck1, q of the tracers
+    if (k <= kmax) {
+#pragma unroll
+      for (int h = 0; h < NT; ++h) x[1 + h] = Qn[h] = horiz(v, h);
+    }
+    quotients(x, rr);
     if (k == kmin) {
 #pragma unroll
-      for (int h = 0; h < kPair; ++h) {
-        Qh[h] = horiz(v, h), q[h] = Qh[h] / r, qm[h] = q[h], Qhm[h] = 0.0, Qmn[h] = Qmx[h] = fl[h] = 0.0;
+      for (int h = 0; h < NT; ++h) {
+        Qh[h][S] = Qn[h], q[h][S] = q[h][Z] = x[1 + h];
+        Qmn[h] = Qmx[h] = fl[h] = 0.0;
       }
     } else {
-      c2 = v.w * P.dt * P.rdgz[k - 1] / rp;  // ck2 of level k-1
-      const VPar vp = vpar(c1, c2, c1n);
+      double c2[1] = {v.w * P.dt * P.rdgz[k - 1]};  // ck2 of level k-1
+      quotients(c2, rp);
+      const VPar vp = vpar(c1, c2[0], x[0]);
       const double af = P.afact[k - 1], bf = P.bfact[k - 1];
 #pragma unroll
-      for (int h = 0; h < kPair; ++h) {
-        double Qn = 0.0, qn = q[h];
-        if (k <= kmax) Qn = horiz(v, h), qn = Qn / r;
+      for (int h = 0; h < NT; ++h) {
+        const double qn = k <= kmax ? x[1 + h] : q[h][Z];  // the ghost above repeats the top level
         double lo, hi;
-        vqout(vp, qm[h], q[h], qn, lo, hi);
-        double qh = af * q[h] + bf * qm[h];
+        vqout(vp, q[h][S], q[h][Z], qn, lo, hi);
+        double qh = af * q[h][Z] + bf * q[h][S];
         if (k - 1 > kmin) qh = vclamp(vp.infl, qh, Qmn[h], Qmx[h], lo, hi);
         const double fu = wk * qh;  // through the face below level k-1
         if (k - 1 > kmin) {
-          const double z = Qhm[h] - (fu - fl[h]) * P.dt * P.rdgz[k - 2];
-          Q[h][(size_t)(k - 2) * g] = z;
-          if (k - 2 == kmin) Q[h][0] = z;
+          const double z = Qh[h][S] - (fu - fl[h]) * P.dt * P.rdgz[k - 2];
+          Q[h][(unsigned)(k - 2) * g + c] = z;
+          if (k - 2 == kmin) Q[h][c] = z;
         }
         fl[h] = fu, Qmn[h] = lo, Qmx[h] = hi;
-        Qhm[h] = Qh[h], Qh[h] = Qn, qm[h] = q[h], q[h] = qn;
+        Qh[h][S] = Qn[h], q[h][S] = qn;
       }
     }
-    c1 = c1n, rp = r, wk = v.w;
-  }
-  // level kmax: the flux through the top face is unlimited
+    c1 = x[0], rp = rr, wk = v.w;
+  };
+  using C0 = std::integral_constant<int, 0>;
+  using C1 = std::integral_constant<int, 1>;
+  auto top = [&](auto slot) {  // level kmax: the flux through the top face is unlimited
+    constexpr int S = decltype(slot)::value, Z = 1 - S;  // S: the ghost level's slot, Z: kmax's
 #pragma unroll
-  for (int h = 0; h < kPair; ++h) {
-    const double qh = P.afact[kmax + 1] * q[h] + P.bfact[kmax + 1] * qm[h];
-    const double z = Qhm[h] - (wk * qh - fl[h]) * P.dt * P.rdgz[kmax];
-    Q[h][(size_t)kmax * g] = z;
-    Q[h][(size_t)(K - 1) * g] = z;
-    if (kmin == kmax) Q[h][0] = z;
+    for (int h = 0; h < NT; ++h) {
+      const double qh = P.afact[kmax + 1] * q[h][S] + P.bfact[kmax + 1] * q[h][Z];
+      const double z = Qh[h][Z] - (wk * qh - fl[h]) * P.dt * P.rdgz[kmax];
+      Q[h][(unsigned)kmax * g + c] = z;
+      Q[h][(unsigned)(K - 1) * g + c] = z;
+      if (kmin == kmax) Q[h][c] = z;
+    }
+  };
+#pragma unroll 1
+  for (int k = kmin;; k += 2) {
+    if (k < kmax + 1) load(B, k + 1, k < kmax);
+    level(A, k, C0{});
+    if (k == kmax + 1) {
+      top(C0{});
+      break;
+    }
+    if (k + 1 < kmax + 1) load(A, k + 2, k + 1 < kmax);
+    level(B, k + 1, C1{});
+    if (k + 1 == kmax + 1) {
+      top(C1{});
+      break;
+    }
   }
+}
+
+// blocks: (tracer pair fastest, column block, region), then the pole columns
+__global__ void __launch_bounds__(kColThreads, 2) k_plain_column(PlainArgs P, int colblk, int nmain) {
+  if ((int)blockIdx.x >= nmain) {
+    const int u = (int)blockIdx.x - nmain;
+    pole_column(P, u % kLallPl, u / kLallPl);
+    return;
+  }
+  const int npair = (P.nt + 1) / 2, t0 = (int)blockIdx.x % npair * 2, cb = (int)blockIdx.x / npair;
+  const int l = cb / colblk, col = cb % colblk * kColThreads + (int)threadIdx.x;
+  if (t0 + 1 < P.nt) column<2>(P, t0, l, col);
+  else column<1>(P, t0, l, col);
 }
 
 // the density: rhog -= sum_m flx_h(m), then -= d(rhogw)/dz dt, ghost levels copied.  One thread per
@@ -771,7 +910,7 @@ int step_plain(StepCtx &S, int ntr, double dt, double *rhog, double *rhog_pl, do
   launch_horizontal_flux<double>(D, fin, fout, S.geo, dt, st);
   launches += 2;
   const int n = D.gmax - D.gmin + 1, NK = D.kmax - D.kmin + 1;
-  const int ncolblk = (D.lall * n * n + kColThreads - 1) / kColThreads;
+  const int colblk = (n * n + kColThreads - 1) / kColThreads;  // column blocks of a region
   for (int t0 = 0; t0 < ntr; t0 += kPlainGroup) {
     PlainArgs P{};
     P.D = D, P.nt = (ntr - t0 < kPlainGroup) ? ntr - t0 : kPlainGroup, P.nb = S.nb, P.ns = S.ns, P.dt = dt;
@@ -787,8 +926,8 @@ int step_plain(StepCtx &S, int ntr, double dt, double *rhog, double *rhog_pl, do
     if (e != cudaSuccess) return set_error(std::string("advect_step: ") + cudaGetErrorString(e)), ICA_ERR_CUDA;
     const long long ns = (long long)P.ns * NK * P.nt;
     k_plain_seam<<<(unsigned)((ns + 127) / 128), 128, 0, st>>>(P);
-    const int npair = (P.nt + kPair - 1) / kPair;
-    k_plain_column<<<(unsigned)(ncolblk * npair + kLallPl * P.nt), kColThreads, 0, st>>>(P, ncolblk);
+    const int nmain = colblk * D.lall * ((P.nt + 1) / 2);
+    k_plain_column<<<(unsigned)(nmain + kLallPl * P.nt), kColThreads, 0, st>>>(P, colblk, nmain);
     launches += 3;
   }
   const long long nr = ((long long)D.lall * n * n + kLallPl) * NK;

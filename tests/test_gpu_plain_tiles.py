@@ -30,3 +30,26 @@ def test_plain_step_every_tile_form(built, glevel, rlevel, kall, ntr):
             np.testing.assert_array_equal(G[k], S[k], err_msg=k)
     finally:
         ctx.close()
+
+
+def test_plain_step_quotients_at_every_magnitude(built):
+    """The step forms several quotients from one reciprocal where that is exact and divides where it
+    is not: mixing ratios of 1e-309 (subnormal), 1e-300, 1e-240 and 1e250, and a zero tracer, against
+    the oracle's divisions, bit for bit."""
+    from icoatmosbenchmark_v1_b200 import api
+    from oracle import oracle as O
+    c = case(4, 0, 8, 5)
+    g, f = c["grid"], c["fields"]
+    scale = np.array([1e-309, 1e-300, 1e-240, 1e250, 0.0]).reshape(5, 1, 1, 1)
+    S = {k: v * scale if k.startswith("rhogq") else v.copy() for k, v in c["state"].items()}
+    G = {k: v.copy() for k, v in S.items()}
+    ctx = api.IcoAdv(4, 0, 6)
+    try:
+        ctx.set_grid(g)
+        O.step(c["dims"], g.have_sgp, c["topo"], c["dt"], S, f, g.arrays, nthreads=8)
+        ctx.advect_step(c["dt"], G["rhog"], G["rhog_pl"], G["rhogq"], G["rhogq_pl"], f["rhogvx"], f["rhogvx_pl"],
+                        f["rhogvy"], f["rhogvy_pl"], f["rhogvz"], f["rhogvz_pl"], f["rhogw"], f["rhogw_pl"])
+        for k in S:
+            np.testing.assert_array_equal(G[k], S[k], err_msg=k)
+    finally:
+        ctx.close()
