@@ -367,7 +367,7 @@ int vlim_dev(Ctx *c, T *q_h, T *q_h_pl, const T *q, const T *q_pl, const T *d, c
   if (!q_h || !q_h_pl || !q || !q_pl || !d || !d_pl || !ck || !ck_pl)
     return set_error("vertical_limiter_thuburn: NULL argument"), ICA_ERR_ARG;
   launch_vlim<T>(c->D, q_h, q_h_pl, q, q_pl, d, d_pl, ck, ck_pl, c->stream);
-  if (c->D.kmax > c->D.kmin) c->launches += c->D.have_pl ? 2 : 1;
+  if (c->D.kmax > c->D.kmin) c->launches += 1;
   return c->check_launch("vertical_limiter_thuburn");
 }
 

@@ -403,21 +403,31 @@ __global__ void k_hlim_apply_pl(Dims D, LimIn<T> in, T *q_a_pl, const T *Qout_pl
 }
 
 // ---------------------------------------------------------------------------
-// vertical_limiter_thuburn: one thread per column g, the k-recurrence in registers
+// vertical_limiter_thuburn: one thread per column and kVlimLevels consecutive half levels.  A half
+// level needs the Qout of the levels on both sides and nothing else of the column, so the columns
+// are cut into chunks that share one Qout at each cut (one in kVlimLevels is formed twice).  With a
+// column per thread a glevel-6 grid gave the card 341 blocks and a chain of 40 dependent levels
+// (69 us, and 56 us more for the 12 pole columns in a launch behind it); now bound by memory:
+// 170 us for glevel 7, kall 96 (0.78 GB, 120 us at the copy rate; 8 and 16 levels a thread alike,
+// 4 levels 188), and below the call's host time at glevel 6 (132 -> 27 us a call).
+constexpr int kVlimLevels = 8, kVlimThreads = 128;
+
+template <typename T>
+struct VlimLevel {  // what Qout of a level reads: its own values and q and ck1 around it
+  T q, d, c1, c2;
+};
 template <typename T, bool POLE>
-__device__ __forceinline__ void vlim_qout(const T *q, const T *d, const T *ck1, const T *ck2, size_t s, int k,
-                                          T &inflagL, T &Qmin, T &Qmax) {
+__device__ __forceinline__ void vlim_qout(T qm, const VlimLevel<T> &v, T qp, T c1p, T &inflagL, T &Qmin, T &Qmax) {
   const T BIG = Num<T>::big(), EPS = Num<T>::eps();
-  inflagL = T(0.5) - fsign(T(0.5), ck1[(size_t)k * s]);
-  const T inflagU = T(0.5) + fsign(T(0.5), ck1[(size_t)(k + 1) * s]);
-  const T qk = q[(size_t)k * s], qm = q[(size_t)(k - 1) * s], qp = q[(size_t)(k + 1) * s];
+  inflagL = T(0.5) - fsign(T(0.5), v.c1);
+  const T inflagU = T(0.5) + fsign(T(0.5), c1p);
+  const T qk = v.q, c1 = v.c1, c2 = v.c2;
   const T minL = mn(qk, qm) + (T(1) - inflagL) * BIG;
   const T minU = mn(qk, qp) + (T(1) - inflagU) * BIG;
   const T maxL = mx(qk, qm) - (T(1) - inflagL) * BIG;
   const T maxU = mx(qk, qp) - (T(1) - inflagU) * BIG;
   const T qnmin = mn(mn(minL, minU), qk);
   const T qnmax = mx(mx(maxL, maxU), qk);
-  const T c1 = ck1[(size_t)k * s], c2 = ck2[(size_t)k * s];
   const T Cin = inflagL * c1 + inflagU * c2;
   const T Cout = (T(1) - inflagL) * c1 + (T(1) - inflagU) * c2;
   T CQmin, CQmax;
@@ -429,32 +439,64 @@ __device__ __forceinline__ void vlim_qout(const T *q, const T *d, const T *ck1, 
     CQmax = inflagL * c1 * maxL + inflagU * c2 * maxU;
   }
   const T zerosw = T(0.5) - fsign(T(0.5), fabs(Cout) - EPS);
-  const T dv = d[(size_t)k * s];
-  Qmin = ((qk - qnmax) + qnmax * (Cin + Cout - dv) - CQmax) / (Cout + zerosw) * (T(1) - zerosw) + qk * zerosw;
-  Qmax = ((qk - qnmin) + qnmin * (Cin + Cout - dv) - CQmin) / (Cout + zerosw) * (T(1) - zerosw) + qk * zerosw;
+  Qmin = ((qk - qnmax) + qnmax * (Cin + Cout - v.d) - CQmax) / (Cout + zerosw) * (T(1) - zerosw) + qk * zerosw;
+  Qmax = ((qk - qnmin) + qnmin * (Cin + Cout - v.d) - CQmin) / (Cout + zerosw) * (T(1) - zerosw) + qk * zerosw;
 }
 
+// half levels [k0, k0 + kVlimLevels) (0-based, below kmax) of one column; arrays at the column's
+// first level, g elements from level to level, ck2 at ck + ck2off.  Levels kmin - 1 and kmax + 1
+// lie inside the arrays of a grid with ghost levels; without them the nearest level is read.
 template <typename T, bool POLE>
-__global__ void k_vlim(int ncol, int colsize, int kall, int kmin, int kmax, T *q_h, const T *q, const T *d,
-                       const T *ck) {
-  // column index t -> (l, g); fields (g,k,l) with stride colsize between levels
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ncol) return;
-  const int l = t / colsize, g = t % colsize;
-  const size_t base = (size_t)l * kall * colsize + g;
-  const size_t ck2off = (size_t)(ncol / colsize) * kall * colsize;
-  const T *ck1 = ck + base, *ck2 = ck + ck2off + base;
-  T fl, Qmin_km1, Qmax_km1;
-  vlim_qout<T, POLE>(q + base, d + base, ck1, ck2, colsize, kmin - 1, fl, Qmin_km1, Qmax_km1);
-  for (int k = kmin; k <= kmax - 1; ++k) {  // 0-based k = Fortran kmin+1 .. kmax
+__device__ __forceinline__ void vlim_chunk(unsigned g, int k0, int kmax, int kall, T *qh, const T *q, const T *d,
+                                           const T *ck, size_t ck2off) {
+  const T *ck2 = ck + ck2off;
+  const int k1 = min(k0 + kVlimLevels, kmax);
+  auto at = [&](int k) { return (unsigned)min(max(k, 0), kall - 1) * g; };
+  auto level = [&](int k) { return VlimLevel<T>{q[at(k)], d[at(k)], ck[at(k)], ck2[at(k)]}; };
+  VlimLevel<T> m = level(k0 - 1), v = level(k0);
+  T qp = q[at(k0 + 1)], c1p = ck[at(k0 + 1)], qm = q[at(k0 - 2)], fl, Qmin_m, Qmax_m;
+  vlim_qout<T, POLE>(qm, m, v.q, v.c1, fl, Qmin_m, Qmax_m);
+  qm = m.q;
+#pragma unroll 4
+  for (int k = k0; k < k1; ++k) {
+    VlimLevel<T> n{qp, T(0), c1p, T(0)};
+    T qn = T(0), c1n = T(0);
+    if (k + 1 < k1) {  // the next level's inputs
+      n.d = d[at(k + 1)], n.c2 = ck2[at(k + 1)];
+      qn = q[at(k + 2)], c1n = ck[at(k + 2)];
+    }
+    T &o = qh[at(k)];
+    const T h = o;
     T inflagL, Qmin, Qmax;
-    vlim_qout<T, POLE>(q + base, d + base, ck1, ck2, colsize, k, inflagL, Qmin, Qmax);
-    const size_t e = base + (size_t)k * colsize;
-    const T qh = q_h[e];
-    q_h[e] = inflagL * mx(mn(qh, Qmax_km1), Qmin_km1) + (T(1) - inflagL) * mx(mn(qh, Qmax), Qmin);
-    Qmin_km1 = Qmin;
-    Qmax_km1 = Qmax;
+    vlim_qout<T, POLE>(qm, v, qp, c1p, inflagL, Qmin, Qmax);
+    o = inflagL * mx(mn(h, Qmax_m), Qmin_m) + (T(1) - inflagL) * mx(mn(h, Qmax), Qmin);
+    Qmin_m = Qmin, Qmax_m = Qmax;
+    qm = v.q, v = n, qp = qn, c1p = c1n;
   }
+}
+
+// blocks: column blocks of a region fastest, then its chunks, then the regions; the last blocks take
+// the pole columns
+template <typename T>
+__global__ void __launch_bounds__(kVlimThreads) k_vlim(Dims D, int nchunk, int colblk, int nmain, T *q_h, const T *q,
+                                                       const T *d, const T *ck, T *q_h_pl, const T *q_pl,
+                                                       const T *d_pl, const T *ck_pl) {
+  const int b = blockIdx.x;
+  if (b < nmain) {
+    const int u = b % colblk * kVlimThreads + (int)threadIdx.x;
+    if (u >= D.gall) return;
+    const int l = b / colblk / nchunk, k0 = D.kmin + b / colblk % nchunk * kVlimLevels;  // 0-based kmin+1 ..
+    const size_t base = (size_t)l * D.kall * D.gall + u;
+    vlim_chunk<T, false>(D.gall, k0, D.kmax, D.kall, q_h + base, q + base, d + base, ck + base,
+                         (size_t)D.lall * D.kall * D.gall);
+    return;
+  }
+  const int t = (b - nmain) * kVlimThreads + (int)threadIdx.x;
+  if (t >= kLallPl * kGallPl * nchunk) return;
+  const int col = t % (kLallPl * kGallPl), k0 = D.kmin + t / (kLallPl * kGallPl) * kVlimLevels;
+  const size_t base = (size_t)(col / kGallPl) * D.kall * kGallPl + col % kGallPl;
+  vlim_chunk<T, true>(kGallPl, k0, D.kmax, D.kall, q_h_pl + base, q_pl + base, d_pl + base, ck_pl + base,
+                      (size_t)kLallPl * D.kall * kGallPl);
 }
 
 // ---------------------------------------------------------------------------
@@ -509,10 +551,11 @@ template <typename T>
 void launch_vlim(const Dims &D, T *q_h, T *q_h_pl, const T *q, const T *q_pl, const T *d, const T *d_pl,
                  const T *ck, const T *ck_pl, cudaStream_t s) {
   if (D.kmax <= D.kmin) return;
-  const int ncol = D.gall * D.lall;
-  k_vlim<T, false><<<(ncol + 127) / 128, 128, 0, s>>>(ncol, D.gall, D.kall, D.kmin, D.kmax, q_h, q, d, ck);
-  const int ncp = kGallPl * kLallPl;
-  if (D.have_pl) k_vlim<T, true><<<1, 32, 0, s>>>(ncp, kGallPl, D.kall, D.kmin, D.kmax, q_h_pl, q_pl, d_pl, ck_pl);
+  const int nchunk = (D.kmax - D.kmin + kVlimLevels - 1) / kVlimLevels;
+  const int colblk = (D.gall + kVlimThreads - 1) / kVlimThreads, nmain = colblk * nchunk * D.lall;
+  const int npole = D.have_pl ? (kLallPl * kGallPl * nchunk + kVlimThreads - 1) / kVlimThreads : 0;
+  k_vlim<T><<<(unsigned)(nmain + npole), kVlimThreads, 0, s>>>(D, nchunk, colblk, nmain, q_h, q, d, ck, q_h_pl, q_pl,
+                                                               d_pl, ck_pl);
 }
 
 template <typename T>
