@@ -44,157 +44,135 @@ template <typename T> __device__ __forceinline__ T fsign(T a, T b) { return copy
 
 // ---------------------------------------------------------------------------
 // horizontal_flux
-struct TriVal {
-  double r, x, y, z;
-};
-template <typename T> struct Tri {
-  T r, x, y, z;
-};
+// One thread per cell, kFluxLevels levels one after the other.  A cell's three faces need four
+// triangles (AI = TJ(i,j-1) + TI(i,j), AIJ = TI(i,j) + TJ(i,j), AJ = TJ(i,j) + TI(i-1,j)), formed once
+// each from the fields of the six cells they touch, each field loaded once; the cell's weights,
+// normals, arc midpoints and areas stay in registers from level to level.  Forming the triangles
+// face by face took 72 field loads and 1000 instructions a cell and level; these are 570, and what
+// bounds the kernel is the latency of a level's loads at 4 blocks per SM, so each thread asks for its
+// own cell's fields of the next level one level ahead (its neighbours' are other threads' own).
+// glevel 7, rlevel 1, kall 61 (1.6 GB, 248 us at the copy rate): 642 -> 359 us; 433 without the
+// prefetch, 371 at 3 blocks, 452 with 4 levels a thread; with the geometry in shared memory 470 and more.
+constexpr int kFluxThreads = 128, kFluxLevels = 8;
 
 template <typename T>
-__device__ __forceinline__ Tri<T> tri_TI(const Dims &D, const FluxIn<T> &in, const Geo<T> &g, int l,
-                                         size_t off, int ij) {
-  // rhot_TI(ij) = rho(ij)*W1 + rho(ip1j)*W2, then + rho(ip1jp1)*W3   (:146-153, :171-174)
-  const size_t gw = (size_t)D.gall * D.lall;
-  const T w1 = g.GMTR_t[(size_t)(W1 - 1) * 2 * gw + (size_t)(TI - 1) * gw + (size_t)l * D.gall + (ij - 1)];
-  const T w2 = g.GMTR_t[(size_t)(W2 - 1) * 2 * gw + (size_t)(TI - 1) * gw + (size_t)l * D.gall + (ij - 1)];
-  const T w3 = g.GMTR_t[(size_t)(W3 - 1) * 2 * gw + (size_t)(TI - 1) * gw + (size_t)l * D.gall + (ij - 1)];
-  const int a = ij - 1, b = ij, c = ij + D.gall_1d;
-  Tri<T> t;
-  t.r = in.rho[off + a] * w1 + in.rho[off + b] * w2;
-  t.x = in.rhovx[off + a] * w1 + in.rhovx[off + b] * w2;
-  t.y = in.rhovy[off + a] * w1 + in.rhovy[off + b] * w2;
-  t.z = in.rhovz[off + a] * w1 + in.rhovz[off + b] * w2;
-  t.r = t.r + in.rho[off + c] * w3;
-  t.x = t.x + in.rhovx[off + c] * w3;
-  t.y = t.y + in.rhovy[off + c] * w3;
-  t.z = t.z + in.rhovz[off + c] * w3;
+struct Vec4 {  // rho, rhovx, rhovy, rhovz of a cell or triangle
+  T v[4];
+};
+
+// triangle value f0 w1 + f1 w2 + f2 w3 (:146-183); TI(ij) takes (ij, ip1j, ip1jp1), TJ(ij) takes
+// (ij, ip1jp1, ijp1)
+template <typename T>
+__device__ __forceinline__ Vec4<T> tri(const Vec4<T> &f0, const Vec4<T> &f1, const Vec4<T> &f2, const T (&w)[3]) {
+  Vec4<T> t;
+#pragma unroll
+  for (int x = 0; x < 4; ++x) t.v[x] = f0.v[x] * w[0] + f1.v[x] * w[1] + f2.v[x] * w[2];
   return t;
 }
 
 template <typename T>
-__device__ __forceinline__ Tri<T> tri_TJ(const Dims &D, const FluxIn<T> &in, const Geo<T> &g, int l,
-                                         size_t off, int ij) {
-  // rhot_TJ(ij) = rho(ij)*W1, then + rho(ip1jp1)*W2 + rho(ijp1)*W3   (:155-158, :176-183)
-  const size_t gw = (size_t)D.gall * D.lall;
-  const T w1 = g.GMTR_t[(size_t)(W1 - 1) * 2 * gw + (size_t)(TJ - 1) * gw + (size_t)l * D.gall + (ij - 1)];
-  const T w2 = g.GMTR_t[(size_t)(W2 - 1) * 2 * gw + (size_t)(TJ - 1) * gw + (size_t)l * D.gall + (ij - 1)];
-  const T w3 = g.GMTR_t[(size_t)(W3 - 1) * 2 * gw + (size_t)(TJ - 1) * gw + (size_t)l * D.gall + (ij - 1)];
-  const int a = ij - 1, c = ij + D.gall_1d, e = ij + D.gall_1d - 1;
-  Tri<T> t;
-  t.r = in.rho[off + a] * w1;
-  t.x = in.rhovx[off + a] * w1;
-  t.y = in.rhovy[off + a] * w1;
-  t.z = in.rhovz[off + a] * w1;
-  t.r = t.r + in.rho[off + c] * w2 + in.rho[off + e] * w3;
-  t.x = t.x + in.rhovx[off + c] * w2 + in.rhovx[off + e] * w3;
-  t.y = t.y + in.rhovy[off + c] * w2 + in.rhovy[off + e] * w3;
-  t.z = t.z + in.rhovz[off + c] * w2 + in.rhovz[off + e] * w3;
-  return t;
-}
+__device__ __forceinline__ void pole_flux(const Dims &D, const FluxIn<T> &in, const FluxOut<T> &out, const Geo<T> &g,
+                                          T dt, int l, int k);
 
-// TI with the singular-point override rhot_TI(gmin-1,gmin-1) = rhot_TJ(gmin,gmin-1)   (:188-201)
+// blocks: level blocks fastest (a cell block's geometry is read from L2 after the first), then cell
+// blocks, then regions; the last blocks take the poles, one thread per (pole, level)
 template <typename T>
-__device__ __forceinline__ Tri<T> tri_TI_s(const Dims &D, const FluxIn<T> &in, const Geo<T> &g, int l,
-                                           size_t off, int i, int j, bool sgp) {
-  const int ij = (j - 1) * D.gall_1d + i;
-  if (sgp && i == D.gmin - 1 && j == D.gmin - 1) return tri_TJ(D, in, g, l, off, ij + 1);
-  return tri_TI(D, in, g, l, off, ij);
-}
-
-template <typename T>
-__global__ void k_horizontal_flux(Dims D, FluxIn<T> in, FluxOut<T> out, Geo<T> g, T dt) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y;  // l*kall + k
-  const int l = kl / D.kall;
-  const int i = c % D.gall_1d + 1, j = c / D.gall_1d + 1;
-  const int ij = c + 1, G = D.gall_1d, gmin = D.gmin, gmax = D.gmax;
-  const size_t off = (size_t)kl * D.gall;                  // (k,l) slab of a 3-D field
-  const size_t fs = (size_t)D.lall * D.kall * D.gall;      // stride of the last dimension
-  const size_t gw = (size_t)D.gall * D.lall;               // geometry stride
+__global__ void __launch_bounds__(kFluxThreads, 4) k_horizontal_flux(Dims D, FluxIn<T> in, FluxOut<T> out, Geo<T> g, T dt,
+                                                                  int nlb, int cellblk, int nmain) {
+  if ((int)blockIdx.x >= nmain) {
+    const int t = ((int)blockIdx.x - nmain) * kFluxThreads + (int)threadIdx.x;
+    if (t < D.kall * kLallPl) pole_flux(D, in, out, g, dt, t / D.kall, t % D.kall);
+    return;
+  }
+  const int lb = (int)blockIdx.x % nlb, l = (int)blockIdx.x / nlb / cellblk;
+  const int ci = (int)blockIdx.x / nlb % cellblk * kFluxThreads + (int)threadIdx.x;
+  if (ci >= D.gall) return;
+  const int G = D.gall_1d, gmin = D.gmin, gmax = D.gmax;
+  const int i = ci % G + 1, j = ci / G + 1;
+  const unsigned c = ci;
+  const size_t fs = (size_t)D.lall * D.kall * D.gall;  // stride of the last dimension
+  const size_t gw = (size_t)D.gall * D.lall, lg = (size_t)l * D.gall;
   const bool sgp = D.have_sgp[l] != 0;
   const T EPS = Num<T>::eps();
-  const T rarea_ij = g.GMTR_p[(size_t)(P_RAREA - 1) * gw + (size_t)l * D.gall + c];
-  auto HN = [&](int cell, int a, int h) -> T {
-    return g.GMTR_a[((size_t)(h - 1) * 3 + (a - 1)) * gw + (size_t)l * D.gall + (cell - 1)];
-  };
-  auto XR = [&](int cell, int a, int x) -> T {
-    return g.GRD_xr[((size_t)(x - 1) * 3 + (a - 1)) * gw + (size_t)l * D.gall + (cell - 1)];
-  };
-  auto store_xc = [&](int a, T x, T y, T z) {
-    out.GRD_xc[((size_t)0 * 3 + (a - 1)) * fs + off + c] = x;
-    out.GRD_xc[((size_t)1 * 3 + (a - 1)) * fs + off + c] = y;
-    out.GRD_xc[((size_t)2 * 3 + (a - 1)) * fs + off + c] = z;
-  };
-  auto face = [&](const Tri<T> &p, const Tri<T> &q, int a, T &rrhoa2, T &vx, T &vy, T &vz) -> T {
-    rrhoa2 = T(1) / mx(p.r + q.r, EPS);
-    vx = p.x + q.x;
-    vy = p.y + q.y;
-    vz = p.z + q.z;
-    return T(0.5) * (vx * HN(ij, a, HNX) + vy * HN(ij, a, HNY) + vz * HN(ij, a, HNZ));
-  };
   const bool inI = (i >= gmin && i <= gmax), inJ = (j >= gmin && j <= gmax);
-  const bool extI = (i >= gmin - 1 && i <= gmax), extJ = (j >= gmin - 1 && j <= gmax);
-  // AI face of (i,j): flx_h(ij,1), flx_h(ip1j,4), GRD_xc(ij,AI)   (:235-257)
-  if (inJ && extI) {
-    T r2, vx, vy, vz;
-    const Tri<T> tj = tri_TJ(D, in, g, l, off, ij - G);  // TJ(ijm1): j-1 >= gmin-1, never singular
-    const Tri<T> ti = tri_TI_s(D, in, g, l, off, i, j, sgp);
-    const T flux = face(tj, ti, AI, r2, vx, vy, vz);
-    out.flx_h[(size_t)0 * fs + off + c] = flux * rarea_ij * dt;
-    const T rarea_n = g.GMTR_p[(size_t)(P_RAREA - 1) * gw + (size_t)l * D.gall + c + 1];
-    out.flx_h[(size_t)3 * fs + off + c + 1] = -flux * rarea_n * dt;
-    store_xc(AI, XR(ij, AI, 1) - vx * r2 * dt * T(0.5), XR(ij, AI, 2) - vy * r2 * dt * T(0.5),
-             XR(ij, AI, 3) - vz * r2 * dt * T(0.5));
-  } else {
-    out.flx_h[(size_t)0 * fs + off + c] = T(0);
-    store_xc(AI, T(0), T(0), T(0));
+  const bool ext = (i >= gmin - 1 && i <= gmax && j >= gmin - 1 && j <= gmax);
+  const bool face[3] = {ext && inJ, ext, ext && inI};
+  // flx_h(:,4:6) elements no face writes: this cell writes them itself
+  const bool in1 = i - 1 >= gmin - 1 && i - 1 <= gmax, jn1 = j - 1 >= gmin - 1 && j - 1 <= gmax;
+  const bool own[3] = {!(inJ && in1), !(in1 && jn1), !(inI && jn1)};
+  // TI(gmin-1,gmin-1) of a singular region is TJ(gmin,gmin-1) (:188-201): read by the AIJ face of
+  // (gmin-1,gmin-1) and the AJ face of (gmin,gmin-1), whose flx_h(gmin,gmin,6) is zero (:311-320)
+  const bool singI = sgp && i == gmin - 1 && j == gmin - 1, singJ = sgp && i == gmin && j == gmin - 1;
+  T wI[3] = {}, wJ[3] = {}, wJm[3] = {}, wIm[3] = {}, wS[3] = {}, hn[3][3] = {}, xr[3][3] = {}, ra[4] = {};
+  if (ext) {
+    auto weights = [&](int t, unsigned cell, T (&w)[3]) {
+#pragma unroll
+      for (int n = 0; n < 3; ++n) w[n] = (g.GMTR_t + ((size_t)(W1 - 1 + n) * 2 + (t - 1)) * gw + lg)[cell];
+    };
+    weights(TI, c, wI), weights(TJ, c, wJ);
+    if (inJ) weights(TJ, c - G, wJm);
+    if (inI) weights(TI, c - 1, wIm);
+    if (singI) weights(TJ, c + 1, wS);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        hn[a][x] = (g.GMTR_a + ((size_t)x * 3 + a) * gw + lg)[c];
+        xr[a][x] = (g.GRD_xr + ((size_t)x * 3 + a) * gw + lg)[c];
+      }
+    const T *rarea = g.GMTR_p + (size_t)(P_RAREA - 1) * gw + lg;
+    ra[0] = rarea[c], ra[1] = rarea[c + 1], ra[2] = rarea[c + G + 1], ra[3] = rarea[c + G];
   }
-  // flx_h(ij,4) when no AI face of im1j writes it
-  if (!(inJ && i - 1 >= gmin - 1 && i - 1 <= gmax)) out.flx_h[(size_t)3 * fs + off + c] = T(0);
-  // AIJ face: flx_h(ij,2), flx_h(ip1jp1,5), GRD_xc(ij,AIJ)   (:261-283)
-  if (extI && extJ) {
-    T r2, vx, vy, vz;
-    const Tri<T> ti = tri_TI_s(D, in, g, l, off, i, j, sgp);
-    const Tri<T> tj = tri_TJ(D, in, g, l, off, ij);
-    const T flux = face(ti, tj, AIJ, r2, vx, vy, vz);
-    out.flx_h[(size_t)1 * fs + off + c] = flux * rarea_ij * dt;
-    const T rarea_n = g.GMTR_p[(size_t)(P_RAREA - 1) * gw + (size_t)l * D.gall + c + G + 1];
-    out.flx_h[(size_t)4 * fs + off + c + G + 1] = -flux * rarea_n * dt;
-    store_xc(AIJ, XR(ij, AIJ, 1) - vx * r2 * dt * T(0.5), XR(ij, AIJ, 2) - vy * r2 * dt * T(0.5),
-             XR(ij, AIJ, 3) - vz * r2 * dt * T(0.5));
-  } else {
-    out.flx_h[(size_t)1 * fs + off + c] = T(0);
-    store_xc(AIJ, T(0), T(0), T(0));
+  const int k1 = min((lb + 1) * kFluxLevels, D.kall);
+#pragma unroll 1
+  for (int k = lb * kFluxLevels; k < k1; ++k) {
+    const size_t off = ((size_t)l * D.kall + k) * D.gall;
+    auto cell = [&](unsigned p) {
+      return Vec4<T>{{(in.rho + off)[p], (in.rhovx + off)[p], (in.rhovy + off)[p], (in.rhovz + off)[p]}};
+    };
+    if (k + 1 < k1) {
+      const size_t on = off + D.gall;
+      for (const T *q : {in.rho, in.rhovx, in.rhovy, in.rhovz})
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(q + on + c));
+    }
+    Vec4<T> tI{}, tJ{}, tJm{}, tIm{};
+    if (ext) {
+      const Vec4<T> f00 = cell(c), f10 = cell(c + 1), f11 = cell(c + G + 1), f01 = cell(c + G);
+      Vec4<T> f0m{}, fm0{};
+      if (inJ) f0m = cell(c - G);
+      if (inI) fm0 = cell(c - 1);
+      tI = tri(f00, f10, f11, wI), tJ = tri(f00, f11, f01, wJ);
+      tJm = tri(f0m, f10, f00, wJm), tIm = tri(fm0, f00, f01, wIm);
+      if (singI) tI = tri(f10, cell(c + G + 2), f11, wS);
+      if (singJ) tIm = tJ;
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      T *flx = out.flx_h + (size_t)a * fs + off, *fln = out.flx_h + (size_t)(a + 3) * fs + off;
+      T f = T(0), x[3] = {T(0), T(0), T(0)};
+      if (face[a]) {  // :235-309
+        const Vec4<T> &p = (a == 0) ? tJm : (a == 1 ? tI : tJ), &q = (a == 0) ? tI : (a == 1 ? tJ : tIm);
+        const T rrhoa2 = T(1) / mx(p.v[0] + q.v[0], EPS);
+        const T v[3] = {p.v[1] + q.v[1], p.v[2] + q.v[2], p.v[3] + q.v[3]};
+        const T flux = T(0.5) * (v[0] * hn[a][0] + v[1] * hn[a][1] + v[2] * hn[a][2]);
+        f = flux * ra[0] * dt;
+        const unsigned nb = c + (a == 0 ? 1 : (a == 1 ? G + 1 : G));
+        fln[nb] = (a == 2 && singJ) ? T(0) : -flux * ra[a + 1] * dt;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) x[d] = xr[a][d] - v[d] * rrhoa2 * dt * T(0.5);
+      }
+      flx[c] = f;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) (out.GRD_xc + ((size_t)d * 3 + a) * fs + off)[c] = x[d];
+      if (own[a]) fln[c] = T(0);
+    }
   }
-  if (!(i - 1 >= gmin - 1 && i - 1 <= gmax && j - 1 >= gmin - 1 && j - 1 <= gmax))
-    out.flx_h[(size_t)4 * fs + off + c] = T(0);
-  // AJ face: flx_h(ij,3), flx_h(ijp1,6), GRD_xc(ij,AJ)   (:286-309), singular flx_h(gmin,gmin,6)=0 (:311-320)
-  if (inI && extJ) {
-    T r2, vx, vy, vz;
-    const Tri<T> tj = tri_TJ(D, in, g, l, off, ij);
-    const Tri<T> ti = tri_TI_s(D, in, g, l, off, i - 1, j, sgp);
-    const T flux = face(tj, ti, AJ, r2, vx, vy, vz);
-    out.flx_h[(size_t)2 * fs + off + c] = flux * rarea_ij * dt;
-    const T rarea_n = g.GMTR_p[(size_t)(P_RAREA - 1) * gw + (size_t)l * D.gall + c + G];
-    const bool sing6 = sgp && i == gmin && j + 1 == gmin;
-    out.flx_h[(size_t)5 * fs + off + c + G] = sing6 ? T(0) : -flux * rarea_n * dt;
-    store_xc(AJ, XR(ij, AJ, 1) - vx * r2 * dt * T(0.5), XR(ij, AJ, 2) - vy * r2 * dt * T(0.5),
-             XR(ij, AJ, 3) - vz * r2 * dt * T(0.5));
-  } else {
-    out.flx_h[(size_t)2 * fs + off + c] = T(0);
-    store_xc(AJ, T(0), T(0), T(0));
-  }
-  if (!(inI && j - 1 >= gmin - 1 && j - 1 <= gmax)) out.flx_h[(size_t)5 * fs + off + c] = T(0);
 }
 
+// one level of a pole (:326-374)
 template <typename T>
-__global__ void k_horizontal_flux_pl(Dims D, FluxIn<T> in, FluxOut<T> out, Geo<T> g, T dt) {
-  // poles (:326-374): one thread per (k, pole)
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= D.kall * kLallPl) return;
-  const int k = t % D.kall, l = t / D.kall;
+__device__ __forceinline__ void pole_flux(const Dims &D, const FluxIn<T> &in, const FluxOut<T> &out, const Geo<T> &g,
+                                          T dt, int l, int k) {
   const T EPS = Num<T>::eps();
   const size_t off = ((size_t)l * D.kall + k) * kGallPl;
   const size_t fsp = (size_t)kLallPl * D.kall * kGallPl;
@@ -530,8 +508,10 @@ static inline dim3 slab_grid(const Dims &D, int threads) {
 template <typename T>
 void launch_horizontal_flux(const Dims &D, const FluxIn<T> &in, const FluxOut<T> &out, const Geo<T> &g, T dt,
                             cudaStream_t s) {
-  k_horizontal_flux<T><<<slab_grid(D, 128), 128, 0, s>>>(D, in, out, g, dt);
-  if (D.have_pl) k_horizontal_flux_pl<T><<<(D.kall * kLallPl + 63) / 64, 64, 0, s>>>(D, in, out, g, dt);
+  const int nlb = (D.kall + kFluxLevels - 1) / kFluxLevels, cellblk = (D.gall + kFluxThreads - 1) / kFluxThreads;
+  const int nmain = nlb * cellblk * D.lall;
+  const int npole = D.have_pl ? (D.kall * kLallPl + kFluxThreads - 1) / kFluxThreads : 0;
+  k_horizontal_flux<T><<<(unsigned)(nmain + npole), kFluxThreads, 0, s>>>(D, in, out, g, dt, nlb, cellblk, nmain);
 }
 
 template <typename T>
