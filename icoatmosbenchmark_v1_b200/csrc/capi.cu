@@ -119,6 +119,18 @@ int ica_init(const ica_dims *dims, ica_ctx **out) {
     cudaMemcpy(p.dst, d.data(), sizeof(int) * p.n, cudaMemcpyHostToDevice);
     cudaMemcpy(p.src, sr.data(), sizeof(int) * p.n, cudaMemcpyHostToDevice);
   }
+  {  // the fill as a map from every point to its source (itself where no list writes it)
+    std::vector<int> d, sr, m((size_t)t.npoints());
+    rc = t.build_plan(false, d, sr);
+    if (rc) { delete c; return set_error("halo plan: a source is also a destination"), rc; }
+    for (size_t p = 0; p < m.size(); ++p) m[p] = (int)p;
+    for (size_t p = 0; p < d.size(); ++p) m[d[p]] = sr[p];
+    if (cudaMalloc(&c->halo_src, sizeof(int) * m.size()) != cudaSuccess) {
+      delete c;
+      return set_error("cudaMalloc(halo sources)"), ICA_ERR_NOMEM;
+    }
+    cudaMemcpy(c->halo_src, m.data(), sizeof(int) * m.size(), cudaMemcpyHostToDevice);
+  }
   if (cudaMalloc(&c->d_have_sgp, sizeof(int) * t.nrgn) != cudaSuccess) {
     delete c;
     return set_error("cudaMalloc(have_sgp)"), ICA_ERR_NOMEM;
@@ -235,6 +247,7 @@ Ctx::~Ctx() {
     if (geo32[i]) cudaFree(geo32[i]);
   }
   if (d_have_sgp) cudaFree(d_have_sgp);
+  if (halo_src) cudaFree(halo_src);
   for (void *p : stepgeo)
     if (p) cudaFree(p);
   for (void *p : {(void *)fast.bsrc, (void *)fast.blist, (void *)fast.ring, (void *)fast.carry, (void *)fast.cg32,
@@ -315,7 +328,7 @@ int comm_dev(Ctx *c, T *var, T *var_pl, int kmax, int vmax, bool pole_fill) {
 template <typename T>
 int hlim_dev(Ctx *c, T *q_a, T *q_a_pl, const T *q, const T *q_pl, const T *d, const T *d_pl, const T *ch,
              const T *ch_pl, const T *cmask, const T *cmask_pl, T *Qout_prev, T *Qout_prev_pl, const T *Qout_post,
-             const T *Qout_post_pl, T *scratch_Qout, T *scratch_Qout_pl, T *scratch_Qin_pl) {
+             const T *Qout_post_pl, T *scratch_Qin_pl) {
   if (!q_a || !q_a_pl || !q || !q_pl || !d || !d_pl || !ch || !ch_pl || !cmask || !cmask_pl || !Qout_prev ||
       !Qout_prev_pl || ((Qout_post == nullptr) != (Qout_post_pl == nullptr)))
     return set_error("horizontal_limiter_thuburn: bad argument"), ICA_ERR_ARG;
@@ -323,42 +336,29 @@ int hlim_dev(Ctx *c, T *q_a, T *q_a_pl, const T *q, const T *q_pl, const T *d, c
     int rc = c->need_grid("horizontal_limiter_thuburn with Qout_post = NULL");
     if (rc) return rc;
   }
-  const size_t n2 = (size_t)c->sz.gall * c->sz.kall * c->sz.lall * 2, n2p = (size_t)kGallPl * c->sz.kall * kLallPl * 2;
   LimIn<T> in{q, q_pl, d, d_pl, ch, ch_pl, cmask, cmask_pl};
   launch_hlim_qout<T>(c->D, in, Qout_prev, Qout_prev_pl, scratch_Qin_pl, c->stream);
-  c->launches += c->D.have_pl ? 2 : 1;
-  const T *Qo = Qout_post, *Qo_pl = Qout_post_pl;
-  if (!Qout_post) {  // NICAM: COMM_data_transfer(Qout, Qout_pl) on a copy of the pre-fill Qout
-    cudaError_t e = cudaMemcpyAsync(scratch_Qout, Qout_prev, n2 * sizeof(T), cudaMemcpyDeviceToDevice, c->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "horizontal_limiter_thuburn: copy of Qout");
-    e = cudaMemcpyAsync(scratch_Qout_pl, Qout_prev_pl, n2p * sizeof(T), cudaMemcpyDeviceToDevice, c->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "horizontal_limiter_thuburn: copy of Qout_pl");
-    const Plan &p = c->plan[0];
-    launch_gather<T>(c->D, p.n, p.dst, p.src, c->sz.kall, 2, scratch_Qout, scratch_Qout_pl, c->stream);
-    c->launches += 1;
-    Qo = scratch_Qout;
-    Qo_pl = scratch_Qout_pl;
-  }
-  launch_hlim_apply<T>(c->D, in, q_a, q_a_pl, Qo, Qo_pl, scratch_Qin_pl, c->stream);
-  c->launches += c->D.have_pl ? 2 : 1;
+  // without Qout_post (NICAM's COMM_data_transfer(Qout, Qout_pl)) the apply reads halo cells from
+  // the cells the fill would copy
+  launch_hlim_apply<T>(c->D, in, q_a, q_a_pl, Qout_post ? Qout_post : Qout_prev, Qout_post ? Qout_post_pl : Qout_prev_pl,
+                       scratch_Qin_pl, Qout_post ? nullptr : c->halo_src, c->stream);
+  c->launches += 2;
   return c->check_launch("horizontal_limiter_thuburn");
 }
 
 template int hlim_dev<double>(Ctx *, double *, double *, const double *, const double *, const double *,
                               const double *, const double *, const double *, const double *, const double *,
-                              double *, double *, const double *, const double *, double *, double *, double *);
+                              double *, double *, const double *, const double *, double *);
 
 template <typename T>
 int hlim_dev_alloc(Ctx *c, T *q_a, T *q_a_pl, const T *q, const T *q_pl, const T *d, const T *d_pl, const T *ch,
                    const T *ch_pl, const T *cmask, const T *cmask_pl, T *Qout_prev, T *Qout_prev_pl,
                    const T *Qout_post, const T *Qout_post_pl) {
-  const size_t n2 = (size_t)c->sz.gall * c->sz.kall * c->sz.lall * 2, n2p = (size_t)kGallPl * c->sz.kall * kLallPl * 2;
-  T *sq = (T *)c->buf(sizeof(T) == 8 ? "lim_qout64" : "lim_qout32", n2 * sizeof(T));
-  T *sqp = (T *)c->buf(sizeof(T) == 8 ? "lim_qoutpl64" : "lim_qoutpl32", n2p * sizeof(T));
-  T *sqin = (T *)c->buf(sizeof(T) == 8 ? "lim_qinpl64" : "lim_qinpl32", n2p * 2 * sizeof(T));
-  if (!sq || !sqp || !sqin) return set_error("horizontal_limiter_thuburn: cudaMalloc(scratch)"), ICA_ERR_NOMEM;
+  const size_t n4p = (size_t)kGallPl * c->sz.kall * kLallPl * 4;
+  T *sqin = (T *)c->buf(sizeof(T) == 8 ? "lim_qinpl64" : "lim_qinpl32", n4p * sizeof(T));
+  if (!sqin) return set_error("horizontal_limiter_thuburn: cudaMalloc(scratch)"), ICA_ERR_NOMEM;
   return hlim_dev<T>(c, q_a, q_a_pl, q, q_pl, d, d_pl, ch, ch_pl, cmask, cmask_pl, Qout_prev, Qout_prev_pl,
-                     Qout_post, Qout_post_pl, sq, sqp, sqin);
+                     Qout_post, Qout_post_pl, sqin);
 }
 
 template <typename T>

@@ -62,6 +62,7 @@ struct Ctx {
   cudaStream_t copy_in = nullptr, copy_out = nullptr;  // host-link copies of the chunked host path
   int host_chunk = 0;                                   // tracers per chunk of that path, 0: by size
   Plan plan[2];               // [0] COMM_data_transfer, [1] COMM_var
+  int *halo_src = nullptr;    // COMM_data_transfer as a map: each point's source (or itself)
   int *d_have_sgp = nullptr;
   void *geo64[8] = {};        // GRD_xr, _pl, GMTR_p, _pl, GMTR_t, _pl, GMTR_a, _pl
   void *geo32[8] = {};
@@ -94,13 +95,12 @@ struct Ctx {
 
 int cuda_fail(cudaError_t e, const char *what);
 
-// horizontal_limiter_thuburn on device buffers with caller-provided scratch: the Qout copy
-// the halo fill runs on (gall*kall*lall*2 and 6*kall*2*2 values) and the pole inflow bounds
+// horizontal_limiter_thuburn on device buffers with caller-provided scratch: the pole inflow bounds
 // (6*kall*2*4 values).  Instantiated for double in capi.cu.
 template <typename T>
 int hlim_dev(Ctx *c, T *q_a, T *q_a_pl, const T *q, const T *q_pl, const T *d, const T *d_pl, const T *ch,
              const T *ch_pl, const T *cmask, const T *cmask_pl, T *Qout_prev, T *Qout_prev_pl, const T *Qout_post,
-             const T *Qout_post_pl, T *scratch_Qout, T *scratch_Qout_pl, T *scratch_Qin_pl);
+             const T *Qout_post_pl, T *scratch_Qin_pl);
 
 // Device address of the noalloc limiter's fixed scratch array in the current device's
 // context.  Looking it up loads the module that holds the array, so its device memory is

@@ -1,13 +1,12 @@
 // horizontal_limiter_thuburn for callers that cannot allocate device memory.
 //
-// The ordinary entry points take their scratch (the copy of Qout that the
-// halo fill runs on, and the pole-ring inflow bounds) from buffers the
-// context allocates with cudaMalloc on first use.  Some callers cannot let a
-// library do that: a host model that hands the whole GPU to its own pool
+// The ordinary entry points take their scratch (the pole-ring inflow bounds) from a
+// buffer the context allocates with cudaMalloc on first use.  Some callers cannot
+// let a library do that: a host model that hands the whole GPU to its own pool
 // allocator at start-up and allocates every array exactly once (the usual
 // shape of a Fortran climate model), or a run whose device-memory footprint
 // must not change once it has started.  For them this file keeps the scratch
-// in a fixed-size array in the library's own device memory (about 32.1 MiB):
+// in a fixed-size array in the library's own device memory (96 KiB):
 // ica_init looks up its address, which loads it on the context's device, so
 // the context must be created before the host's pool claims the GPU.  From then
 // on every GPU with a context holds the array until the process exits, and
@@ -22,11 +21,9 @@
 
 namespace icoadv {
 
-constexpr size_t kRegionScratch = (size_t)2 * ICA_NOALLOC_MAX_CELLS;        // Qout copy, 2 values per cell
-constexpr size_t kPoleQout = (size_t)kGallPl * kLallPl * 2 * ICA_NOALLOC_MAX_KALL;  // Qout_pl copy
-constexpr size_t kPoleQin = (size_t)kGallPl * kLallPl * 4 * ICA_NOALLOC_MAX_KALL;   // Qin_pl(min/max, face set)
+constexpr size_t kPoleQin = (size_t)kGallPl * kLallPl * 4 * ICA_NOALLOC_MAX_KALL;  // Qin_pl(min/max, face set)
 
-static __device__ __align__(256) double g_noalloc_scratch[kRegionScratch + kPoleQout + kPoleQin];
+static __device__ __align__(256) double g_noalloc_scratch[kPoleQin];
 
 // The host-side symbol g_noalloc_scratch is only a stand-in, never a device address:
 // the address is looked up in the current device's context.
@@ -61,7 +58,6 @@ extern "C" int ica_horizontal_limiter_thuburn_noalloc(ica_ctx *ctx, double *q_a,
     int rc = noalloc_scratch_address(&c->noalloc_scratch);
     if (rc) return rc;
   }
-  double *s = c->noalloc_scratch;
   return hlim_dev<double>(c, q_a, q_a_pl, q, q_pl, d, d_pl, ch, ch_pl, cmask, cmask_pl, Qout_prev, Qout_prev_pl,
-                          Qout_post, Qout_post_pl, s, s + kRegionScratch, s + kRegionScratch + kPoleQout);
+                          Qout_post, Qout_post_pl, c->noalloc_scratch);
 }

@@ -24,6 +24,7 @@
 #include <cstdint>
 
 #include "plain_kernels.cuh"
+#include "quotients.cuh"
 
 namespace icoadv {
 
@@ -203,92 +204,125 @@ __device__ __forceinline__ void pole_flux(const Dims &D, const FluxIn<T> &in, co
 // ---------------------------------------------------------------------------
 // horizontal_limiter_thuburn
 
-// 4-point bounds of face a (AI, AIJ, AJ) of cell c = (i,j) in one (k,l) slab,
-// including the index clamps im1j = max(im1j,1), ijm1 = max(ijm1,1) of
-// :152-153 and the singular AIJ stencil of :192-214.
+// Qout as the halo fill would leave it, read from where it would copy it: src maps every point
+// (regions, then the 12 pole slots) to its source, or to itself; null: Qout is filled already.
 template <typename T>
-__device__ __forceinline__ void face_bounds(const Dims &D, const T *q, int i, int j, int a, bool sgp,
-                                            T &qmin, T &qmax) {
-  const int G = D.gall_1d, ij = (j - 1) * G + i;
-  const int ip1j = ij + 1, ip1jp1 = ij + G + 1, ijp1 = ij + G;
-  int im1j = ij - 1, ijm1 = ij - G;
-  if (im1j < 1) im1j = 1;
-  if (ijm1 < 1) ijm1 = 1;
-  const T q0 = q[ij - 1];
-  T b, c, d;
-  if (a == AI) {
-    b = q[ijm1 - 1], c = q[ip1j - 1], d = q[ip1jp1 - 1];
-  } else if (a == AIJ) {
-    if (sgp && i == D.gmin - 1 && j == D.gmin - 1) b = q[ip1jp1 - 1], c = q[ij + G + 2 - 1], d = q[ijp1 - 1];
-    else b = q[ip1j - 1], c = q[ip1jp1 - 1], d = q[ijp1 - 1];
-  } else {
-    b = q[ip1jp1 - 1], c = q[ijp1 - 1], d = q[im1j - 1];
+struct HaloSource {
+  const int *src;
+  const T *Qout;
+  __device__ __forceinline__ void load(const Dims &D, const T *Q, const T *Q_pl, int p, int k, T &lo, T &hi) const {
+    const int npt = D.lall * D.gall;
+    const T *a = p < npt ? Q + ((size_t)(p / D.gall) * D.kall + k) * D.gall + p % D.gall
+                         : Q_pl + ((size_t)((p - npt) / kGallPl) * D.kall + k) * kGallPl + (p - npt) % kGallPl;
+    lo = a[0];
+    hi = a[p < npt ? (size_t)npt * D.kall : (size_t)kLallPl * kGallPl * D.kall];
   }
-  qmin = mn(mn(mn(q0, b), c), d);
-  qmax = mx(mx(mx(q0, b), c), d);
-}
+};
+
+// One thread per (cell, level) in both kernels, the poles in the last blocks of the same launches;
+// addresses are a slab base that is the same for the block and a 32-bit offset in the slab.  Bound by
+// memory: glevel 7, kall 96 takes 368 us for Qout (104 bytes a cell, 260 us at the copy rate) and 375
+// for the apply (120 bytes, 300 us); 486 + 383 us before, and 125 us more for the copy of Qout and
+// its halo fill, which the apply now does without.
+
+template <typename T> __device__ __forceinline__ T mn4(T a, T b, T c, T d) { return mn(mn(mn(a, b), c), d); }
+template <typename T> __device__ __forceinline__ T mx4(T a, T b, T c, T d) { return mx(mx(mx(a, b), c), d); }
 
 template <typename T>
-__global__ void k_hlim_qout(Dims D, LimIn<T> in, T *Qout) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall;
-  const int i = c % D.gall_1d + 1, j = c / D.gall_1d + 1, G = D.gall_1d;
+__device__ __forceinline__ void pole_qout(const Dims &D, const LimIn<T> &in, T *Qout_pl, T *Qin_pl, int l, int k);
+template <typename T>
+__device__ __forceinline__ void pole_apply(const Dims &D, const LimIn<T> &in, T *q_a_pl, const T *Qout_pl,
+                                           const T *Qin_pl, const HaloSource<T> &H, int v, int l, int k);
+
+constexpr int kLimThreads = 128;
+
+// Qout of a cell from the 4-point bounds of its six faces (:152-282).  Faces 4-6 are faces 1-3 of the
+// cells (i-1,j), (i-1,j-1), (i,j-1); an interior cell's stencil needs none of the index clamps of
+// :152-153.
+template <typename T>
+__global__ void __launch_bounds__(kLimThreads, 7) k_hlim_qout(Dims D, LimIn<T> in, T *Qout, T *Qout_pl, T *Qin_pl,
+                                                           int cellblk, int nmain) {
+  if ((int)blockIdx.x >= nmain) {
+    const int t = ((int)blockIdx.x - nmain) * kLimThreads + (int)threadIdx.x;
+    if (t < D.kall * kLallPl) pole_qout(D, in, Qout_pl, Qin_pl, t / D.kall, t % D.kall);
+    return;
+  }
+  const int ci = (int)blockIdx.x % cellblk * kLimThreads + (int)threadIdx.x, kl = (int)blockIdx.x / cellblk;
+  if (ci >= D.gall) return;
+  const int l = kl / D.kall, G = D.gall_1d;
+  const int i = ci % G + 1, j = ci / G + 1;
+  const unsigned c = ci;
   const size_t off = (size_t)kl * D.gall;
   const size_t fs = (size_t)D.lall * D.kall * D.gall;
   const T *q = in.q + off;
   const T q0 = q[c];
+  T *Qmin = Qout + off, *Qmax = Qout + fs + off;
   if (i < D.gmin || i > D.gmax || j < D.gmin || j > D.gmax) {  // halo: Qout = q   (:288-301)
-    Qout[0 * fs + off + c] = q0;
-    Qout[1 * fs + off + c] = q0;
+    Qmin[c] = q0;
+    Qmax[c] = q0;
     return;
   }
-  const bool sgp = D.have_sgp[l] != 0;
+  const T *cm1 = in.cmask + off, *cm2 = in.cmask + fs + off, *cm3 = in.cmask + 2 * fs + off;
+  const T cc[7] = {T(0), cm1[c], cm2[c], cm3[c], cm1[c - 1], cm2[c - G - 1], cm3[c - G]};
+  T ch[7];
+#pragma unroll
+  for (int f = 1; f <= 6; ++f) ch[f] = (in.ch + (size_t)(f - 1) * fs + off)[c];
+  const T dv = (in.d + off)[c];
+  const T n1 = q[c + 1], n2 = q[c + G + 1], n3 = q[c + G], n4 = q[c - 1], n5 = q[c - G - 1], n6 = q[c - G];
   const T BIG = Num<T>::big(), EPS = Num<T>::eps();
-  auto cm = [&](int cell0, int m) { return in.cmask[(size_t)(m - 1) * fs + off + cell0]; };
-  // Qin(ij,.,1..3) from the faces of ij; Qin(ij,.,4..6) from the faces of im1j, im1jm1, ijm1
-  T qin_min[7], qin_max[7];
-  {
-    T lo, hi, cc;
-    face_bounds(D, q, i, j, AI, sgp, lo, hi); cc = cm(c, 1);
-    qin_min[1] = cc * lo + (T(1) - cc) * BIG; qin_max[1] = cc * hi + (T(1) - cc) * (-BIG);
-    face_bounds(D, q, i, j, AIJ, sgp, lo, hi); cc = cm(c, 2);
-    qin_min[2] = cc * lo + (T(1) - cc) * BIG; qin_max[2] = cc * hi + (T(1) - cc) * (-BIG);
-    face_bounds(D, q, i, j, AJ, sgp, lo, hi); cc = cm(c, 3);
-    qin_min[3] = cc * lo + (T(1) - cc) * BIG; qin_max[3] = cc * hi + (T(1) - cc) * (-BIG);
-    face_bounds(D, q, i - 1, j, AI, sgp, lo, hi); cc = cm(c - 1, 1);
-    qin_min[4] = cc * BIG + (T(1) - cc) * lo; qin_max[4] = cc * (-BIG) + (T(1) - cc) * hi;
-    face_bounds(D, q, i - 1, j - 1, AIJ, sgp, lo, hi); cc = cm(c - G - 1, 2);
-    qin_min[5] = cc * BIG + (T(1) - cc) * lo; qin_max[5] = cc * (-BIG) + (T(1) - cc) * hi;
-    face_bounds(D, q, i, j - 1, AJ, sgp, lo, hi); cc = cm(c - G, 3);
-    qin_min[6] = cc * BIG + (T(1) - cc) * lo; qin_max[6] = cc * (-BIG) + (T(1) - cc) * hi;
-  }
-  T qnext_min = q0, qnext_max = q0;
-  for (int f = 1; f <= 6; ++f) qnext_min = mn(qnext_min, qin_min[f]);
-  for (int f = 1; f <= 6; ++f) qnext_max = mx(qnext_max, qin_max[f]);
-  T ch[7], cmk[7];
+  const bool sing = i == D.gmin && j == D.gmin && D.have_sgp[l] != 0;  // the AIJ stencil of :192-214
+  const T b5 = sing ? q0 : n6, c5 = sing ? n1 : q0;
+  const T lo[7] = {T(0), mn4(q0, n6, n1, n2), mn4(q0, n1, n2, n3), mn4(q0, n2, n3, n4),
+                   mn4(n4, n5, q0, n3),       mn4(n5, b5, c5, n4), mn4(n6, n1, q0, n5)};
+  const T hi[7] = {T(0), mx4(q0, n6, n1, n2), mx4(q0, n1, n2, n3), mx4(q0, n2, n3, n4),
+                   mx4(n4, n5, q0, n3),       mx4(n5, b5, c5, n4), mx4(n6, n1, q0, n5)};
+  // cmask is 0 or 1 where it comes from a Courant number: an inflow face's bound enters as it is, and an
+  // outflow face's, +-BIG, binds nothing and has no part in CQ unless its Courant number says inflow
+  bool simple = true, inflow[7];
+  T chm[7];
+#pragma unroll
   for (int f = 1; f <= 6; ++f) {
-    ch[f] = in.ch[(size_t)(f - 1) * fs + off + c];
-    cmk[f] = mn(ch[f], T(0));
+    inflow[f] = cc[f] == (f <= 3 ? T(1) : T(0));
+    chm[f] = mn(ch[f], T(0));
+    simple = simple && (inflow[f] || (cc[f] == (f <= 3 ? T(0) : T(1)) && chm[f] == T(0)));
   }
-  const T Cin = cmk[1] + cmk[2] + cmk[3] + cmk[4] + cmk[5] + cmk[6];
-  const T Cout = ch[1] - cmk[1] + ch[2] - cmk[2] + ch[3] - cmk[3] + ch[4] - cmk[4] + ch[5] - cmk[5] + ch[6] - cmk[6];
-  const T CQmin = cmk[1] * qin_min[1] + cmk[2] * qin_min[2] + cmk[3] * qin_min[3] + cmk[4] * qin_min[4] +
-                  cmk[5] * qin_min[5] + cmk[6] * qin_min[6];
-  const T CQmax = cmk[1] * qin_max[1] + cmk[2] * qin_max[2] + cmk[3] * qin_max[3] + cmk[4] * qin_max[4] +
-                  cmk[5] * qin_max[5] + cmk[6] * qin_max[6];
-  const T zerosw = T(0.5) - fsign(T(0.5), fabs(Cout) - EPS);
-  const T dv = in.d[off + c];
-  Qout[0 * fs + off + c] = (q0 - CQmax - qnext_max * (T(1) - Cin - Cout + dv)) / (Cout + zerosw) * (T(1) - zerosw) + q0 * zerosw;
-  Qout[1 * fs + off + c] = (q0 - CQmin - qnext_min * (T(1) - Cin - Cout + dv)) / (Cout + zerosw) * (T(1) - zerosw) + q0 * zerosw;
+  T qnext_min = q0, qnext_max = q0, Cin = chm[1], Cout = ch[1] - chm[1], CQmin, CQmax;
+#pragma unroll
+  for (int f = 2; f <= 6; ++f) Cin = Cin + chm[f], Cout = Cout + ch[f] - chm[f];
+  if (simple) {
+    CQmin = chm[1] * lo[1], CQmax = chm[1] * hi[1];
+#pragma unroll
+    for (int f = 1; f <= 6; ++f) {
+      qnext_min = (inflow[f] && lo[f] < qnext_min) ? lo[f] : qnext_min;
+      qnext_max = (inflow[f] && hi[f] > qnext_max) ? hi[f] : qnext_max;
+      if (f > 1) CQmin = CQmin + chm[f] * lo[f], CQmax = CQmax + chm[f] * hi[f];
+    }
+  } else {
+    CQmin = CQmax = T(0);
+#pragma unroll
+    for (int f = 1; f <= 6; ++f) {
+      T qmin, qmax;
+      if (f <= 3) {
+        qmin = cc[f] * lo[f] + (T(1) - cc[f]) * BIG, qmax = cc[f] * hi[f] + (T(1) - cc[f]) * (-BIG);
+      } else {
+        qmin = cc[f] * BIG + (T(1) - cc[f]) * lo[f], qmax = cc[f] * (-BIG) + (T(1) - cc[f]) * hi[f];
+      }
+      qnext_min = mn(qnext_min, qmin), qnext_max = mx(qnext_max, qmax);
+      CQmin = (f == 1) ? chm[f] * qmin : CQmin + chm[f] * qmin;
+      CQmax = (f == 1) ? chm[f] * qmax : CQmax + chm[f] * qmax;
+    }
+  }
+  const T zerosw = T(0.5) - fsign(T(0.5), fabs(Cout) - EPS), omc = T(1) - Cin - Cout + dv;
+  T o[2] = {q0 - CQmax - qnext_max * omc, q0 - CQmin - qnext_min * omc};
+  if constexpr (sizeof(T) == 8) quotients(o, recip(Cout + zerosw));
+  else o[0] = o[0] / (Cout + zerosw), o[1] = o[1] / (Cout + zerosw);
+  Qmin[c] = o[0] * (T(1) - zerosw) + q0 * zerosw;
+  Qmax[c] = o[1] * (T(1) - zerosw) + q0 * zerosw;
 }
 
+// (:307-367): Qout_pl(n) from the 5 ring faces; Qout_pl(2:6) = 0; keep Qin_pl for the apply
 template <typename T>
-__global__ void k_hlim_qout_pl(Dims D, LimIn<T> in, T *Qout_pl, T *Qin_pl) {
-  // (:307-367): Qout_pl(n) from the 5 ring faces; Qout_pl(2:6) = 0; keep Qin_pl for the apply
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= D.kall * kLallPl) return;
-  const int k = t % D.kall, l = t / D.kall;
+__device__ __forceinline__ void pole_qout(const Dims &D, const LimIn<T> &in, T *Qout_pl, T *Qin_pl, int l, int k) {
   const T BIG = Num<T>::big(), EPS = Num<T>::eps();
   const size_t off = ((size_t)l * D.kall + k) * kGallPl;
   const size_t fsp = (size_t)kLallPl * D.kall * kGallPl;
@@ -330,53 +364,81 @@ __global__ void k_hlim_qout_pl(Dims D, LimIn<T> in, T *Qout_pl, T *Qin_pl) {
   }
 }
 
+// (:378-410): cells (i,j) in [gmin-1,gmax]^2, faces 1..3, mirrored to 4..6.  With H.src the halo
+// cells' Qout is read from the cells the fill would copy it from, which saves the copy of Qout and
+// the fill (a pass over 4 of the kernel's 15 values, and a launch).
 template <typename T>
-__global__ void k_hlim_apply(Dims D, LimIn<T> in, T *q_a, const T *Qout) {
-  // (:378-410): cells (i,j) in [gmin-1,gmax]^2, faces 1..3, mirrored to 4..6
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall;
-  const int i = c % D.gall_1d + 1, j = c / D.gall_1d + 1, G = D.gall_1d;
+__global__ void __launch_bounds__(kLimThreads) k_hlim_apply(Dims D, LimIn<T> in, T *q_a, T *q_a_pl, const T *Qout,
+                                                            const T *Qout_pl, const T *Qin_pl, HaloSource<T> H,
+                                                            int cellblk, int nmain) {
+  if ((int)blockIdx.x >= nmain) {
+    const int t = ((int)blockIdx.x - nmain) * kLimThreads + (int)threadIdx.x, kl = t / 5;
+    if (kl < D.kall * kLallPl) pole_apply(D, in, q_a_pl, Qout_pl, Qin_pl, H, t % 5 + 2, kl / D.kall, kl % D.kall);
+    return;
+  }
+  const int ci = (int)blockIdx.x % cellblk * kLimThreads + (int)threadIdx.x, kl = (int)blockIdx.x / cellblk;
+  if (ci >= D.gall) return;
+  const int l = kl / D.kall, G = D.gall_1d;
+  const int i = ci % G + 1, j = ci / G + 1;
   if (i < D.gmin - 1 || i > D.gmax || j < D.gmin - 1 || j > D.gmax) return;
+  const unsigned c = ci, nb[3] = {c + 1, c + G + 1, c + G};
   const size_t off = (size_t)kl * D.gall;
   const size_t fs = (size_t)D.lall * D.kall * D.gall;
-  const bool sgp = D.have_sgp[l] != 0;
   const T BIG = Num<T>::big();
   const T *q = in.q + off;
-  const int nbs[4] = {0, c + 1, c + G + 1, c + G};
-  const int faces[4] = {0, AI, AIJ, AJ};
-  for (int m = 1; m <= 3; ++m) {
-    const int nb = nbs[m];
-    T lo, hi;
-    face_bounds(D, q, i, j, faces[m], sgp, lo, hi);
-    const T cc = in.cmask[(size_t)(m - 1) * fs + off + c];
-    const T own_min = cc * lo + (T(1) - cc) * BIG, own_max = cc * hi + (T(1) - cc) * (-BIG);
-    const T nb_min = cc * BIG + (T(1) - cc) * lo, nb_max = cc * (-BIG) + (T(1) - cc) * hi;
-    T v = q_a[(size_t)(m - 1) * fs + off + c];
-    v = cc * mn(mx(v, own_min), own_max) + (T(1) - cc) * mn(mx(v, nb_min), nb_max);
-    const T on_max = Qout[1 * fs + off + nb], on_min = Qout[0 * fs + off + nb];
-    const T os_max = Qout[1 * fs + off + c], os_min = Qout[0 * fs + off + c];
-    v = cc * mx(mn(v, on_max), on_min) + (T(1) - cc) * mx(mn(v, os_max), os_min);
-    q_a[(size_t)(m - 1) * fs + off + c] = v;
-    q_a[(size_t)(m + 2) * fs + off + nb] = v;
+  T cc[3], v[3], os_min, os_max, on_min[3], on_max[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) cc[m] = (in.cmask + m * fs + off)[c], v[m] = (q_a + m * fs + off)[c];
+  const T q0 = q[c], n1 = q[nb[0]], n2 = q[nb[1]], n3 = q[nb[2]];
+  const T n4 = q[ci > 0 ? c - 1 : 0], n6 = q[ci >= G ? c - G : 0];  // the index clamps of :152-153
+  const T *Qmin = Qout + off, *Qmax = Qout + fs + off;
+  if (H.src && (i < D.gmin || i == D.gmax || j < D.gmin || j == D.gmax)) {
+    const int k = kl % D.kall, *src = H.src + (size_t)l * D.gall;
+    H.load(D, Qout, Qout_pl, src[c], k, os_min, os_max);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) H.load(D, Qout, Qout_pl, src[nb[m]], k, on_min[m], on_max[m]);
+  } else {
+    os_min = Qmin[c], os_max = Qmax[c];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) on_min[m] = Qmin[nb[m]], on_max[m] = Qmax[nb[m]];
+  }
+  T lo[3] = {mn4(q0, n6, n1, n2), mn4(q0, n1, n2, n3), mn4(q0, n2, n3, n4)};
+  T hi[3] = {mx4(q0, n6, n1, n2), mx4(q0, n1, n2, n3), mx4(q0, n2, n3, n4)};
+  if (i == D.gmin - 1 && j == D.gmin - 1 && D.have_sgp[l] != 0) {  // the singular AIJ stencil of :192-214
+    const T ns = q[c + G + 2];
+    lo[1] = mn4(q0, n2, ns, n3), hi[1] = mx4(q0, n2, ns, n3);
+  }
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const T own_min = cc[m] * lo[m] + (T(1) - cc[m]) * BIG, own_max = cc[m] * hi[m] + (T(1) - cc[m]) * (-BIG);
+    const T nb_min = cc[m] * BIG + (T(1) - cc[m]) * lo[m], nb_max = cc[m] * (-BIG) + (T(1) - cc[m]) * hi[m];
+    T x = cc[m] * mn(mx(v[m], own_min), own_max) + (T(1) - cc[m]) * mn(mx(v[m], nb_min), nb_max);
+    x = cc[m] * mx(mn(x, on_max[m]), on_min[m]) + (T(1) - cc[m]) * mx(mn(x, os_max), os_min);
+    (q_a + m * fs + off)[c] = x;
+    (q_a + (m + 3) * fs + off)[nb[m]] = x;
   }
 }
 
+// (:412-425)
 template <typename T>
-__global__ void k_hlim_apply_pl(Dims D, LimIn<T> in, T *q_a_pl, const T *Qout_pl, const T *Qin_pl) {
-  // (:412-425)
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= D.kall * kLallPl * 5) return;
-  const int v = t % 5 + 2, kl = t / 5;
-  const size_t off = (size_t)kl * kGallPl;
+__device__ __forceinline__ void pole_apply(const Dims &D, const LimIn<T> &in, T *q_a_pl, const T *Qout_pl,
+                                           const T *Qin_pl, const HaloSource<T> &H, int v, int l, int k) {
+  const size_t off = ((size_t)l * D.kall + k) * kGallPl;
   const size_t fsp = (size_t)kLallPl * D.kall * kGallPl;
   const T c = in.cmask_pl[off + v - 1];
-  T x = q_a_pl[off + v - 1];
+  T x = q_a_pl[off + v - 1], ring_min, ring_max, mid_min, mid_max;
+  if (H.src) {
+    const int *src = H.src + D.lall * D.gall + l * kGallPl;
+    H.load(D, H.Qout, Qout_pl, src[v - 1], k, ring_min, ring_max);
+    H.load(D, H.Qout, Qout_pl, src[0], k, mid_min, mid_max);
+  } else {
+    ring_min = Qout_pl[off + v - 1], ring_max = Qout_pl[fsp + off + v - 1];
+    mid_min = Qout_pl[off], mid_max = Qout_pl[fsp + off];
+  }
   const T i1min = Qin_pl[((size_t)0 * 2 + 0) * fsp + off + v - 1], i2min = Qin_pl[((size_t)0 * 2 + 1) * fsp + off + v - 1];
   const T i1max = Qin_pl[((size_t)1 * 2 + 0) * fsp + off + v - 1], i2max = Qin_pl[((size_t)1 * 2 + 1) * fsp + off + v - 1];
   x = c * mn(mx(x, i1min), i1max) + (T(1) - c) * mn(mx(x, i2min), i2max);
-  x = c * mx(mn(x, Qout_pl[1 * fsp + off + v - 1]), Qout_pl[0 * fsp + off + v - 1]) +
-      (T(1) - c) * mx(mn(x, Qout_pl[1 * fsp + off + 0]), Qout_pl[0 * fsp + off + 0]);
+  x = c * mx(mn(x, ring_max), ring_min) + (T(1) - c) * mx(mn(x, mid_max), mid_min);
   q_a_pl[off + v - 1] = x;
 }
 
@@ -501,10 +563,6 @@ __global__ void k_gather(int nent, const int *__restrict__ dst, const int *__res
 
 // ---------------------------------------------------------------------------
 // launchers
-static inline dim3 slab_grid(const Dims &D, int threads) {
-  return dim3((D.gall + threads - 1) / threads, D.kall * D.lall);
-}
-
 template <typename T>
 void launch_horizontal_flux(const Dims &D, const FluxIn<T> &in, const FluxOut<T> &out, const Geo<T> &g, T dt,
                             cudaStream_t s) {
@@ -516,15 +574,18 @@ void launch_horizontal_flux(const Dims &D, const FluxIn<T> &in, const FluxOut<T>
 
 template <typename T>
 void launch_hlim_qout(const Dims &D, const LimIn<T> &in, T *Qout, T *Qout_pl, T *Qin_pl, cudaStream_t s) {
-  k_hlim_qout<T><<<slab_grid(D, 128), 128, 0, s>>>(D, in, Qout);
-  if (D.have_pl) k_hlim_qout_pl<T><<<(D.kall * kLallPl + 63) / 64, 64, 0, s>>>(D, in, Qout_pl, Qin_pl);
+  const int cellblk = (D.gall + kLimThreads - 1) / kLimThreads, nmain = cellblk * D.kall * D.lall;
+  const int npole = D.have_pl ? (D.kall * kLallPl + kLimThreads - 1) / kLimThreads : 0;
+  k_hlim_qout<T><<<(unsigned)(nmain + npole), kLimThreads, 0, s>>>(D, in, Qout, Qout_pl, Qin_pl, cellblk, nmain);
 }
 
 template <typename T>
 void launch_hlim_apply(const Dims &D, const LimIn<T> &in, T *q_a, T *q_a_pl, const T *Qout, const T *Qout_pl,
-                       const T *Qin_pl, cudaStream_t s) {
-  k_hlim_apply<T><<<slab_grid(D, 128), 128, 0, s>>>(D, in, q_a, Qout);
-  if (D.have_pl) k_hlim_apply_pl<T><<<(D.kall * kLallPl * 5 + 63) / 64, 64, 0, s>>>(D, in, q_a_pl, Qout_pl, Qin_pl);
+                       const T *Qin_pl, const int *halo_src, cudaStream_t s) {
+  const int cellblk = (D.gall + kLimThreads - 1) / kLimThreads, nmain = cellblk * D.kall * D.lall;
+  const int npole = D.have_pl ? (D.kall * kLallPl * 5 + kLimThreads - 1) / kLimThreads : 0;
+  k_hlim_apply<T><<<(unsigned)(nmain + npole), kLimThreads, 0, s>>>(D, in, q_a, q_a_pl, Qout, Qout_pl, Qin_pl,
+                                                                    HaloSource<T>{halo_src, Qout}, cellblk, nmain);
 }
 
 template <typename T>
@@ -554,7 +615,7 @@ void launch_gather(const Dims &D, int nent, const int *dst, const int *src, int 
                                           T, cudaStream_t);                                                   \
   template void launch_hlim_qout<T>(const Dims &, const LimIn<T> &, T *, T *, T *, cudaStream_t);             \
   template void launch_hlim_apply<T>(const Dims &, const LimIn<T> &, T *, T *, const T *, const T *,          \
-                                     const T *, cudaStream_t);                                                \
+                                     const T *, const int *, cudaStream_t);                                                \
   template void launch_vlim<T>(const Dims &, T *, T *, const T *, const T *, const T *, const T *, const T *, \
                                const T *, cudaStream_t);                                                      \
   template void launch_gather<T>(const Dims &, int, const int *, const int *, int, int, T *, T *, cudaStream_t);

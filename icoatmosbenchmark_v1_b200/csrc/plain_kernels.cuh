@@ -42,9 +42,10 @@ void launch_horizontal_flux(const Dims &D, const FluxIn<T> &in, const FluxOut<T>
 // Qout (pre-fill) for regions and poles; Qin_pl(6,kall,2,2,2) is kept for the apply
 template <typename T>
 void launch_hlim_qout(const Dims &D, const LimIn<T> &in, T *Qout, T *Qout_pl, T *Qin_pl, cudaStream_t s);
+// halo_src: null if Qout is halo filled, else each point's source in the fill (HaloSource)
 template <typename T>
 void launch_hlim_apply(const Dims &D, const LimIn<T> &in, T *q_a, T *q_a_pl, const T *Qout, const T *Qout_pl,
-                       const T *Qin_pl, cudaStream_t s);
+                       const T *Qin_pl, const int *halo_src, cudaStream_t s);
 template <typename T>
 void launch_vlim(const Dims &D, T *q_h, T *q_h_pl, const T *q, const T *q_pl, const T *d, const T *d_pl,
                  const T *ck, const T *ck_pl, cudaStream_t s);

@@ -22,6 +22,7 @@
 #include <cfloat>
 #include <type_traits>
 
+#include "quotients.cuh"
 #include "step.cuh"
 
 namespace icoadv {
@@ -203,39 +204,6 @@ __device__ __forceinline__ double mx4(double a, double b, double c, double d) { 
 __device__ __forceinline__ bool upmask(double f, double r) {
   if (r >= 0x1p-900) return f < DBL_EPSILON * r;
   return 0.5 - sgn(0.5, f / r - DBL_EPSILON) != 0.0;
-}
-
-// Several quotients with one divisor, each correctly rounded: y = 1/b is correctly rounded (an
-// IEEE division), q1 = q0 + (a - b q0) y is faithful, and one more such step with its exact
-// residual is a/b correctly rounded (Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", 1990).  The residuals are exact while nothing under- or overflows:
-// quotients outside [2^-800, 2^1000) other than those of a zero, and divisors outside
-// [2^-100, 2^101), take the division itself.
-struct Recip {
-  double b, y;
-  bool ok;
-};
-__device__ __forceinline__ bool recip_ok(double b) {
-  return ((unsigned)__double2hiint(b) & 0x7fffffffu) - 0x39b00000u < 0x0c900000u;
-}
-__device__ __forceinline__ Recip recip(double b) { return Recip{b, 1.0 / b, recip_ok(b)}; }
-template <int N>
-__device__ __forceinline__ void quotients(double (&a)[N], const Recip &d) {
-  double q[N];
-  bool ok = d.ok;
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const double q0 = a[i] * d.y, q1 = __fma_rn(__fma_rn(-d.b, q0, a[i]), d.y, q0);
-    q[i] = __fma_rn(__fma_rn(-d.b, q1, a[i]), d.y, q1);
-    ok = ok && (((unsigned)__double2hiint(q[i]) & 0x7fffffffu) - 0x0df00000u < 0x70800000u || a[i] == 0.0);
-  }
-  if (ok) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) a[i] = q[i];
-  } else {
-#pragma unroll
-    for (int i = 0; i < N; ++i) a[i] = a[i] / d.b;
-  }
 }
 
 // pole centre (p, k) of tracer t: gradient and Qout (mod_src_tracer.f90:307-367) into bb

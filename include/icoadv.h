@@ -183,9 +183,8 @@ int ica_horizontal_limiter_thuburn_f32(ica_ctx *ctx,
 /* ica_horizontal_limiter_thuburn_dev without any device allocation.  No reference
  * counterpart: it serves callers that cannot let a library allocate device memory
  * after start-up (a host model whose pool allocator owns the GPU, a run whose
- * footprint must stay fixed).  The scratch (the Qout copy the halo fill runs on and
- * the pole inflow bounds) is a fixed array in the library's device memory, about
- * 32.1 MiB.  ica_init looks up its address on the context's device, which loads it
+ * footprint must stay fixed).  The scratch (the pole inflow bounds) is a fixed array
+ * in the library's device memory, 96 KiB.  ica_init looks up its address on the context's device, which loads it
  * there, so create the context before a pool allocator claims the GPU; every GPU
  * with a context then holds the array until the process exits.  (Should that lookup
  * fail, the first call repeats it: make that call before any stream capture.)  Grids with
