@@ -109,6 +109,24 @@ int ica_init(const ica_dims *dims, ica_ctx **out) {
     std::vector<int> d, sr;
     rc = t.build_plan(pf != 0, d, sr);
     if (rc) { delete c; return set_error("halo plan: a source is also a destination"), rc; }
+    // The fill as a map from every point to its source (itself where no list writes it), and its
+    // entries in the order of the points they write: the halo columns on both sides of a row end are
+    // neighbours in memory, so a warp's stores (and mostly its loads) share sectors.  The fill reads
+    // no point it writes, so its order is free.
+    std::vector<int> m((size_t)t.npoints());
+    for (size_t q = 0; q < m.size(); ++q) m[q] = (int)q;
+    for (size_t q = 0; q < d.size(); ++q) m[d[q]] = sr[q];
+    size_t ne = 0;
+    for (size_t q = 0; q < m.size(); ++q)
+      if (m[q] != (int)q) d[ne] = (int)q, sr[ne] = m[q], ++ne;
+    d.resize(ne), sr.resize(ne);
+    if (pf == 0) {
+      if (cudaMalloc(&c->halo_src, sizeof(int) * m.size()) != cudaSuccess) {
+        delete c;
+        return set_error("cudaMalloc(halo sources)"), ICA_ERR_NOMEM;
+      }
+      cudaMemcpy(c->halo_src, m.data(), sizeof(int) * m.size(), cudaMemcpyHostToDevice);
+    }
     Plan &p = c->plan[pf];
     p.n = (int)d.size();
     if (cudaMalloc(&p.dst, sizeof(int) * (p.n + 1)) != cudaSuccess ||
@@ -118,18 +136,6 @@ int ica_init(const ica_dims *dims, ica_ctx **out) {
     }
     cudaMemcpy(p.dst, d.data(), sizeof(int) * p.n, cudaMemcpyHostToDevice);
     cudaMemcpy(p.src, sr.data(), sizeof(int) * p.n, cudaMemcpyHostToDevice);
-  }
-  {  // the fill as a map from every point to its source (itself where no list writes it)
-    std::vector<int> d, sr, m((size_t)t.npoints());
-    rc = t.build_plan(false, d, sr);
-    if (rc) { delete c; return set_error("halo plan: a source is also a destination"), rc; }
-    for (size_t p = 0; p < m.size(); ++p) m[p] = (int)p;
-    for (size_t p = 0; p < d.size(); ++p) m[d[p]] = sr[p];
-    if (cudaMalloc(&c->halo_src, sizeof(int) * m.size()) != cudaSuccess) {
-      delete c;
-      return set_error("cudaMalloc(halo sources)"), ICA_ERR_NOMEM;
-    }
-    cudaMemcpy(c->halo_src, m.data(), sizeof(int) * m.size(), cudaMemcpyHostToDevice);
   }
   if (cudaMalloc(&c->d_have_sgp, sizeof(int) * t.nrgn) != cudaSuccess) {
     delete c;
@@ -1209,9 +1215,9 @@ static int advect_fast_impl(Ctx *c, int ntr, double dt, const double *rhog_in, c
   if (e != cudaSuccess) return cuda_fail(e, "ica_advect_fast");
   if (parts & 2u) {  // the halo fill of the new state (a sharded rank: its own copies only)
     const Plan &p = c->fast.sharded ? c->fast.local : c->plan[0];
-    launch_gather<double>(c->D, p.n, p.dst, p.src, c->sz.kall, 1, rhog_out, rhog_out_pl, c->stream);
-    launch_gather<double>(c->D, p.n, p.dst, p.src, c->sz.kall, ntr, rhogq_out, rhogq_out_pl, c->stream);
-    c->launches += 2;
+    launch_gather<double>(c->D, p.n, p.dst, p.src, c->sz.kall, ntr, rhogq_out, rhogq_out_pl, c->stream, rhog_out,
+                          rhog_out_pl);
+    c->launches += 1;
   }
   return c->check_launch("ica_advect_fast");
 }
@@ -1466,10 +1472,9 @@ static int batch_enqueue(ica_batch *b, const MultiInst &M, const Args *args) {
   for (int i = 0; i < M.n; ++i) {
     Ctx *c = b->ctx[i];
     const Plan &p = c->plan[0];
-    launch_gather<double>(c->D, p.n, p.dst, p.src, c->sz.kall, 1, args[i].rhog_out, args[i].rhog_out_pl, c0->stream);
     launch_gather<double>(c->D, p.n, p.dst, p.src, c->sz.kall, args[i].ntr, args[i].rhogq_out, args[i].rhogq_out_pl,
-                          c0->stream);
-    launches += 2;
+                          c0->stream, args[i].rhog_out, args[i].rhog_out_pl);
+    launches += 1;
   }
   c0->launches += launches;
   return c0->check_launch("ica_batch step");

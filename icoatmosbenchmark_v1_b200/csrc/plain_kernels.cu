@@ -540,25 +540,41 @@ __global__ void __launch_bounds__(kVlimThreads) k_vlim(Dims D, int nchunk, int c
 }
 
 // ---------------------------------------------------------------------------
-// halo/pole fill as one gather: var(dst) = var(src) for every (entry, k, v)
+// halo/pole fill as one gather: var(dst) = var(src) for every (entry, k, v), of one array or of two
+// (a step's rhogq and rhog).  A thread takes one entry through kGatherPlanes (k, v) planes: the
+// points' addresses are worked out once and that many loads are in flight.
+constexpr int kGatherThreads = 128, kGatherPlanes = 4;
+
 template <typename T>
-__global__ void k_gather(int nent, const int *__restrict__ dst, const int *__restrict__ src, int npt_rgn, int gall,
-                         int lall, int kmax, int vmax, T *var, T *var_pl) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)nent * kmax * vmax;
-  if (t >= total) return;
-  const int e = (int)(t % nent);
-  const int kv = (int)(t / nent);
-  const int k = kv % kmax, v = kv / kmax;
-  auto addr = [&](int p) -> T * {
-    if (p < npt_rgn) {
-      const int l = p / gall, ij0 = p % gall;
-      return var + (((size_t)v * lall + l) * kmax + k) * gall + ij0;
-    }
-    const int qd = p - npt_rgn, lp = qd / kGallPl, vv = qd % kGallPl;
-    return var_pl + (((size_t)v * kLallPl + lp) * kmax + k) * kGallPl + vv;
+__global__ void __launch_bounds__(kGatherThreads) k_gather(int nent, const int *__restrict__ dst,
+                                                           const int *__restrict__ src, int entblk, int gall, int lall,
+                                                           int kmax, int vmax, int planes, T *var, T *var_pl, T *var2,
+                                                           T *var2_pl) {
+  const int e = (int)blockIdx.x % entblk * kGatherThreads + (int)threadIdx.x;
+  const int p0 = (int)blockIdx.x / entblk * kGatherPlanes, n = min(kGatherPlanes, planes - p0);
+  if (e >= nent) return;
+  const int npt = lall * gall, pd = dst[e], ps = src[e];
+  const bool dpl = pd >= npt, spl = ps >= npt;
+  // the points' offsets at level 0 of a variable, and their steps from level to level
+  auto offset = [&](int p) {
+    return p < npt ? (size_t)(p / gall) * kmax * gall + p % gall
+                   : (size_t)((p - npt) / kGallPl) * kmax * kGallPl + (p - npt) % kGallPl;
   };
-  *addr(dst[e]) = *addr(src[e]);
+  const size_t od = offset(pd), os = offset(ps), kd = dpl ? kGallPl : gall, ks = spl ? kGallPl : gall;
+  const size_t vr = (size_t)npt * kmax, vp = (size_t)kLallPl * kGallPl * kmax;  // a variable of var and of var_pl
+  int k = p0 % kmax, v = p0 / kmax;  // variable vmax is var2
+  T x[kGatherPlanes], *to[kGatherPlanes];
+#pragma unroll
+  for (int u = 0; u < kGatherPlanes; ++u)
+    if (u < n) {
+      T *r = v < vmax ? var + v * vr : var2, *p = v < vmax ? var_pl + v * vp : var2_pl;
+      to[u] = (dpl ? p : r) + od + k * kd;
+      x[u] = ((spl ? p : r) + os)[k * ks];
+      if (++k == kmax) k = 0, ++v;
+    }
+#pragma unroll
+  for (int u = 0; u < kGatherPlanes; ++u)
+    if (u < n) *to[u] = x[u];
 }
 
 // ---------------------------------------------------------------------------
@@ -601,13 +617,12 @@ void launch_vlim(const Dims &D, T *q_h, T *q_h_pl, const T *q, const T *q_pl, co
 
 template <typename T>
 void launch_gather(const Dims &D, int nent, const int *dst, const int *src, int kmax, int vmax, T *var, T *var_pl,
-                   cudaStream_t s) {
-  const long long total = (long long)nent * kmax * vmax;
-  if (total == 0) return;
-  const int threads = 256;
-  const long long blocks = (total + threads - 1) / threads;
-  k_gather<T><<<(unsigned)blocks, threads, 0, s>>>(nent, dst, src, D.gall * D.lall, D.gall, D.lall, kmax, vmax, var,
-                                                   var_pl);
+                   cudaStream_t s, T *var2, T *var2_pl) {
+  const int planes = kmax * (vmax + (var2 ? 1 : 0));
+  if (nent == 0 || planes == 0) return;
+  const int entblk = (nent + kGatherThreads - 1) / kGatherThreads, chunks = (planes + kGatherPlanes - 1) / kGatherPlanes;
+  k_gather<T><<<(unsigned)(entblk * chunks), kGatherThreads, 0, s>>>(nent, dst, src, entblk, D.gall, D.lall, kmax, vmax,
+                                                                     planes, var, var_pl, var2, var2_pl);
 }
 
 #define INSTANTIATE(T)                                                                                        \
@@ -618,7 +633,8 @@ void launch_gather(const Dims &D, int nent, const int *dst, const int *src, int 
                                      const T *, const int *, cudaStream_t);                                                \
   template void launch_vlim<T>(const Dims &, T *, T *, const T *, const T *, const T *, const T *, const T *, \
                                const T *, cudaStream_t);                                                      \
-  template void launch_gather<T>(const Dims &, int, const int *, const int *, int, int, T *, T *, cudaStream_t);
+  template void launch_gather<T>(const Dims &, int, const int *, const int *, int, int, T *, T *, cudaStream_t, \
+                                 T *, T *);
 INSTANTIATE(double)
 INSTANTIATE(float)
 

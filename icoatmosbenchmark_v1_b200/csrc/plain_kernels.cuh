@@ -49,8 +49,9 @@ void launch_hlim_apply(const Dims &D, const LimIn<T> &in, T *q_a, T *q_a_pl, con
 template <typename T>
 void launch_vlim(const Dims &D, T *q_h, T *q_h_pl, const T *q, const T *q_pl, const T *d, const T *d_pl,
                  const T *ck, const T *ck_pl, cudaStream_t s);
+// halo fill of var (kmax levels, vmax variables) and, if given, of var2 (kmax levels, one variable)
 template <typename T>
 void launch_gather(const Dims &D, int nent, const int *dst, const int *src, int kmax, int vmax, T *var, T *var_pl,
-                   cudaStream_t s);
+                   cudaStream_t s, T *var2 = nullptr, T *var2_pl = nullptr);
 
 }  // namespace icoadv

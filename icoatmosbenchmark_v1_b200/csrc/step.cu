@@ -900,9 +900,8 @@ int step_plain(StepCtx &S, int ntr, double dt, double *rhog, double *rhog_pl, do
   }
   const long long nr = ((long long)D.lall * n * n + kLallPl) * NK;
   k_plain_rho<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(D, dt, S.flx, S.flx_pl, w, w_pl, S.rdgz, rhog, rhog_pl);
-  launch_gather<double>(D, S.plan.n, S.plan.dst, S.plan.src, D.kall, 1, rhog, rhog_pl, st);
-  launch_gather<double>(D, S.plan.n, S.plan.dst, S.plan.src, D.kall, ntr, rhogq, rhogq_pl, st);
-  launches += 3;
+  launch_gather<double>(D, S.plan.n, S.plan.dst, S.plan.src, D.kall, ntr, rhogq, rhogq_pl, st, rhog, rhog_pl);
+  launches += 2;
   return ICA_OK;
 }
 
