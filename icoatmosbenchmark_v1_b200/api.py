@@ -127,6 +127,20 @@ def apply_plan_numpy(plan, var, var_pl):
 
 
 # ---- the context ------------------------------------------------------------------
+_TORCH = None  # torch.Tensor and torch's dtype of a numpy one, once a tensor has been seen
+
+
+def _torch_types():
+    global _TORCH
+    if _TORCH is None:
+        try:
+            import torch
+        except ImportError:  # pragma: no cover
+            raise TypeError("unsupported array type")
+        _TORCH = (torch.Tensor, {np.float64: torch.float64, np.float32: torch.float32}, torch.cuda)
+    return _TORCH
+
+
 def _ptr(a, want):
     """Pointer of a numpy array (host) or a torch CUDA tensor (device)."""
     if a is None:
@@ -135,16 +149,37 @@ def _ptr(a, want):
         if a.dtype != want or not a.flags.c_contiguous:
             raise TypeError(f"expected C-contiguous {want} array, got {a.dtype}")
         return a.ctypes.data_as(C.c_void_p), False
-    try:
-        import torch
-    except ImportError:  # pragma: no cover
-        raise TypeError("unsupported array type")
-    if isinstance(a, torch.Tensor):
-        tw = {np.float64: torch.float64, np.float32: torch.float32}[np.dtype(want).type]
+    tensor, dtypes, _ = _TORCH or _torch_types()
+    if isinstance(a, tensor):
+        tw = dtypes.get(want) or dtypes[np.dtype(want).type]
         if a.dtype != tw or not a.is_contiguous() or not a.is_cuda:
             raise TypeError(f"expected contiguous CUDA tensor of {tw}, got {a.dtype} on {a.device}")
         return C.c_void_p(a.data_ptr()), True
     raise TypeError(f"unsupported array type {type(a)}")
+
+
+class _Ordered:
+    """Stream order of a device call against torch's current stream: the context stream waits for
+    what torch queued before it, torch waits for the call (two library calls; torch's own
+    wait_stream makes an event object for each, about 10 us a call)."""
+
+    __slots__ = ("ctx", "cur")
+
+    def __init__(self, ctx):
+        self.ctx = ctx
+
+    def __enter__(self):
+        cuda = (_TORCH or _torch_types())[2]
+        self.cur = C.c_void_p(cuda.current_stream(self.ctx.device).cuda_stream)
+        _check("ica_stream_order", lib().ica_stream_order(self.ctx.h, self.cur, 0))
+
+    def __exit__(self, kind, value, tb):
+        if kind is None:
+            _check("ica_stream_order", lib().ica_stream_order(self.ctx.h, self.cur, 1))
+        return False
+
+
+_UNORDERED = contextlib.nullcontext()
 
 
 class IcoAdv:
@@ -158,7 +193,6 @@ class IcoAdv:
         _check("ica_get_sizes", lib().ica_get_sizes(self.h, C.byref(s)))
         self.sizes = s
         self.glevel, self.rlevel, self.vlayer, self.device = glevel, rlevel, vlayer, device
-        self._ext = None
 
     @classmethod
     def regions(cls, gall_1d, kall, kmin, kmax, lall, have_pl, have_sgp, device=0):
@@ -178,15 +212,13 @@ class IcoAdv:
         self.sizes = s
         self.glevel = self.rlevel = None
         self.vlayer, self.device = kall - 2, device
-        self._ext = None
         return self
 
     def close(self):
         if self.h:
             lib().ica_finalize(self.h)
             self.h = C.c_void_p()
-            self._ext = None
-
+    
     def __del__(self):
         try:
             self.close()
@@ -197,20 +229,8 @@ class IcoAdv:
     def stream(self):
         return lib().ica_stream(self.h)
 
-    @contextlib.contextmanager
     def _ordered(self, dev=True):
-        """Stream order of a device call against torch's current stream: the context
-        stream waits for what torch queued before it, torch waits for the call."""
-        if not dev:
-            yield
-            return
-        import torch
-        if self._ext is None:
-            self._ext = torch.cuda.ExternalStream(self.stream, device=self.device)
-        cur = torch.cuda.current_stream(self.device)
-        self._ext.wait_stream(cur)
-        yield
-        cur.wait_stream(self._ext)
+        return _Ordered(self) if dev else _UNORDERED
 
     @property
     def launch_count(self):
@@ -222,11 +242,16 @@ class IcoAdv:
         _check("ica_set_geometry", lib().ica_set_geometry(self.h, *[_ptr(a, np.float64)[0] for a in keep]))
 
     def _call(self, name, dtype, arrays, *scalars):
-        ptrs, kinds = zip(*[_ptr(a, dtype) for a in arrays])
-        dev = {k for k in kinds if k is not None}
-        if len(dev) != 1:
+        ptrs, dev = [], None
+        for a in arrays:
+            p, d = _ptr(a, dtype)
+            if d is not None and d is not dev:
+                if dev is not None:
+                    raise TypeError("mix of host and device arrays")
+                dev = d
+            ptrs.append(p)
+        if dev is None:
             raise TypeError("mix of host and device arrays")
-        dev = dev.pop()
         suffix = "_dev" if dev else ""
         if dtype == np.float32:
             if dev:
@@ -240,8 +265,8 @@ class IcoAdv:
     def _dtype(a):
         if isinstance(a, np.ndarray):
             return a.dtype.type
-        import torch
-        return {torch.float64: np.float64, torch.float32: np.float32}[a.dtype]
+        d64, d32 = _torch_types()[1].values()
+        return {d64: np.float64, d32: np.float32}[a.dtype]
 
     def horizontal_flux(self, flx_h, flx_h_pl, GRD_xc, GRD_xc_pl, rho, rho_pl, rhovx, rhovx_pl,
                         rhovy, rhovy_pl, rhovz, rhovz_pl, dt):

@@ -221,6 +221,18 @@ int ica_get_sizes(const ica_ctx *c, ica_sizes *out) {
 }
 
 void *ica_stream(ica_ctx *c) { return c ? (void *)c->stream : nullptr; }
+int ica_stream_order(ica_ctx *c, void *stream, int after) {
+  if (!c) return set_error("NULL context"), ICA_ERR_ARG;
+  cudaSetDevice(c->device);
+  const cudaStream_t from = after ? c->stream : (cudaStream_t)stream, to = after ? (cudaStream_t)stream : c->stream;
+  cudaEvent_t ev;  // of this call alone: any number of threads may order the same context
+  cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  if (e != cudaSuccess) return cuda_fail(e, "ica_stream_order");
+  e = cudaEventRecord(ev, from);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(to, ev, 0);
+  cudaEventDestroy(ev);
+  return e == cudaSuccess ? ICA_OK : cuda_fail(e, "ica_stream_order");
+}
 long long ica_launch_count(const ica_ctx *c) { return c ? c->launches : -1; }
 
 int ica_set_geometry(ica_ctx *c, const double *GRD_xr, const double *GRD_xr_pl, const double *GMTR_p,

@@ -82,6 +82,10 @@ int ica_finalize(ica_ctx *ctx);
 int ica_get_sizes(const ica_ctx *ctx, ica_sizes *out);
 /* The context's CUDA stream (a cudaStream_t), for the *_dev entry points. */
 void *ica_stream(ica_ctx *ctx);
+/* Orders the context's stream against another stream of the same device, without waiting on the
+ * host: after = 0, what the context queues next runs after what `stream` holds now; after = 1, what
+ * `stream` is given next runs after what the context has queued. */
+int ica_stream_order(ica_ctx *ctx, void *stream, int after);
 /* Text of the last error on this thread. */
 const char *ica_last_error(void);
 /* Number of kernels this library launched since the context was created. */
