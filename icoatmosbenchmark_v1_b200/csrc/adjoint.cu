@@ -18,16 +18,18 @@
 // outflow side of a masked bound) have no derivative.  rhogw, the geometry
 // and the vertical grid are constants.
 //
-// Transposes of scatter shape (a face handing its adjoint to the cell that
-// bounded it, a halo copy handing its adjoint to the source point) use FP64
-// atomicAdd; the gradient stencil and the triangle interpolation are
-// transposed as gathers.  Sums therefore associate differently from a serial
-// adjoint, at rounding level.
+// The horizontal sub-step is transposed where the forward forms it: by the thread of a
+// face's upwind cell, which holds every operand (k_adj_cells), with the seam faces in
+// a kernel of their own.  What the data decide (a bound handing its adjoint to one of
+// its cells, a halo copy to its source) and sums over tiles and tracers use FP64
+// atomicAdd; the triangle interpolation is transposed as a gather.  Sums therefore
+// associate differently from a serial adjoint, at rounding level.
 #include <cuda_runtime.h>
 
 #include <cfloat>
 
 #include "adjoint.cuh"
+#include "plain_cells.cuh"
 
 namespace icoadv {
 
@@ -35,49 +37,31 @@ namespace {
 
 constexpr double kEps = DBL_EPSILON, kBig = DBL_MAX;
 
-__device__ __forceinline__ double mn(double a, double b) { return (b < a) ? b : a; }
-__device__ __forceinline__ double mx(double a, double b) { return (b > a) ? b : a; }
-__device__ __forceinline__ double sgn(double a, double b) { return copysign(fabs(a), b); }
-
-// which operand of mn(mn(mn(a,b),c),d) / the mx chain is returned (0..3)
-__device__ __forceinline__ int argmin4(const double v[4]) {
-  int i = 0;
-  double s = v[0];
-  if (v[1] < s) s = v[1], i = 1;
-  if (v[2] < s) s = v[2], i = 2;
-  if (v[3] < s) i = 3;
-  return i;
-}
-__device__ __forceinline__ int argmax4(const double v[4]) {
-  int i = 0;
-  double s = v[0];
-  if (v[1] > s) s = v[1], i = 1;
-  if (v[2] > s) s = v[2], i = 2;
-  if (v[3] > s) i = 3;
-  return i;
-}
-
 __device__ __forceinline__ bool inner(const Dims &D, int i, int j) {
   return i >= D.gmin && i <= D.gmax && j >= D.gmin && j <= D.gmax;
 }
 
-// The 4 cells (0-based slab indices) bounding face a (1..3) of owner (i,j): the owner
-// first, with the index clamps and the singular AIJ stencil of the limiter
-// (dyn_horiz_adv_limiter/src/mod_src_tracer.f90:152-214).
-__device__ __forceinline__ void face_points(const Dims &D, int i, int j, int a, bool sgp, int p[4]) {
-  const int G = D.gall_1d, ij = (j - 1) * G + i;
-  int im1j = ij - 1, ijm1 = ij - G;
-  if (im1j < 1) im1j = 1;
-  if (ijm1 < 1) ijm1 = 1;
-  p[0] = ij - 1;
-  if (a == 1) {
-    p[1] = ijm1 - 1, p[2] = ij, p[3] = ij + G;
-  } else if (a == 2) {
-    if (sgp && i == D.gmin - 1 && j == D.gmin - 1) p[1] = ij + G, p[2] = ij + G + 1, p[3] = ij + G - 1;
-    else p[1] = ij, p[2] = ij + G, p[3] = ij + G - 1;
-  } else {
-    p[1] = ij + G, p[2] = ij + G - 1, p[3] = im1j - 1;
-  }
+// The arguments of a group of tracers.
+struct AdjArgs {
+  PlainArgs P;
+  double *aQ, *aQp;      // the group's adjoint of rhogq
+  double *Qh, *Qhp;      // rhogq after the horizontal sub-step (Qh: a_q's memory, until the column pass is done)
+  double *a_q, *a_qp;    // adjoint of q
+  double *a_bb;          // adjoint of the boundary values: gradient x/y/z, Qout min / max
+  double *rh, *rhp, *a_rh, *a_rhp, *a_flx, *a_flxp, *a_xc, *a_xcp, *a_chp, *a_rho, *a_rhop;
+  bool first, last;      // of the step's groups
+  __device__ double *abval(int t, int k, int b) const { return a_bb + (((size_t)t * P.D.kall + k) * P.nb + b) * 5; }
+};
+
+// Limiter apply and remap of a face's value v0 (bounds lo, hi; the upwind cell's Qout Qn, Qx): the
+// limited value, and what it is a copy of (mod_src_tracer.f90:378-410).
+enum Pick { kRemap, kLow, kHigh, kQmin, kQmax };
+__device__ __forceinline__ Pick limited(double v0, double lo, double hi, double Qn, double Qx) {
+  const double v1a = mx(v0, lo), v1 = mn(v1a, hi), v2a = mn(v1, Qx);
+  if (Qn > v2a) return kQmin;
+  if (Qx < v1) return kQmax;
+  if (hi < v1a) return kHigh;
+  return (lo > v0) ? kLow : kRemap;
 }
 
 // ---------------------------------------------------------------------------
@@ -250,29 +234,26 @@ __device__ __forceinline__ void vlim_level_adj(const VLim &v, double qm, double 
   ac2 += a2;
 }
 
-__global__ void __launch_bounds__(kAdjThreads) k_adj_vert(Dims D, double dt, const double *__restrict__ Qh,
-                                                  const double *__restrict__ rh, const double *__restrict__ w,
-                                                  double *__restrict__ aQ, double *__restrict__ a_rh,
-                                                  const double *__restrict__ Qh_pl, const double *__restrict__ rh_pl,
-                                                  const double *__restrict__ w_pl, double *__restrict__ aQ_pl,
-                                                  double *__restrict__ a_rh_pl, const double *__restrict__ rdgz,
-                                                  const double *__restrict__ afact,
-                                                  const double *__restrict__ bfact) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ncol = D.lall * D.gall;
+// Blocks: tracers fastest (they share rh and w in L2), column blocks of a region, regions; the last
+// blocks take the pole columns.
+__global__ void __launch_bounds__(kAdjThreads) k_adj_vert(AdjArgs A, int colblk, int nmain) {
+  const Dims &D = A.P.D;
+  const double dt = A.P.dt, *__restrict__ rdgz = A.P.rdgz, *__restrict__ afact = A.P.afact, *__restrict__ bfact = A.P.bfact;
   const double *QH, *R, *W;
   double *AQ, *ARH;
   size_t s;
-  if (t < ncol) {
-    const int l = t / D.gall, c = t % D.gall, G = D.gall_1d;
-    if (!inner(D, c % G + 1, c / G + 1)) return;  // halo column: passes through
-    const size_t base = (size_t)l * D.kall * D.gall + c;
-    QH = Qh + base, R = rh + base, W = w + base, AQ = aQ + base, ARH = a_rh + base, s = D.gall;
-  } else if (t < ncol + kLallPl) {
-    const size_t base = (size_t)(t - ncol) * D.kall * kGallPl;
-    QH = Qh_pl + base, R = rh_pl + base, W = w_pl + base, AQ = aQ_pl + base, ARH = a_rh_pl + base, s = kGallPl;
+  if ((int)blockIdx.x < nmain) {
+    const int t = (int)blockIdx.x % A.P.nt, cb = (int)blockIdx.x / A.P.nt, l = cb / colblk;
+    const int n = D.gmax - D.gmin + 1, col = cb % colblk * kAdjThreads + (int)threadIdx.x;
+    if (col >= n * n) return;
+    const size_t base = (size_t)l * D.kall * D.gall + (col / n + D.gmin - 1) * D.gall_1d + col % n + D.gmin - 1;
+    const size_t tb = t * A.P.n3() + base;
+    QH = A.Qh + tb, R = A.rh + base, W = A.P.w + base, AQ = A.aQ + tb, ARH = A.a_rh + base, s = D.gall;
   } else {
-    return;
+    const int u = ((int)blockIdx.x - nmain) * kAdjThreads + (int)threadIdx.x;
+    if (u >= kLallPl * A.P.nt) return;
+    const size_t base = (size_t)(u % kLallPl) * D.kall * kGallPl, tb = u / kLallPl * A.P.n3p() + base;
+    QH = A.Qhp + tb, R = A.rhp + base, W = A.P.wp + base, AQ = A.aQp + tb, ARH = A.a_rhp + base, s = kGallPl;
   }
   const int K = D.kall, kmin = D.kmin, kmax = D.kmax;  // 1-based levels below
   auto X = [&](int k) { return (size_t)(k - 1) * s; };
@@ -374,10 +355,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_vert(Dims D, double dt, con
       if (k + 1 == kmax) a += aqcTop;
       const double rR = 1.0 / P.R;
       AQ[X(k + 1)] = P.aO + a * rR;
-      double r = ARH[X(k + 1)];
-      r += -a * P.qc * rR;
-      r += -(ac1P * P.c1 + ac2P * P.c2) * rR;
-      ARH[X(k + 1)] = r;
+      atomicAdd(&ARH[X(k + 1)], -a * P.qc * rR - (ac1P * P.c1 + ac2P * P.c2) * rR);  // the tracers share rh
     }
     // shift the window down one level
     P = Z, Z = M, M = M2;
@@ -396,10 +374,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_vert(Dims D, double dt, con
     a += aqcBot;
     const double rR = 1.0 / P.R;
     AQ[X(kmin)] = P.aO + a * rR;
-    double r = ARH[X(kmin)];
-    r += -a * P.qc * rR;
-    r += -(ac1P * P.c1 + ac2P * P.c2) * rR;
-    ARH[X(kmin)] = r;
+    atomicAdd(&ARH[X(kmin)], -a * P.qc * rR - (ac1P * P.c1 + ac2P * P.c2) * rR);
   }
   AQ[X(1)] = 0.0;
   AQ[X(K)] = 0.0;
@@ -407,408 +382,502 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_vert(Dims D, double dt, con
 }
 
 // ---------------------------------------------------------------------------
-// Forward recompute of rhogq after the horizontal sub-step, Qh = Q - sum_m flx(m) qa(m),
-// with each face's limited value formed from the pre-limit remap value in the
-// same operation sequence as the limiter apply (mod_src_tracer.f90:378-410), so
-// Qh equals the forward step's value bit for bit without storing the limited faces.
-__device__ __forceinline__ double limited_face(const Dims &D, const double *qs, const double *qa0,
-                                               const double *qo, const double *cm, size_t off, size_t fs, int oi,
-                                               int oj, int a, bool sgp) {
-  const int G = D.gall_1d, o = (oj - 1) * G + oi - 1;
-  const int nb = (a == 1) ? o + 1 : ((a == 2) ? o + G + 1 : o + G);
-  int p[4];
-  face_points(D, oi, oj, a, sgp, p);
-  const double lo = mn(mn(mn(qs[p[0]], qs[p[1]]), qs[p[2]]), qs[p[3]]);
-  const double hi = mx(mx(mx(qs[p[0]], qs[p[1]]), qs[p[2]]), qs[p[3]]);
-  const double cc = cm[(size_t)(a - 1) * fs + off + o];
-  const double own_min = cc * lo + (1.0 - cc) * kBig, own_max = cc * hi + (1.0 - cc) * (-kBig);
-  const double nb_min = cc * kBig + (1.0 - cc) * lo, nb_max = cc * (-kBig) + (1.0 - cc) * hi;
-  double v = qa0[(size_t)(a - 1) * fs + off + o];
-  v = cc * mn(mx(v, own_min), own_max) + (1.0 - cc) * mn(mx(v, nb_min), nb_max);
-  const double on_max = qo[fs + off + nb], on_min = qo[off + nb];
-  const double os_max = qo[fs + off + o], os_min = qo[off + o];
-  return cc * mx(mn(v, on_max), on_min) + (1.0 - cc) * mx(mn(v, os_max), os_min);
+// The horizontal sub-step.  The forward's own kernels (plain_faces) recompute every limited face value
+// fv and the boundary values bb; the gradient, bounds and Qout of a cell are formed again where they
+// are transposed, from q in shared memory as the forward forms them, and never stored.
+
+// One of the five faces of pole p at level k (v = 1..5: ring slot), tracer t: forward values.
+struct PoleFace {
+  double q[kGallPl], lo, hi, v0;
+  int up;            // the upwind point's slot, 0: the centre
+  const double *bv;  // its gradient and Qout
+};
+__device__ __forceinline__ PoleFace pole_face(const PlainArgs &P, int t, int p, int k, int v) {
+  const size_t off = ((size_t)p * P.D.kall + k) * kGallPl, n3p = P.n3p();
+  PoleFace f;
+#pragma unroll
+  for (int x = 0; x < kGallPl; ++x) f.q[x] = P.Qp[t * n3p + off + x] / P.rhop[off + x];
+  const int vp = (v == 5) ? 1 : v + 1, vm = (v == 1) ? 5 : v - 1;
+  auto q = [&](int x) { return P.Qp[t * n3p + off + x] / P.rhop[off + x]; };
+  const double qv = q(v), qm = q(vm), qp = q(vp);
+  f.up = upmask(P.flxp[off + v], P.rhop[off]) ? v : 0;
+  f.bv = P.bval(t, k, f.up ? P.ring[p * kVlink + v - 1] : P.nb - 2 + p);
+  f.lo = mn4(f.q[0], qv, qm, qp), f.hi = mx4(f.q[0], qv, qm, qp);
+  f.v0 = f.up ? qv : f.q[0];
+  for (int d = 0; d < 3; ++d)
+    f.v0 = f.v0 + f.bv[d] * (P.xcp[d * n3p + off + v] - P.GRD_xp[((size_t)d * kLallPl + p) * kGallPl + f.up]);
+  return f;
 }
 
-__global__ void k_adj_qh(Dims D, const double *__restrict__ q, const double *__restrict__ qa0,
-                         const double *__restrict__ qo, const double *__restrict__ cm,
-                         const double *__restrict__ flx, const double *__restrict__ Q, double *Qh) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
-  const int i = c % G + 1, j = c / G + 1;
-  if (!inner(D, i, j)) return;
-  const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall;
-  const bool sgp = D.have_sgp[l] != 0;
-  const double *qs = q + off;
-  // faces 1..3 are owned by (i,j); 4..6 by (i-1,j), (i-1,j-1), (i,j-1) as their faces 1..3
-  const int oi[6] = {i, i, i, i - 1, i - 1, i}, oj[6] = {j, j, j, j, j - 1, j - 1};
-  double s = flx[off + c] * limited_face(D, qs, qa0, qo, cm, off, fs, oi[0], oj[0], 1, sgp);
-  for (int m = 1; m < 6; ++m)
-    s = s + flx[(size_t)m * fs + off + c] * limited_face(D, qs, qa0, qo, cm, off, fs, oi[m], oj[m], m % 3 + 1, sgp);
-  Qh[off + c] = Q[off + c] - s;
-}
-
-// pole centres (mod_src_tracer.f90:412-425 with the Qin bounds kept by the Qout pass)
-__global__ void k_adj_qh_pl(int kall, const double *qa0_pl, const double *cm_pl, const double *qo_pl,
-                            const double *qin_pl, const double *flx_pl, const double *Qp, double *Qh_pl) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kLallPl * kall) return;
-  const size_t off = (size_t)t * kGallPl, fsp = (size_t)kLallPl * kall * kGallPl;
-  double s = 0.0;
-  for (int v = 2; v <= 6; ++v) {
-    const double c = cm_pl[off + v - 1];
-    double x = qa0_pl[off + v - 1];
-    const double i1min = qin_pl[0 * fsp + off + v - 1], i2min = qin_pl[1 * fsp + off + v - 1];
-    const double i1max = qin_pl[2 * fsp + off + v - 1], i2max = qin_pl[3 * fsp + off + v - 1];
-    x = c * mn(mx(x, i1min), i1max) + (1.0 - c) * mn(mx(x, i2min), i2max);
-    x = c * mx(mn(x, qo_pl[fsp + off + v - 1]), qo_pl[off + v - 1]) +
-        (1.0 - c) * mx(mn(x, qo_pl[fsp + off]), qo_pl[off]);
-    s = (v == 2) ? flx_pl[off + v - 1] * x : s + flx_pl[off + v - 1] * x;
-  }
-  Qh_pl[off] = Qp[off] - s;
-}
-
-// ---------------------------------------------------------------------------
-// One face (owner (i,j), a = 1..3): the horizontal update, the limiter apply
-// (mod_src_tracer.f90:378-410) and the upwind remap, transposed together.
-__global__ void k_adj_face(Dims D, const double *__restrict__ q, const double *__restrict__ qa0,
-                           const double *__restrict__ qo, const double *__restrict__ cm,
-                           const double *__restrict__ flx, const double *__restrict__ aQ,
-                           const double *__restrict__ xc, const double *__restrict__ GRD_x,
-                           const double *__restrict__ gr, double *a_flx, double *a_xc, double *a_qo, double *a_q,
-                           double *a_gr) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
-  const int i = c % G + 1, j = c / G + 1;
-  if (i < D.gmin - 1 || i > D.gmax || j < D.gmin - 1 || j > D.gmax) return;
-  const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall, gw = (size_t)D.lall * D.gall;
-  const bool sgp = D.have_sgp[l] != 0;
-  const double *qs = q + off;
-  const bool inC = inner(D, i, j);
-  const double aC = inC ? aQ[off + c] : 0.0;
-  const int nbs[3] = {c + 1, c + G + 1, c + G};
-  const int ni[3] = {i + 1, i + 1, i}, nj[3] = {j, j + 1, j + 1};
-  for (int m = 1; m <= 3; ++m) {
-    const int nb = nbs[m - 1];
-    const bool inN = inner(D, ni[m - 1], nj[m - 1]);
-    if (!inC && !inN) continue;
-    const double aN = inN ? aQ[off + nb] : 0.0;
-    int p[4];
-    face_points(D, i, j, m, sgp, p);
-    const double qv[4] = {qs[p[0]], qs[p[1]], qs[p[2]], qs[p[3]]};
-    const double lo = mn(mn(mn(qv[0], qv[1]), qv[2]), qv[3]);
-    const double hi = mx(mx(mx(qv[0], qv[1]), qv[2]), qv[3]);
-    const size_t fm = (size_t)(m - 1) * fs + off;
-    const double cc = cm[fm + c];
-    const double v0 = qa0[fm + c];
-    const double v1a = mx(v0, lo);
-    int s1 = (lo > v0) ? 1 : 0;
-    const double v1 = mn(v1a, hi);
-    if (hi < v1a) s1 = 2;
-    const int up = (cc != 0.0) ? nb : c;
-    const double Qx = qo[fs + off + up], Qn = qo[off + up];
-    const double v2a = mn(v1, Qx);
-    int s2 = (Qx < v1) ? 1 : 0;
-    const double v2 = mx(v2a, Qn);
-    if (Qn > v2a) s2 = 2;
-    // rhogq -= sum_m flx(m) qa(m) at the owner (face m) and at the neighbour (face m+3)
-    const size_t fn = (size_t)(m + 2) * fs + off;
-    const double t1 = inC ? -aC * flx[fm + c] : 0.0;
-    const double t2 = inN ? -aN * flx[fn + nb] : 0.0;
-    const double av = t1 + t2;
-    if (inC) a_flx[fm + c] += -aC * v2;
-    if (inN) a_flx[fn + nb] += -aN * v2;
-    if (av == 0.0) continue;
-    if (s2 == 1) {
-      atomicAdd(&a_qo[fs + off + up], av);
-    } else if (s2 == 2) {
-      atomicAdd(&a_qo[off + up], av);
-    } else if (s1 == 1) {
-      atomicAdd(&a_q[off + p[argmin4(qv)]], av);
-    } else if (s1 == 2) {
-      atomicAdd(&a_q[off + p[argmax4(qv)]], av);
-    } else {  // remap: qa = q(up) + grad(up) . (xc - x(up))
-      atomicAdd(&a_q[off + up], av);
-      for (int x = 0; x < 3; ++x) {
-        const size_t xi = ((size_t)x * 3 + (m - 1)) * fs + off + c;
-        atomicAdd(&a_gr[(size_t)x * fs + off + up], av * (xc[xi] - GRD_x[(size_t)x * gw + (size_t)l * D.gall + up]));
-        a_xc[xi] += av * gr[(size_t)x * fs + off + up];
+// rhogq after the horizontal sub-step from the face values (one thread per cell and level, the
+// group's tracers one after the other), and with the first group the density after it.  The last
+// blocks take the pole centres.
+__global__ void __launch_bounds__(128) k_adj_qh(AdjArgs A, int cellblk, int nmain) {
+  const PlainArgs &P = A.P;
+  const Dims &D = P.D;
+  const size_t n3 = P.n3(), n3p = P.n3p();
+  const int K = D.kall;
+  if ((int)blockIdx.x >= nmain) {
+    const int u = ((int)blockIdx.x - nmain) * 128 + (int)threadIdx.x;
+    if (u >= P.nt * kLallPl * K) return;
+    const int k = u % K, p = u / K % kLallPl, t = u / K / kLallPl;
+    const size_t off = ((size_t)p * K + k) * kGallPl;
+    double s = 0.0, r = 0.0;
+    for (int v = 1; v <= 5; ++v) {
+      const double f = P.flxp[off + v];
+      r = (v == 1) ? f : r + f;
+      if (k >= D.kmin - 1 && k < D.kmax) {
+        const PoleFace F = pole_face(P, t, p, k, v);
+        const double x = mx(mn(mn(mx(F.v0, F.lo), F.hi), F.bv[4]), F.bv[3]);
+        s = (v == 1) ? f * x : s + f * x;
       }
     }
+    A.Qhp[t * n3p + off] = P.Qp[t * n3p + off] - s;
+    if (t == 0) A.rhp[off] = P.rhop[off] - r;
+    return;
+  }
+  const int ci = (int)blockIdx.x % cellblk * 128 + (int)threadIdx.x, kl = (int)blockIdx.x / cellblk, k = kl % K;
+  const int G = D.gall_1d;
+  if (ci >= D.gall || !inner(D, ci % G + 1, ci / G + 1)) return;
+  const unsigned c = ci;
+  const size_t off = (size_t)kl * D.gall;
+  double f[6];
+#pragma unroll
+  for (int m = 0; m < 6; ++m) f[m] = (P.flx + m * n3 + off)[c];
+  if (A.first) A.rh[off + c] = P.rho[off + c] - (f[0] + f[1] + f[2] + f[3] + f[4] + f[5]);
+  if (k < D.kmin - 1 || k >= D.kmax) return;
+  for (int t = 0; t < P.nt; ++t) {
+    const double *fv = P.fv + (size_t)t * 3 * n3 + off;
+    double s = f[0] * fv[c];
+    s = s + f[1] * (fv + n3)[c];
+    s = s + f[2] * (fv + 2 * n3)[c];
+    s = s + f[3] * fv[c - 1];
+    s = s + f[4] * (fv + n3)[c - G - 1];
+    s = s + f[5] * (fv + 2 * n3)[c - G];
+    (A.Qh + t * n3 + off)[c] = (P.Q + t * n3 + off)[c] - s;
   }
 }
 
-// pole faces (mod_src_tracer.f90:412-425), one thread per (pole, level, ring face v)
-__global__ void k_adj_face_pl(int kall, const double *q_pl, const double *qa0_pl, const double *qo_pl,
-                              const double *cm_pl, const double *flx_pl, const double *aQ_pl, const double *xc_pl,
-                              const double *GRD_x_pl, const double *gr_pl, double *a_flx_pl, double *a_xc_pl,
-                              double *a_qo_pl, double *a_q_pl, double *a_gr_pl) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kLallPl * kall * 5) return;
-  const int v = t % 5 + 2, kl = t / 5, l = kl / kall;
-  const size_t off = (size_t)kl * kGallPl, fsp = (size_t)kLallPl * kall * kGallPl;
-  const int vp = (v == 6) ? 2 : v + 1, vm = (v == 2) ? 6 : v - 1;
-  const int p[4] = {0, v - 1, vm - 1, vp - 1};
-  const double qv[4] = {q_pl[off + p[0]], q_pl[off + p[1]], q_pl[off + p[2]], q_pl[off + p[3]]};
-  const double lo = mn(mn(mn(qv[0], qv[1]), qv[2]), qv[3]);
-  const double hi = mx(mx(mx(qv[0], qv[1]), qv[2]), qv[3]);
-  const double cc = cm_pl[off + v - 1], v0 = qa0_pl[off + v - 1];
-  const double v1a = mx(v0, lo);
-  int s1 = (lo > v0) ? 1 : 0;
-  const double v1 = mn(v1a, hi);
-  if (hi < v1a) s1 = 2;
-  const int up = (cc != 0.0) ? v - 1 : 0;
-  const double Qx = qo_pl[fsp + off + up], Qn = qo_pl[off + up];
-  const double v2a = mn(v1, Qx);
-  int s2 = (Qx < v1) ? 1 : 0;
-  const double v2 = mx(v2a, Qn);
-  if (Qn > v2a) s2 = 2;
-  const double a = aQ_pl[off];
-  const double av = -a * flx_pl[off + v - 1];
-  a_flx_pl[off + v - 1] += -a * v2;
-  if (av == 0.0) return;
-  if (s2 == 1) {
-    atomicAdd(&a_qo_pl[fsp + off + up], av);
-  } else if (s2 == 2) {
-    atomicAdd(&a_qo_pl[off + up], av);
-  } else if (s1 == 1) {
-    atomicAdd(&a_q_pl[off + p[argmin4(qv)]], av);
-  } else if (s1 == 2) {
-    atomicAdd(&a_q_pl[off + p[argmax4(qv)]], av);
+// which of four values mn4 / mx4 returns
+__device__ __forceinline__ int arg4(const double (&v)[4], bool high) {
+  int i = 0;
+  double s = v[0];
+#pragma unroll
+  for (int n = 1; n < 4; ++n)
+    if (high ? v[n] > s : v[n] < s) s = v[n], i = n;
+  return i;
+}
+
+// Faces with a halo cell on one side, one thread per (face, level), the group's tracers one after the
+// other: the adjoint of the upwind cell's gradient and Qout goes to the cell whose values the halo
+// stands for (a_bb).  The last threads take the pole faces.
+__global__ void __launch_bounds__(128) k_adj_seam(AdjArgs A) {
+  const PlainArgs &P = A.P;
+  const Dims &D = P.D;
+  const int NK = D.kmax - D.kmin + 1, K = D.kall, G = D.gall_1d;
+  const size_t n3 = P.n3(), n3p = P.n3p();
+  const long long u = (long long)blockIdx.x * 128 + threadIdx.x, nseam = (long long)P.ns * NK;
+  if (u >= nseam) {
+    const int w = (int)(u - nseam);
+    if (w >= kLallPl * NK * 5 * P.nt) return;
+    const int v = w % 5 + 1, k = D.kmin - 1 + w / 5 % NK, p = w / 5 / NK % kLallPl, t = w / 5 / NK / kLallPl;
+    const size_t off = ((size_t)p * K + k) * kGallPl;
+    const double a = A.aQp[t * n3p + off], av = -a * P.flxp[off + v];
+    const PoleFace f = pole_face(P, t, p, k, v);
+    atomicAdd(&A.a_flxp[off + v], -a * mx(mn(mn(mx(f.v0, f.lo), f.hi), f.bv[4]), f.bv[3]));
+    if (av == 0.0) return;
+    double *aq = A.a_qp + t * n3p + off, *ab = A.a_bb + (f.bv - P.bb);
+    const Pick pick = limited(f.v0, f.lo, f.hi, f.bv[3], f.bv[4]);
+    if (pick == kQmax || pick == kQmin) {
+      atomicAdd(&ab[pick == kQmax ? 4 : 3], av);
+    } else if (pick == kLow || pick == kHigh) {
+      const int pt[4] = {0, v, (v == 1) ? 5 : v - 1, (v == 5) ? 1 : v + 1};
+      const double qv[4] = {f.q[pt[0]], f.q[pt[1]], f.q[pt[2]], f.q[pt[3]]};
+      atomicAdd(&aq[pt[arg4(qv, pick == kHigh)]], av);
+    } else {
+      atomicAdd(&aq[f.up], av);
+      for (int d = 0; d < 3; ++d) {
+        const size_t xi = d * n3p + off + v;
+        atomicAdd(&ab[d], av * (P.xcp[xi] - P.GRD_xp[((size_t)d * kLallPl + p) * kGallPl + f.up]));
+        atomicAdd(&A.a_xcp[xi], av * f.bv[d]);
+      }
+    }
+    return;
+  }
+  const int e = (int)(u % P.ns), k = D.kmin - 1 + (int)(u / P.ns), code = P.seam[e];
+  const int a = code % 3, o = code / 3 % D.gall, l = code / 3 / D.gall;
+  const int i = o % G + 1, j = o / G + 1, nb = o + face_step(a, G);
+  const bool inO = P.inner(i, j), inN = P.inner(a < 2 ? i + 1 : i, a > 0 ? j + 1 : j);
+  if (!inO && !inN) return;  // no interior cell reads it
+  const size_t off = ((size_t)l * K + k) * D.gall, gw = (size_t)D.lall * D.gall;
+  const double *rho = P.rho + off;
+  int p[4] = {o, 0, 0, 0};
+  if (a == 0) {
+    p[1] = max(o - G, 0), p[2] = o + 1, p[3] = o + G + 1;
+  } else if (a == 1) {
+    const bool sing = D.have_sgp[l] != 0 && i == D.gmin - 1 && j == D.gmin - 1;
+    p[1] = sing ? o + G + 1 : o + 1, p[2] = sing ? o + G + 2 : o + G + 1, p[3] = o + G;
   } else {
-    atomicAdd(&a_q_pl[off + up], av);
-    for (int x = 0; x < 3; ++x) {
-      const size_t xi = (size_t)x * fsp + off + v - 1;
-      atomicAdd(&a_gr_pl[(size_t)x * fsp + off + up],
-                av * (xc_pl[xi] - GRD_x_pl[((size_t)x * kLallPl + l) * kGallPl + up]));
-      a_xc_pl[xi] += av * gr_pl[(size_t)x * fsp + off + up];
+    p[1] = o + G + 1, p[2] = o + G, p[3] = max(o - 1, 0);
+  }
+  const double fo = P.flx[a * n3 + off + o], fn = P.flx[(a + 3) * n3 + off + nb];
+  const int up = upmask(fo, rho[o]) ? nb : o, b = P.bsrc[(size_t)l * D.gall + up];
+  double disp[3], ax[3] = {0.0, 0.0, 0.0};
+  for (int d = 0; d < 3; ++d) disp[d] = P.xc[(d * 3 + a) * n3 + off + o] - P.GRD_x[d * gw + (size_t)l * D.gall + up];
+  for (int t = 0; t < P.nt; ++t) {
+    const double *Q = P.Q + t * n3 + off, *aQ = A.aQ + t * n3 + off;
+    const double t1 = inO ? -aQ[o] * fo : 0.0, t2 = inN ? -aQ[nb] * fn : 0.0, av = t1 + t2;
+    if (av == 0.0) continue;
+    const double qv[4] = {Q[p[0]] / rho[p[0]], Q[p[1]] / rho[p[1]], Q[p[2]] / rho[p[2]], Q[p[3]] / rho[p[3]]};
+    const double qu = Q[up] / rho[up];
+    // a halo point no list fills has no gradient, and Qout = q
+    const double none[5] = {0.0, 0.0, 0.0, qu, qu}, *bv = b >= 0 ? P.bval(t, k, b) : none;
+    double v0 = qu;
+    for (int d = 0; d < 3; ++d) v0 = v0 + bv[d] * disp[d];
+    const Pick pick = limited(v0, mn4(qv[0], qv[1], qv[2], qv[3]), mx4(qv[0], qv[1], qv[2], qv[3]), bv[3], bv[4]);
+    double *aq = A.a_q + t * n3 + off;
+    if (pick == kLow || pick == kHigh) {
+      atomicAdd(&aq[p[arg4(qv, pick == kHigh)]], av);
+    } else if (pick == kRemap) {
+      atomicAdd(&aq[up], av);
+      for (int d = 0; d < 3; ++d) {
+        if (b >= 0) atomicAdd(A.abval(t, k, b) + d, av * disp[d]);
+        ax[d] += av * bv[d];
+      }
+    } else if (b >= 0) {
+      atomicAdd(A.abval(t, k, b) + (pick == kQmax ? 4 : 3), av);
+    } else {
+      atomicAdd(&aq[up], av);
     }
   }
-}
-
-// ---------------------------------------------------------------------------
-// Qout of one cell (mod_src_tracer.f90:219-301): halo Qout = q, interior the
-// Thuburn bounds from the 6 faces' Qin and the Courant numbers.
-__global__ void k_adj_qout(Dims D, const double *__restrict__ q, const double *__restrict__ cm,
-                           const double *__restrict__ ch, const double *__restrict__ a_qo, double *a_q,
-                           double *a_ch) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
-  const int i = c % G + 1, j = c / G + 1;
-  const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall;
-  const double aQn = a_qo[off + c], aQx = a_qo[fs + off + c];
-  if (aQn == 0.0 && aQx == 0.0) return;
-  if (!inner(D, i, j)) {
-    atomicAdd(&a_q[off + c], aQn + aQx);
-    return;
-  }
-  const bool sgp = D.have_sgp[l] != 0;
-  const double *qs = q + off;
-  const int oi[7] = {0, i, i, i, i - 1, i - 1, i}, oj[7] = {0, j, j, j, j, j - 1, j - 1};
-  const int fo[7] = {0, 1, 2, 3, 1, 2, 3};
-  double qmn[7], qmx[7], chv[7], chm[7];
-  int pmn[7], pmx[7];
-  for (int f = 1; f <= 6; ++f) {
-    int p[4];
-    face_points(D, oi[f], oj[f], fo[f], sgp, p);
-    const double qv[4] = {qs[p[0]], qs[p[1]], qs[p[2]], qs[p[3]]};
-    const double lo = mn(mn(mn(qv[0], qv[1]), qv[2]), qv[3]);
-    const double hi = mx(mx(mx(qv[0], qv[1]), qv[2]), qv[3]);
-    const double cmo = cm[(size_t)(fo[f] - 1) * fs + off + p[0]];
-    const bool in = (f <= 3) ? (cmo != 0.0) : (cmo == 0.0);
-    qmn[f] = in ? lo : kBig;
-    qmx[f] = in ? hi : -kBig;
-    pmn[f] = in ? p[argmin4(qv)] : -1;
-    pmx[f] = in ? p[argmax4(qv)] : -1;
-    chv[f] = ch[(size_t)(f - 1) * fs + off + c];
-    chm[f] = mn(chv[f], 0.0);
-  }
-  const double q0 = qs[c];
-  double qnmin = q0, qnmax = q0;
-  int snmin = 0, snmax = 0;
-  for (int f = 1; f <= 6; ++f) {
-    if (qmn[f] < qnmin) qnmin = qmn[f], snmin = f;
-    if (qmx[f] > qnmax) qnmax = qmx[f], snmax = f;
-  }
-  const double Cin = chm[1] + chm[2] + chm[3] + chm[4] + chm[5] + chm[6];
-  const double Cout = chv[1] - chm[1] + chv[2] - chm[2] + chv[3] - chm[3] + chv[4] - chm[4] + chv[5] - chm[5] +
-                      chv[6] - chm[6];
-  const double zerosw = 0.5 - sgn(0.5, fabs(Cout) - kEps);
-  if (zerosw != 0.0) {
-    atomicAdd(&a_q[off + c], aQn + aQx);
-    return;
-  }
-  double CQmin = 0.0, CQmax = 0.0;
-  for (int f = 1; f <= 6; ++f) CQmin += chm[f] * qmn[f], CQmax += chm[f] * qmx[f];
-  const double S = 1.0 - Cin - Cout;
-  const double Nmn = q0 - CQmax - qnmax * S, Nmx = q0 - CQmin - qnmin * S;
-  const double Dn = Cout;
-  const double aNmn = aQn / Dn, aNmx = aQx / Dn, aD = -(aQn * Nmn + aQx * Nmx) / (Dn * Dn);
-  double a_q0 = aNmn + aNmx;
-  const double a_qnmax = -aNmn * S, a_qnmin = -aNmx * S;
-  const double aS = -aNmn * qnmax - aNmx * qnmin;
-  const double aCQmax = -aNmn, aCQmin = -aNmx, aCin = -aS, aCout = -aS + aD;
-  if (snmax == 0) a_q0 += a_qnmax;
-  else if (pmx[snmax] >= 0) atomicAdd(&a_q[off + pmx[snmax]], a_qnmax);
-  if (snmin == 0) a_q0 += a_qnmin;
-  else if (pmn[snmin] >= 0) atomicAdd(&a_q[off + pmn[snmin]], a_qnmin);
-  atomicAdd(&a_q[off + c], a_q0);
-  for (int f = 1; f <= 6; ++f) {
-    double achm = aCin;
-    if (pmn[f] >= 0) atomicAdd(&a_q[off + pmn[f]], aCQmin * chm[f]), achm += aCQmin * qmn[f];
-    if (pmx[f] >= 0) atomicAdd(&a_q[off + pmx[f]], aCQmax * chm[f]), achm += aCQmax * qmx[f];
-    const double dchm = (0.0 < chv[f]) ? 0.0 : 1.0;
-    a_ch[(size_t)(f - 1) * fs + off + c] += aCout * (1.0 - dchm) + achm * dchm;
+  for (int d = 0; d < 3; ++d) {
+    double &x = A.a_xc[(d * 3 + a) * n3 + off + o];
+    x = A.first ? ax[d] : x + ax[d];
   }
 }
 
-// pole centre Qout (mod_src_tracer.f90:307-367), one thread per (pole, level)
-__global__ void k_adj_qout_pl(int kall, const double *q_pl, const double *cm_pl, const double *ch_pl,
-                              const double *a_qo_pl, double *a_q_pl, double *a_ch_pl) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kLallPl * kall) return;
-  const size_t off = (size_t)t * kGallPl, fsp = (size_t)kLallPl * kall * kGallPl;
-  const double aQn = a_qo_pl[off], aQx = a_qo_pl[fsp + off];
-  if (aQn == 0.0 && aQx == 0.0) return;
-  const double *qs = q_pl + off;
-  double qmn[7], qmx[7];
-  int pmn[7], pmx[7];
-  for (int v = 2; v <= 6; ++v) {
-    const int vp = (v == 6) ? 2 : v + 1, vm = (v == 2) ? 6 : v - 1;
-    const int p[4] = {0, v - 1, vm - 1, vp - 1};
-    const double qv[4] = {qs[p[0]], qs[p[1]], qs[p[2]], qs[p[3]]};
-    const double lo = mn(mn(mn(qv[0], qv[1]), qv[2]), qv[3]);
-    const double hi = mx(mx(mx(qv[0], qv[1]), qv[2]), qv[3]);
-    const bool in = cm_pl[off + v - 1] != 0.0;
-    qmn[v] = in ? lo : kBig;
-    qmx[v] = in ? hi : -kBig;
-    pmn[v] = in ? p[argmin4(qv)] : -1;
-    pmx[v] = in ? p[argmax4(qv)] : -1;
+// pole centre (t, p, k): Qout (mod_src_tracer.f90:307-367) and gradient, transposed
+__device__ __forceinline__ void adj_pole_centre(const AdjArgs &A, int t, int p, int k) {
+  const PlainArgs &P = A.P;
+  const size_t off = ((size_t)p * P.D.kall + k) * kGallPl, n3p = P.n3p();
+  const double *ab = A.abval(t, k, P.nb - 2 + p);
+  double *a_q = A.a_qp + t * n3p + off;
+  for (int x = 0; x < 3; ++x) {
+    const double *cx = P.cgp + ((size_t)p * 3 + x) * 6;
+    for (int v = 0; v < kGallPl; ++v) a_q[v] += cx[v] * ab[x];
   }
-  const double q0 = qs[0];
-  double qnmin = q0, qnmax = q0;
+  const double aQn = ab[3], aQx = ab[4];
+  if (aQn == 0.0 && aQx == 0.0) return;
+  double qs[kGallPl], qmn[6], qmx[6], chm[6], ch[6];
+  int pmn[6], pmx[6];
+  for (int v = 0; v < kGallPl; ++v) qs[v] = P.Qp[t * n3p + off + v] / P.rhop[off + v];
+  double qnmin = qs[0], qnmax = qs[0], Cin = 0.0, Cout = 0.0, CQmax = 0.0, CQmin = 0.0;
   int snmin = 0, snmax = 0;
-  for (int v = 2; v <= 6; ++v) {
+  for (int v = 1; v <= 5; ++v) {
+    const int pt[4] = {0, v, (v == 1) ? 5 : v - 1, (v == 5) ? 1 : v + 1};
+    const double qv[4] = {qs[pt[0]], qs[pt[1]], qs[pt[2]], qs[pt[3]]};
+    const bool in = upmask(P.flxp[off + v], P.rhop[off]);
+    qmn[v] = in ? mn4(qv[0], qv[1], qv[2], qv[3]) : kBig;
+    qmx[v] = in ? mx4(qv[0], qv[1], qv[2], qv[3]) : -kBig;
+    pmn[v] = in ? pt[arg4(qv, false)] : -1;
+    pmx[v] = in ? pt[arg4(qv, true)] : -1;
     if (qmn[v] < qnmin) qnmin = qmn[v], snmin = v;
     if (qmx[v] > qnmax) qnmax = qmx[v], snmax = v;
+    ch[v] = P.flxp[off + v] / P.rhop[off];
+    chm[v] = in ? ch[v] : 0.0;
+    Cin = Cin + chm[v];
+    Cout = Cout - chm[v] + ch[v];
+    CQmin = CQmin + chm[v] * qmn[v];
+    CQmax = CQmax + chm[v] * qmx[v];
   }
-  double Cin = 0.0, Cout = 0.0, CQmax = 0.0, CQmin = 0.0, chmk[7];
-  for (int v = 2; v <= 6; ++v) {
-    chmk[v] = cm_pl[off + v - 1] * ch_pl[off + v - 1];
-    Cin = Cin + chmk[v];
-    Cout = Cout - chmk[v] + ch_pl[off + v - 1];
-    CQmin = CQmin + chmk[v] * qmn[v];
-    CQmax = CQmax + chmk[v] * qmx[v];
-  }
-  const double zerosw = 0.5 - sgn(0.5, fabs(Cout) - kEps);
-  if (zerosw != 0.0) {
-    a_q_pl[off] += aQn + aQx;
+  if (0.5 - sgn(0.5, fabs(Cout) - kEps) != 0.0) {
+    a_q[0] += aQn + aQx;
     return;
   }
   const double S = 1.0 - Cin - Cout, Dn = Cout;
-  const double Nmn = q0 - CQmax - qnmax * S, Nmx = q0 - CQmin - qnmin * S;
+  const double Nmn = qs[0] - CQmax - qnmax * S, Nmx = qs[0] - CQmin - qnmin * S;
   const double aNmn = aQn / Dn, aNmx = aQx / Dn, aD = -(aQn * Nmn + aQx * Nmx) / (Dn * Dn);
-  double a_q0 = aNmn + aNmx;
-  const double a_qnmax = -aNmn * S, a_qnmin = -aNmx * S;
-  const double aS = -aNmn * qnmax - aNmx * qnmin;
+  const double a_qnmax = -aNmn * S, a_qnmin = -aNmx * S, aS = -aNmn * qnmax - aNmx * qnmin;
   const double aCQmax = -aNmn, aCQmin = -aNmx, aCin = -aS, aCout = -aS + aD;
-  if (snmax == 0) a_q0 += a_qnmax;
-  else if (pmx[snmax] >= 0) a_q_pl[off + pmx[snmax]] += a_qnmax;
-  if (snmin == 0) a_q0 += a_qnmin;
-  else if (pmn[snmin] >= 0) a_q_pl[off + pmn[snmin]] += a_qnmin;
-  a_q_pl[off] += a_q0;
-  for (int v = 2; v <= 6; ++v) {
-    const double cc = cm_pl[off + v - 1];
+  a_q[0] += aNmn + aNmx;
+  a_q[snmax ? pmx[snmax] : 0] += a_qnmax;
+  a_q[snmin ? pmn[snmin] : 0] += a_qnmin;
+  for (int v = 1; v <= 5; ++v) {
     double achm = aCin - aCout;
-    if (pmn[v] >= 0) a_q_pl[off + pmn[v]] += aCQmin * chmk[v], achm += aCQmin * qmn[v];
-    if (pmx[v] >= 0) a_q_pl[off + pmx[v]] += aCQmax * chmk[v], achm += aCQmax * qmx[v];
-    a_ch_pl[off + v - 1] += aCout + achm * cc;
+    if (pmn[v] >= 0) {
+      a_q[pmn[v]] += aCQmin * chm[v], a_q[pmx[v]] += aCQmax * chm[v];
+      achm += aCQmin * qmn[v] + aCQmax * qmx[v];
+    }
+    atomicAdd(&A.a_chp[off + v], aCout + (pmn[v] >= 0 ? achm : 0.0));
   }
 }
 
-// ---------------------------------------------------------------------------
-// gradient stencil (mod_oprt.f90:499-734 coefficients), transposed as a gather:
-// point p collects coef(c, n) a_grad(c) from the interior cells c whose n-th
-// stencil point it is.
-__global__ void k_adj_grad(Dims D, const double *__restrict__ cg, const double *__restrict__ a_gr, double *a_q) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
-  const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall;
-  const int d[7] = {0, 1, G + 1, G, -1, -G - 1, -G};
-  double s = 0.0;
-  bool any = false;
-  for (int n = 0; n < 7; ++n) {
-    const int c = p - d[n];
-    if (c < 0 || c >= D.gall || !inner(D, c % G + 1, c / G + 1)) continue;
-    for (int x = 0; x < 3; ++x) {
-      const double a = a_gr[(size_t)x * fs + off + c];
-      if (a == 0.0) continue;
-      s += cg[(((size_t)l * 3 + x) * 7 + n) * D.gall + c] * a;
-      any = true;
+// The cells.  The upwind cell of a face holds every operand of its value, so the face, the remap, the
+// cell's Qout and its gradient are transposed by that cell's thread: the adjoints of its gradient and
+// Qout are registers, those of the tracer-independent inputs (fluxes, face centroids, Courant
+// numbers) are summed over the tracers on chip, and a tracer's adjoint of q leaves as seven values a
+// cell that the tile adds up in shared memory.  Only what a bound hands to one of its cells, which
+// the data decide, goes to memory one by one (atomicAdd).
+// Bound by latency at 12 warps an SM (168 registers and 75 KB a block): 1.9 ms for 8 tracers of glevel
+// 6, kall 42; with the per-thread sums in registers two blocks fit and it took 2.3, or three that
+// spilled, 3.0.
+constexpr int kAdjCells = 128;  // threads, one per cell of a TX x (128 / TX) tile
+constexpr int kAdjBlocks = 3;   // per SM
+
+// cells bounding face f (0..5: faces 1-6, 6: face 5 of a singular corner) as neighbours of the cell, the
+// owner first (mod_src_tracer.f90:152-214), and the neighbours' steps in i and j
+__constant__ signed char kFacePts[7][4] = {{0, 6, 1, 2}, {0, 1, 2, 3}, {0, 2, 3, 4}, {4, 5, 0, 3},
+                                           {5, 6, 0, 4}, {6, 1, 0, 5}, {5, 0, 1, 4}};
+__constant__ signed char kStepI[7] = {0, 1, 1, 0, -1, -1, 0}, kStepJ[7] = {0, 0, 1, 1, 0, -1, -1};
+
+template <int TX>
+struct AdjCellSmem : CellSmem<TX, kAdjCells> {  // q[0]: q of the window, q[1]: adjoint of rhogq there
+  double part[7][kAdjCells];  // adjoints of q of a cell and its neighbours
+  // each thread's own, here for want of registers: fluxes of its faces and their adjoints, adjoints of
+  // the chosen outflow faces' centroids and of the Courant numbers
+  double flx[6][kAdjCells], aflx[6][kAdjCells], axc[9][kAdjCells], ach[6][kAdjCells];
+};
+
+template <int TX>
+__global__ void __launch_bounds__(kAdjCells, kAdjBlocks) k_adj_cells(AdjArgs A, int ntx, int nty, int nlb, int lpb) {
+  using Tile = CellTile<TX, kAdjCells>;
+  using S = AdjCellSmem<TX>;
+  extern __shared__ __align__(16) unsigned char raw[];
+  S &s = *reinterpret_cast<S *>(raw);
+  const PlainArgs &P = A.P;
+  const Dims &D = P.D;
+  const int G = D.gall_1d, tid = threadIdx.x, nmain = ntx * nty * D.lall * nlb;
+  if ((int)blockIdx.x >= nmain) {
+    const int u = ((int)blockIdx.x - nmain) * kAdjCells + tid, NK = D.kmax - D.kmin + 1;
+    if (u < P.nt * kLallPl * NK) adj_pole_centre(A, u / NK / kLallPl, u / NK % kLallPl, D.kmin - 1 + u % NK);
+    return;
+  }
+  const int lb = (int)blockIdx.x % nlb;
+  Tile T;
+  T.init(P, s, (int)blockIdx.x / nlb, ntx, nty);
+  const int c = T.c;
+  const size_t n3 = P.n3();
+  const int k0 = D.kmin - 1 + lb * lpb, k1 = min(k0 + lpb, D.kmax);
+  for (int k = k0; k < k1; ++k) {
+    const size_t off = ((size_t)T.l * D.kall + k) * D.gall;
+    double Qw[Tile::NSLOT][1], aw[Tile::NSLOT];
+    auto load = [&](int t) {
+      const double *Qs = P.Q + (size_t)t * n3 + off, *as = A.aQ + (size_t)t * n3 + off;
+#pragma unroll
+      for (int r = 0; r < Tile::NSLOT; ++r)
+        if (T.wc[r] >= 0) Qw[r][0] = Qs[T.wc[r]], aw[r] = as[T.wc[r]];
+    };
+    load(0);
+    CellFlow F;
+    double fo[3];
+    {
+      Recip rw[Tile::NSLOT];
+      double flx[6];
+      T.level(P, s, off, rw, F, flx);
+#pragma unroll
+      for (int m = 0; m < 6; ++m) s.flx[m][tid] = flx[m], s.aflx[m][tid] = s.ach[m][tid] = 0.0;
+#pragma unroll
+      for (int m = 0; m < 9; ++m) s.axc[m][tid] = 0.0;
+    }
+    // the flux of the chosen outflow faces as their other cell has it, with this cell's own
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const bool f = (F.side >> a) & 1u;
+      fo[a] = F.st[a] >= 0 ? (P.flx + (size_t)(f ? a : a + 3) * n3 + off)[f ? F.st[a] : c + face_step(a, G)] : 0.0;
+      if (A.first && ((F.again >> a) & 1u))
+        for (int d = 0; d < 3; ++d) (A.a_xc + (size_t)(d * 3 + a) * n3 + off)[c - face_step(a, G)] = 0.0;
+    }
+    for (int t = 0; t < P.nt; ++t) {
+      double *a_q = A.a_q + (size_t)t * n3 + off;
+#pragma unroll
+      for (int r = 0; r < Tile::NSLOT; ++r)
+        if (T.wc[r] >= 0) {
+          const int e = tid + r * kAdjCells;
+          const double rho = s.rho[e];
+          quotients(Qw[r], Recip{rho, s.y[e], recip_ok(rho)});
+          s.q[0][e] = Qw[r][0];
+          s.q[1][e] = aw[r];
+        }
+      if (t + 1 < P.nt) load(t + 1);
+      {  // the fluxes of the cell's faces, in Qh = Q - sum_m flx(m) fv(m)
+        const double *fv = P.fv + (size_t)t * 3 * n3 + off, aH = T.act ? (A.aQ + (size_t)t * n3 + off)[c] : 0.0;
+        const double f[6] = {fv[c], (fv + n3)[c], (fv + 2 * n3)[c], fv[c - 1], (fv + n3)[c - G - 1], (fv + 2 * n3)[c - G]};
+#pragma unroll
+        for (int m = 0; m < 6; ++m) s.aflx[m][tid] += -aH * f[m];
+      }
+      __syncthreads();
+      double n[7], g[3];
+      T.gradient(s, 0, n, g);
+      CellLimits L;
+      cell_limits(n, F, T.sing, L);
+      double aself = 0.0, ag[3] = {0.0, 0.0, 0.0}, aQn = 0.0, aQx = 0.0;
+      if (T.bs >= 0) {  // what seam and pole faces hand to this cell's values
+        const double *o = A.abval(t, k, T.bs);
+        ag[0] = o[0], ag[1] = o[1], ag[2] = o[2], aQn = o[3], aQx = o[4];
+      }
+      const double aH = s.q[1][T.ew];
+      // the cell (as a neighbour of this one) that face f's lower or upper bound is a copy of
+      auto bound = [&](int f, bool high) {
+        const signed char *pt = kFacePts[(f == 4 && T.sing) ? 6 : f];
+        int at = pt[0];
+        double best = s.q[0][T.ew + kStepJ[at] * S::WW + kStepI[at]];
+        for (int x = 1; x < 4; ++x) {
+          const int q = pt[x];
+          const double v = s.q[0][T.ew + kStepJ[q] * S::WW + kStepI[q]];
+          if (high ? v > best : v < best) best = v, at = q;
+        }
+        return c + kStepJ[at] * G + kStepI[at];
+      };
+      // outflow face m (of faces a + 1 and a + 4): own flux fm, the other cell's fn and its adjoint aN
+      auto face = [&](int a, int m, double lo, double hi, double fn, int slot, auto centroid) {
+        const double fm = s.flx[m - 1][tid], aN = s.q[1][T.ew + (m > 3 ? Tile::wstep(a + 4) : Tile::wstep(a + 1))];
+        const double av = -aH * fm + -aN * fn;
+        if (av == 0.0) return;
+        double v0 = n[0], disp[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) disp[d] = s.disp[a * 3 + d][slot], v0 = v0 + g[d] * disp[d];
+        const Pick pick = limited(v0, lo, hi, L.Qmin, L.Qmax);
+        if (pick == kRemap) {
+          aself += av;
+#pragma unroll
+          for (int d = 0; d < 3; ++d) ag[d] += av * disp[d], centroid(d, av * g[d]);
+        } else if (pick == kQmin) {
+          aQn += av;
+        } else if (pick == kQmax) {
+          aQx += av;
+        } else {
+          atomicAdd(&a_q[bound(m - 1, pick == kHigh)], av);
+        }
+      };
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (F.st[a] < 0) continue;
+        const bool f = (F.side >> a) & 1u;
+        face(a, f ? a + 4 : a + 1, f ? L.lo[a + 4] : L.lo[a + 1], f ? L.hi[a + 4] : L.hi[a + 1], fo[a], F.sl[a],
+             [&](int d, double x) { s.axc[a * 3 + d][tid] += x; });
+      }
+      if (F.again) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if ((F.again >> a) & 1u) {
+            const int oc = c - face_step(a, G);
+            face(a, a + 4, L.lo[a + 4], L.hi[a + 4], (P.flx + (size_t)a * n3 + off)[oc], T.ow - Tile::slot_back(a),
+                 [&](int d, double x) { (A.a_xc + (size_t)(d * 3 + a) * n3 + off)[oc] += x; });
+          }
+      }
+      // Qout (mod_src_tracer.f90:219-282): a cell whose bounds bind no face has nothing to hand on
+      if (T.act && (aQn != 0.0 || aQx != 0.0)) {
+        if (F.zsw) {
+          aself += aQn + aQx;
+        } else {
+          const double Dn = F.den.b, O = F.omc;
+          const double Nmn = n[0] - L.CQmax - L.qnmax * O, Nmx = n[0] - L.CQmin - L.qnmin * O;
+          const double aNmn = aQn / Dn, aNmx = aQx / Dn, aD = -(aQn * Nmn + aQx * Nmx) / (Dn * Dn);
+          const double aS = -aNmn * L.qnmax - aNmx * L.qnmin;
+          const double aCQmax = -aNmn, aCQmin = -aNmx, aCin = -aS, aCout = -aS + aD;
+          aself += aNmn + aNmx;
+          int fmin = 0, fmax = 0;  // the face whose bound is qnmin / qnmax, 0: the cell itself
+          double lowest = n[0], highest = n[0];
+#pragma unroll
+          for (int m = 1; m <= 6; ++m) {
+            const bool f = (F.in >> m) & 1u;
+            if (f && L.lo[m] < lowest) lowest = L.lo[m], fmin = m;
+            if (f && L.hi[m] > highest) highest = L.hi[m], fmax = m;
+            double achm = aCin;
+            if (f) {
+              atomicAdd(&a_q[bound(m - 1, false)], aCQmin * F.chm[m]);
+              atomicAdd(&a_q[bound(m - 1, true)], aCQmax * F.chm[m]);
+              achm += aCQmin * L.lo[m] + aCQmax * L.hi[m];
+            }
+            s.ach[m - 1][tid] += (s.flx[m - 1][tid] / s.rho[T.ew] > 0.0) ? aCout : achm;
+          }
+          if (fmax) atomicAdd(&a_q[bound(fmax - 1, true)], -aNmn * O);
+          else aself += -aNmn * O;
+          if (fmin) atomicAdd(&a_q[bound(fmin - 1, false)], -aNmx * O);
+          else aself += -aNmx * O;
+        }
+      }
+      // the gradient's stencil; the tile's cells are added up, one atomic per window cell
+#pragma unroll
+      for (int m = 0; m < 7; ++m) {
+        double x = s.cg[m][tid] * ag[0];
+        x += s.cg[7 + m][tid] * ag[1];
+        x += s.cg[14 + m][tid] * ag[2];
+        s.part[m][tid] = T.act ? (m == 0 ? aself + x : x) : 0.0;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < Tile::NSLOT; ++r)
+        if (T.wc[r] >= 0) {
+          const int e = tid + r * kAdjCells, wx = e % S::WW - 1, wy = e / S::WW - 1;  // in the tile's frame
+          double sum = 0.0;
+#pragma unroll
+          for (int m = 0; m < 7; ++m) {
+            constexpr int DX[7] = {0, 1, 1, 0, -1, -1, 0}, DY[7] = {0, 0, 1, 1, 0, -1, -1};
+            const int x = wx - DX[m], y = wy - DY[m];
+            if (x >= 0 && x < TX && y >= 0 && y < S::TY) sum += s.part[m][y * TX + x];
+          }
+          if (sum != 0.0) atomicAdd(&a_q[T.wc[r]], sum);
+        }
+    }
+    // ---- the level's sums over the tracers
+    if (T.act) {
+      const double rc = s.rho[T.ew], ah = A.last ? A.a_rh[off + c] : 0.0;
+      double ar = ah;
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        const double a = s.ach[m][tid];
+        double f = s.aflx[m][tid] - ah;
+        if (a != 0.0) f += a / rc, ar += -a * (s.flx[m][tid] / rc) / rc;
+        double &o = (A.a_flx + (size_t)m * n3 + off)[c];
+        o = A.first ? f : o + f;
+      }
+      if (ar != 0.0) A.a_rho[off + c] += ar;
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        if (F.st[a] >= 0) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            double &o = (A.a_xc + (size_t)(d * 3 + a) * n3 + off)[F.st[a]];
+            o = A.first ? s.axc[a * 3 + d][tid] : o + s.axc[a * 3 + d][tid];
+          }
+        }
     }
   }
-  if (any) a_q[off + p] += s;
-}
-__global__ void k_adj_grad_pl(int kall, const double *cg_pl, const double *a_gr_pl, double *a_q_pl) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kLallPl * kall) return;
-  const int l = t / kall;
-  const size_t off = (size_t)t * kGallPl, fsp = (size_t)kLallPl * kall * kGallPl;
-  for (int x = 0; x < 3; ++x) {
-    const double a = a_gr_pl[(size_t)x * fsp + off];
-    const double *cx = cg_pl + ((size_t)l * 3 + x) * 6;
-    a_q_pl[off] += cx[0] * a;
-    for (int v = 2; v <= 6; ++v) a_q_pl[off + v - 1] += cx[v - 1] * a;
-  }
 }
 
-// q = Q / rho: a_Q += a_q / rho, a_rho -= a_q q / rho (regions and poles in one launch)
-__global__ void k_adj_div(long long n3, int n3p, const double *a_q, const double *q, const double *rho,
-                          const double *a_q_pl, const double *q_pl, const double *rho_pl, double *aQ, double *aQp,
-                          double *a_rho, double *a_rho_pl) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n3) {
-    const double a = a_q[t];
-    if (a == 0.0) return;
-    aQ[t] += a / rho[t];
-    a_rho[t] += -a * q[t] / rho[t];
-  } else if (t < n3 + n3p) {
-    const long long u = t - n3;
-    const double a = a_q_pl[u];
-    if (a == 0.0) return;
-    aQp[u] += a / rho_pl[u];
-    a_rho_pl[u] += -a * q_pl[u] / rho_pl[u];
+// q = Q / rho: a_Q += a_q / rho, a_rho -= a_q q / rho, over the group's tracers (regions and poles in
+// one launch, physical levels)
+__global__ void __launch_bounds__(256) k_adj_div(AdjArgs A) {
+  const PlainArgs &P = A.P;
+  const Dims &D = P.D;
+  const int NK = D.kmax - D.kmin + 1;
+  const long long u = (long long)blockIdx.x * 256 + threadIdx.x, nreg = (long long)D.lall * NK * D.gall;
+  const double *rho, *aq, *Q;
+  double *aQ, *ar;
+  size_t ts;
+  if (u < nreg) {
+    const size_t o = ((size_t)(u / D.gall / NK) * D.kall + D.kmin - 1 + u / D.gall % NK) * D.gall + u % D.gall;
+    rho = P.rho + o, aq = A.a_q + o, Q = P.Q + o, aQ = A.aQ + o, ar = A.a_rho + o, ts = P.n3();
+  } else {
+    const int w = (int)(u - nreg);
+    if (w >= kLallPl * NK * kGallPl) return;
+    const size_t o = ((size_t)(w / kGallPl / NK) * D.kall + D.kmin - 1 + w / kGallPl % NK) * kGallPl + w % kGallPl;
+    rho = P.rhop + o, aq = A.a_qp + o, Q = P.Qp + o, aQ = A.aQp + o, ar = A.a_rhop + o, ts = P.n3p();
   }
+  const double r = *rho;
+  double sum = 0.0;
+  for (int t = 0; t < P.nt; ++t) {
+    const double a = aq[t * ts];
+    if (a == 0.0) continue;
+    aQ[t * ts] += a / r;
+    sum += -a * (Q[t * ts] / r) / r;
+  }
+  if (sum != 0.0) *ar += sum;
 }
 
-// rho_h = rho - sum_m flx(m) and ch(m) = flx(m) / rho: adjoints to flx and rho
-__global__ void k_adj_rhoh_ch(Dims D, const double *rho, const double *ch, const double *a_rh, const double *a_ch,
-                              double *a_flx, double *a_rho) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, G = D.gall_1d;
-  const size_t off = (size_t)kl * D.gall + c, fs = (size_t)D.lall * D.kall * D.gall;
-  const double ah = a_rh[off];
-  double ar = a_rho[off] + ah;
-  const bool in = inner(D, c % G + 1, c / G + 1);
-  const double r = rho[off];
-  for (int m = 0; m < 6; ++m) {
-    double f = a_flx[m * fs + off];
-    if (in) f += -ah;
-    const double a = a_ch[m * fs + off];
-    if (a != 0.0) {
-      f += a / r;
-      ar += -a * ch[m * fs + off] / r;
-    }
-    a_flx[m * fs + off] = f;
-  }
-  a_rho[off] = ar;
-}
-__global__ void k_adj_rhoh_ch_pl(int kall, const double *rho_pl, const double *ch_pl, const double *a_rh_pl,
+// pole centres: rho_h = rho - sum_m flx(m) and ch(m) = flx(m) / rho
+__global__ void k_adj_rhoh_ch_pl(int kall, const double *rho_pl, const double *flx_pl, const double *a_rh_pl,
                                  const double *a_ch_pl, double *a_flx_pl, double *a_rho_pl) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= kLallPl * kall) return;
@@ -821,7 +890,7 @@ __global__ void k_adj_rhoh_ch_pl(int kall, const double *rho_pl, const double *c
     const double a = a_ch_pl[off + v - 1];
     if (a == 0.0) continue;
     a_flx_pl[off + v - 1] += a / r;
-    a_rho_pl[off] += -a * ch_pl[off + v - 1] / r;
+    a_rho_pl[off] += -a * (flx_pl[off + v - 1] / r) / r;
   }
 }
 
@@ -859,6 +928,7 @@ __device__ __forceinline__ Tv triI(const Dims &D, const Fld &F, const double *GT
 __device__ __forceinline__ void face_adj(const Dims &D, const Geo<double> &g, const double *a_flx,
                                          const double *a_xc, double dt, int l, size_t off, size_t fs, int o, int a,
                                          bool sgp, const Tv &p, const Tv &q, Tv &ap) {
+  // a_flx and a_xc hold what an interior cell on either side contributed; a face has them only there
   const size_t gw = (size_t)D.gall * D.lall;
   const int G = D.gall_1d;
   const int nb = (a == 1) ? o + 1 : ((a == 2) ? o + G + 1 : o + G);
@@ -866,9 +936,11 @@ __device__ __forceinline__ void face_adj(const Dims &D, const Geo<double> &g, co
   double vs[3];
   for (int x = 0; x < 3; ++x) vs[x] = p.v[x + 1] + q.v[x + 1];
   const double rr = 1.0 / mx(rsum, kEps);
-  double aflux = a_flx[(size_t)(a - 1) * fs + off + o] * g.GMTR_p[(size_t)(P_RAREA - 1) * gw + (size_t)l * D.gall + o] * dt;
+  const bool inO = inner(D, o % G + 1, o / G + 1), inN = inner(D, nb % G + 1, nb / G + 1);
+  if (!inO && !inN) return;
+  double aflux = !inO ? 0.0 : a_flx[(size_t)(a - 1) * fs + off + o] * g.GMTR_p[(size_t)(P_RAREA - 1) * gw + (size_t)l * D.gall + o] * dt;
   const bool sg0 = sgp && a == 3 && nb == (D.gmin - 1) * G + (D.gmin - 1);
-  if (!sg0)
+  if (!sg0 && inN)
     aflux += -a_flx[(size_t)(a + 2) * fs + off + nb] * g.GMTR_p[(size_t)(P_RAREA - 1) * gw + (size_t)l * D.gall + nb] *
              dt;
   double avs[3], arr = 0.0;
@@ -892,6 +964,8 @@ __global__ void k_adj_tri(Dims D, Geo<double> g, Fld F, const double *a_flx, con
   const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
   const int i = c % G + 1, j = c / G + 1;
   const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall;
+  const int k = kl % D.kall;
+  if (k < D.kmin - 1 || k >= D.kmax) return;  // the ghost levels have no part in the step
   Tv aI{}, aJ{};
   const int lo = D.gmin - 1, hi = D.gmax;
   if (i >= lo && i <= hi && j >= lo && j <= hi) {
@@ -926,6 +1000,7 @@ __global__ void k_adj_fields(Dims D, const double *GT, const double *aT, double 
   const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
   const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall, gw = (size_t)D.gall * D.lall;
   const bool sgp = D.have_sgp[l] != 0;
+  if (kl % D.kall < D.kmin - 1 || kl % D.kall >= D.kmax) return;
   const int sg = (D.gmin - 2) * G + (D.gmin - 2);
   auto ok = [&](int c) {
     if (c < 0 || c >= D.gall) return false;
@@ -998,6 +1073,21 @@ __global__ void k_adj_flux_pl(int kall, Geo<double> g, Fld F, const double *a_fl
 
 dim3 slab(const Dims &D, int th) { return dim3((D.gall + th - 1) / th, D.kall * D.lall); }
 
+template <int TX>
+cudaError_t launch_adj_cells(const AdjArgs &A, cudaStream_t st) {
+  const Dims &D = A.P.D;
+  using S = AdjCellSmem<TX>;
+  const int n = D.gmax - D.gmin + 1, ntx = (n + TX - 1) / TX, nty = (n + S::TY - 1) / S::TY;
+  const int tiles = ntx * nty * D.lall, NK = D.kmax - D.kmin + 1;
+  int lpb = 8;  // levels a block, as in the forward's cell kernel
+  while (lpb > 1 && (long long)tiles * ((NK + lpb - 1) / lpb) < 2 * kAdjBlocks * 148) lpb /= 2;
+  const int nlb = (NK + lpb - 1) / lpb, npole = (A.P.nt * kLallPl * NK + kAdjCells - 1) / kAdjCells;
+  cudaError_t e = cudaFuncSetAttribute(k_adj_cells<TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(S));
+  if (e != cudaSuccess) return e;
+  k_adj_cells<TX><<<(unsigned)(tiles * nlb + npole), kAdjCells, sizeof(S), st>>>(A, ntx, nty, nlb, lpb);
+  return cudaGetLastError();
+}
+
 void fill_adj(const StepCtx &S, double *a, double *a_pl, int vmax, cudaStream_t st) {
   const Dims &D = S.D;
   const long long total = (long long)S.plan.n * D.kall * vmax;
@@ -1015,80 +1105,63 @@ int step_adjoint(StepCtx &S, const AdjScratch &A, int ntr, double dt, const doub
                  double *a_vx, double *a_vx_pl, double *a_vy, double *a_vy_pl, double *a_vz, double *a_vz_pl,
                  cudaStream_t st, long long &launches) {
   const Dims &D = S.D;
-  if (D.kall < 4 || D.kmax <= D.kmin) return ICA_ERR_ARG;
+  if (D.kall < 4 || D.kmax <= D.kmin) return set_error("adjoint: bad vertical grid"), ICA_ERR_ARG;
   const size_t n3 = (size_t)D.gall * D.kall * D.lall, n3p = (size_t)kGallPl * D.kall * kLallPl;
   const size_t B = sizeof(double);
-  const int T = 128;
+  const int T = 128, n = D.gmax - D.gmin + 1, NK = D.kmax - D.kmin + 1;
   const unsigned nbl = (unsigned)((kLallPl * D.kall + 127) / 128);
-  // ---- forward recompute of the step-level intermediates
+  // ---- the step-level forward values, the final halo fill, the density part of the vertical sub-step
   FluxIn<double> fin{rhog, rhog_pl, vx, vx_pl, vy, vy_pl, vz, vz_pl};
   FluxOut<double> fout{S.flx, S.flx_pl, S.xc, S.xc_pl};
   launch_horizontal_flux<double>(D, fin, fout, S.geo, dt, st);
-  launch_courant(S, rhog, rhog_pl, st);
-  cudaMemcpyAsync(A.rh, rhog, n3 * B, cudaMemcpyDeviceToDevice, st);
-  cudaMemcpyAsync(A.rh_pl, rhog_pl, n3p * B, cudaMemcpyDeviceToDevice, st);
-  launch_update_rho(S, A.rh, A.rh_pl, st);
-  cudaMemsetAsync(A.a_flx, 0, 6 * n3 * B, st);
   cudaMemsetAsync(A.a_flx_pl, 0, n3p * B, st);
-  cudaMemsetAsync(A.a_xc, 0, 9 * n3 * B, st);
   cudaMemsetAsync(A.a_xc_pl, 0, 3 * n3p * B, st);
-  cudaMemsetAsync(A.a_ch, 0, 6 * n3 * B, st);
   cudaMemsetAsync(A.a_ch_pl, 0, n3p * B, st);
-  launches += 6;
-  // ---- the final halo fill and the density part of the vertical sub-step
   fill_adj(S, a_rhog, a_rhog_pl, 1, st);
   fill_adj(S, a_rhogq, a_rhogq_pl, ntr, st);
   const int npt = D.lall * D.gall + kLallPl * kGallPl;
   k_adj_vrho<<<(npt + 127) / 128, 128, 0, st>>>(D, a_rhog, a_rhog_pl, A.a_rh, A.a_rh_pl);
-  launches += 3;
-  // ---- tracer by tracer: recompute the horizontal sub-step, then transpose it
-  LimIn<double> lin{S.q, S.q_pl, S.zero, S.zero_pl, S.ch, S.ch_pl, S.cm, S.cm_pl};
-  const int ncol = D.lall * D.gall + kLallPl;
-  for (int t = 0; t < ntr; ++t) {
-    const double *Q = rhogq + t * n3, *Qp = rhogq_pl + t * n3p;
-    double *aQ = a_rhogq + t * n3, *aQp = a_rhogq_pl + t * n3p;
-    launch_divide(S, Q, Qp, rhog, rhog_pl, st);
-    launch_gradient(S, st);
-    launch_remap(S, st);
-    launch_hlim_qout<double>(D, lin, S.qout, S.qout_pl, S.qin_pl, st);
-    launch_gather<double>(D, S.plan.n, S.plan.dst, S.plan.src, D.kall, 2, S.qout, S.qout_pl, st);
-    k_adj_qh<<<slab(D, T), T, 0, st>>>(D, S.q, S.qa, S.qout, S.cm, S.flx, Q, A.Qh);
-    k_adj_qh_pl<<<nbl, 128, 0, st>>>(D.kall, S.qa_pl, S.cm_pl, S.qout_pl, S.qin_pl, S.flx_pl, Qp, A.Qh_pl);
+  launches += 4;
+  // ---- the tracers, a group at a time: recompute the faces, then transpose the two sub-steps
+  for (int t0 = 0; t0 < ntr; t0 += kPlainGroup) {
+    AdjArgs a{};
+    // the forward's launches only read rhogq here
+    a.P = plain_group(S, t0, ntr, dt, rhog, rhog_pl, const_cast<double *>(rhogq), const_cast<double *>(rhogq_pl), w, w_pl);
+    const int nt = a.P.nt;
+    a.aQ = a_rhogq + t0 * n3, a.aQp = a_rhogq_pl + t0 * n3p;
+    a.Qh = A.a_q, a.Qhp = A.Qh_pl, a.a_q = A.a_q, a.a_qp = A.a_q_pl, a.a_bb = A.a_bb;
+    a.rh = A.rh, a.rhp = A.rh_pl, a.a_rh = A.a_rh, a.a_rhp = A.a_rh_pl;
+    a.a_flx = A.a_flx, a.a_flxp = A.a_flx_pl, a.a_xc = A.a_xc, a.a_xcp = A.a_xc_pl, a.a_chp = A.a_ch_pl;
+    a.a_rho = a_rhog, a.a_rhop = a_rhog_pl;
+    a.first = t0 == 0, a.last = t0 + nt >= ntr;
+    const int rc = plain_faces(a.P, st, launches);
+    if (rc) return rc;
+    const int cellblk = (D.gall + T - 1) / T, nqh = cellblk * D.kall * D.lall;
+    k_adj_qh<<<(unsigned)(nqh + (nt * kLallPl * D.kall + T - 1) / T), T, 0, st>>>(a, cellblk, nqh);
     // vertical sub-step: aQ becomes the adjoint of rhogq after the horizontal sub-step
-    k_adj_vert<<<(ncol + kAdjThreads - 1) / kAdjThreads, kAdjThreads, (int)sizeof(AdjRing), st>>>(D, dt, A.Qh, A.rh, w, aQ, A.a_rh, A.Qh_pl, A.rh_pl, w_pl, aQp,
-                                                   A.a_rh_pl, S.rdgz, S.afact, S.bfact);
-    cudaMemsetAsync(A.a_q, 0, n3 * B, st);
-    cudaMemsetAsync(A.a_q_pl, 0, n3p * B, st);
-    cudaMemsetAsync(A.a_gr, 0, 3 * n3 * B, st);
-    cudaMemsetAsync(A.a_gr_pl, 0, 3 * n3p * B, st);
-    cudaMemsetAsync(A.a_qo, 0, 2 * n3 * B, st);
-    cudaMemsetAsync(A.a_qo_pl, 0, 2 * n3p * B, st);
-    k_adj_face<<<slab(D, T), T, 0, st>>>(D, S.q, S.qa, S.qout, S.cm, S.flx, aQ, S.xc, S.GRD_x, S.grad, A.a_flx,
-                                         A.a_xc, A.a_qo, A.a_q, A.a_gr);
-    k_adj_face_pl<<<(unsigned)((kLallPl * D.kall * 5 + 127) / 128), 128, 0, st>>>(
-        D.kall, S.q_pl, S.qa_pl, S.qout_pl, S.cm_pl, S.flx_pl, aQp, S.xc_pl, S.GRD_x_pl, S.grad_pl, A.a_flx_pl,
-        A.a_xc_pl, A.a_qo_pl, A.a_q_pl, A.a_gr_pl);
-    fill_adj(S, A.a_qo, A.a_qo_pl, 2, st);
-    k_adj_qout<<<slab(D, T), T, 0, st>>>(D, S.q, S.cm, S.ch, A.a_qo, A.a_q, A.a_ch);
-    k_adj_qout_pl<<<nbl, 128, 0, st>>>(D.kall, S.q_pl, S.cm_pl, S.ch_pl, A.a_qo_pl, A.a_q_pl, A.a_ch_pl);
-    fill_adj(S, A.a_gr, A.a_gr_pl, 3, st);
-    k_adj_grad<<<slab(D, T), T, 0, st>>>(D, S.cg, A.a_gr, A.a_q);
-    k_adj_grad_pl<<<nbl, 128, 0, st>>>(D.kall, S.cg_pl, A.a_gr_pl, A.a_q_pl);
-    k_adj_div<<<(unsigned)((n3 + n3p + 255) / 256), 256, 0, st>>>((long long)n3, (int)n3p, A.a_q, S.q, rhog,
-                                                                  A.a_q_pl, S.q_pl, rhog_pl, aQ, aQp, a_rhog,
-                                                                  a_rhog_pl);
-    launches += 27;
+    const int colblk = (n * n + kAdjThreads - 1) / kAdjThreads, ncol = colblk * D.lall * nt;
+    k_adj_vert<<<(unsigned)(ncol + (nt * kLallPl + kAdjThreads - 1) / kAdjThreads), kAdjThreads, sizeof(AdjRing), st>>>(
+        a, colblk, ncol);
+    cudaMemsetAsync(A.a_q, 0, nt * n3 * B, st);
+    cudaMemsetAsync(A.a_q_pl, 0, nt * n3p * B, st);
+    cudaMemsetAsync(A.a_bb, 0, (size_t)nt * D.kall * S.nb * 5 * B, st);
+    const long long nsm = (long long)S.ns * NK + (long long)kLallPl * NK * 5 * nt;
+    k_adj_seam<<<(unsigned)((nsm + 127) / 128), 128, 0, st>>>(a);
+    const cudaError_t e = n >= 32 ? launch_adj_cells<32>(a, st) : launch_adj_cells<16>(a, st);
+    if (e != cudaSuccess) return set_error(std::string("adjoint: ") + cudaGetErrorString(e)), ICA_ERR_CUDA;
+    const long long nd = (long long)NK * (D.lall * D.gall + kLallPl * kGallPl);
+    k_adj_div<<<(unsigned)((nd + 255) / 256), 256, 0, st>>>(a);
+    launches += 5;
   }
-  // ---- density update and Courant numbers, then horizontal_flux
-  k_adj_rhoh_ch<<<slab(D, T), T, 0, st>>>(D, rhog, S.ch, A.a_rh, A.a_ch, A.a_flx, a_rhog);
-  k_adj_rhoh_ch_pl<<<nbl, 128, 0, st>>>(D.kall, rhog_pl, S.ch_pl, A.a_rh_pl, A.a_ch_pl, A.a_flx_pl, a_rhog_pl);
+  // ---- the poles' density update and Courant numbers, then horizontal_flux
+  k_adj_rhoh_ch_pl<<<nbl, 128, 0, st>>>(D.kall, rhog_pl, S.flx_pl, A.a_rh_pl, A.a_ch_pl, A.a_flx_pl, a_rhog_pl);
   const Fld F{{rhog, vx, vy, vz}};
   const Fld Fp{{rhog_pl, vx_pl, vy_pl, vz_pl}};
   k_adj_tri<<<slab(D, T), T, 0, st>>>(D, S.geo, F, A.a_flx, A.a_xc, dt, A.aT);
   k_adj_fields<<<slab(D, T), T, 0, st>>>(D, S.geo.GMTR_t, A.aT, a_rhog, a_vx, a_vy, a_vz);
   k_adj_flux_pl<<<nbl, 128, 0, st>>>(D.kall, S.geo, Fp, A.a_flx_pl, A.a_xc_pl, dt, a_rhog_pl, a_vx_pl, a_vy_pl,
                                      a_vz_pl);
-  launches += 5;
+  launches += 4;
   return ICA_OK;
 }
 

@@ -7,13 +7,12 @@ namespace icoadv {
 
 // Device scratch of one adjoint step, besides the forward scratch of StepCtx.
 struct AdjScratch {
-  double *rh, *rh_pl;          // rhog after the horizontal sub-step
-  double *qa1, *qa1_pl;        // limited face values of the current tracer
-  double *Qh, *Qh_pl;          // rhogq after the horizontal sub-step, current tracer
-  double *a_q, *a_q_pl;        // adjoint of q = rhogq / rhog, current tracer
-  double *aT;                  // triangle adjoints of horizontal_flux (8 fields; aliases qa1 | Qh | a_q)
-  double *a_flx, *a_flx_pl, *a_xc, *a_xc_pl, *a_ch, *a_ch_pl, *a_rh, *a_rh_pl;
-  double *a_gr, *a_gr_pl, *a_qo, *a_qo_pl;
+  double *rh, *rh_pl;      // rhog after the horizontal sub-step
+  // a group of tracers: rhogq after the horizontal sub-step (poles), the adjoint of q = rhogq / rhog
+  // (a_q holds rhogq after the horizontal sub-step until the column pass has read it) and of bb
+  double *Qh_pl, *a_q, *a_q_pl, *a_bb;
+  double *aT;              // triangle adjoints of horizontal_flux (8 fields, over a_q)
+  double *a_flx, *a_flx_pl, *a_xc, *a_xc_pl, *a_ch_pl, *a_rh, *a_rh_pl;
 };
 
 // One adjoint step.  In: the step's input state (rhog, rhogq and their pole

@@ -619,25 +619,11 @@ int Ctx::step_ctx(StepCtx &S) {
     const char *name;
     size_t n;
   } bl[] = {{&S.flx, "st_flx", n3 * 6}, {&S.flx_pl, "st_flxp", n3p}, {&S.xc, "st_xc", n3 * 9},
-            {&S.xc_pl, "st_xcp", n3p * 3}, {&S.fv, "st_work", n3 * 3 * kPlainGroup}, {&S.ch_pl, "st_chp", n3p},
-            {&S.cm_pl, "st_cmp", n3p}, {&S.zero, "st_zero", n3},
-            {&S.zero_pl, "st_zerop", n3p}, {&S.q_pl, "st_qp", n3p},
-            {&S.grad_pl, "st_gradp", n3p * 3},
-            {&S.qa_pl, "st_qap", n3p}, {&S.qout_pl, "st_qoutp", n3p * 2},
-            {&S.qin_pl, "st_qinp", n3p * 4},
+            {&S.xc_pl, "st_xcp", n3p * 3}, {&S.fv, "st_fv", n3 * 3 * kPlainGroup},
             {&S.bb, "st_bb", (size_t)kPlainGroup * sz.kall * fast.nb * 5}};
-  bool fresh_zero = bufs.find("st_zero") == bufs.end();
   for (auto &b : bl) {
     *b.p = (double *)buf(b.name, b.n * sizeof(double));
     if (!*b.p) return set_error(std::string("cudaMalloc ") + b.name), ICA_ERR_NOMEM;
-  }
-  // the adjoint's fields of one tracer share the face values' memory: 24 fields
-  static_assert(3 * kPlainGroup == 24, "ch 6, cm 6, q 1, grad 3, qa 6, qout 2");
-  S.ch = S.fv, S.cm = S.fv + 6 * n3, S.q = S.fv + 12 * n3, S.grad = S.fv + 13 * n3, S.qa = S.fv + 16 * n3;
-  S.qout = S.fv + 22 * n3;
-  if (fresh_zero) {
-    cudaMemsetAsync(S.zero, 0, n3 * sizeof(double), stream);
-    cudaMemsetAsync(S.zero_pl, 0, n3p * sizeof(double), stream);
   }
   return ICA_OK;
 }
@@ -733,20 +719,18 @@ static int adj_scratch(Ctx *c, AdjScratch &A) {
     double **p;
     const char *name;
     size_t n;
-  } bl[] = {{&A.rh, "adj_rh", n3},         {&A.rh_pl, "adj_rhp", n3p},     {&A.qa1, "adj_tr", 8 * n3},
-            {&A.qa1_pl, "adj_qa1p", n3p},  {&A.Qh_pl, "adj_Qhp", n3p},     {&A.a_q_pl, "adj_aqp", n3p},
+  } bl[] = {{&A.rh, "adj_rh", n3}, {&A.rh_pl, "adj_rhp", n3p},
+            {&A.a_q, "adj_aq", kPlainGroup * n3}, {&A.a_q_pl, "adj_aqp", kPlainGroup * n3p},
+            {&A.Qh_pl, "adj_Qhp", kPlainGroup * n3p}, {&A.a_bb, "adj_abb", (size_t)kPlainGroup * c->sz.kall * c->fast.nb * 5},
             {&A.a_flx, "adj_aflx", 6 * n3}, {&A.a_flx_pl, "adj_aflxp", n3p}, {&A.a_xc, "adj_axc", 9 * n3},
-            {&A.a_xc_pl, "adj_axcp", 3 * n3p}, {&A.a_ch, "adj_ach", 6 * n3}, {&A.a_ch_pl, "adj_achp", n3p},
-            {&A.a_rh, "adj_arh", n3},      {&A.a_rh_pl, "adj_arhp", n3p},  {&A.a_gr, "adj_agr", 3 * n3},
-            {&A.a_gr_pl, "adj_agrp", 3 * n3p}, {&A.a_qo, "adj_aqo", 2 * n3}, {&A.a_qo_pl, "adj_aqop", 2 * n3p}};
+            {&A.a_xc_pl, "adj_axcp", 3 * n3p}, {&A.a_ch_pl, "adj_achp", n3p},
+            {&A.a_rh, "adj_arh", n3}, {&A.a_rh_pl, "adj_arhp", n3p}};
   for (auto &b : bl) {
     *b.p = (double *)c->buf(b.name, b.n * sizeof(double));
     if (!*b.p) return set_error(std::string("cudaMalloc ") + b.name), ICA_ERR_NOMEM;
   }
-  // qa1 | Qh | a_q are one block, reused as the 8 triangle-adjoint fields after the tracers
-  A.Qh = A.qa1 + 6 * n3;
-  A.a_q = A.qa1 + 7 * n3;
-  A.aT = A.qa1;
+  static_assert(kPlainGroup == 8, "the 8 triangle-adjoint fields reuse a_q after the tracers");
+  A.aT = A.a_q;
   return ICA_OK;
 }
 
@@ -798,7 +782,7 @@ int ica_advect_step_adjoint_dev(ica_ctx *c, int ntr, double dt, const double *rh
   rc = step_adjoint(S, A, ntr, dt, rhog, rhog_pl, rhogq, rhogq_pl, vx, vx_pl, vy, vy_pl, vz, vz_pl, w, w_pl, a_rhog,
                     a_rhog_pl, a_rhogq, a_rhogq_pl, a_vx, a_vx_pl, a_vy, a_vy_pl, a_vz, a_vz_pl, c->stream,
                     c->launches);
-  if (rc) return set_error("ica_advect_step_adjoint: bad vertical grid"), rc;
+  if (rc) return rc;
   return c->check_launch("ica_advect_step_adjoint");
 }
 
@@ -899,7 +883,7 @@ int ica_adjoint_sweep(ica_ctx *c, const double *vx, const double *vx_pl, const d
       rc = step_adjoint(S, A, T.ntr, T.dt, st[u].r, st[u].rp, st[u].q, st[u].qp, vx, vx_pl, vy, vy_pl, vz, vz_pl, w,
                         w_pl, a_rhog, a_rhog_pl, a_rhogq, a_rhogq_pl, a_vx, a_vx_pl, a_vy, a_vy_pl, a_vz, a_vz_pl,
                         c->stream, c->launches);
-      if (rc) return set_error("ica_adjoint_sweep: bad vertical grid"), rc;
+      if (rc) return rc;
     }
   }
   return c->check_launch("ica_adjoint_sweep");
@@ -909,9 +893,8 @@ int ica_adjoint_release(ica_ctx *c) {
   CTX_OK(c);
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  for (const char *n : {"adj_ckpt", "adj_seg", "adj_rh", "adj_rhp", "adj_tr", "adj_qa1p", "adj_Qhp", "adj_aqp",
-                        "adj_aflx", "adj_aflxp", "adj_axc", "adj_axcp", "adj_ach", "adj_achp", "adj_arh", "adj_arhp",
-                        "adj_agr", "adj_agrp", "adj_aqo", "adj_aqop"})
+  for (const char *n : {"adj_ckpt", "adj_seg", "adj_rh", "adj_rhp", "adj_aq", "adj_aqp", "adj_Qhp", "adj_abb",
+                        "adj_aflx", "adj_aflxp", "adj_axc", "adj_axcp", "adj_achp", "adj_arh", "adj_arhp"})
     c->release(n);
   c->tape = AdjTape{};
   return ICA_OK;

@@ -1,8 +1,7 @@
 // The composed tracer step, plain FP64 path: the reference kernels' operations
 // with the pieces the reference leaves out (Courant numbers, gradient, remap,
 // rhogq update, vertical flux), fused into three launches per group of tracers
-// (below).  The one-kernel-per-piece forms that come first serve the adjoint's
-// recompute.  The FP32 / FP64 batched path is fast_kernels.cu.
+// (below).  The FP32 / FP64 batched path is fast_kernels.cu.
 //
 // The composition (horizontal sub-step, then vertical sub-step, then the halo
 // fill of the state) and every formula match the CPU oracle's definition of
@@ -22,138 +21,9 @@
 #include <cfloat>
 #include <type_traits>
 
-#include "quotients.cuh"
-#include "step.cuh"
+#include "plain_cells.cuh"
 
 namespace icoadv {
-
-__device__ __forceinline__ double sgn(double a, double b) { return copysign(fabs(a), b); }
-
-// ch, cmask for every (face, cell, level, region); poles: ring faces v = 2..6, ch(1) = 0
-__global__ void k_courant(int n3, const double *flx, const double *rho, double *ch, double *cm) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 6LL * n3) return;
-  const double c = flx[t] / rho[t % n3];
-  ch[t] = c;
-  cm[t] = 0.5 - sgn(0.5, c - DBL_EPSILON);
-}
-__global__ void k_courant_pl(int kall, const double *flx_pl, const double *rho_pl, double *ch_pl, double *cm_pl) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kLallPl * kall * kGallPl) return;
-  const int v = t % kGallPl, kl = t / kGallPl;
-  const double c = (v == 0) ? 0.0 : flx_pl[t] / rho_pl[kl * kGallPl];
-  ch_pl[t] = c;
-  cm_pl[t] = 0.5 - sgn(0.5, c - DBL_EPSILON);
-}
-
-// q = rhogq / rhog (regions and poles in one launch)
-__global__ void k_divide(long long n3, int n3p, const double *Q, const double *rho, const double *Qp,
-                         const double *rhop, double *q, double *qp) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n3) q[t] = Q[t] / rho[t];
-  else if (t < n3 + n3p) qp[t - n3] = Qp[t - n3] / rhop[t - n3];
-}
-
-// gradient at interior cells, 0 elsewhere; coef_grad(gall,0:6,3,lall)
-__global__ void k_gradient(Dims D, const double *q, const double *cg, double *grad) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
-  const int i = c % G + 1, j = c / G + 1;
-  const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall;
-  if (i < D.gmin || i > D.gmax || j < D.gmin || j > D.gmax) {
-    for (int x = 0; x < 3; ++x) grad[x * fs + off + c] = 0.0;
-    return;
-  }
-  const int nb[7] = {c, c + 1, c + G + 1, c + G, c - 1, c - G - 1, c - G};
-  const double *qs = q + off;
-  for (int x = 0; x < 3; ++x) {
-    const double *cx = cg + ((size_t)l * 3 + x) * 7 * D.gall + c;
-    double s = cx[0] * qs[nb[0]];
-    for (int n = 1; n <= 6; ++n) s = s + cx[(size_t)n * D.gall] * qs[nb[n]];
-    grad[x * fs + off + c] = s;
-  }
-}
-__global__ void k_gradient_pl(int kall, const double *q_pl, const double *cg_pl, double *grad_pl) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kLallPl * kall) return;
-  const int l = t / kall;
-  const size_t off = (size_t)t * kGallPl, fsp = (size_t)kLallPl * kall * kGallPl;
-  for (int x = 0; x < 3; ++x) {
-    const double *cx = cg_pl + ((size_t)l * 3 + x) * 6;
-    double s = cx[0] * q_pl[off];
-    for (int v = 2; v <= 6; ++v) s = s + cx[v - 1] * q_pl[off + v - 1];
-    for (int v = 0; v < kGallPl; ++v) grad_pl[x * fsp + off + v] = (v == 0) ? s : 0.0;
-  }
-}
-
-// upwind remap of the three faces attached to (i,j) in [gmin-1,gmax]^2
-__global__ void k_remap(Dims D, const double *q, const double *grad, const double *cm, const double *xc,
-                        const double *GRD_x, double *qa) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
-  const int i = c % G + 1, j = c / G + 1;
-  if (i < D.gmin - 1 || i > D.gmax || j < D.gmin - 1 || j > D.gmax) return;
-  const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall;
-  const size_t gw = (size_t)D.lall * D.gall;
-  const int nbs[4] = {0, c + 1, c + G + 1, c + G};
-  for (int m = 1; m <= 3; ++m) {
-    const int nb = nbs[m];
-    const double cc = cm[(size_t)(m - 1) * fs + off + c];
-    double vu = q[off + nb], vs = q[off + c];
-    for (int x = 0; x < 3; ++x) {
-      const double xcv = xc[((size_t)x * 3 + (m - 1)) * fs + off + c];
-      vu = vu + grad[x * fs + off + nb] * (xcv - GRD_x[x * gw + (size_t)l * D.gall + nb]);
-    }
-    for (int x = 0; x < 3; ++x) {
-      const double xcv = xc[((size_t)x * 3 + (m - 1)) * fs + off + c];
-      vs = vs + grad[x * fs + off + c] * (xcv - GRD_x[x * gw + (size_t)l * D.gall + c]);
-    }
-    const double v = cc * vu + (1.0 - cc) * vs;
-    qa[(size_t)(m - 1) * fs + off + c] = v;
-    qa[(size_t)(m + 2) * fs + off + nb] = v;
-  }
-}
-__global__ void k_remap_pl(int kall, const double *q_pl, const double *grad_pl, const double *cm_pl,
-                           const double *xc_pl, const double *GRD_x_pl, double *qa_pl) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kLallPl * kall * kGallPl) return;
-  const int v = t % kGallPl, kl = t / kGallPl, l = kl / kall;
-  const size_t off = (size_t)kl * kGallPl, fsp = (size_t)kLallPl * kall * kGallPl;
-  if (v == 0) {
-    qa_pl[off] = 0.0;
-    return;
-  }
-  const double cc = cm_pl[off + v];
-  double vu = q_pl[off + v], vs = q_pl[off];
-  for (int x = 0; x < 3; ++x)
-    vu = vu + grad_pl[x * fsp + off + v] * (xc_pl[x * fsp + off + v] - GRD_x_pl[((size_t)x * kLallPl + l) * kGallPl + v]);
-  for (int x = 0; x < 3; ++x)
-    vs = vs + grad_pl[x * fsp + off] * (xc_pl[x * fsp + off + v] - GRD_x_pl[((size_t)x * kLallPl + l) * kGallPl]);
-  qa_pl[off + v] = cc * vu + (1.0 - cc) * vs;
-}
-
-// rhog -= sum_m flx_h(m)
-__global__ void k_update_rho(Dims D, const double *flx, double *rho) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, G = D.gall_1d;
-  const int i = c % G + 1, j = c / G + 1;
-  if (i < D.gmin || i > D.gmax || j < D.gmin || j > D.gmax) return;
-  const size_t off = (size_t)kl * D.gall + c, fs = (size_t)D.lall * D.kall * D.gall;
-  double s = flx[off];
-  for (int m = 1; m < 6; ++m) s = s + flx[m * fs + off];
-  rho[off] = rho[off] - s;
-}
-__global__ void k_update_rho_pl(int kall, const double *flx_pl, double *rho_pl) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kLallPl * kall) return;
-  const size_t off = (size_t)t * kGallPl;
-  double s = flx_pl[off + 1];
-  for (int v = 3; v <= 6; ++v) s = s + flx_pl[off + v - 1];
-  rho_pl[off] = rho_pl[off] - s;
-}
 
 // ---------------------------------------------------------------------------
 // The step itself: the tracers go through in groups of up to kPlainGroup, three launches a group.
@@ -177,34 +47,6 @@ __global__ void k_update_rho_pl(int kall, const double *flx_pl, double *rho_pl) 
 // (c a + (1 - c) b), the chosen side is taken, which is the same number.
 constexpr int kTileCells = 256;  // threads of k_plain_cells: one per cell of a TX x (256 / TX) tile
 constexpr int kCellBlocks = 2;   // its blocks per SM: 128 registers a thread, which hold one tracer's values
-
-struct PlainArgs {
-  Dims D;
-  int nt, nb, ns;                    // tracers of the group; boundary entries, seam faces
-  double dt;
-  double *Q, *Qp;                    // the group's rhogq
-  const double *rho, *rhop, *w, *wp, *flx, *flxp, *xc, *xcp;
-  const double *GRD_x, *GRD_xp, *cg, *cgp, *rdgz, *afact, *bfact;
-  const int *bsrc, *seam, *ring;     // boundary entry of a point, seam face codes, pole ring's entries
-  double *fv;                        // (nt, 3, lall, kall, gall): limited values of faces AI, AIJ, AJ of their owner
-  double *bb;                        // (nt, kall, nb, 5): gradient x/y/z, Qout min / max
-  __device__ size_t n3() const { return (size_t)D.lall * D.kall * D.gall; }
-  __device__ size_t n3p() const { return (size_t)kLallPl * D.kall * kGallPl; }
-  __device__ double *bval(int t, int k, int b) const { return bb + (((size_t)t * D.kall + k) * nb + b) * 5; }
-  __device__ bool inner(int i, int j) const { return i >= D.gmin && i <= D.gmax && j >= D.gmin && j <= D.gmax; }
-};
-
-__device__ __forceinline__ double mn(double a, double b) { return (b < a) ? b : a; }
-__device__ __forceinline__ double mx(double a, double b) { return (b > a) ? b : a; }
-__device__ __forceinline__ double mn4(double a, double b, double c, double d) { return mn(mn(mn(a, b), c), d); }
-__device__ __forceinline__ double mx4(double a, double b, double c, double d) { return mx(mx(mx(a, b), c), d); }
-// cmask of the Courant number f / r: true where it is 1 (the face's neighbour is its upwind cell),
-// which is where the rounded quotient is below EPS.  EPS is a power of two, so for an ordinary
-// density that is f < EPS r, without the division.
-__device__ __forceinline__ bool upmask(double f, double r) {
-  if (r >= 0x1p-900) return f < DBL_EPSILON * r;
-  return 0.5 - sgn(0.5, f / r - DBL_EPSILON) != 0.0;
-}
 
 // pole centre (p, k) of tracer t: gradient and Qout (mod_src_tracer.f90:307-367) into bb
 __device__ __forceinline__ void pole_centre(const PlainArgs &P, int t, int p, int k) {
@@ -238,18 +80,6 @@ __device__ __forceinline__ void pole_centre(const PlainArgs &P, int t, int p, in
   o[4] = (q[0] - CQmin - qnmin * (1.0 - Cin - Cout + dn)) / (Cout + zsw) * (1.0 - zsw) + q[0] * zsw;
 }
 
-template <int TX>
-struct CellSmem {
-  static constexpr int TY = kTileCells / TX, WW = TX + 2, NW = WW * (TY + 2);  // window: the tile and one ring
-  static constexpr int OW = TX + 1, NO = OW * (TY + 1);                        // owners of the tile's faces
-  double cg[21][kTileCells];
-  // xc of the face [face * 3 + x][owner]; its upwind cell's thread turns it into xc - x(upwind cell)
-  // and is the one that reads it
-  double disp[9][NO];
-  double rho[NW], y[NW];  // rhog and its reciprocal
-  double q[2][NW];
-};
-
 // Bound by instruction issue (FP64 compare-and-selects of the bounds, then the gradient): 1.62 ms
 // of the 3.61.  One tracer per pass of the loop and two blocks per SM keep every value in
 // registers; two tracers, or three blocks, spill and take 2.5-2.6 ms.
@@ -257,7 +87,8 @@ struct CellSmem {
 // after the first), then the pole centres
 template <int TX>
 __global__ void __launch_bounds__(kTileCells, kCellBlocks) k_plain_cells(PlainArgs P, int ntx, int nty, int nlb, int lpb) {
-  using S = CellSmem<TX>;
+  using Tile = CellTile<TX, kTileCells>;
+  using S = typename Tile::Smem;
   extern __shared__ __align__(16) unsigned char raw[];
   S &s = *reinterpret_cast<S *>(raw);
   const Dims &D = P.D;
@@ -268,214 +99,67 @@ __global__ void __launch_bounds__(kTileCells, kCellBlocks) k_plain_cells(PlainAr
     if (u < P.nt * kLallPl * D.kall) pole_centre(P, u / (kLallPl * D.kall), u / D.kall % kLallPl, u % D.kall);
     return;
   }
-  const int lb = (int)blockIdx.x % nlb, tile = (int)blockIdx.x / nlb;
-  const int l = tile / (ntx * nty), tr = tile % (ntx * nty);
-  const int i0 = D.gmin + (tr % ntx) * TX, j0 = D.gmin + (tr / ntx) * S::TY;  // first cell, 1-based
-  const int x = tid % TX, y = tid / TX, i = i0 + x, j = j0 + y;
-  // regions 32 or more cells wide are whole tiles; in a smaller one a thread without a cell works on
-  // the region's last cell and stores nothing
-  const bool act = TX == 32 || (i <= D.gmax && j <= D.gmax);
-  const int ci = TX == 32 ? i : min(i, D.gmax), cj = TX == 32 ? j : min(j, D.gmax);
-  const int c = (cj - 1) * G + (ci - 1);
-  const bool sing = D.have_sgp[l] != 0 && ci == D.gmin && cj == D.gmin;
-  const int bs = act ? P.bsrc[(size_t)l * D.gall + c] : -1;
-  const size_t n3 = P.n3(), gw = (size_t)D.lall * D.gall;
-#pragma unroll
-  for (int n = 0; n < 21; ++n) s.cg[n][tid] = P.cg[((size_t)l * 21 + n) * D.gall + c];
-  // this thread's window slots and their cells (-1: none)
-  constexpr int NSLOT = (S::NW + kTileCells - 1) / kTileCells;
-  int wc[NSLOT];
-#pragma unroll
-  for (int r = 0; r < NSLOT; ++r) {
-    const int e = tid + r * kTileCells, wi = i0 - 1 + e % S::WW, wj = j0 - 1 + e / S::WW;  // >= 1
-    wc[r] = (e < S::NW && wi <= G && wj <= G) ? (wj - 1) * G + (wi - 1) : -1;
-  }
-  // owner slots of the faces: this cell's, and for the first threads one of the row and column
-  // before the tile
-  const int cx = ci - i0, cy = cj - j0;
-  const int ew = (cy + 1) * S::WW + cx + 1, ow = (cy + 1) * S::OW + cx + 1;
-  const int wn[7] = {ew, ew + 1, ew + S::WW + 1, ew + S::WW, ew - 1, ew - S::WW - 1, ew - S::WW};
-  int oslot = -1, ocell = 0;
-  if (tid < TX + S::TY + 1) {
-    const int ox = tid <= TX ? tid - 1 : -1, oy = tid <= TX ? -1 : tid - TX - 1;
-    if (i0 + ox <= D.gmax && j0 + oy <= D.gmax)
-      oslot = (oy + 1) * S::OW + ox + 1, ocell = (j0 + oy - 1) * G + (i0 + ox - 1);
-  }
-  unsigned both = 0;  // bit m: the cell across face m is interior too (not a seam face)
-  {
-    constexpr int DX[7] = {0, 1, 1, 0, -1, -1, 0}, DY[7] = {0, 0, 1, 1, 0, -1, -1};
-#pragma unroll
-    for (int m = 1; m <= 6; ++m) both |= act && P.inner(ci + DX[m], cj + DY[m]) ? 1u << m : 0u;
-  }
-  const double X[3] = {P.GRD_x[(size_t)l * D.gall + c], P.GRD_x[gw + (size_t)l * D.gall + c],
-                       P.GRD_x[2 * gw + (size_t)l * D.gall + c]};
+  const int lb = (int)blockIdx.x % nlb;
+  Tile T;
+  T.init(P, s, (int)blockIdx.x / nlb, ntx, nty);
+  const int c = T.c;
+  const size_t n3 = P.n3();
   const int kfirst = D.kmin - 1, kend = D.kmax;  // physical levels, 0-based
   const int k0 = kfirst + lb * lpb, k1 = min(k0 + lpb, kend);
   for (int k = k0; k < k1; ++k) {
-    const size_t off = ((size_t)l * D.kall + k) * D.gall;
-    double Qw[NSLOT][1];
+    const size_t off = ((size_t)T.l * D.kall + k) * D.gall;
+    double Qw[Tile::NSLOT][1];
     auto load = [&](int t) {
       const double *Qs = P.Q + (size_t)t * n3 + off;
 #pragma unroll
-      for (int r = 0; r < NSLOT; ++r)
-        if (wc[r] >= 0) Qw[r][0] = Qs[wc[r]];
+      for (int r = 0; r < Tile::NSLOT; ++r)
+        if (T.wc[r] >= 0) Qw[r][0] = Qs[T.wc[r]];
     };
-    // ---- every global load of the level's set-up before the first wait
-    load(0);
-    double ch[6], fo[3], rv[NSLOT];
-    const double *flx = P.flx + off;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) ch[m] = (flx + m * n3)[c];
-    fo[0] = flx[c - 1], fo[1] = (flx + n3)[c - G - 1], fo[2] = (flx + 2 * n3)[c - G];  // owners of faces 4-6
-#pragma unroll
-    for (int r = 0; r < NSLOT; ++r) rv[r] = wc[r] >= 0 ? P.rho[off + wc[r]] : 1.0;
-    __syncthreads();  // the previous level's shared data is read
-    {
-      const double *xc = P.xc + off;
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          if (act) s.disp[a * 3 + d][ow] = (xc + (d * 3 + a) * n3)[c];
-          if (oslot >= 0) s.disp[a * 3 + d][oslot] = (xc + (d * 3 + a) * n3)[ocell];
-        }
-    }
-    Recip rw[NSLOT];
-#pragma unroll
-    for (int r = 0; r < NSLOT; ++r) {
-      rw[r] = recip(rv[r]);
-      if (wc[r] >= 0) s.rho[tid + r * kTileCells] = rv[r], s.y[tid + r * kTileCells] = rw[r].y;
-    }
-    __syncthreads();
-    // ---- tracer-independent: Courant numbers, upwind sides, outflow sums, displacements
-    double chm[7], omc;
-    Recip den;
-    unsigned in = 0, out = 0;
-    bool odd = false;  // an inflow Courant number at a face whose mask says outflow (rounding-level fluxes)
-    bool zsw;
-    {
-      const double rc = s.rho[ew];
-#pragma unroll
-      for (int m = 1; m <= 6; ++m) {
-        // the owner's mask: 1 takes the owner's neighbour as the upwind cell
-        const bool cm = (m <= 3) ? upmask(ch[m - 1], rc) : upmask(fo[m - 4], s.rho[wn[m]]);
-        if (cm == (m <= 3)) in |= 1u << m;
-        else if ((both >> m) & 1u) out |= 1u << m;
-      }
-      quotients(ch, Recip{rc, s.y[ew], recip_ok(rc)});
-#pragma unroll
-      for (int m = 1; m <= 6; ++m) {
-        chm[m] = mn(ch[m - 1], 0.0);
-        odd = odd || (!((in >> m) & 1u) && chm[m] != 0.0);
-      }
-      const double Cin = chm[1] + chm[2] + chm[3] + chm[4] + chm[5] + chm[6];
-      const double Cout = ch[0] - chm[1] + ch[1] - chm[2] + ch[2] - chm[3] + ch[3] - chm[4] + ch[4] - chm[5] + ch[5] -
-                          chm[6];
-      const double dv = 0.0, z = 0.5 - sgn(0.5, fabs(Cout) - DBL_EPSILON);
-      zsw = z != 0.0;
-      den = recip(Cout + z);
-      omc = 1.0 - Cin - Cout + dv;
-    }
-    // Of two opposite faces a and a + 3 a cell usually has one outflow face: sl / st are its owner's
-    // slot and cell (a's own where neither flows out; st < 0 then).  Cells with both go through the
-    // second one again below (again).
-    int sl[3], st[3];
-    unsigned side = 0, again = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const int so = ow - (a == 0 ? 1 : (a == 1 ? S::OW + 1 : S::OW)), sc = c - (a == 0 ? 1 : (a == 1 ? G + 1 : G));
-      const bool o1 = (out >> (a + 1)) & 1u, o2 = (out >> (a + 4)) & 1u;
-      if (!o1 && o2) side |= 1u << a;
-      if (o1 && o2) again |= 1u << a;
-      sl[a] = (!o1 && o2) ? so : ow;
-      st[a] = o1 ? c : (o2 ? sc : -1);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        if (o1 || o2) s.disp[a * 3 + d][sl[a]] -= X[d];
-        if (o1 && o2) s.disp[a * 3 + d][so] -= X[d];
-      }
-    }
+    load(0);  // with the level's other global loads, before the first wait
+    Recip rw[Tile::NSLOT];
+    CellFlow F;
+    double flx[6];
+    T.level(P, s, off, rw, F, flx);
     // ---- the tracers; their q alternates between two buffers
     for (int t = 0; t < P.nt; ++t) {
       const int b = t & 1;
 #pragma unroll
-      for (int r = 0; r < NSLOT; ++r)
-        if (wc[r] >= 0) {
+      for (int r = 0; r < Tile::NSLOT; ++r)
+        if (T.wc[r] >= 0) {
           quotients(Qw[r], rw[r]);
           s.q[b][tid + r * kTileCells] = Qw[r][0];
         }
       if (t + 1 < P.nt) load(t + 1);
       __syncthreads();
-      const double c0 = s.q[b][wn[0]], n1 = s.q[b][wn[1]], n2 = s.q[b][wn[2]], n3v = s.q[b][wn[3]], n4 = s.q[b][wn[4]],
-                   n5 = s.q[b][wn[5]], n6 = s.q[b][wn[6]];
-      const double n[7] = {c0, n1, n2, n3v, n4, n5, n6};
-      double g[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        g[d] = s.cg[d * 7][tid] * n[0];
-#pragma unroll
-        for (int m = 1; m < 7; ++m) g[d] = g[d] + s.cg[d * 7 + m][tid] * n[m];
-      }
-      // 4-point bounds of the six faces (mod_src_tracer.f90:152-214): the cell and three
-      // consecutive neighbours, of which each pair is compared once
-      const double l12 = mn(n1, n2), l34 = mn(n3v, n4), l56 = mn(n5, n6);
-      const double h12 = mx(n1, n2), h34 = mx(n3v, n4), h56 = mx(n5, n6);
-      double lo[7], hi[7];
-      lo[1] = mn(c0, mn(n6, l12)), hi[1] = mx(c0, mx(n6, h12));
-      lo[2] = mn(c0, mn(l12, n3v)), hi[2] = mx(c0, mx(h12, n3v));
-      lo[3] = mn(c0, mn(n2, l34)), hi[3] = mx(c0, mx(n2, h34));
-      lo[4] = mn(c0, mn(l34, n5)), hi[4] = mx(c0, mx(h34, n5));
-      lo[5] = mn(c0, mn(n4, l56)), hi[5] = mx(c0, mx(n4, h56));
-      lo[6] = mn(c0, mn(l56, n1)), hi[6] = mx(c0, mx(h56, n1));
-      if (sing) lo[5] = mn4(n5, c0, n1, n4), hi[5] = mx4(n5, c0, n1, n4);  // the singular point's shifted stencil
-      // Qout (:219-282, d = 0).  An outflow face's +-BIG bound never binds, and its term of CQ is
-      // zero with its Courant number, except at an odd face
-      double qnmin = c0, qnmax = c0, CQmin = chm[1] * lo[1], CQmax = chm[1] * hi[1];
-#pragma unroll
-      for (int m = 1; m <= 6; ++m) {
-        const bool f = (in >> m) & 1u;
-        qnmin = (f && lo[m] < qnmin) ? lo[m] : qnmin;
-        qnmax = (f && hi[m] > qnmax) ? hi[m] : qnmax;
-        if (m > 1) CQmin = CQmin + chm[m] * lo[m], CQmax = CQmax + chm[m] * hi[m];
-      }
-      if (odd) {
-#pragma unroll
-        for (int m = 1; m <= 6; ++m) {
-          const bool f = (in >> m) & 1u;
-          const double tmin = chm[m] * (f ? lo[m] : DBL_MAX), tmax = chm[m] * (f ? hi[m] : -DBL_MAX);
-          CQmin = (m == 1) ? tmin : CQmin + tmin;
-          CQmax = (m == 1) ? tmax : CQmax + tmax;
-        }
-      }
-      double Qo[2] = {c0 - CQmax - qnmax * omc, c0 - CQmin - qnmin * omc};
-      quotients(Qo, den);
-      const double Qmin = zsw ? c0 : Qo[0], Qmax = zsw ? c0 : Qo[1];
+      double n[7], g[3];
+      T.gradient(s, b, n, g);
+      CellLimits L;
+      cell_limits(n, F, T.sing, L);
       double *fv = P.fv + (size_t)t * 3 * n3 + off;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        const bool f = (side >> a) & 1u;
-        double v = c0;
+        const bool f = (F.side >> a) & 1u;
+        double v = n[0];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) v = v + g[d] * s.disp[a * 3 + d][sl[a]];
-        v = mn(mx(v, f ? lo[a + 4] : lo[a + 1]), f ? hi[a + 4] : hi[a + 1]);
-        v = mx(mn(v, Qmax), Qmin);
-        if (st[a] >= 0) (fv + a * n3)[st[a]] = v;
+        for (int d = 0; d < 3; ++d) v = v + g[d] * s.disp[a * 3 + d][F.sl[a]];
+        v = mn(mx(v, f ? L.lo[a + 4] : L.lo[a + 1]), f ? L.hi[a + 4] : L.hi[a + 1]);
+        v = mx(mn(v, L.Qmax), L.Qmin);
+        if (F.st[a] >= 0) (fv + a * n3)[F.st[a]] = v;
       }
-      if (again) {
+      if (F.again) {
 #pragma unroll
         for (int a = 0; a < 3; ++a)
-          if ((again >> a) & 1u) {
-            const int so = a == 0 ? 1 : (a == 1 ? S::OW + 1 : S::OW), sc = a == 0 ? 1 : (a == 1 ? G + 1 : G);
-            double v = c0;
+          if ((F.again >> a) & 1u) {
+            double v = n[0];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) v = v + g[d] * s.disp[a * 3 + d][ow - so];
-            v = mn(mx(v, lo[a + 4]), hi[a + 4]);
-            (fv + a * n3)[c - sc] = mx(mn(v, Qmax), Qmin);
+            for (int d = 0; d < 3; ++d) v = v + g[d] * s.disp[a * 3 + d][T.ow - Tile::slot_back(a)];
+            v = mn(mx(v, L.lo[a + 4]), L.hi[a + 4]);
+            (fv + a * n3)[c - face_step(a, G)] = mx(mn(v, L.Qmax), L.Qmin);
           }
       }
-      if (bs >= 0) {
-        double *o = P.bval(t, k, bs);
-        o[0] = g[0], o[1] = g[1], o[2] = g[2], o[3] = Qmin, o[4] = Qmax;
+      if (T.bs >= 0) {
+        double *o = P.bval(t, k, T.bs);
+        o[0] = g[0], o[1] = g[1], o[2] = g[2], o[3] = L.Qmin, o[4] = L.Qmax;
       }
     }
   }
@@ -810,49 +494,13 @@ __global__ void k_plain_rho(Dims D, double dt, const double *flx, const double *
 }
 
 // ---------------------------------------------------------------------------
-static dim3 slab(const Dims &D, int th) { return dim3((D.gall + th - 1) / th, D.kall * D.lall); }
-static constexpr int kSlabThreads = 128;
-
 static size_t n3_of(const Dims &D) { return (size_t)D.gall * D.kall * D.lall; }
 static size_t n3p_of(const Dims &D) { return (size_t)kGallPl * D.kall * kLallPl; }
-
-void launch_courant(const StepCtx &S, const double *rhog, const double *rhog_pl, cudaStream_t st) {
-  const size_t n3 = n3_of(S.D), n3p = n3p_of(S.D);
-  k_courant<<<(unsigned)((6 * n3 + 255) / 256), 256, 0, st>>>((int)n3, S.flx, rhog, S.ch, S.cm);
-  k_courant_pl<<<(unsigned)((n3p + 255) / 256), 256, 0, st>>>(S.D.kall, S.flx_pl, rhog_pl, S.ch_pl, S.cm_pl);
-}
-
-void launch_divide(const StepCtx &S, const double *Q, const double *Qp, const double *rhog, const double *rhog_pl,
-                   cudaStream_t st) {
-  const size_t n3 = n3_of(S.D), n3p = n3p_of(S.D);
-  k_divide<<<(unsigned)((n3 + n3p + 255) / 256), 256, 0, st>>>((long long)n3, (int)n3p, Q, rhog, Qp, rhog_pl, S.q,
-                                                               S.q_pl);
-}
-
-void launch_gradient(const StepCtx &S, cudaStream_t st) {
-  const Dims &D = S.D;
-  k_gradient<<<slab(D, kSlabThreads), kSlabThreads, 0, st>>>(D, S.q, S.cg, S.grad);
-  k_gradient_pl<<<(unsigned)((kLallPl * D.kall + 255) / 256), 256, 0, st>>>(D.kall, S.q_pl, S.cg_pl, S.grad_pl);
-  launch_gather<double>(D, S.plan.n, S.plan.dst, S.plan.src, D.kall, 3, S.grad, S.grad_pl, st);
-}
-
-void launch_remap(const StepCtx &S, cudaStream_t st) {
-  const Dims &D = S.D;
-  k_remap<<<slab(D, kSlabThreads), kSlabThreads, 0, st>>>(D, S.q, S.grad, S.cm, S.xc, S.GRD_x, S.qa);
-  k_remap_pl<<<(unsigned)((n3p_of(D) + 255) / 256), 256, 0, st>>>(D.kall, S.q_pl, S.grad_pl, S.cm_pl, S.xc_pl,
-                                                                   S.GRD_x_pl, S.qa_pl);
-}
-
-void launch_update_rho(const StepCtx &S, double *rho, double *rho_pl, cudaStream_t st) {
-  const Dims &D = S.D;
-  k_update_rho<<<slab(D, kSlabThreads), kSlabThreads, 0, st>>>(D, S.flx, rho);
-  k_update_rho_pl<<<(unsigned)((kLallPl * D.kall + 255) / 256), 256, 0, st>>>(D.kall, S.flx_pl, rho_pl);
-}
 
 template <int TX>
 static cudaError_t launch_cells(const PlainArgs &P, cudaStream_t st) {
   const Dims &D = P.D;
-  using S = CellSmem<TX>;
+  using S = typename CellTile<TX, kTileCells>::Smem;
   const int n = D.gmax - D.gmin + 1, ntx = (n + TX - 1) / TX, nty = (n + S::TY - 1) / S::TY;
   const int tiles = ntx * nty * D.lall, NK = D.kmax - D.kmin + 1;
   // up to 8 levels a block (the gradient coefficients are loaded once per block), fewer while
@@ -867,36 +515,50 @@ static cudaError_t launch_cells(const PlainArgs &P, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+PlainArgs plain_group(const StepCtx &S, int t0, int ntr, double dt, const double *rhog, const double *rhog_pl,
+                      double *rhogq, double *rhogq_pl, const double *w, const double *w_pl) {
+  const Dims &D = S.D;
+  PlainArgs P{};
+  P.D = D, P.nt = (ntr - t0 < kPlainGroup) ? ntr - t0 : kPlainGroup, P.nb = S.nb, P.ns = S.ns, P.dt = dt;
+  P.Q = rhogq + t0 * n3_of(D), P.Qp = rhogq_pl + t0 * n3p_of(D);
+  P.rho = rhog, P.rhop = rhog_pl, P.w = w, P.wp = w_pl;
+  P.flx = S.flx, P.flxp = S.flx_pl, P.xc = S.xc, P.xcp = S.xc_pl;
+  P.GRD_x = S.GRD_x, P.GRD_xp = S.GRD_x_pl, P.cg = S.cg, P.cgp = S.cg_pl;
+  P.rdgz = S.rdgz, P.afact = S.afact, P.bfact = S.bfact;
+  P.bsrc = S.bsrc, P.seam = S.seam, P.ring = S.ring;
+  P.fv = S.fv, P.bb = S.bb;
+  return P;
+}
+
+int plain_faces(const PlainArgs &P, cudaStream_t st, long long &launches) {
+  const int n = P.D.gmax - P.D.gmin + 1, NK = P.D.kmax - P.D.kmin + 1;
+  // 32 x 8 tiles need no partial tile in any region 32 or more cells wide (a region is a power of two wide)
+  const cudaError_t e = n >= 32 ? launch_cells<32>(P, st) : launch_cells<16>(P, st);
+  if (e != cudaSuccess) return set_error(std::string("advect_step: ") + cudaGetErrorString(e)), ICA_ERR_CUDA;
+  const long long ns = (long long)P.ns * NK * P.nt;
+  k_plain_seam<<<(unsigned)((ns + 127) / 128), 128, 0, st>>>(P);
+  launches += 2;
+  return ICA_OK;
+}
+
 int step_plain(StepCtx &S, int ntr, double dt, double *rhog, double *rhog_pl, double *rhogq, double *rhogq_pl,
                const double *vx, const double *vx_pl, const double *vy, const double *vy_pl, const double *vz,
                const double *vz_pl, const double *w, const double *w_pl, cudaStream_t st, long long &launches) {
   const Dims &D = S.D;
   if (D.kall > kColThreads) return set_error("advect_step: kall above 128"), ICA_ERR_ARG;
-  const size_t n3 = n3_of(D), n3p = n3p_of(D);
   FluxIn<double> fin{rhog, rhog_pl, vx, vx_pl, vy, vy_pl, vz, vz_pl};
   FluxOut<double> fout{S.flx, S.flx_pl, S.xc, S.xc_pl};
   launch_horizontal_flux<double>(D, fin, fout, S.geo, dt, st);
-  launches += 2;
+  launches += 1;
   const int n = D.gmax - D.gmin + 1, NK = D.kmax - D.kmin + 1;
   const int colblk = (n * n + kColThreads - 1) / kColThreads;  // column blocks of a region
   for (int t0 = 0; t0 < ntr; t0 += kPlainGroup) {
-    PlainArgs P{};
-    P.D = D, P.nt = (ntr - t0 < kPlainGroup) ? ntr - t0 : kPlainGroup, P.nb = S.nb, P.ns = S.ns, P.dt = dt;
-    P.Q = rhogq + t0 * n3, P.Qp = rhogq_pl + t0 * n3p;
-    P.rho = rhog, P.rhop = rhog_pl, P.w = w, P.wp = w_pl;
-    P.flx = S.flx, P.flxp = S.flx_pl, P.xc = S.xc, P.xcp = S.xc_pl;
-    P.GRD_x = S.GRD_x, P.GRD_xp = S.GRD_x_pl, P.cg = S.cg, P.cgp = S.cg_pl;
-    P.rdgz = S.rdgz, P.afact = S.afact, P.bfact = S.bfact;
-    P.bsrc = S.bsrc, P.seam = S.seam, P.ring = S.ring;
-    P.fv = S.fv, P.bb = S.bb;
-    // 32 x 8 tiles need no partial tile in any region 32 or more cells wide (a region is a power of two wide)
-    const cudaError_t e = n >= 32 ? launch_cells<32>(P, st) : launch_cells<16>(P, st);
-    if (e != cudaSuccess) return set_error(std::string("advect_step: ") + cudaGetErrorString(e)), ICA_ERR_CUDA;
-    const long long ns = (long long)P.ns * NK * P.nt;
-    k_plain_seam<<<(unsigned)((ns + 127) / 128), 128, 0, st>>>(P);
+    const PlainArgs P = plain_group(S, t0, ntr, dt, rhog, rhog_pl, rhogq, rhogq_pl, w, w_pl);
+    const int rc = plain_faces(P, st, launches);
+    if (rc) return rc;
     const int nmain = colblk * D.lall * ((P.nt + 1) / 2);
     k_plain_column<<<(unsigned)(nmain + kLallPl * P.nt), kColThreads, 0, st>>>(P, colblk, nmain);
-    launches += 3;
+    launches += 1;
   }
   const long long nr = ((long long)D.lall * n * n + kLallPl) * NK;
   k_plain_rho<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(D, dt, S.flx, S.flx_pl, w, w_pl, S.rdgz, rhog, rhog_pl);

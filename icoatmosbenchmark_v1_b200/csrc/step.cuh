@@ -17,27 +17,17 @@ struct StepCtx {
   DevPlan plan;
   const double *GRD_x, *GRD_x_pl, *cg, *cg_pl, *rdgz, *afact, *bfact;
   // shared per step
-  double *flx, *flx_pl, *xc, *xc_pl, *ch, *ch_pl, *cm, *cm_pl, *zero, *zero_pl;
-  // per tracer
-  double *q, *q_pl, *grad, *grad_pl, *qa, *qa_pl, *qout, *qout_pl, *qin_pl;
-  // step_plain: boundary tables (Ctx::build_fast_tables), limited face values (kPlainGroup tracers,
-  // over the memory of ch .. qout, which only the adjoint uses) and boundary values
+  double *flx, *flx_pl, *xc, *xc_pl;
+  // boundary tables (Ctx::build_fast_tables), limited face values of a group of tracers and their
+  // boundary values
   int nb, ns;
   const int *bsrc, *seam, *ring;
   double *fv, *bb;
 };
 
-// tracers a group of the plain step takes through its launches: their face values (3 fields a
-// tracer) fill the 24 fields that the adjoint's recompute keeps per step and tracer
+// Tracers a group of the step takes through its launches.  The face values of a group are 3 fields
+// a tracer: 8 tracers keep the step's scratch at 39 fields however many tracers there are.
 constexpr int kPlainGroup = 8;
-
-// Pieces of the step used by the adjoint's forward recompute.
-void launch_courant(const StepCtx &S, const double *rhog, const double *rhog_pl, cudaStream_t st);  // flx -> ch, cm
-void launch_divide(const StepCtx &S, const double *Q, const double *Qp, const double *rhog, const double *rhog_pl,
-                   cudaStream_t st);                                  // q = Q / rhog
-void launch_gradient(const StepCtx &S, cudaStream_t st);             // q -> grad, halo filled
-void launch_remap(const StepCtx &S, cudaStream_t st);                // q, grad -> qa
-void launch_update_rho(const StepCtx &S, double *rho, double *rho_pl, cudaStream_t st);  // rho -= sum flx
 
 int step_plain(StepCtx &S, int ntr, double dt, double *rhog, double *rhog_pl, double *rhogq, double *rhogq_pl,
                const double *vx, const double *vx_pl, const double *vy, const double *vy_pl, const double *vz,
