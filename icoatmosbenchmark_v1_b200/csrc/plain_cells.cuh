@@ -76,7 +76,6 @@ __device__ __forceinline__ void cell_limits(const double (&n)[7], const CellFlow
   L.lo[4] = mn(c0, mn(l34, n5)), L.hi[4] = mx(c0, mx(h34, n5));
   L.lo[5] = mn(c0, mn(n4, l56)), L.hi[5] = mx(c0, mx(n4, h56));
   L.lo[6] = mn(c0, mn(l56, n1)), L.hi[6] = mx(c0, mx(h56, n1));
-  if (sing) L.lo[5] = mn4(n5, c0, n1, n4), L.hi[5] = mx4(n5, c0, n1, n4);  // the singular point's shifted stencil
   // Qout (:219-282, d = 0).  An outflow face's +-BIG bound never binds, and its term of CQ is
   // zero with its Courant number, except at an odd face
   double qnmin = c0, qnmax = c0, CQmin = F.chm[1] * L.lo[1], CQmax = F.chm[1] * L.hi[1];
@@ -87,10 +86,14 @@ __device__ __forceinline__ void cell_limits(const double (&n)[7], const CellFlow
     qnmax = (f && L.hi[m] > qnmax) ? L.hi[m] : qnmax;
     if (m > 1) CQmin = CQmin + F.chm[m] * L.lo[m], CQmax = CQmax + F.chm[m] * L.hi[m];
   }
-  if (F.odd) {
+  if (F.odd || sing) {
+    if (sing) L.lo[5] = mn4(n5, c0, n1, n4), L.hi[5] = mx4(n5, c0, n1, n4);  // the singular point's shifted stencil
+    qnmin = qnmax = c0;
 #pragma unroll
     for (int m = 1; m <= 6; ++m) {
       const bool f = (F.in >> m) & 1u;
+      qnmin = (f && L.lo[m] < qnmin) ? L.lo[m] : qnmin;
+      qnmax = (f && L.hi[m] > qnmax) ? L.hi[m] : qnmax;
       const double tmin = F.chm[m] * (f ? L.lo[m] : DBL_MAX), tmax = F.chm[m] * (f ? L.hi[m] : -DBL_MAX);
       CQmin = (m == 1) ? tmin : CQmin + tmin;
       CQmax = (m == 1) ? tmax : CQmax + tmax;
@@ -101,6 +104,13 @@ __device__ __forceinline__ void cell_limits(const double (&n)[7], const CellFlow
   L.Qmin = F.zsw ? c0 : Qo[0], L.Qmax = F.zsw ? c0 : Qo[1];
   L.qnmin = qnmin, L.qnmax = qnmax, L.CQmin = CQmin, L.CQmax = CQmax;
 }
+
+// store x to p where on, without a branch
+__device__ __forceinline__ void store_if(bool on, double *p, double x) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q st.global.f64 [%0], %1;\n}\n" ::"l"(p), "d"(x), "r"((int)on)
+               : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const double *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 template <int TX, int NTH>
 struct CellSmem {
@@ -123,6 +133,8 @@ struct CellTile {
   static __device__ constexpr int wstep(int m) {  // window slots from a cell to its neighbour m
     return m == 0 ? 0 : m == 1 ? 1 : m == 2 ? Smem::WW + 1 : m == 3 ? Smem::WW : m == 4 ? -1 : m == 5 ? -Smem::WW - 1 : -Smem::WW;
   }
+  // window slot r of this thread holds a cell (the first one always in a region of whole tiles)
+  __device__ __forceinline__ bool has(int r) const { return (TX == 32 && r == 0) || wc[r] >= 0; }
   int l, c, ew, ow, bs, oslot, ocell, wc[NSLOT];
   bool act, sing;
   unsigned both;  // bit m: the cell across face m is interior too (not a seam face)
@@ -180,7 +192,7 @@ struct CellTile {
     for (int m = 0; m < 6; ++m) ch[m] = flx[m] = (fx + m * n3)[c];
     fo[0] = fx[c - 1], fo[1] = (fx + n3)[c - G - 1], fo[2] = (fx + 2 * n3)[c - G];  // owners of faces 4-6
 #pragma unroll
-    for (int r = 0; r < NSLOT; ++r) rv[r] = wc[r] >= 0 ? P.rho[off + wc[r]] : 1.0;
+    for (int r = 0; r < NSLOT; ++r) rv[r] = has(r) ? P.rho[off + wc[r]] : 1.0;
     __syncthreads();  // the previous level's shared data is read
     const double *xc = P.xc + off;
 #pragma unroll
@@ -193,7 +205,7 @@ struct CellTile {
 #pragma unroll
     for (int r = 0; r < NSLOT; ++r) {
       rw[r] = recip(rv[r]);
-      if (wc[r] >= 0) s.rho[tid + r * NTH] = rv[r], s.y[tid + r * NTH] = rw[r].y;
+      if (has(r)) s.rho[tid + r * NTH] = rv[r], s.y[tid + r * NTH] = rw[r].y;
     }
     __syncthreads();
     unsigned out = 0;
@@ -235,6 +247,17 @@ struct CellTile {
         if (o1 && o2) s.disp[a * 3 + d][so] -= X[d];
       }
     }
+  }
+
+  // asks L2 for the next level's set-up inputs and its first tracer's q
+  __device__ __forceinline__ void prefetch(const PlainArgs &P, size_t off) const {
+    const size_t n3 = P.n3();
+#pragma unroll
+    for (int m = 0; m < 6; ++m) prefetch_l2(P.flx + m * n3 + off + c);
+#pragma unroll
+    for (int m = 0; m < 9; ++m) prefetch_l2(P.xc + m * n3 + off + c);
+    prefetch_l2(P.rho + off + c);
+    prefetch_l2(P.Q + off + c);
   }
 
   // q of the cell and its neighbours from buffer b of the window, and the cell's gradient

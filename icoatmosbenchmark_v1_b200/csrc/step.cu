@@ -41,8 +41,8 @@ namespace icoadv {
 //
 // A face value travels once through memory (24 bytes written and read per update); gradient,
 // remap value, Courant number, mask and Qout never do.  Against one launch per piece and tracer
-// (14 launches a tracer, a column's levels in local memory): 9.90 -> 3.61 ms for glevel 7, kall 61,
-// 5 tracers, 1.59 -> 0.35 ms for glevel 5, kall 42, 8 tracers.  Every value is the result of the
+// (14 launches a tracer, a column's levels in local memory): 9.90 -> 3.25 ms for glevel 7, kall 61,
+// 5 tracers, 1.59 -> 0.30 ms for glevel 5, kall 42, 8 tracers.  Every value is the result of the
 // reference's operation sequence; where the reference blends two sides by a mask of 0 or 1
 // (c a + (1 - c) b), the chosen side is taken, which is the same number.
 constexpr int kTileCells = 256;  // threads of k_plain_cells: one per cell of a TX x (256 / TX) tile
@@ -80,9 +80,10 @@ __device__ __forceinline__ void pole_centre(const PlainArgs &P, int t, int p, in
   o[4] = (q[0] - CQmin - qnmin * (1.0 - Cin - Cout + dn)) / (Cout + zsw) * (1.0 - zsw) + q[0] * zsw;
 }
 
-// Bound by instruction issue (FP64 compare-and-selects of the bounds, then the gradient): 1.62 ms
-// of the 3.61.  One tracer per pass of the loop and two blocks per SM keep every value in
-// registers; two tracers, or three blocks, spill and take 2.5-2.6 ms.
+// Bound by instruction issue and latency: 1.67 ms of the 3.25, of which the set-up of a level (620
+// instructions a cell against 550 per tracer) is a third.  One tracer per pass of the loop and two
+// blocks per SM keep every value in registers; two tracers, or three blocks, spill and take 2.5-2.6
+// ms.  The next level's set-up inputs are asked for while a level's tracers go through (1.72 without).
 // grid: blocks 0 .. ntile*nlb-1 (level block fastest: a tile's gradient coefficients come from L2
 // after the first), then the pole centres
 template <int TX>
@@ -109,33 +110,35 @@ __global__ void __launch_bounds__(kTileCells, kCellBlocks) k_plain_cells(PlainAr
   for (int k = k0; k < k1; ++k) {
     const size_t off = ((size_t)T.l * D.kall + k) * D.gall;
     double Qw[Tile::NSLOT][1];
-    auto load = [&](int t) {
-      const double *Qs = P.Q + (size_t)t * n3 + off;
+    const double *Qs = P.Q + off;
+    auto load = [&] {
 #pragma unroll
       for (int r = 0; r < Tile::NSLOT; ++r)
-        if (T.wc[r] >= 0) Qw[r][0] = Qs[T.wc[r]];
+        if (T.has(r)) Qw[r][0] = Qs[T.wc[r]];
     };
-    load(0);  // with the level's other global loads, before the first wait
+    load();  // with the level's other global loads, before the first wait
     Recip rw[Tile::NSLOT];
     CellFlow F;
     double flx[6];
     T.level(P, s, off, rw, F, flx);
+    if (k + 1 < k1) T.prefetch(P, off + D.gall);
     // ---- the tracers; their q alternates between two buffers
-    for (int t = 0; t < P.nt; ++t) {
+    double *fv = P.fv + off;
+    for (int t = 0; t < P.nt; ++t, fv += 3 * n3) {
       const int b = t & 1;
 #pragma unroll
       for (int r = 0; r < Tile::NSLOT; ++r)
-        if (T.wc[r] >= 0) {
+        if (T.has(r)) {
           quotients(Qw[r], rw[r]);
           s.q[b][tid + r * kTileCells] = Qw[r][0];
         }
-      if (t + 1 < P.nt) load(t + 1);
+      Qs += n3;
+      if (t + 1 < P.nt) load();
       __syncthreads();
       double n[7], g[3];
       T.gradient(s, b, n, g);
       CellLimits L;
       cell_limits(n, F, T.sing, L);
-      double *fv = P.fv + (size_t)t * 3 * n3 + off;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         const bool f = (F.side >> a) & 1u;
@@ -144,7 +147,7 @@ __global__ void __launch_bounds__(kTileCells, kCellBlocks) k_plain_cells(PlainAr
         for (int d = 0; d < 3; ++d) v = v + g[d] * s.disp[a * 3 + d][F.sl[a]];
         v = mn(mx(v, f ? L.lo[a + 4] : L.lo[a + 1]), f ? L.hi[a + 4] : L.hi[a + 1]);
         v = mx(mn(v, L.Qmax), L.Qmin);
-        if (F.st[a] >= 0) (fv + a * n3)[F.st[a]] = v;
+        store_if(F.st[a] >= 0, fv + a * n3 + F.st[a], v);
       }
       if (F.again) {
 #pragma unroll
@@ -240,12 +243,19 @@ __device__ __forceinline__ double vclamp(double infl, double h, double mnL, doub
   return infl * b1 + (1.0 - infl) * b2;
 }
 
-constexpr int kColThreads = 128;
+constexpr int kColThreads = 128, kColStages = 2, kColBlocks = 3;
+constexpr int kColSmem = kColStages * (8 + 7 * 2) * kColThreads * (int)sizeof(double);
+
+__device__ __forceinline__ void copy_async(double *dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
 
 // the two sub-steps of one pole column (p, tracer t): a thread per level, every stage level-parallel
 __device__ __forceinline__ void pole_column(const PlainArgs &P, int p, int t) {
-  __shared__ double sq[kColThreads], sh[kColThreads], s1[kColThreads], s2[kColThreads], smn[kColThreads],
-      smx[kColThreads];
+  extern __shared__ __align__(16) double ring[];  // the memory of the other blocks' input stages
+  double *sq = ring, *sh = sq + kColThreads, *s1 = sh + kColThreads, *s2 = s1 + kColThreads, *smn = s2 + kColThreads,
+         *smx = smn + kColThreads;
   const Dims &D = P.D;
   const int K = D.kall, k = threadIdx.x, kmin = D.kmin - 1, kmax = D.kmax - 1;
   const size_t off = ((size_t)p * K + k) * kGallPl, n3p = P.n3p();
@@ -311,10 +321,11 @@ __device__ __forceinline__ void pole_column(const PlainArgs &P, int p, int t) {
 }
 
 // One column per thread and two tracers (an odd group's last one alone): the two share the column's
-// density, w and limiter parameters and fill each other's latencies (5 tracers at glevel 7, kall 61:
-// 0.92 ms, one tracer per thread 0.97 ms at 4 blocks per SM).  A column block's tracer pairs are
-// consecutive blocks and share rhog, rhogw and the fluxes in L2; the next level's inputs are loaded
-// while a level is worked on.
+// density, w and limiter parameters and fill each other's latencies.  The next level's inputs are
+// copied to shared memory while a level is worked on, which leaves the registers for three blocks an
+// SM: 0.81 ms for 5 tracers at glevel 7, kall 61 (the next level's inputs in registers, two blocks:
+// 0.89; one tracer a thread 0.97; a third stage takes the L1 cache away: 1.08).  A column block's
+// tracer pairs are consecutive blocks and share rhog, rhogw and the fluxes in L2.
 // Level k gives Qout of level k-1 and the limited flux of the face below it, which finish level k-2;
 // levels alternate between two slots, so nothing is copied from level to level.
 template <int NT>
@@ -331,47 +342,69 @@ __device__ __forceinline__ void column(const PlainArgs &P, int t0, int l, int co
   const double *fv[NT];
 #pragma unroll
   for (int h = 0; h < NT; ++h) Q[h] = P.Q + (size_t)(t0 + h) * n3 + base, fv[h] = P.fv + (size_t)(t0 + h) * 3 * n3 + base;
+  // the inputs of kColStages levels, each thread's own copies (cp.async: no barrier, no registers)
   struct In {
-    double Q[NT], f[NT][6], flx[6], rho, w;
+    double flx[6], rho, w, x[NT][7];  // x: Q, then the six face values
   };
-  auto load = [&](In &v, int k, bool phys) {
-    const unsigned o = (unsigned)k * g + c;
+  constexpr int NV = 8 + 7 * NT;
+  extern __shared__ __align__(16) double ring[];  // [stage][value][thread]
+  auto issue = [&](int k, bool phys) {
+    if (k <= K - 1) {
+      double *to = ring + (size_t)(k % kColStages) * NV * kColThreads + threadIdx.x;
+      const unsigned o = (unsigned)k * g + c;
 #pragma unroll
-    for (int m = 0; m < 6; ++m) v.flx[m] = (flx + m * n3)[o];
-    v.rho = rho[o], v.w = W[o];
-    if (phys) {
-      const unsigned o4 = o - 1, o5 = o - G - 1, o6 = o - G;
+      for (int m = 0; m < 6; ++m) copy_async(to + m * kColThreads, flx + m * n3 + o);
+      copy_async(to + 6 * kColThreads, rho + o), copy_async(to + 7 * kColThreads, W + o);
+      if (phys) {
+        const unsigned o4 = o - 1, o5 = o - G - 1, o6 = o - G;
 #pragma unroll
-      for (int h = 0; h < NT; ++h) {
-        v.Q[h] = Q[h][o];
-        v.f[h][0] = fv[h][o], v.f[h][1] = (fv[h] + n3)[o], v.f[h][2] = (fv[h] + 2 * n3)[o];
-        v.f[h][3] = fv[h][o4], v.f[h][4] = (fv[h] + n3)[o5], v.f[h][5] = (fv[h] + 2 * n3)[o6];
+        for (int h = 0; h < NT; ++h) {
+          double *th = to + (8 + 7 * h) * kColThreads;
+          copy_async(th, Q[h] + o);
+          copy_async(th + kColThreads, fv[h] + o), copy_async(th + 2 * kColThreads, fv[h] + n3 + o);
+          copy_async(th + 3 * kColThreads, fv[h] + 2 * n3 + o), copy_async(th + 4 * kColThreads, fv[h] + o4);
+          copy_async(th + 5 * kColThreads, fv[h] + n3 + o5), copy_async(th + 6 * kColThreads, fv[h] + 2 * n3 + o6);
+        }
       }
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  auto load = [&](In &v, int k) {  // level k, copied kColStages - 1 levels ago
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kColStages - 2) : "memory");
+    const double *from = ring + (size_t)(k % kColStages) * NV * kColThreads + threadIdx.x;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) v.flx[m] = from[m * kColThreads];
+    v.rho = from[6 * kColThreads], v.w = from[7 * kColThreads];
+#pragma unroll
+    for (int h = 0; h < NT; ++h)
+#pragma unroll
+      for (int m = 0; m < 7; ++m) v.x[h][m] = from[(8 + 7 * h + m) * kColThreads];
   };
   auto horiz = [&](const In &v, int h) {  // rhogq after the horizontal sub-step
-    double s = v.flx[0] * v.f[h][0];
+    double s = v.flx[0] * v.x[h][1];
 #pragma unroll
-    for (int m = 1; m < 6; ++m) s = s + v.flx[m] * v.f[h][m];
-    return v.Q[h] - s;
+    for (int m = 1; m < 6; ++m) s = s + v.flx[m] * v.x[h][m + 1];
+    return v.x[h][0] - s;
   };
   const int kmin = D.kmin - 1, kmax = D.kmax - 1;
-  In A, B;
-  load(A, kmin, true);
+#pragma unroll
+  for (int d = 0; d < kColStages - 1; ++d) issue(kmin + d, kmin + d <= kmax);
   if (K == 1) {
-    double x[NT];
+    In v;
+    load(v, kmin);
 #pragma unroll
-    for (int h = 0; h < NT; ++h) x[h] = horiz(A, h);
-#pragma unroll
-    for (int h = 0; h < NT; ++h) Q[h][c] = x[h];
+    for (int h = 0; h < NT; ++h) Q[h][c] = horiz(v, h);
     return;
   }
   // slot s of a window: the level being worked on (before: level k-2); slot 1 - s: level k-1
   double q[NT][2], Qh[NT][2], Qmn[NT], Qmx[NT], fl[NT];
   double c1 = 0.0, wk = 0.0;  // ck1 and w of level k-1
   Recip rp{1.0, 1.0, true};   // its density
-  auto level = [&](const In &v, int k, auto slot) {
+  auto level = [&](int k, auto slot) {
     constexpr int S = decltype(slot)::value, Z = 1 - S;
+    In v;
+    load(v, k);
+    issue(k + kColStages - 1, k + kColStages - 1 <= kmax);  // into the stage of level k - 1
     double r = v.flx[0];
 #pragma unroll
     for (int m = 1; m < 6; ++m) r = r + v.flx[m];
@@ -427,23 +460,22 @@ __device__ __forceinline__ void column(const PlainArgs &P, int t0, int l, int co
   };
 #pragma unroll 1
   for (int k = kmin;; k += 2) {
-    if (k < kmax + 1) load(B, k + 1, k < kmax);
-    level(A, k, C0{});
+    level(k, C0{});
     if (k == kmax + 1) {
       top(C0{});
       break;
     }
-    if (k + 1 < kmax + 1) load(A, k + 2, k + 1 < kmax);
-    level(B, k + 1, C1{});
+    level(k + 1, C1{});
     if (k + 1 == kmax + 1) {
       top(C1{});
       break;
     }
   }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
 // blocks: (tracer pair fastest, column block, region), then the pole columns
-__global__ void __launch_bounds__(kColThreads, 2) k_plain_column(PlainArgs P, int colblk, int nmain) {
+__global__ void __launch_bounds__(kColThreads, kColBlocks) k_plain_column(PlainArgs P, int colblk, int nmain) {
   if ((int)blockIdx.x >= nmain) {
     const int u = (int)blockIdx.x - nmain;
     pole_column(P, u % kLallPl, u / kLallPl);
@@ -552,12 +584,14 @@ int step_plain(StepCtx &S, int ntr, double dt, double *rhog, double *rhog_pl, do
   launches += 1;
   const int n = D.gmax - D.gmin + 1, NK = D.kmax - D.kmin + 1;
   const int colblk = (n * n + kColThreads - 1) / kColThreads;  // column blocks of a region
+  const cudaError_t e = cudaFuncSetAttribute(k_plain_column, cudaFuncAttributeMaxDynamicSharedMemorySize, kColSmem);
+  if (e != cudaSuccess) return set_error(std::string("advect_step: ") + cudaGetErrorString(e)), ICA_ERR_CUDA;
   for (int t0 = 0; t0 < ntr; t0 += kPlainGroup) {
     const PlainArgs P = plain_group(S, t0, ntr, dt, rhog, rhog_pl, rhogq, rhogq_pl, w, w_pl);
     const int rc = plain_faces(P, st, launches);
     if (rc) return rc;
     const int nmain = colblk * D.lall * ((P.nt + 1) / 2);
-    k_plain_column<<<(unsigned)(nmain + kLallPl * P.nt), kColThreads, 0, st>>>(P, colblk, nmain);
+    k_plain_column<<<(unsigned)(nmain + kLallPl * P.nt), kColThreads, kColSmem, st>>>(P, colblk, nmain);
     launches += 1;
   }
   const long long nr = ((long long)D.lall * n * n + kLallPl) * NK;
