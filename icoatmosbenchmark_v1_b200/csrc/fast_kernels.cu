@@ -162,7 +162,9 @@ __global__ void k_fast_boundary(const __grid_constant__ MultiInst M) {
   const int oi[7] = {0, i, i, i, i - 1, i - 1, i}, oj[7] = {0, j, j, j, j, j - 1, j - 1};
   const int fa[7] = {0, AI, AIJ, AJ, AI, AIJ, AJ};
   const double rho_c = f(0, i, j), ra_c = rarea(I, l, i, j);
-  double ch[7], chm[7], cmk[7];
+  double ch[7], chm[7];
+  unsigned in = 0;   // bit m: face m is an inflow face (its mask; the owner's, 1 takes the owner's neighbour)
+  bool odd = false;  // an inflow Courant number at a face whose mask says outflow (rounding-level fluxes)
   for (int m = 1; m <= 6; ++m) {
     double xcv[3];
     const bool ex = face_exists(I, oi[m], oj[m], fa[m]);
@@ -171,7 +173,9 @@ __global__ void k_fast_boundary(const __grid_constant__ MultiInst M) {
     ch[m] = flx / rho_c;
     chm[m] = mn64(ch[m], 0.0);
     const double ch_own = (m <= 3) ? ch[m] : (fl * rarea(I, l, oi[m], oj[m]) * I.dt) / f(0, oi[m], oj[m]);
-    cmk[m] = 0.5 - fsg(0.5, ch_own - EPS);
+    const bool cm = 0.5 - fsg(0.5, ch_own - EPS) != 0.0;
+    if (cm == (m <= 3)) in |= 1u << m;
+    else odd = odd || chm[m] != 0.0;
   }
   const double Cin = chm[1] + chm[2] + chm[3] + chm[4] + chm[5] + chm[6];
   const double Cout =
@@ -233,23 +237,25 @@ __global__ void k_fast_boundary(const __grid_constant__ MultiInst M) {
     if (sgp5) b4(5, Q(-1, -1), Q(0, 0), Q(1, 0), Q(-1, 0));  // AIJ of the singular corner
     else b4(5, Q(-1, -1), Q(0, -1), Q(0, 0), Q(-1, 0));      // AIJ of (i-1, j-1)
     b4(6, Q(0, -1), Q(1, 0), Q(0, 0), Q(-1, -1));   // AJ of (i, j-1)
-    double qmn[7], qmx[7];
-#pragma unroll
-    for (int m = 1; m <= 6; ++m) {
-      const double cm = cmk[m];
-      if (m <= 3) qmn[m] = cm * lo[m] + (1.0 - cm) * BIG, qmx[m] = cm * hi[m] + (1.0 - cm) * (-BIG);
-      else qmn[m] = cm * BIG + (1.0 - cm) * lo[m], qmx[m] = cm * (-BIG) + (1.0 - cm) * hi[m];
-    }
+    // an outflow face's +-BIG bound binds nothing, and its term of CQ is zero with its Courant
+    // number, except at an odd face
     const double q0 = q9[1][1];
     double qnmin = q0, qnmax = q0;
 #pragma unroll
-    for (int m = 1; m <= 6; ++m) qnmin = mn64(qnmin, qmn[m]);
+    for (int m = 1; m <= 6; ++m) {
+      const bool f = (in >> m) & 1u;
+      qnmin = (f && lo[m] < qnmin) ? lo[m] : qnmin;
+      qnmax = (f && hi[m] > qnmax) ? hi[m] : qnmax;
+    }
+    if (odd) {
 #pragma unroll
-    for (int m = 1; m <= 6; ++m) qnmax = mx64(qnmax, qmx[m]);
-    const double CQmin = chm[1] * qmn[1] + chm[2] * qmn[2] + chm[3] * qmn[3] + chm[4] * qmn[4] + chm[5] * qmn[5] +
-                         chm[6] * qmn[6];
-    const double CQmax = chm[1] * qmx[1] + chm[2] * qmx[2] + chm[3] * qmx[3] + chm[4] * qmx[4] + chm[5] * qmx[5] +
-                         chm[6] * qmx[6];
+      for (int m = 1; m <= 6; ++m)
+        if (!((in >> m) & 1u)) lo[m] = BIG, hi[m] = -BIG;
+    }
+    const double CQmin = chm[1] * lo[1] + chm[2] * lo[2] + chm[3] * lo[3] + chm[4] * lo[4] + chm[5] * lo[5] +
+                         chm[6] * lo[6];
+    const double CQmax = chm[1] * hi[1] + chm[2] * hi[2] + chm[3] * hi[3] + chm[4] * hi[4] + chm[5] * hi[5] +
+                         chm[6] * hi[6];
     out[3] = (q0 - CQmax - qnmax * omc) * rden + q0 * zerosw;
     out[4] = (q0 - CQmin - qnmin * omc) * rden + q0 * zerosw;
     double *dst = dst0 + t * dstride;
@@ -283,11 +289,12 @@ __global__ void k_fast_seam(const __grid_constant__ MultiInst M) {
   I.sflux[(size_t)k * I.ns + sidx] = fl;
   const int ni = (a == AI || a == AIJ) ? i + 1 : i, nj = (a == AIJ || a == AJ) ? j + 1 : j;
   const double ch = (fl * rarea(I, l, i, j) * I.dt) / gf(0, i, j);
-  const double cm = 0.5 - fsg(0.5, ch - DBL_EPSILON);
-  const int bo = I.bsrc[(size_t)l * I.gall + (j - 1) * G + (i - 1)];
-  const int bn = I.bsrc[(size_t)l * I.gall + (nj - 1) * G + (ni - 1)];
-  double dxo[3], dxn[3];
-  for (int x = 0; x < 3; ++x) dxo[x] = xc[x] - gx(I, l, i, j, x), dxn[x] = xc[x] - gx(I, l, ni, nj, x);
+  // the upwind cell: the owner's neighbour where the mask is 1
+  const bool cm = 0.5 - fsg(0.5, ch - DBL_EPSILON) != 0.0;
+  const int ui = cm ? ni : i, uj = cm ? nj : j;
+  const int bu = I.bsrc[(size_t)l * I.gall + (uj - 1) * G + (ui - 1)];
+  double dxu[3];
+  for (int x = 0; x < 3; ++x) dxu[x] = xc[x] - gx(I, l, ui, uj, x);
   // the 4 cells of the face's bounds (bounds64's selection) and 1/rho there; the owner is [0]
   int pc[4];
   {
@@ -303,26 +310,25 @@ __global__ void k_fast_seam(const __grid_constant__ MultiInst M) {
     } else pc[1] = ij + G + 1, pc[2] = ij + G, pc[3] = im1j;
   }
   const size_t slab = ((size_t)l * I.K + k) * I.gall, tstride = (size_t)I.lall * I.K * I.gall;
-  const size_t on = (size_t)(nj - 1) * G + (ni - 1);
+  const size_t ou = (size_t)(uj - 1) * G + (ui - 1);
   double rv[4];
   for (int n = 0; n < 4; ++n) rv[n] = 1.0 / I.rho_in[slab + pc[n] - 1];
-  const double rn = 1.0 / I.rho_in[slab + on];
-  const double BIG = DBL_MAX;
+  const double ru = 1.0 / I.rho_in[slab + ou];
   // the tracer's inputs one tracer ahead: the next tracer's loads are issued before this
   // tracer's store (which the compiler may not move them across).  Per-tracer strides are
-  // applied to base pointers (the index products stay out of the tracer loop).
-  double rq[5], rgo[5], rgn[5];
+  // applied to base pointers (the index products stay out of the tracer loop).  Of the gradient and
+  // Qout only the upwind side's are read: half of the pass's traffic.
+  double rq[5], rg[5];
   const double *Qt = I.Q_in + slab;
   const size_t bstride = (size_t)I.K * I.nb * 5, vstride = (size_t)I.K * I.ns;
-  const double *bvo = I.bbuf + ((size_t)k * I.nb + (bo >= 0 ? bo : 0)) * 5;
-  const double *bvn = I.bbuf + ((size_t)k * I.nb + (bn >= 0 ? bn : 0)) * 5;
+  const double *bvu = I.bbuf + ((size_t)k * I.nb + (bu >= 0 ? bu : 0)) * 5;
   auto fetch = [&]() {
 #pragma unroll
     for (int n = 0; n < 4; ++n) rq[n] = Qt[pc[n] - 1];
-    rq[4] = Qt[on];
+    rq[4] = Qt[ou];
 #pragma unroll
-    for (int x = 0; x < 5; ++x) rgo[x] = bo >= 0 ? bvo[x] : 0.0, rgn[x] = bn >= 0 ? bvn[x] : 0.0;
-    Qt += tstride, bvo += bstride, bvn += bstride;
+    for (int x = 0; x < 5; ++x) rg[x] = bu >= 0 ? bvu[x] : 0.0;
+    Qt += tstride, bvu += bstride;
   };
   fetch();
   const size_t vbase = (size_t)k * I.ns + sidx;
@@ -332,24 +338,18 @@ __global__ void k_fast_seam(const __grid_constant__ MultiInst M) {
     double qv[4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) qv[n] = rq[n] * rv[n];
-    const double qo = qv[0], qn = rq[4] * rn;
-    // gradient and Qout of both cells (boundary or halo cells of this region)
-    double go[5] = {0, 0, 0, 0, 0}, gn[5] = {0, 0, 0, 0, 0};
-    if (bo >= 0) for (int x = 0; x < 5; ++x) go[x] = rgo[x];
-    else go[3] = go[4] = qo;  // halo point no list reaches: Qout = q, grad = 0 (as after the reference fill)
-    if (bn >= 0) for (int x = 0; x < 5; ++x) gn[x] = rgn[x];
-    else gn[3] = gn[4] = qn;
+    const double qu = rq[4] * ru;
+    double g[5];
+#pragma unroll
+    for (int x = 0; x < 5; ++x) g[x] = rg[x];
+    if (bu < 0) g[3] = g[4] = qu;  // halo point no list reaches: Qout = q, grad = 0 (as after the reference fill)
     if (t + 1 < I.ntr) fetch();
-    double vu = qn, vs = qo;
-    for (int x = 0; x < 3; ++x) vu = vu + gn[x] * dxn[x];
-    for (int x = 0; x < 3; ++x) vs = vs + go[x] * dxo[x];
-    double v = cm * vu + (1.0 - cm) * vs;
+    double v = qu;
+    for (int x = 0; x < 3; ++x) v = v + g[x] * dxu[x];
     const double lo = mn64(mn64(mn64(qv[0], qv[1]), qv[2]), qv[3]);
     const double hi = mx64(mx64(mx64(qv[0], qv[1]), qv[2]), qv[3]);
-    const double own_min = cm * lo + (1.0 - cm) * BIG, own_max = cm * hi + (1.0 - cm) * (-BIG);
-    const double nb_min = cm * BIG + (1.0 - cm) * lo, nb_max = cm * (-BIG) + (1.0 - cm) * hi;
-    v = cm * mn64(mx64(v, own_min), own_max) + (1.0 - cm) * mn64(mx64(v, nb_min), nb_max);
-    v = cm * mx64(mn64(v, gn[4]), gn[3]) + (1.0 - cm) * mx64(mn64(v, go[4]), go[3]);
+    v = mn64(mx64(v, lo), hi);
+    v = mx64(mn64(v, g[4]), g[3]);
     if (I.f64) *sv64 = v, sv64 += vstride;
     else *sv32 = (float)v, sv32 += vstride;
   }
@@ -1124,19 +1124,35 @@ __global__ void __launch_bounds__(TileGeo<TX, TY>::NT, (sizeof(R) == 8 ? 1 : 2))
   }
 }
 
-// one grid: one CTA per (tile, kLevelsPerCta consecutive levels) (grid x = level block, y = tile:
+// one grid: one CTA per (tile, lpc consecutive levels) (grid x = level block, y = tile:
 // a tile's level blocks run side by side, so its level-invariant coefficients are read from L2
 // by all but the first, and a CTA keeps them in registers over its levels)
 constexpr int kLevelsPerCta = 8;
+// FP64 holds one CTA an SM, so a grid of few CTAs runs in waves of whole ones, and of the splits up to
+// 8 levels the one whose last wave is fullest is the fastest: glevel 6, rlevel 1, kall 42, 13
+// tracers (160 tiles) 1.65 -> 1.59 ms a step with 4 levels (10.8 waves of 148) for 8 (5.4).  A CTA's own
+// set-up counts as a third of a level; past eight waves the last one no longer matters.
+static int levels_per_cta(long long tiles, int levels, int slots) {
+  int best = kLevelsPerCta;
+  double least = 0.0;
+  for (int l = kLevelsPerCta; l >= 1; --l) {
+    const long long ctas = tiles * ((levels + l - 1) / l);
+    const double cost = ctas > 8LL * slots ? ((double)tiles * levels + 0.3 * (double)ctas) / slots
+                                           : (double)((ctas + slots - 1) / slots) * (l + 0.3);
+    if (l == kLevelsPerCta || cost < least) best = l, least = cost;
+  }
+  return best;
+}
 template <int TX, int TY, int TB, typename R>
 __global__ void __launch_bounds__(TileGeo<TX, TY>::NT, (sizeof(R) == 8 ? 1 : 2))
-    k_fast_horiz1(const __grid_constant__ FastInst I, const __grid_constant__ TileMaps T) {
+    k_fast_horiz1(const __grid_constant__ FastInst I, const __grid_constant__ TileMaps T, int levels) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   auto &s = tile_smem<TX, TY, TB, R>(smem_raw);
   tile_smem_init(s);
   unsigned phase = 0;
   const int tile = I.l0 * I.ntx * I.nty + (int)blockIdx.y, tr = (int)blockIdx.y % (I.ntx * I.nty);
-  const int k0 = 1 + (int)blockIdx.x * kLevelsPerCta, k1 = min(k0 + kLevelsPerCta, I.K - 1);
+  const int lpc = sizeof(R) == 8 ? levels : kLevelsPerCta;
+  const int k0 = 1 + (int)blockIdx.x * lpc, k1 = min(k0 + lpc, I.K - 1);
   if (edge_tile<TX, TY>(I, I.gmin + (tr % I.ntx) * TX, I.gmin + (tr / I.ntx) * TY))
     horiz_levels<TX, TY, TB, R, true>(I, &T, tile, k0, k1, s, phase);
   else
@@ -1567,10 +1583,10 @@ static cudaError_t launch_tile_n(const MultiInst &M, cudaStream_t st) {
     nwork += (long long)(M.inst[i].l1 - M.inst[i].l0) * M.inst[i].ntx * M.inst[i].nty * (M.inst[i].K - 2);
   if (ONE) {
     const FastInst &I = M.inst[0];
-    if ((long long)(I.l1 - I.l0) * I.ntx * I.nty > 65535) return cudaErrorInvalidConfiguration;  // grid y
-    k_fast_horiz1<TX, TY, TB, R>
-        <<<dim3((unsigned)((I.K - 2 + kLevelsPerCta - 1) / kLevelsPerCta), (unsigned)((I.l1 - I.l0) * I.ntx * I.nty)),
-           NT, smem, st>>>(I, T.m[0]);
+    const long long tiles = (long long)(I.l1 - I.l0) * I.ntx * I.nty;
+    if (tiles > 65535) return cudaErrorInvalidConfiguration;  // grid y
+    const int lpc = sizeof(R) == 8 ? levels_per_cta(tiles, I.K - 2, nsm * per_sm[dev]) : kLevelsPerCta;
+    k_fast_horiz1<TX, TY, TB, R><<<dim3((unsigned)((I.K - 2 + lpc - 1) / lpc), (unsigned)tiles), NT, smem, st>>>(I, T.m[0], lpc);
   } else {
     const long long grid = nwork < (long long)nsm * per_sm[dev] ? nwork : (long long)nsm * per_sm[dev];
     e = cudaMemsetAsync(M.inst[0].work_next, 0, sizeof(unsigned long long), st);
