@@ -158,21 +158,52 @@ __global__ void k_fast_boundary(const __grid_constant__ MultiInst M) {
   const bool sgp = I.have_sgp[l] != 0;
   const GFields f{&I, l, k};
   const double BIG = DBL_MAX, EPS = DBL_EPSILON;
-  // tracer-independent: Courant numbers and upwind masks of the 6 faces, 1/rho on the 3x3 block
-  const int oi[7] = {0, i, i, i, i - 1, i - 1, i}, oj[7] = {0, j, j, j, j, j - 1, j - 1};
-  const int fa[7] = {0, AI, AIJ, AJ, AI, AIJ, AJ};
-  const double rho_c = f(0, i, j), ra_c = rarea(I, l, i, j);
+  // tracer-independent: Courant numbers and upwind masks of the 6 faces, 1/rho on the 3x3 block.  The
+  // six triangles around the cell are formed once each, every face being two neighbours of them
+  // (face by face they took 12 triangles and 108 field loads, half of this pass at 13 tracers);
+  // every face of an interior cell exists, and TI(gmin-1,gmin-1) of a singular region is
+  // TJ(gmin,gmin-1).
+  const bool sgp5 = sgp && i == I.gmin && j == I.gmin;
+  const size_t slab = ((size_t)l * I.K + k) * I.gall, gw = (size_t)I.lall * I.gall, lg = (size_t)l * I.gall;
+  const int cw[7] = {c, c + 1, c + G + 1, c + G, c - 1, c - G - 1, c - G};  // the cell and its six neighbours
+  double fv[3][7];
+#pragma unroll
+  for (int x = 0; x < 3; ++x)
+#pragma unroll
+    for (int n = 0; n < 7; ++n) fv[x][n] = fld(I, x, slab + cw[n]);
+  // triangle t (TI, TJ) of owner o with corners (cells of cw): rhov x/y/z
+  auto triangle = [&](int o, int t, int c0, int c1, int c2, double (&v)[3]) {
+    const double w1 = I.GMTR_t[((size_t)(W1 - 1) * 2 + (t - 1)) * gw + lg + o];
+    const double w2 = I.GMTR_t[((size_t)(W2 - 1) * 2 + (t - 1)) * gw + lg + o];
+    const double w3 = I.GMTR_t[((size_t)(W3 - 1) * 2 + (t - 1)) * gw + lg + o];
+#pragma unroll
+    for (int x = 0; x < 3; ++x) v[x] = fv[x][c0] * w1 + fv[x][c1] * w2 + fv[x][c2] * w3;
+  };
+  double tI[3], tJ[3], tIw[3], tIsw[3], tJsw[3], tJs[3];
+  triangle(c, TI, 0, 1, 2, tI), triangle(c, TJ, 0, 2, 3, tJ);
+  triangle(c - 1, TI, 4, 0, 3, tIw);
+  triangle(c - G - 1, TI, 5, 6, 0, tIsw), triangle(c - G - 1, TJ, 5, 0, 4, tJsw);
+  triangle(c - G, TJ, 6, 1, 0, tJs);
+  if (sgp5) {
+#pragma unroll
+    for (int x = 0; x < 3; ++x) tIsw[x] = tJs[x];
+  }
+  const double rho_c = I.rho_in[slab + c], ra_c = rarea(I, l, i, j);
   double ch[7], chm[7];
   unsigned in = 0;   // bit m: face m is an inflow face (its mask; the owner's, 1 takes the owner's neighbour)
   bool odd = false;  // an inflow Courant number at a face whose mask says outflow (rounding-level fluxes)
+#pragma unroll
   for (int m = 1; m <= 6; ++m) {
-    double xcv[3];
-    const bool ex = face_exists(I, oi[m], oj[m], fa[m]);
-    const double fl = ex ? face_geo(I, l, oi[m], oj[m], fa[m], sgp, f, xcv) : 0.0;
-    const double flx = ex ? cell_flx(I, l, i, j, m, sgp, fl, ra_c) : 0.0;
-    ch[m] = flx / rho_c;
+    // faces 1-3 are the cell's own, 4-6 faces 1-3 of the neighbours 4-6
+    const double *pa = (m == 1) ? tJs : (m == 2) ? tI : (m == 3) ? tJ : (m == 4) ? tJsw : (m == 5) ? tIsw : tJs;
+    const double *pb = (m == 1) ? tI : (m == 2) ? tJ : (m == 3) ? tIw : (m == 4) ? tIw : (m == 5) ? tJsw : tIsw;
+    const int o = (m <= 3) ? c : cw[m], a = (m - 1) % 3;
+    const double *hn = I.GMTR_a + (size_t)a * gw + lg + o;
+    const double fl = 0.5 * ((pa[0] + pb[0]) * hn[0] + (pa[1] + pb[1]) * hn[3 * gw] + (pa[2] + pb[2]) * hn[6 * gw]);
+    ch[m] = cell_flx(I, l, i, j, m, sgp, fl, ra_c) / rho_c;
     chm[m] = mn64(ch[m], 0.0);
-    const double ch_own = (m <= 3) ? ch[m] : (fl * rarea(I, l, oi[m], oj[m]) * I.dt) / f(0, oi[m], oj[m]);
+    const double ch_own = (m <= 3) ? ch[m]
+                                   : (fl * I.GMTR_p[(size_t)(P_RAREA - 1) * gw + lg + o] * I.dt) / I.rho_in[slab + o];
     const bool cm = 0.5 - fsg(0.5, ch_own - EPS) != 0.0;
     if (cm == (m <= 3)) in |= 1u << m;
     else odd = odd || chm[m] != 0.0;
@@ -193,7 +224,6 @@ __global__ void k_fast_boundary(const __grid_constant__ MultiInst M) {
   // block: a region-boundary cell lies in [gmin, gmax]^2, so every point is in the block and
   // no index clamp applies.  Face 5's owner is the singular corner (gmin-1, gmin-1) when the
   // cell is (gmin, gmin) of a region with the singular point: then its points shift.
-  const bool sgp5 = sgp && i == I.gmin && j == I.gmin;
   // rhogq of the 3x3 block, one tracer ahead: the next tracer's loads are issued before this
   // tracer's stores (which the compiler may not move them across)
   const double *Q0 = I.Q_in + ((size_t)l * I.K + k) * I.gall + (size_t)(j - 2) * G + (i - 2);
