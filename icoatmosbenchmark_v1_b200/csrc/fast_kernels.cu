@@ -10,7 +10,6 @@
 //                    and pole passes read them.  One thread per (cell, level): the
 //                    face geometry once, then the tracers.
 //   k_fast_seam      FP64 flux and limited value of every seam face (below), all tracers.
-//   k_fast_pole      the two pole centres (horizontal + vertical), FP64.
 //   k_fast_faces     per (owner cell, level): the flux of its three faces (FP32 triangle
 //                    values; the seam pass's FP64 value on seams), the owner-side upwind
 //                    mask and the remap displacement of each face's upwind cell.
@@ -23,8 +22,9 @@
 //                    FP64 update of the tile cells and q of the next batch from its TMA window.
 //   k_fast_vert      vertical sub-step: one thread per (column, 4 tracers) streaming the
 //                    levels through a 3-level shared-memory ring of its own cp.async copies,
-//                    limiter two levels behind, FP64 update in place.
-//   k_fast_carry     halo points that no halo list writes keep their input values.
+//                    limiter two levels behind, FP64 update in place.  Its last blocks take the
+//                    two pole centres (horizontal + vertical, FP64; pole_columns) and the halo
+//                    points that no halo list writes, which keep their input values.
 //   gather           halo/pole fill of the new state (the COMM plan).
 //
 // Faces are "seam" faces when one of their two cells is a halo cell; the
@@ -433,103 +433,140 @@ __device__ __forceinline__ R eps_thr() { return (R)DBL_EPSILON; }
 // cell, i.e. the fixed per-face offset GRD_xr - GRD_x of its side plus the centroid
 // displacement -rhov rr dt / 2.  One thread per (owner cell, level); every tile that needs a
 // face reads these values, so the face's two cells see the same flux and mask.
-template <typename R>
-__global__ void k_fast_faces(const __grid_constant__ MultiInst M) {
+// A thread takes a cell through up to LV levels with its weights, normals and area in registers, and asks
+// L2 for its own fields of the next level; a thread per level loaded the 16 geometry values each time
+// (FP32, uneven batch: 584 -> 468 us; FP64, glevel 6, rlevel 1, kall 42: 141 -> 102).  8 levels, or 2 where
+// 8 would leave the card fewer threads than it holds.
+constexpr int kFaceLevels = 8, kFaceLevelsSmall = 2;
+constexpr long long kFaceThreads = 148LL * 1024;
+__host__ __device__ inline int face_level_blocks(int K, int lv) { return (K - 2 + lv - 1) / lv; }
+template <typename R, int LV>
+__global__ void __launch_bounds__(128) k_fast_faces(const __grid_constant__ MultiInst M) {
   using A = Arith<R>;
   long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int ii = find_inst(M, w, [](const FastInst &I) { return (long long)(I.l1 - I.l0) * (I.K - 2) * I.gall; });
+  const int ii = find_inst(M, w, [](const FastInst &I) { return (long long)(I.l1 - I.l0) * face_level_blocks(I.K, LV) * I.gall; });
   if (ii < 0) return;
   const FastInst &I = M.inst[ii];
   // 32-bit index arithmetic throughout (a 64-bit division or product is several times the
   // cost of this thread's arithmetic); the host keeps 3 * lall * kall * gall below 2^31
-  const unsigned wu = (unsigned)w, gall = (unsigned)I.gall, kin = (unsigned)(I.K - 2), Gu = (unsigned)I.G;
+  const unsigned wu = (unsigned)w, gall = (unsigned)I.gall, nkb = (unsigned)face_level_blocks(I.K, LV), Gu = (unsigned)I.G;
   const int G = I.G, c = (int)(wu % gall);
   const unsigned lk = wu / gall;
-  const int k = 1 + (int)(lk % kin), l = I.l0 + (int)(lk / kin);
+  const int kb = (int)(lk % nkb), l = I.l0 + (int)(lk / nkb);
   const int i = (int)((unsigned)c % Gu) + 1, j = (int)((unsigned)c / Gu) + 1;
-  const unsigned n3 = (unsigned)I.lall * (unsigned)I.K * gall, o = ((unsigned)l * (unsigned)I.K + (unsigned)k) * gall + c;
+  const unsigned n3 = (unsigned)I.lall * (unsigned)I.K * gall;
   const R dtf = (R)I.dt;
   auto interior = [&](int a, int b) { return a >= I.gmin && a <= I.gmax && b >= I.gmin && b <= I.gmax; };
   // faces between interior cells take the FP32 triangle form, seam faces the FP64 value of
   // k_fast_seam; AI = TJ(i,j-1) + TI(i,j), AIJ = TI(i,j) + TJ(i,j), AJ = TJ(i,j) + TI(i-1,j),
   // so the four triangles are formed once each, before any store
   bool ex[3], inner[3];
+  int sid[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const int ni = (a < 2) ? i + 1 : i, nj = (a > 0) ? j + 1 : j;
     ex[a] = i < G && j < G && face_exists(I, i, j, a + 1);
     inner[a] = ex[a] && interior(i, j) && interior(ni, nj);
+    sid[a] = (ex[a] && !inner[a]) ? I.seam_id[((unsigned)l * gall + c) * 3 + a] : 0;
   }
-  // the per-column face geometry of this region (see k_fast_offsets) and the fields of the six
-  // cells the four triangles touch: (i,j), (i+1,j), (i+1,j+1), (i,j+1), (i,j-1), (i-1,j); an
+  // the per-column face geometry of this region (see k_fast_offsets) and, per level, the fields of the
+  // six cells the four triangles touch: (i,j), (i+1,j), (i+1,j+1), (i,j+1), (i,j-1), (i-1,j); an
   // inner face has all six inside the region's array
   const R *geo = fast_face_geo(sizeof(R) == 8 ? (const R *)(const void *)I.off64 : (const R *)(const void *)I.off32, I) +
                  (unsigned)l * kFaceGeoPlanes * gall + c;
-  auto cellf = [&](int off, R f[4]) {
-    const unsigned q = (unsigned)((int)o + off);
-    f[0] = (R)I.rho_in[q];
-    if (sizeof(R) == 8) f[1] = (R)I.vx64[q], f[2] = (R)I.vy64[q], f[3] = (R)I.vz64[q];
-    else f[1] = (R)I.vx[q], f[2] = (R)I.vy[q], f[3] = (R)I.vz[q];
-  };
-  // triangle value v = f0 w1 + f1 w2 + f2 w3 with the weights at geometry offset gofs
-  auto tri = [&](const R f0[4], const R f1[4], const R f2[4], int gofs, int wp, R v[4]) {
-    const R w1 = geo[(int)wp * (int)gall + gofs], w2 = geo[(int)(wp + 1) * (int)gall + gofs],
-            w3 = geo[(int)(wp + 2) * (int)gall + gofs];
+  const bool any = inner[0] || inner[1] || inner[2];
+  R wI[3] = {}, wJ[3] = {}, wJm[3] = {}, wIm[3] = {}, hn[9] = {};
+  const R ra = geo[15 * gall];
+  if (any) {
 #pragma unroll
-    for (int x = 0; x < 4; ++x) v[x] = f0[x] * w1 + f1[x] * w2 + f2[x] * w3;
-  };
-  R tIij[4] = {}, tJij[4] = {}, tJm[4] = {}, tIm[4] = {};
-  if (inner[0] || inner[1] || inner[2]) {
-    R f00[4], f10[4], f11[4], f01[4], f0m[4], fm0[4];
-    cellf(0, f00), cellf(1, f10), cellf(G + 1, f11), cellf(G, f01);
-    if (inner[0]) cellf(-G, f0m);
-    if (inner[2]) cellf(-1, fm0);
-    if (inner[0] || inner[1]) tri(f00, f10, f11, 0, 0, tIij);   // TI(i,j)
-    if (inner[1] || inner[2]) tri(f00, f11, f01, 0, 3, tJij);   // TJ(i,j)
-    if (inner[0]) tri(f0m, f10, f00, -G, 3, tJm);               // TJ(i,j-1)
-    if (inner[2]) tri(fm0, f00, f01, -1, 0, tIm);               // TI(i-1,j)
-  }
-  double F[3];
-  R d[3][3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    F[a] = 0.0;
-    d[a][0] = d[a][1] = d[a][2] = R(0.0);
-    if (inner[a]) {
-      const R *p = (a == 0) ? tJm : (a == 1 ? tIij : tJij);
-      const R *q = (a == 0) ? tIij : (a == 1 ? tJij : tIm);
-      const R vx = p[1] + q[1], vy = p[2] + q[2], vz = p[3] + q[3];
-      const R rr = R(1.0) / A::mx(p[0] + q[0], A::RR_EPS);
-      const R Ff = R(0.5) * (vx * geo[(6 + 3 * a) * gall] + vy * geo[(7 + 3 * a) * gall] + vz * geo[(8 + 3 * a) * gall]);
-      F[a] = (double)Ff;
-      d[a][0] = -(vx * rr * dtf * R(0.5));
-      d[a][1] = -(vy * rr * dtf * R(0.5));
-      d[a][2] = -(vz * rr * dtf * R(0.5));
-    } else if (ex[a]) {  // seam face
-      const int sid = I.seam_id[((unsigned)l * gall + c) * 3 + a];
-      F[a] = I.sflux[(unsigned)k * (unsigned)I.ns + sid];
+    for (int n = 0; n < 3; ++n) {
+      wI[n] = geo[n * gall], wJ[n] = geo[(3 + n) * gall];
+      if (inner[0]) wJm[n] = geo[(int)((3 + n) * gall) - G];
+      if (inner[2]) wIm[n] = geo[(int)(n * gall) - 1];
     }
+#pragma unroll
+    for (int n = 0; n < 9; ++n) hn[n] = geo[(6 + n) * gall];
   }
-  // the owner's Courant number of each face and its upwind mask, in the form the tile kernel
-  // used to form them (FP32 flux, rarea and 1/rho of the owner), and the upwind side's offset
-  const R ra = geo[15 * gall], rinv = (R)(1.0 / I.rho_in[o]);
-  const R EPSf = eps_thr<R>();
   const R *offs = (sizeof(R) == 8 ? (const R *)(const void *)I.off64 : (const R *)(const void *)I.off32) +
                   (unsigned)l * kOffPlanes * gall + c;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    I.Fg[a * n3 + o] = F[a];
-    const R chown = ((R)F[a] * ra * dtf) * rinv;
-    const bool cm = (R(0.5) - A::sgn(R(0.5), chown - EPSf)) != R(0.0);
-    R v[3] = {R(0.0), R(0.0), R(0.0)};
-    if (inner[a]) {
-      const R *ob = offs + (a * 6 + (cm ? 3 : 0)) * gall;
-#pragma unroll
-      for (int x = 0; x < 3; ++x) v[x] = ob[x * gall] + d[a][x];
+  const R EPSf = eps_thr<R>();
+  const int k1 = min(1 + (kb + 1) * LV, I.K - 1);
+#pragma unroll 1
+  for (int k = 1 + kb * LV; k < k1; ++k) {
+    const unsigned o = ((unsigned)l * (unsigned)I.K + (unsigned)k) * gall + c;
+    if (k + 1 < k1) {
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(I.rho_in + o + gall));
+      if (sizeof(R) == 8) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(I.vx64 + o + gall));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(I.vy64 + o + gall));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(I.vz64 + o + gall));
+      } else {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(I.vx + o + gall));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(I.vy + o + gall));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(I.vz + o + gall));
+      }
     }
-    const R wm = cm ? R(1.0) : R(0.0);
-    if (sizeof(R) == 8) I.dupc64[a * n3 + o] = make_double4(v[0], v[1], v[2], wm);
-    else I.dupc[a * n3 + o] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)wm);
+    auto cellf = [&](int off, R f[4]) {
+      const unsigned q = (unsigned)((int)o + off);
+      f[0] = (R)I.rho_in[q];
+      if (sizeof(R) == 8) f[1] = (R)I.vx64[q], f[2] = (R)I.vy64[q], f[3] = (R)I.vz64[q];
+      else f[1] = (R)I.vx[q], f[2] = (R)I.vy[q], f[3] = (R)I.vz[q];
+    };
+    // triangle value v = f0 w1 + f1 w2 + f2 w3
+    auto tri = [&](const R f0[4], const R f1[4], const R f2[4], const R (&w)[3], R v[4]) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x) v[x] = f0[x] * w[0] + f1[x] * w[1] + f2[x] * w[2];
+    };
+    R tIij[4] = {}, tJij[4] = {}, tJm[4] = {}, tIm[4] = {};
+    const double rho_c = I.rho_in[o];
+    if (any) {
+      R f00[4], f10[4], f11[4], f01[4], f0m[4], fm0[4];
+      cellf(0, f00), cellf(1, f10), cellf(G + 1, f11), cellf(G, f01);
+      if (inner[0]) cellf(-G, f0m);
+      if (inner[2]) cellf(-1, fm0);
+      if (inner[0] || inner[1]) tri(f00, f10, f11, wI, tIij);   // TI(i,j)
+      if (inner[1] || inner[2]) tri(f00, f11, f01, wJ, tJij);   // TJ(i,j)
+      if (inner[0]) tri(f0m, f10, f00, wJm, tJm);               // TJ(i,j-1)
+      if (inner[2]) tri(fm0, f00, f01, wIm, tIm);               // TI(i-1,j)
+    }
+    double F[3];
+    R d[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      F[a] = 0.0;
+      d[a][0] = d[a][1] = d[a][2] = R(0.0);
+      if (inner[a]) {
+        const R *p = (a == 0) ? tJm : (a == 1 ? tIij : tJij);
+        const R *q = (a == 0) ? tIij : (a == 1 ? tJij : tIm);
+        const R vx = p[1] + q[1], vy = p[2] + q[2], vz = p[3] + q[3];
+        const R rr = R(1.0) / A::mx(p[0] + q[0], A::RR_EPS);
+        const R Ff = R(0.5) * (vx * hn[3 * a] + vy * hn[3 * a + 1] + vz * hn[3 * a + 2]);
+        F[a] = (double)Ff;
+        d[a][0] = -(vx * rr * dtf * R(0.5));
+        d[a][1] = -(vy * rr * dtf * R(0.5));
+        d[a][2] = -(vz * rr * dtf * R(0.5));
+      } else if (ex[a]) {  // seam face
+        F[a] = I.sflux[(unsigned)k * (unsigned)I.ns + sid[a]];
+      }
+    }
+    // the owner's Courant number of each face and its upwind mask, in the form the tile kernel
+    // used to form them (FP32 flux, rarea and 1/rho of the owner), and the upwind side's offset
+    const R rinv = (R)(1.0 / rho_c);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      I.Fg[a * n3 + o] = F[a];
+      const R chown = ((R)F[a] * ra * dtf) * rinv;
+      const bool cm = (R(0.5) - A::sgn(R(0.5), chown - EPSf)) != R(0.0);
+      R v[3] = {R(0.0), R(0.0), R(0.0)};
+      if (inner[a]) {
+        const R *ob = offs + (a * 6 + (cm ? 3 : 0)) * gall;
+#pragma unroll
+        for (int x = 0; x < 3; ++x) v[x] = ob[x * gall] + d[a][x];
+      }
+      const R wm = cm ? R(1.0) : R(0.0);
+      if (sizeof(R) == 8) I.dupc64[a * n3 + o] = make_double4(v[0], v[1], v[2], wm);
+      else I.dupc[a * n3 + o] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)wm);
+    }
   }
 }
 
@@ -1385,48 +1422,22 @@ __device__ __forceinline__ void vert_block(const FastInst &I, long long blk) {
   }
   cp_async_wait_all();  // the trailing groups are empty; nothing is left in flight at exit
 }
-template <int TV, typename R>
-__global__ void __launch_bounds__(256, 2) k_fast_vert1(FastInst I) {
-  vert_block<TV, R>(I, blockIdx.x);
-}
-
-template <int TV, typename R>
-__global__ void __launch_bounds__(256, 2) k_fast_vert(const __grid_constant__ MultiInst M) {
-  // blocks of an instance: (tracer group fastest, column block)
-  long long blk = blockIdx.x;
-  const int ii = find_inst(M, blk, [](const FastInst &J) {
-    const long long nc = (long long)(J.l1 - J.l0) * (J.gmax - J.gmin + 1) * (J.gmax - J.gmin + 1);
-    return (long long)((J.ntr + TV - 1) / TV) * ((nc + 255) / 256);
-  });
-  switch (ii) {
-    case 0: vert_block<TV, R>(M.inst[0], blk); break;
-    case 1: vert_block<TV, R>(M.inst[1], blk); break;
-    case 2: vert_block<TV, R>(M.inst[2], blk); break;
-    case 3: vert_block<TV, R>(M.inst[3], blk); break;
-    default: break;
-  }
-}
-
 // ---- the two pole centres, FP64: one CTA per (pole, tracer), one thread per level ----------
 // The horizontal sub-step of every level, then the vertical one of the column: its Qout of a
 // level needs only q and the Courant numbers, so every stage is level-parallel.  Each value
 // takes the operations of the column form; this file allows FMA contraction, so results
 // can differ from that form at FP64 rounding.
-template <int KMAX>
-__global__ void __launch_bounds__(KMAX) k_fast_pole(const __grid_constant__ MultiInst M) {
-  long long tl = blockIdx.x;
-  const int ii = find_inst(M, tl, [](const FastInst &J) { return J.poles ? (long long)kLallPl * J.ntr : 0LL; });
-  if (ii < 0) return;  // whole CTA
-  const FastInst &I = M.inst[ii];
-  const int t = (int)tl;
-  const int p = t % kLallPl, tr = t / kLallPl;
+// Its own function, so that the column kernels, whose last blocks run it, keep their registers; sm: 9 x
+// kPoleLevels values.
+constexpr int kPoleLevels = 128;
+__device__ __noinline__ void pole_columns(const FastInst &I, int p, int tr, double *sm) {
   const int K = I.K, k = threadIdx.x;
   const int kmin = 1, kmax = K - 2;
   const size_t toff = (size_t)tr * kLallPl * K * kGallPl;
   const double rarea = I.GMTR_p_pl[((size_t)(P_RAREA - 1) * kLallPl + p) * kGallPl];
   const double BIG = DBL_MAX, EPS = DBL_EPSILON;
-  __shared__ double sQh[KMAX], srh[KMAX], sq[KMAX], sqh[KMAX], sck1[KMAX], sck2[KMAX], sQmn[KMAX], sQmx[KMAX],
-      sinfl[KMAX];
+  double *sQh = sm, *srh = sm + kPoleLevels, *sq = srh + kPoleLevels, *sqh = sq + kPoleLevels, *sck1 = sqh + kPoleLevels,
+         *sck2 = sck1 + kPoleLevels, *sQmn = sck2 + kPoleLevels, *sQmx = sQmn + kPoleLevels, *sinfl = sQmx + kPoleLevels;
   // ---- horizontal sub-step of level k
   if (k >= kmin && k <= kmax) {
     const size_t off = ((size_t)p * K + k) * kGallPl;
@@ -1525,17 +1536,61 @@ __global__ void __launch_bounds__(KMAX) k_fast_pole(const __grid_constant__ Mult
 }
 
 // ---- halo points no list writes keep their input values (the reference never touches them)
-__global__ void k_fast_carry(const __grid_constant__ MultiInst M) {
-  long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int ii = find_inst(M, tid, [](const FastInst &J) { return (long long)J.ncarry * J.K; });
-  if (ii < 0) return;
-  const FastInst &I = M.inst[ii];
-  const int p = I.carry[tid % I.ncarry], k = (int)(tid / I.ncarry);
+__device__ __forceinline__ void carry_point(const FastInst &I, long long u) {
+  const int p = I.carry[u % I.ncarry], k = (int)(u / I.ncarry);
   if (p < 0 || !owns_point(I, p)) return;
   const int l = p / I.gall, c = p % I.gall;
   const size_t off = ((size_t)l * I.K + k) * I.gall + c, tstride = (size_t)I.lall * I.K * I.gall;
   I.rho_out[off] = I.rho_in[off];
   for (int t = 0; t < I.ntr; ++t) I.Q_out[(size_t)t * tstride + off] = I.Q_in[(size_t)t * tstride + off];
+}
+
+// ---- the column launch: column blocks, then one block per (pole, tracer), then the carried points (which
+// used to be two small launches behind one another, 14 us of every step)
+template <int TV>
+__host__ __device__ __forceinline__ long long vert_blocks(const FastInst &J) {
+  const long long nc = (long long)(J.l1 - J.l0) * (J.gmax - J.gmin + 1) * (J.gmax - J.gmin + 1);
+  return (long long)((J.ntr + TV - 1) / TV) * ((nc + 255) / 256);
+}
+__host__ __device__ __forceinline__ long long pole_blocks(const FastInst &J) {
+  return J.poles ? (long long)kLallPl * J.ntr : 0LL;
+}
+__host__ __device__ __forceinline__ long long carry_blocks(const FastInst &J) {
+  return ((long long)J.ncarry * J.K + 255) / 256;
+}
+// block blk of the poles' and carried points' blocks of one instance
+__device__ __forceinline__ void vert_rest(const FastInst &I, long long blk) {
+  extern __shared__ __align__(16) unsigned char vraw[];
+  const long long np = pole_blocks(I);
+  if (blk < np) {
+    pole_columns(I, (int)(blk % kLallPl), (int)(blk / kLallPl), (double *)vraw);
+    return;
+  }
+  const long long u = (blk - np) * 256 + threadIdx.x;
+  if (u < (long long)I.ncarry * I.K) carry_point(I, u);
+}
+
+template <int TV, typename R>
+__global__ void __launch_bounds__(256, 2) k_fast_vert1(const __grid_constant__ FastInst I) {
+  const long long n = vert_blocks<TV>(I);
+  if (blockIdx.x < n) vert_block<TV, R>(I, blockIdx.x);
+  else vert_rest(I, blockIdx.x - n);
+}
+
+template <int TV, typename R>
+__global__ void __launch_bounds__(256, 2) k_fast_vert(const __grid_constant__ MultiInst M) {
+  // blocks of an instance: (tracer group fastest, column block)
+  long long blk = blockIdx.x;
+  const int ii = find_inst(M, blk, [](const FastInst &J) { return vert_blocks<TV>(J); });
+  switch (ii) {
+    case 0: vert_block<TV, R>(M.inst[0], blk); return;
+    case 1: vert_block<TV, R>(M.inst[1], blk); return;
+    case 2: vert_block<TV, R>(M.inst[2], blk); return;
+    case 3: vert_block<TV, R>(M.inst[3], blk); return;
+    default: break;
+  }
+  const int ir = find_inst(M, blk, [](const FastInst &J) { return pole_blocks(J) + carry_blocks(J); });
+  if (ir >= 0) vert_rest(M.inst[ir], blk);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1657,40 +1712,35 @@ cudaError_t fast_step_multi(const MultiInst &M, int shape, cudaStream_t st, cuda
   if (M.n < 1 || M.n > kMaxInst) return cudaErrorInvalidValue;
   for (int i = 0; i < M.n; ++i)
     if (M.inst[i].l0 < 0 || M.inst[i].l1 > M.inst[i].lall || M.inst[i].l1 <= M.inst[i].l0) return cudaErrorInvalidValue;
-  long long nbk = 0, nsk = 0, npl = 0, nc = 0, nvb = 0, nvb64 = 0, nfk = 0;
+  long long nbk = 0, nsk = 0, nvb = 0, nvb64 = 0, nfk = 0, nfk2 = 0;
   int kmax = 0;
   constexpr int TV = 4, TV64 = 2;  // tracers per column thread: FP32, FP64 variant
   for (int i = 0; i < M.n; ++i) {
     const FastInst &I = M.inst[i];
-    const long long n = I.gmax - I.gmin + 1, ncol = (long long)(I.l1 - I.l0) * n * n;
     nbk += (long long)I.nb * (I.K - 2);
     nsk += (long long)I.ns * (I.K - 2);
-    nfk += (long long)(I.l1 - I.l0) * (I.K - 2) * I.gall;
-    npl += I.poles ? (long long)kLallPl * I.ntr : 0LL;
-    nc += (long long)I.ncarry * I.K;
-    nvb += (long long)((I.ntr + TV - 1) / TV) * ((ncol + 255) / 256);
-    nvb64 += (long long)((I.ntr + TV64 - 1) / TV64) * ((ncol + 255) / 256);
+    nfk += (long long)(I.l1 - I.l0) * face_level_blocks(I.K, kFaceLevels) * I.gall;
+    nfk2 += (long long)(I.l1 - I.l0) * face_level_blocks(I.K, kFaceLevelsSmall) * I.gall;
+    const long long rest = pole_blocks(I) + carry_blocks(I);
+    nvb += vert_blocks<TV>(I) + rest;
+    nvb64 += vert_blocks<TV64>(I) + rest;
     kmax = I.K > kmax ? I.K : kmax;
   }
-  if (kmax > 128) return cudaErrorInvalidValue;
+  if (kmax > kPoleLevels) return cudaErrorInvalidValue;
   if (parts & 1u) {  // the boundary values other regions read (exchanged between ranks when sharded)
     k_fast_boundary<<<(unsigned)((nbk + 127) / 128), 128, 0, st>>>(M);
     launches += 1;
   }
   if (!(parts & 2u)) return cudaGetLastError();
   k_fast_seam<<<(unsigned)((nsk + 127) / 128), 128, 0, st>>>(M);
-  if (npl > 0) {
-    if (kmax <= 64) k_fast_pole<64><<<(unsigned)npl, 64, 0, st>>>(M);
-    else k_fast_pole<128><<<(unsigned)npl, 128, 0, st>>>(M);
-    launches += 1;
-  }
   if (ev0) cudaEventRecord(ev0, st);
   const bool f64 = M.inst[0].f64 != 0;
   for (int i = 1; i < M.n; ++i)
     if ((M.inst[i].f64 != 0) != f64) return cudaErrorInvalidValue;  // one precision per batch
   cudaError_t e;
   if (!f64) {
-    k_fast_faces<float><<<(unsigned)((nfk + 127) / 128), 128, 0, st>>>(M);
+    if (nfk >= kFaceThreads) k_fast_faces<float, kFaceLevels><<<(unsigned)((nfk + 127) / 128), 128, 0, st>>>(M);
+    else k_fast_faces<float, kFaceLevelsSmall><<<(unsigned)((nfk2 + 127) / 128), 128, 0, st>>>(M);
     switch (shape) {
       case 0: e = launch_tile<16, 16, 4, float>(M, st); break;
       case 1: e = launch_tile<16, 16, 8, float>(M, st); break;
@@ -1703,7 +1753,8 @@ cudaError_t fast_step_multi(const MultiInst &M, int shape, cudaStream_t st, cuda
       default: return cudaErrorInvalidValue;
     }
   } else {  // FP64 variant: the same tiles, 2 tracers per batch (FP64 shared data and registers)
-    k_fast_faces<double><<<(unsigned)((nfk + 127) / 128), 128, 0, st>>>(M);
+    if (nfk >= kFaceThreads) k_fast_faces<double, kFaceLevels><<<(unsigned)((nfk + 127) / 128), 128, 0, st>>>(M);
+    else k_fast_faces<double, kFaceLevelsSmall><<<(unsigned)((nfk2 + 127) / 128), 128, 0, st>>>(M);
     switch (shape) {
       case 0: case 1: case 2: e = launch_tile<16, 16, 2, double>(M, st); break;
       case 3: e = launch_tile<14, 14, 2, double>(M, st); break;
@@ -1717,6 +1768,7 @@ cudaError_t fast_step_multi(const MultiInst &M, int shape, cudaStream_t st, cuda
   if (ev1) cudaEventRecord(ev1, st);
   if (e != cudaSuccess) return e;
   constexpr int vsm = (int)sizeof(VertRing<TV, float>), vsm64 = (int)sizeof(VertRing<TV64, double>);
+  static_assert(vsm >= 9 * kPoleLevels * 8 && vsm64 >= 9 * kPoleLevels * 8, "the poles' blocks use the ring's memory");
   static_assert(vsm <= 48 * 1024 && vsm64 <= 48 * 1024, "the column ring fits the default shared-memory limit");
   if (!f64) {
     if (M.n == 1) k_fast_vert1<TV, float><<<(unsigned)nvb, 256, vsm, st>>>(M.inst[0]);
@@ -1725,8 +1777,7 @@ cudaError_t fast_step_multi(const MultiInst &M, int shape, cudaStream_t st, cuda
     if (M.n == 1) k_fast_vert1<TV64, double><<<(unsigned)nvb64, 256, vsm64, st>>>(M.inst[0]);
     else k_fast_vert<TV64, double><<<(unsigned)nvb64, 256, vsm64, st>>>(M);
   }
-  k_fast_carry<<<(unsigned)((nc + 127) / 128), 128, 0, st>>>(M);
-  launches += 5;
+  launches += 4;
   return cudaGetLastError();
 }
 
