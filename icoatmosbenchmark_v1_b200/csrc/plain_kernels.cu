@@ -161,13 +161,13 @@ __global__ void __launch_bounds__(kFluxThreads, 4) k_horizontal_flux(Dims D, Flu
         const T flux = T(0.5) * (v[0] * hn[a][0] + v[1] * hn[a][1] + v[2] * hn[a][2]);
         f = flux * ra[0] * dt;
         const unsigned nb = c + (a == 0 ? 1 : (a == 1 ? G + 1 : G));
-        fln[nb] = (a == 2 && singJ) ? T(0) : -flux * ra[a + 1] * dt;
+        __stcs(fln + nb, (a == 2 && singJ) ? T(0) : -flux * ra[a + 1] * dt);
 #pragma unroll
         for (int d = 0; d < 3; ++d) x[d] = xr[a][d] - v[d] * rrhoa2 * dt * T(0.5);
       }
-      flx[c] = f;
+      __stcs(flx + c, f);
 #pragma unroll
-      for (int d = 0; d < 3; ++d) (out.GRD_xc + ((size_t)d * 3 + a) * fs + off)[c] = x[d];
+      for (int d = 0; d < 3; ++d) __stcs(out.GRD_xc + ((size_t)d * 3 + a) * fs + off + c, x[d]);
       if (own[a]) fln[c] = T(0);
     }
   }
