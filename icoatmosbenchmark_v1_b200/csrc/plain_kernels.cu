@@ -450,9 +450,8 @@ __device__ __forceinline__ void pole_apply(const Dims &D, const LimIn<T> &in, T 
 // level needs the Qout of the levels on both sides and nothing else of the column, so the columns
 // are cut into chunks that share one Qout at each cut (one in kVlimLevels is formed twice).  With a
 // column per thread a glevel-6 grid gave the card 341 blocks and a chain of 40 dependent levels
-// (69 us, and 56 us more for the 12 pole columns in a launch behind it); now bound by memory:
-// 170 us for glevel 7, kall 96 (0.78 GB, 120 us at the copy rate; 8 and 16 levels a thread alike,
-// 4 levels 188), and below the call's host time at glevel 6 (132 -> 27 us a call).
+// (69 us, and 56 us more for the 12 pole columns in a launch behind it).  Now 23 us there, of the 13.5
+// its 88 MB need (4 levels a thread 25, 13 levels 28), and 170 us for glevel 7, kall 96 (0.78 GB, 120 us).
 constexpr int kVlimLevels = 8, kVlimThreads = 128;
 
 template <typename T>
@@ -482,8 +481,11 @@ __device__ __forceinline__ void vlim_qout(T qm, const VlimLevel<T> &v, T qp, T c
     CQmax = inflagL * c1 * maxL + inflagU * c2 * maxU;
   }
   const T zerosw = T(0.5) - fsign(T(0.5), fabs(Cout) - EPS);
-  Qmin = ((qk - qnmax) + qnmax * (Cin + Cout - v.d) - CQmax) / (Cout + zerosw) * (T(1) - zerosw) + qk * zerosw;
-  Qmax = ((qk - qnmin) + qnmin * (Cin + Cout - v.d) - CQmin) / (Cout + zerosw) * (T(1) - zerosw) + qk * zerosw;
+  T o[2] = {(qk - qnmax) + qnmax * (Cin + Cout - v.d) - CQmax, (qk - qnmin) + qnmin * (Cin + Cout - v.d) - CQmin};
+  if constexpr (sizeof(T) == 8) quotients(o, recip(Cout + zerosw));
+  else o[0] = o[0] / (Cout + zerosw), o[1] = o[1] / (Cout + zerosw);
+  Qmin = o[0] * (T(1) - zerosw) + qk * zerosw;
+  Qmax = o[1] * (T(1) - zerosw) + qk * zerosw;
 }
 
 // half levels [k0, k0 + kVlimLevels) (0-based, below kmax) of one column; arrays at the column's
