@@ -52,8 +52,9 @@ template <typename T> __device__ __forceinline__ T fsign(T a, T b) { return copy
 // face by face took 72 field loads and 1000 instructions a cell and level; these are 570, and what
 // bounds the kernel is the latency of a level's loads at 4 blocks per SM, so each thread asks for its
 // own cell's fields of the next level one level ahead (its neighbours' are other threads' own).
-// glevel 7, rlevel 1, kall 61 (1.6 GB, 248 us at the copy rate): 642 -> 359 us; 433 without the
-// prefetch, 371 at 3 blocks, 452 with 4 levels a thread; with the geometry in shared memory 470 and more.
+// glevel 7, rlevel 1, kall 61 (1.6 GB, 248 us at the copy rate): 642 -> 344 us, 359 of it
+// before the outputs took the streaming hint; then 433 without the prefetch, 371 at 3 blocks, 452 with 4
+// levels a thread; with the geometry in shared memory 470 and more.
 constexpr int kFluxThreads = 128, kFluxLevels = 8;
 
 template <typename T>
@@ -547,7 +548,10 @@ __global__ void __launch_bounds__(kVlimThreads) k_vlim(Dims D, int nchunk, int c
 // ---------------------------------------------------------------------------
 // halo/pole fill as one gather: var(dst) = var(src) for every (entry, k, v), of one array or of two
 // (a step's rhogq and rhog).  A thread takes one entry through kGatherPlanes (k, v) planes: the
-// points' addresses are worked out once and that many loads are in flight.
+// points' addresses are worked out once and that many loads are in flight.  Bound by DRAM
+// sectors: a point of a region's i-edge column costs 64 bytes read and 64 written for its 16.  One element
+// a thread -> 4 planes: 143 -> 122 us (glevel 7, kall 96, 16 arrays), 298 -> 255 (glevel 8), 13.6 -> 11.6
+// (glevel 6, kall 42, 8 arrays); 8 and 16 planes were slower.
 constexpr int kGatherThreads = 128, kGatherPlanes = 4;
 
 template <typename T>

@@ -41,7 +41,7 @@ namespace icoadv {
 //
 // A face value travels once through memory (24 bytes written and read per update); gradient,
 // remap value, Courant number, mask and Qout never do.  Against one launch per piece and tracer
-// (14 launches a tracer, a column's levels in local memory): 9.90 -> 3.25 ms for glevel 7, kall 61,
+// (14 launches a tracer, a column's levels in local memory): 9.90 -> 3.17 ms for glevel 7, kall 61,
 // 5 tracers, 1.59 -> 0.30 ms for glevel 5, kall 42, 8 tracers.  Every value is the result of the
 // reference's operation sequence; where the reference blends two sides by a mask of 0 or 1
 // (c a + (1 - c) b), the chosen side is taken, which is the same number.
@@ -80,7 +80,7 @@ __device__ __forceinline__ void pole_centre(const PlainArgs &P, int t, int p, in
   o[4] = (q[0] - CQmin - qnmin * (1.0 - Cin - Cout + dn)) / (Cout + zsw) * (1.0 - zsw) + q[0] * zsw;
 }
 
-// Bound by instruction issue and latency: 1.67 ms of the 3.25, of which the set-up of a level (620
+// Bound by instruction issue and latency: 1.67 ms of the 3.17, of which the set-up of a level (620
 // instructions a cell against 550 per tracer) is a third.  One tracer per pass of the loop and two
 // blocks per SM keep every value in registers; two tracers, or three blocks, spill and take 2.5-2.6
 // ms.  The next level's set-up inputs are asked for while a level's tracers go through (1.72 without).
