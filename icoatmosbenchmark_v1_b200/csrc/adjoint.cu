@@ -898,7 +898,18 @@ __global__ void k_adj_rhoh_ch_pl(int kall, const double *rho_pl, const double *f
 // horizontal_flux.  Triangle values (:141-201): TI(ij) from (ij, ip1j, ip1jp1),
 // TJ(ij) from (ij, ip1jp1, ijp1), TI(gmin-1,gmin-1) = TJ(gmin,gmin-1) on a
 // singular region.  A face sums its two triangles: AI(ij) = TJ(ijm1) + TI(ij),
-// AIJ(ij) = TI(ij) + TJ(ij), AJ(ij) = TJ(ij) + TI(im1j).
+// AIJ(ij) = TI(ij) + TJ(ij), AJ(ij) = TJ(ij) + TI(im1j), and hands both of them the
+// same adjoint, so each face is transposed once (k_adj_tri) and the fields gather from
+// the faces of the six triangles around a point (k_adj_fields).  Both kernels stream a
+// cell's levels with its weights and normals in registers, as the forward does, and ask
+// for the next level's planes while a level is worked on: the latency of a level's loads
+// bounds them.  One thread per triangle pair and level (each face transposed five times,
+// twelve triangle values a cell) took 2.38 + 1.03 ms at glevel 7, kall 96.  At glevel 6,
+// kall 42: 119 + 112 us a step, of 70 + 45 at the copy rate; k_adj_tri at 3 blocks per SM
+// 136, without the prefetch 145, 5 blocks 206 (spills), 16 levels a thread 170;
+// k_adj_fields without the prefetch 122.
+constexpr int kAdjFluxThreads = 128, kAdjFluxLevels = 8;  // levels a thread
+
 struct Fld {
   const double *f[4];  // rho, rhovx, rhovy, rhovz
 };
@@ -906,122 +917,159 @@ struct Tv {
   double v[4];
 };
 
-__device__ __forceinline__ Tv tri(const Dims &D, const Fld &F, const double *GT, int l, size_t off, int c, int t) {
-  // t = 1 (TI), 2 (TJ); c 0-based owner
-  const size_t gw = (size_t)D.gall * D.lall;
-  const int G = D.gall_1d;
-  const double w1 = GT[((size_t)(W1 - 1) * 2 + (t - 1)) * gw + (size_t)l * D.gall + c];
-  const double w2 = GT[((size_t)(W2 - 1) * 2 + (t - 1)) * gw + (size_t)l * D.gall + c];
-  const double w3 = GT[((size_t)(W3 - 1) * 2 + (t - 1)) * gw + (size_t)l * D.gall + c];
-  const int b = (t == 1) ? c + 1 : c + G + 1, e = (t == 1) ? c + G + 1 : c + G;
+__device__ __forceinline__ Tv tri(const Tv &f0, const Tv &f1, const Tv &f2, const double (&w)[3]) {
   Tv r;
-  for (int x = 0; x < 4; ++x) r.v[x] = F.f[x][off + c] * w1 + F.f[x][off + b] * w2 + F.f[x][off + e] * w3;
+#pragma unroll
+  for (int x = 0; x < 4; ++x) r.v[x] = f0.v[x] * w[0] + f1.v[x] * w[1] + f2.v[x] * w[2];
   return r;
 }
-__device__ __forceinline__ Tv triI(const Dims &D, const Fld &F, const double *GT, int l, size_t off, int c, bool sgp) {
-  const int G = D.gall_1d;
-  if (sgp && c == (D.gmin - 2) * G + (D.gmin - 2)) return tri(D, F, GT, l, off, c + 1, 2);
-  return tri(D, F, GT, l, off, c, 1);
-}
 
-// adjoint of one face's (flux, xc) -> its two triangles (aT gets += for both)
-__device__ __forceinline__ void face_adj(const Dims &D, const Geo<double> &g, const double *a_flx,
-                                         const double *a_xc, double dt, int l, size_t off, size_t fs, int o, int a,
-                                         bool sgp, const Tv &p, const Tv &q, Tv &ap) {
-  // a_flx and a_xc hold what an interior cell on either side contributed; a face has them only there
-  const size_t gw = (size_t)D.gall * D.lall;
-  const int G = D.gall_1d;
-  const int nb = (a == 1) ? o + 1 : ((a == 2) ? o + G + 1 : o + G);
-  const double rsum = p.v[0] + q.v[0];
-  double vs[3];
-  for (int x = 0; x < 3; ++x) vs[x] = p.v[x + 1] + q.v[x + 1];
-  const double rr = 1.0 / mx(rsum, kEps);
-  const bool inO = inner(D, o % G + 1, o / G + 1), inN = inner(D, nb % G + 1, nb / G + 1);
-  if (!inO && !inN) return;
-  double aflux = !inO ? 0.0 : a_flx[(size_t)(a - 1) * fs + off + o] * g.GMTR_p[(size_t)(P_RAREA - 1) * gw + (size_t)l * D.gall + o] * dt;
-  const bool sg0 = sgp && a == 3 && nb == (D.gmin - 1) * G + (D.gmin - 1);
-  if (!sg0 && inN)
-    aflux += -a_flx[(size_t)(a + 2) * fs + off + nb] * g.GMTR_p[(size_t)(P_RAREA - 1) * gw + (size_t)l * D.gall + nb] *
-             dt;
-  double avs[3], arr = 0.0;
-  for (int x = 0; x < 3; ++x)
-    avs[x] = 0.5 * aflux * g.GMTR_a[((size_t)x * 3 + (a - 1)) * gw + (size_t)l * D.gall + o];
-  for (int x = 0; x < 3; ++x) {
-    const double ax = a_xc[((size_t)x * 3 + (a - 1)) * fs + off + o];
-    avs[x] += -ax * rr * dt * 0.5;
-    arr += -ax * vs[x] * dt * 0.5;
-  }
-  const double ars = (rsum > kEps) ? -arr * rr * rr : 0.0;
-  ap.v[0] += ars;
-  for (int x = 0; x < 3; ++x) ap.v[x + 1] += avs[x];
-}
-
-// triangle adjoints of owner p: TI(p) from AI(p), AIJ(p), AJ(p+1); TJ(p) from AI(p+G), AIJ(p), AJ(p)
-__global__ void k_adj_tri(Dims D, Geo<double> g, Fld F, const double *a_flx, const double *a_xc, double dt,
-                          double *aT) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
-  const int i = c % G + 1, j = c / G + 1;
-  const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall;
-  const int k = kl % D.kall;
-  if (k < D.kmin - 1 || k >= D.kmax) return;  // the ghost levels have no part in the step
-  Tv aI{}, aJ{};
-  const int lo = D.gmin - 1, hi = D.gmax;
-  if (i >= lo && i <= hi && j >= lo && j <= hi) {
-    const bool sgp = D.have_sgp[l] != 0;
-    const double *GT = g.GMTR_t;
-    const Tv tI = triI(D, F, GT, l, off, c, sgp), tJ = tri(D, F, GT, l, off, c, 2);
-    if (j >= D.gmin) face_adj(D, g, a_flx, a_xc, dt, l, off, fs, c, 1, sgp, tri(D, F, GT, l, off, c - G, 2), tI, aI);
-    {
-      Tv a2{};
-      face_adj(D, g, a_flx, a_xc, dt, l, off, fs, c, 2, sgp, tI, tJ, a2);
-      for (int x = 0; x < 4; ++x) aI.v[x] += a2.v[x], aJ.v[x] += a2.v[x];
-    }
-    if (i + 1 >= D.gmin && i + 1 <= hi)
-      face_adj(D, g, a_flx, a_xc, dt, l, off, fs, c + 1, 3, sgp, tri(D, F, GT, l, off, c + 1, 2), tI, aI);
-    if (j + 1 >= D.gmin && j + 1 <= hi)
-      face_adj(D, g, a_flx, a_xc, dt, l, off, fs, c + G, 1, sgp, tJ, triI(D, F, GT, l, off, c + G, sgp), aJ);
-    if (i >= D.gmin) face_adj(D, g, a_flx, a_xc, dt, l, off, fs, c, 3, sgp, tJ, triI(D, F, GT, l, off, c - 1, sgp), aJ);
-  }
-  for (int x = 0; x < 4; ++x) {
-    aT[(size_t)x * fs + off + c] = aI.v[x];
-    aT[(size_t)(4 + x) * fs + off + c] = aJ.v[x];
-  }
-}
-
-// fields from the triangles: point p is ij of TI/TJ(p) (W1), ip1j of TI(p-1) (W2),
-// ip1jp1 of TI(p-G-1) (W3) and TJ(p-G-1) (W2), ijp1 of TJ(p-G) (W3); on a singular
-// region TI(gmin-1,gmin-1) is TJ(gmin,gmin-1)
-__global__ void k_adj_fields(Dims D, const double *GT, const double *aT, double *a0, double *a1, double *a2,
-                             double *a3) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= D.gall) return;
-  const int kl = blockIdx.y, l = kl / D.kall, G = D.gall_1d;
-  const size_t off = (size_t)kl * D.gall, fs = (size_t)D.lall * D.kall * D.gall, gw = (size_t)D.gall * D.lall;
+// A face's adjoint of its triangles' (rho, rhovx, rhovy, rhovz) sum: the wind parts take the place of
+// a_xc, which nothing else reads any more, the density part goes to a_rs (3 fields); zero where a cell
+// owns no face.  a_flx and a_xc hold what an interior cell on either side contributed; a face has them
+// only there.  blocks: level blocks fastest, then cell blocks, then regions
+__global__ void __launch_bounds__(kAdjFluxThreads, 4) k_adj_tri(Dims D, Geo<double> g, Fld F, const double *a_flx,
+                                                               double *a_xc, double dt, double *a_rs, int lpb,
+                                                               int nlb, int cellblk) {
+  const int lb = (int)blockIdx.x % nlb, l = (int)blockIdx.x / nlb / cellblk;
+  const int ci = (int)blockIdx.x / nlb % cellblk * kAdjFluxThreads + (int)threadIdx.x;
+  if (ci >= D.gall) return;
+  const int G = D.gall_1d, gmin = D.gmin, gmax = D.gmax;
+  const int i = ci % G + 1, j = ci / G + 1;
+  const unsigned c = ci;
+  const size_t fs = (size_t)D.lall * D.kall * D.gall, gw = (size_t)D.gall * D.lall, lg = (size_t)l * D.gall;
   const bool sgp = D.have_sgp[l] != 0;
-  if (kl % D.kall < D.kmin - 1 || kl % D.kall >= D.kmax) return;
+  const bool inI = i >= gmin && i <= gmax, inJ = j >= gmin && j <= gmax;
+  const bool ext = i >= gmin - 1 && i <= gmax && j >= gmin - 1 && j <= gmax;
+  const bool inO = inI && inJ;
+  const bool inN[3] = {inner(D, i + 1, j), inner(D, i + 1, j + 1), inner(D, i, j + 1)};
+  const bool face[3] = {ext && inJ && (inO || inN[0]), ext && (inO || inN[1]), ext && inI && (inO || inN[2])};
+  const bool singI = sgp && i == gmin - 1 && j == gmin - 1, singJ = sgp && i == gmin && j == gmin - 1;
+  double wI[3] = {}, wJ[3] = {}, wJm[3] = {}, wIm[3] = {}, wS[3] = {}, hn[3][3] = {}, ra[4] = {};
+  if (ext) {
+    auto weights = [&](int t, unsigned cell, double (&w)[3]) {
+#pragma unroll
+      for (int n = 0; n < 3; ++n) w[n] = (g.GMTR_t + ((size_t)(W1 - 1 + n) * 2 + (t - 1)) * gw + lg)[cell];
+    };
+    weights(TI, c, wI), weights(TJ, c, wJ);
+    if (inJ) weights(TJ, c - G, wJm);
+    if (inI) weights(TI, c - 1, wIm);
+    if (singI) weights(TJ, c + 1, wS);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int x = 0; x < 3; ++x) hn[a][x] = (g.GMTR_a + ((size_t)x * 3 + a) * gw + lg)[c];
+    const double *rarea = g.GMTR_p + (size_t)(P_RAREA - 1) * gw + lg;
+    ra[0] = rarea[c], ra[1] = rarea[c + 1], ra[2] = rarea[c + G + 1], ra[3] = rarea[c + G];
+  }
+  const int k0 = D.kmin - 1 + lb * lpb, k1 = min(k0 + lpb, D.kmax);  // the ghost levels have no part in the step
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) {
+    const size_t off = ((size_t)l * D.kall + k) * D.gall;
+    auto cell = [&](unsigned p) { return Tv{{(F.f[0] + off)[p], (F.f[1] + off)[p], (F.f[2] + off)[p], (F.f[3] + off)[p]}}; };
+    if (k + 1 < k1) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x) asm volatile("prefetch.global.L1 [%0];" ::"l"(F.f[x] + off + D.gall + c));
+#pragma unroll
+      for (int x = 0; x < 9; ++x) prefetch_l2(a_xc + (size_t)x * fs + off + D.gall + c);
+#pragma unroll
+      for (int x = 0; x < 6; ++x) prefetch_l2(a_flx + (size_t)x * fs + off + D.gall + c);
+    }
+    double afl[3] = {}, axc[3][3] = {};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const unsigned nb = c + (a == 0 ? 1 : (a == 1 ? G + 1 : G));
+      if (!face[a]) continue;
+      if (inO) afl[a] = (a_flx + (size_t)a * fs + off)[c] * ra[0] * dt;
+      if (inN[a] && !(a == 2 && singJ)) afl[a] += -(a_flx + (size_t)(a + 3) * fs + off)[nb] * ra[a + 1] * dt;
+#pragma unroll
+      for (int x = 0; x < 3; ++x) axc[a][x] = (a_xc + ((size_t)x * 3 + a) * fs + off)[c];
+    }
+    Tv tI{}, tJ{}, tJm{}, tIm{};
+    if (ext) {
+      const Tv f00 = cell(c), f10 = cell(c + 1), f11 = cell(c + G + 1), f01 = cell(c + G);
+      Tv f0m{}, fm0{};
+      if (inJ) f0m = cell(c - G);
+      if (inI) fm0 = cell(c - 1);
+      tI = tri(f00, f10, f11, wI), tJ = tri(f00, f11, f01, wJ);
+      tJm = tri(f0m, f10, f00, wJm), tIm = tri(fm0, f00, f01, wIm);
+      if (singI) tI = tri(f10, cell(c + G + 2), f11, wS);
+      if (singJ) tIm = tJ;
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      double avs[3] = {}, ars = 0.0;
+      if (face[a]) {
+        const Tv &p = (a == 0) ? tJm : (a == 1 ? tI : tJ), &q = (a == 0) ? tI : (a == 1 ? tJ : tIm);
+        const double rsum = p.v[0] + q.v[0], rr = 1.0 / mx(rsum, kEps);
+        double arr = 0.0;
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+          const double ax = axc[a][x];
+          avs[x] = 0.5 * afl[a] * hn[a][x];
+          avs[x] += -ax * rr * dt * 0.5;
+          arr += -ax * (p.v[x + 1] + q.v[x + 1]) * dt * 0.5;
+        }
+        ars = (rsum > kEps) ? -arr * rr * rr : 0.0;
+      }
+      (a_rs + (size_t)a * fs + off)[c] = ars;
+#pragma unroll
+      for (int x = 0; x < 3; ++x) (a_xc + ((size_t)x * 3 + a) * fs + off)[c] = avs[x];
+    }
+  }
+}
+
+// fields from the faces: point p is ij of TI/TJ(p) (W1), ip1j of TI(p-1) (W2),
+// ip1jp1 of TI(p-G-1) (W3) and TJ(p-G-1) (W2), ijp1 of TJ(p-G) (W3); on a singular
+// region TI(gmin-1,gmin-1) is TJ(gmin,gmin-1).  TI(c) has the faces AI(c), AIJ(c), AJ(c+1),
+// TJ(c) the faces AIJ(c), AI(c+G), AJ(c)
+__global__ void __launch_bounds__(kAdjFluxThreads) k_adj_fields(Dims D, const double *GT, const double *a_rs,
+                                                               const double *a_xc, int lpb, int nlb, int cellblk,
+                                                               double *a0, double *a1, double *a2, double *a3) {
+  const int lb = (int)blockIdx.x % nlb, l = (int)blockIdx.x / nlb / cellblk;
+  const int p = (int)blockIdx.x / nlb % cellblk * kAdjFluxThreads + (int)threadIdx.x;
+  if (p >= D.gall) return;
+  const int G = D.gall_1d, i = p % G + 1, j = p / G + 1;
+  const size_t fs = (size_t)D.lall * D.kall * D.gall, gw = (size_t)D.gall * D.lall;
+  const bool sgp = D.have_sgp[l] != 0;
   const int sg = (D.gmin - 2) * G + (D.gmin - 2);
-  auto ok = [&](int c) {
-    if (c < 0 || c >= D.gall) return false;
-    const int i = c % G + 1, j = c / G + 1;
-    return i >= D.gmin - 1 && i <= D.gmax && j >= D.gmin - 1 && j <= D.gmax;
+  const bool i0 = i >= D.gmin - 1 && i <= D.gmax, j0 = j >= D.gmin - 1 && j <= D.gmax;  // p owns triangles
+  const bool im = i >= D.gmin && i - 1 <= D.gmax, jm = j >= D.gmin && j - 1 <= D.gmax;  // ip-1, jp-1 do
+  const bool ok[4] = {i0 && j0, im && j0, im && jm, i0 && jm};
+  auto w = [&](bool on, int c, int t, int wi) {
+    return on ? GT[((size_t)(wi - 1) * 2 + (t - 1)) * gw + (size_t)l * D.gall + c] : 0.0;
   };
-  auto w = [&](int c, int t, int wi) { return GT[((size_t)(wi - 1) * 2 + (t - 1)) * gw + (size_t)l * D.gall + c]; };
-  auto aI = [&](int c, int x) { return (sgp && c == sg) ? 0.0 : aT[(size_t)x * fs + off + c]; };
-  auto aJ = [&](int c, int x) {
-    double v = aT[(size_t)(4 + x) * fs + off + c];
-    if (sgp && c == sg + 1) v += aT[(size_t)x * fs + off + sg];
-    return v;
-  };
-  double *out[4] = {a0, a1, a2, a3};
-  for (int x = 0; x < 4; ++x) {
-    double s = 0.0;
-    if (ok(p)) s += aI(p, x) * w(p, TI, W1) + aJ(p, x) * w(p, TJ, W1);
-    if (ok(p - 1)) s += aI(p - 1, x) * w(p - 1, TI, W2);
-    if (ok(p - G - 1)) s += aI(p - G - 1, x) * w(p - G - 1, TI, W3) + aJ(p - G - 1, x) * w(p - G - 1, TJ, W2);
-    if (ok(p - G)) s += aJ(p - G, x) * w(p - G, TJ, W3);
-    out[x][off + p] += s;
+  const double w0I = w(ok[0], p, TI, W1), w0J = w(ok[0], p, TJ, W1), w1I = w(ok[1], p - 1, TI, W2),
+               w2I = w(ok[2], p - G - 1, TI, W3), w2J = w(ok[2], p - G - 1, TJ, W2), w3J = w(ok[3], p - G, TJ, W3);
+  const int k0 = D.kmin - 1 + lb * lpb, k1 = min(k0 + lpb, D.kmax);
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) {
+    const size_t off = ((size_t)l * D.kall + k) * D.gall;
+    double sum[4];
+    if (k + 1 < k1) {
+#pragma unroll
+      for (int x = 0; x < 9; ++x) prefetch_l2(a_xc + (size_t)x * fs + off + D.gall + p);
+#pragma unroll
+      for (int x = 0; x < 3; ++x) prefetch_l2(a_rs + (size_t)x * fs + off + D.gall + p);
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      auto f = [&](int a, int c) { return ((x == 0 ? a_rs + (size_t)a * fs : a_xc + ((size_t)(x - 1) * 3 + a) * fs) + off)[c]; };
+      auto sumI = [&](int c) { return f(0, c) + f(1, c) + f(2, c + 1); };
+      auto aI = [&](int c) { return (sgp && c == sg) ? 0.0 : sumI(c); };
+      auto aJ = [&](int c) {
+        double v = f(1, c) + f(0, c + G) + f(2, c);
+        if (sgp && c == sg + 1) v += sumI(sg);
+        return v;
+      };
+      double s = 0.0;
+      if (ok[0]) s += aI(p) * w0I + aJ(p) * w0J;
+      if (ok[1]) s += aI(p - 1) * w1I;
+      if (ok[2]) s += aI(p - G - 1) * w2I + aJ(p - G - 1) * w2J;
+      if (ok[3]) s += aJ(p - G) * w3J;
+      sum[x] = s;
+    }
+    a0[off + p] += sum[0], a1[off + p] += sum[1], a2[off + p] += sum[2], a3[off + p] += sum[3];
   }
 }
 
@@ -1070,8 +1118,6 @@ __global__ void k_adj_flux_pl(int kall, Geo<double> g, Fld F, const double *a_fl
     }
   }
 }
-
-dim3 slab(const Dims &D, int th) { return dim3((D.gall + th - 1) / th, D.kall * D.lall); }
 
 template <int TX>
 cudaError_t launch_adj_cells(const AdjArgs &A, cudaStream_t st) {
@@ -1157,8 +1203,15 @@ int step_adjoint(StepCtx &S, const AdjScratch &A, int ntr, double dt, const doub
   k_adj_rhoh_ch_pl<<<nbl, 128, 0, st>>>(D.kall, rhog_pl, S.flx_pl, A.a_rh_pl, A.a_ch_pl, A.a_flx_pl, a_rhog_pl);
   const Fld F{{rhog, vx, vy, vz}};
   const Fld Fp{{rhog_pl, vx_pl, vy_pl, vz_pl}};
-  k_adj_tri<<<slab(D, T), T, 0, st>>>(D, S.geo, F, A.a_flx, A.a_xc, dt, A.aT);
-  k_adj_fields<<<slab(D, T), T, 0, st>>>(D, S.geo.GMTR_t, A.aT, a_rhog, a_vx, a_vy, a_vz);
+  {
+    const int cb = (D.gall + kAdjFluxThreads - 1) / kAdjFluxThreads;
+    int lpb = kAdjFluxLevels;  // fewer where the blocks would not fill the SMs
+    while (lpb > 1 && (long long)cb * D.lall * ((NK + lpb - 1) / lpb) < 4 * 148) lpb /= 2;
+    const int nlb = (NK + lpb - 1) / lpb;
+    const unsigned nb = (unsigned)(cb * D.lall * nlb);
+    k_adj_tri<<<nb, kAdjFluxThreads, 0, st>>>(D, S.geo, F, A.a_flx, A.a_xc, dt, A.a_rs, lpb, nlb, cb);
+    k_adj_fields<<<nb, kAdjFluxThreads, 0, st>>>(D, S.geo.GMTR_t, A.a_rs, A.a_xc, lpb, nlb, cb, a_rhog, a_vx, a_vy, a_vz);
+  }
   k_adj_flux_pl<<<nbl, 128, 0, st>>>(D.kall, S.geo, Fp, A.a_flx_pl, A.a_xc_pl, dt, a_rhog_pl, a_vx_pl, a_vy_pl,
                                      a_vz_pl);
   launches += 4;

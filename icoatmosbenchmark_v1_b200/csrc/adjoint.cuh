@@ -11,7 +11,7 @@ struct AdjScratch {
   // a group of tracers: rhogq after the horizontal sub-step (poles), the adjoint of q = rhogq / rhog
   // (a_q holds rhogq after the horizontal sub-step until the column pass has read it) and of bb
   double *Qh_pl, *a_q, *a_q_pl, *a_bb;
-  double *aT;              // triangle adjoints of horizontal_flux (8 fields, over a_q)
+  double *a_rs;            // adjoint of a face's density sum in horizontal_flux (3 fields, over a_q)
   double *a_flx, *a_flx_pl, *a_xc, *a_xc_pl, *a_ch_pl, *a_rh, *a_rh_pl;
 };
 

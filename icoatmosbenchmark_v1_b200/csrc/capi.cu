@@ -729,8 +729,8 @@ static int adj_scratch(Ctx *c, AdjScratch &A) {
     *b.p = (double *)c->buf(b.name, b.n * sizeof(double));
     if (!*b.p) return set_error(std::string("cudaMalloc ") + b.name), ICA_ERR_NOMEM;
   }
-  static_assert(kPlainGroup == 8, "the 8 triangle-adjoint fields reuse a_q after the tracers");
-  A.aT = A.a_q;
+  static_assert(kPlainGroup >= 3, "the 3 fields of a_rs reuse a_q after the tracers");
+  A.a_rs = A.a_q;
   return ICA_OK;
 }
 
