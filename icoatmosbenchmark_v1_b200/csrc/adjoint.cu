@@ -904,7 +904,7 @@ __global__ void k_adj_rhoh_ch_pl(int kall, const double *rho_pl, const double *f
 // cell's levels with its weights and normals in registers, as the forward does, and ask
 // for the next level's planes while a level is worked on: the latency of a level's loads
 // bounds them.  One thread per triangle pair and level (each face transposed five times,
-// twelve triangle values a cell) took 2.38 + 1.03 ms at glevel 7, kall 96.  At glevel 6,
+// twelve triangle values a cell) took 2.38 + 1.03 ms at glevel 7, kall 96; now 0.96 + 0.93.  At glevel 6,
 // kall 42: 119 + 112 us a step, of 70 + 45 at the copy rate; k_adj_tri at 3 blocks per SM
 // 136, without the prefetch 145, 5 blocks 206 (spills), 16 levels a thread 170;
 // k_adj_fields without the prefetch 122.
