@@ -38,6 +38,20 @@ void *Ctx::buf(const char *name, size_t bytes) {
   return b.ptr;
 }
 
+// A host table of n ints as a new device array in *dst.  Complete on return: a copy from pageable memory may
+// come back with its last bytes still on their way, and a context's stream does not wait for the
+// legacy stream.  On failure *dst is null or the context's to free, and no error is left for a later call.
+static int upload_ints(int **dst, const int *src, size_t n, const char *what) {
+  if (cudaMalloc(dst, sizeof(int) * (n + 1)) != cudaSuccess) {
+    *dst = nullptr;
+    cudaGetLastError();
+    return set_error(std::string("cudaMalloc(") + what + ")"), ICA_ERR_NOMEM;
+  }
+  cudaError_t e = cudaMemcpy(*dst, src, sizeof(int) * n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  return e == cudaSuccess ? ICA_OK : cuda_fail(e, what);
+}
+
 void Ctx::release(const char *name) {
   auto it = bufs.find(name);
   if (it == bufs.end()) return;
@@ -120,28 +134,15 @@ int ica_init(const ica_dims *dims, ica_ctx **out) {
     for (size_t q = 0; q < m.size(); ++q)
       if (m[q] != (int)q) d[ne] = (int)q, sr[ne] = m[q], ++ne;
     d.resize(ne), sr.resize(ne);
-    if (pf == 0) {
-      if (cudaMalloc(&c->halo_src, sizeof(int) * m.size()) != cudaSuccess) {
-        delete c;
-        return set_error("cudaMalloc(halo sources)"), ICA_ERR_NOMEM;
-      }
-      cudaMemcpy(c->halo_src, m.data(), sizeof(int) * m.size(), cudaMemcpyHostToDevice);
-    }
     Plan &p = c->plan[pf];
-    p.n = (int)d.size();
-    if (cudaMalloc(&p.dst, sizeof(int) * (p.n + 1)) != cudaSuccess ||
-        cudaMalloc(&p.src, sizeof(int) * (p.n + 1)) != cudaSuccess) {
-      delete c;
-      return set_error("cudaMalloc(plan)"), ICA_ERR_NOMEM;
-    }
-    cudaMemcpy(p.dst, d.data(), sizeof(int) * p.n, cudaMemcpyHostToDevice);
-    cudaMemcpy(p.src, sr.data(), sizeof(int) * p.n, cudaMemcpyHostToDevice);
+    p.n = (int)ne;
+    if (pf == 0) rc = upload_ints(&c->halo_src, m.data(), m.size(), "halo sources");
+    if (!rc) rc = upload_ints(&p.dst, d.data(), ne, "plan");
+    if (!rc) rc = upload_ints(&p.src, sr.data(), ne, "plan");
+    if (rc) { delete c; return rc; }
   }
-  if (cudaMalloc(&c->d_have_sgp, sizeof(int) * t.nrgn) != cudaSuccess) {
-    delete c;
-    return set_error("cudaMalloc(have_sgp)"), ICA_ERR_NOMEM;
-  }
-  cudaMemcpy(c->d_have_sgp, t.have_sgp.data(), sizeof(int) * t.nrgn, cudaMemcpyHostToDevice);
+  rc = upload_ints(&c->d_have_sgp, t.have_sgp.data(), t.have_sgp.size(), "have_sgp");
+  if (rc) { delete c; return rc; }
   c->D.gall_1d = s.gall_1d;
   c->D.gall = s.gall;
   c->D.gmin = s.gmin;
@@ -188,12 +189,8 @@ int ica_init_regions(int gall_1d, int kall, int kmin, int kmax, int lall, int ha
   s.lall_pl = kLallPl;
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaStreamCreate"); }
-  if (cudaMalloc(&c->d_have_sgp, sizeof(int) * lall) != cudaSuccess) {
-    delete c;
-    return set_error("cudaMalloc(have_sgp)"), ICA_ERR_NOMEM;
-  }
-  e = cudaMemcpy(c->d_have_sgp, have_sgp, sizeof(int) * lall, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaMemcpy(have_sgp)"); }
+  rc = upload_ints(&c->d_have_sgp, have_sgp, (size_t)lall, "have_sgp");
+  if (rc) { delete c; return rc; }
   c->D.gall_1d = s.gall_1d, c->D.gall = s.gall, c->D.gmin = s.gmin, c->D.gmax = s.gmax;
   c->D.kall = s.kall, c->D.kmin = s.kmin, c->D.kmax = s.kmax;
   c->D.lall = s.lall;
