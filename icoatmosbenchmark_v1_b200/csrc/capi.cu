@@ -989,19 +989,18 @@ int Ctx::build_fast_tables() {
   fast.nb = (int)blist.size();
   fast.ncarry = (int)carry.size();
   fast.ns = (int)seam_list.size();
-  if (cudaMalloc(&fast.bsrc, bsrc.size() * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&fast.blist, blist.size() * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&fast.ring, ring.size() * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&fast.carry, carry.size() * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&fast.seam_list, seam_list.size() * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&fast.seam_id, seam_id.size() * sizeof(int)) != cudaSuccess)
-    return set_error("cudaMalloc(fast tables)"), ICA_ERR_NOMEM;
-  cudaMemcpy(fast.bsrc, bsrc.data(), bsrc.size() * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(fast.blist, blist.data(), blist.size() * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(fast.ring, ring.data(), ring.size() * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(fast.carry, carry.data(), carry.size() * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(fast.seam_list, seam_list.data(), seam_list.size() * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(fast.seam_id, seam_id.data(), seam_id.size() * sizeof(int), cudaMemcpyHostToDevice);
+  const struct {
+    int **dst;
+    const std::vector<int> &src;
+  } tables[] = {{&fast.bsrc, bsrc},   {&fast.blist, blist},         {&fast.ring, ring},
+                {&fast.carry, carry}, {&fast.seam_list, seam_list}, {&fast.seam_id, seam_id}};
+  for (auto &x : tables) {
+    rc = upload_ints(x.dst, x.src.data(), x.src.size(), "boundary tables");
+    if (rc) {  // the next call starts over
+      for (auto &y : tables) cudaFree(*y.dst), *y.dst = nullptr;
+      return rc;
+    }
+  }
   fast.built = true;
   return ICA_OK;
 }

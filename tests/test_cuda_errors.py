@@ -137,3 +137,48 @@ def test_init_reports_a_failed_call_and_can_be_repeated(child, kind):
     assert len(out) >= 6  # the halo map, two plans of two lists, the singular-point flags
     for n, (first, live, again) in enumerate(out, 1):
         assert not first and live == 0 and again, (n, first, live, again)
+
+
+STEP = r"""
+kind, out = sys.argv[2], []
+n, shapes = 1, lambda ctx: ((ctx.sizes.lall, ctx.sizes.kall, ctx.sizes.gall), (2, ctx.sizes.kall, 6))
+while True:
+    ctx = api.IcoAdv(2, 0, 4)
+    ctx.set_grid(Grid(2, 0, 6))
+    reg, pol = shapes(ctx)
+    arrs = [np.ones(reg), np.ones(pol), np.ones((2,) + reg), np.ones((2,) + pol)]
+    arrs += [np.ones(s) for _ in range(4) for s in (reg, pol)]
+
+    def step():
+        try:
+            ctx.advect_step(1.0, *arrs)
+            return True
+        except api.IcoAdvError:
+            return False
+
+    fake.fake_reset()
+    fail(kind, n)
+    first = step()
+    if calls(kind) < n:
+        break
+    launched = calls("cudaLaunchKernel")
+    fake.fake_reset()
+    again = step()
+    copies = calls("cudaMemcpy")
+    ctx.close()
+    out.append([first, launched, again, copies, fake.fake_live()])
+    n += 1
+print(json.dumps(out))
+"""
+
+
+@pytest.mark.parametrize("kind", ["cudaMalloc", "cudaMemcpy"])
+def test_plain_step_whose_tables_failed_can_be_repeated(child, kind):
+    """The plain step builds the boundary tables on its first call.  Whatever fails there, nothing is launched on
+    the state, and the next call builds what is missing and succeeds; closing the context frees all of it."""
+    out = child(STEP, kind)
+    assert len(out) >= 6
+    for n, (first, launched, again, copies, live) in enumerate(out, 1):
+        assert not first and launched == 0 and again and live == 0, (n, first, launched, again, live)
+        if kind == "cudaMemcpy":
+            assert copies == 6, (n, copies)
