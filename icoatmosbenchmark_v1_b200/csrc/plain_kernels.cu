@@ -593,9 +593,12 @@ void launch_horizontal_flux(const Dims &D, const FluxIn<T> &in, const FluxOut<T>
                             cudaStream_t s) {
   const int cellblk = (D.gall + kFluxThreads - 1) / kFluxThreads;
   // a grid whose levels fit one wave (4 blocks on each of 148 SMs) in runs of at most 12 takes that
-  // split: 130 x 130 x 42 in one region, 38.4 us a call at 11 levels against 40.2 at 8 (1.35 waves)
-  const int fit = 4 * 148 / (cellblk * D.lall), one = fit > 0 ? (D.kall + fit - 1) / fit : D.kall;
-  const int lpb = one <= 12 ? one : kFluxLevels;
+  // split: 130 x 130 x 42 in one region, 38.4 us a call at 11 levels against 40.2 at 8 (1.35 waves).
+  // Where not one level fits (fit = 0) there is no such split, and runs of 8 in the fixed form are the
+  // faster ones: glevel 7, kall 7, 9 and 12 take 54, 68 and 81 us, in one run of all levels 59, 72
+  // and 92; glevel 8, kall 6 and 12 150 and 287 against 160 and 296, kall 9 (runs of 8 and 1) 231 against 226
+  const int fit = 4 * 148 / (cellblk * D.lall), one = fit > 0 ? (D.kall + fit - 1) / fit : 0;
+  const int lpb = fit > 0 && one <= 12 ? one : kFluxLevels;
   const int nlb = (D.kall + lpb - 1) / lpb;
   const int nmain = nlb * cellblk * D.lall;
   const int npole = D.have_pl ? (D.kall * kLallPl + kFluxThreads - 1) / kFluxThreads : 0;

@@ -20,7 +20,7 @@ FAKE = r"""
 #include <string>
 static std::map<std::string, long> calls, fail_at;
 static cudaError_t last = cudaSuccess;
-static long live = 0;
+static long live = 0, blocks = 0;
 static cudaError_t call(const char *name) {
   const long n = ++calls[name];
   const auto f = fail_at.find(name);
@@ -32,6 +32,7 @@ void fake_reset() { calls.clear(), fail_at.clear(); }
 void fake_fail(const char *name, long nth) { fail_at[name] = nth; }
 long fake_calls(const char *name) { return calls[name]; }
 long fake_live() { return live; }
+long fake_blocks() { return blocks; }  // of the latest launch
 cudaError_t cudaGetLastError() { const cudaError_t e = last; last = cudaSuccess; return e; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
@@ -69,7 +70,10 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = (cudaStr
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
-cudaError_t cudaLaunchKernel(const void *, dim3, dim3, void **, size_t, cudaStream_t) { return call("cudaLaunchKernel"); }
+cudaError_t cudaLaunchKernel(const void *, dim3 g, dim3, void **, size_t, cudaStream_t) {
+  blocks = (long)g.x * g.y * g.z;
+  return call("cudaLaunchKernel");
+}
 }
 """
 
@@ -80,7 +84,7 @@ import numpy as np
 from icoatmosbenchmark_v1_b200 import api
 from icoatmosbenchmark_v1_b200.grid import Grid
 fake = C.CDLL(None)
-for f in (fake.fake_calls, fake.fake_live):
+for f in (fake.fake_calls, fake.fake_live, fake.fake_blocks):
     f.restype = C.c_long
 calls = lambda name: fake.fake_calls(name.encode())
 fail = lambda name, nth: fake.fake_fail(name.encode(), C.c_long(nth))
