@@ -38,17 +38,21 @@ void *Ctx::buf(const char *name, size_t bytes) {
   return b.ptr;
 }
 
-// A host table of n ints as a new device array in *dst.  Complete on return: a copy from pageable memory may
-// come back with its last bytes still on their way, and a context's stream does not wait for the
-// legacy stream.  On failure *dst is null or the context's to free, and no error is left for a later call.
+// A host table of n ints as a new device array in *dst, complete after the uploads_done() that follows it and its
+// neighbours.  On failure *dst is null or the context's to free, and no error is left for a later call.
 static int upload_ints(int **dst, const int *src, size_t n, const char *what) {
   if (cudaMalloc(dst, sizeof(int) * (n + 1)) != cudaSuccess) {
     *dst = nullptr;
     cudaGetLastError();
     return set_error(std::string("cudaMalloc(") + what + ")"), ICA_ERR_NOMEM;
   }
-  cudaError_t e = cudaMemcpy(*dst, src, sizeof(int) * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  const cudaError_t e = cudaMemcpy(*dst, src, sizeof(int) * n, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? ICA_OK : cuda_fail(e, what);
+}
+// A copy from pageable memory may come back with its last bytes still on their way, and a context's
+// stream does not wait for the legacy stream.
+static int uploads_done(const char *what) {
+  const cudaError_t e = cudaStreamSynchronize(nullptr);
   return e == cudaSuccess ? ICA_OK : cuda_fail(e, what);
 }
 
@@ -142,6 +146,7 @@ int ica_init(const ica_dims *dims, ica_ctx **out) {
     if (rc) { delete c; return rc; }
   }
   rc = upload_ints(&c->d_have_sgp, t.have_sgp.data(), t.have_sgp.size(), "have_sgp");
+  if (!rc) rc = uploads_done("ica_init");
   if (rc) { delete c; return rc; }
   c->D.gall_1d = s.gall_1d;
   c->D.gall = s.gall;
@@ -190,6 +195,7 @@ int ica_init_regions(int gall_1d, int kall, int kmin, int kmax, int lall, int ha
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaStreamCreate"); }
   rc = upload_ints(&c->d_have_sgp, have_sgp, (size_t)lall, "have_sgp");
+  if (!rc) rc = uploads_done("ica_init_regions");
   if (rc) { delete c; return rc; }
   c->D.gall_1d = s.gall_1d, c->D.gall = s.gall, c->D.gmin = s.gmin, c->D.gmax = s.gmax;
   c->D.kall = s.kall, c->D.kmin = s.kmin, c->D.kmax = s.kmax;
@@ -994,12 +1000,12 @@ int Ctx::build_fast_tables() {
     const std::vector<int> &src;
   } tables[] = {{&fast.bsrc, bsrc},   {&fast.blist, blist},         {&fast.ring, ring},
                 {&fast.carry, carry}, {&fast.seam_list, seam_list}, {&fast.seam_id, seam_id}};
-  for (auto &x : tables) {
-    rc = upload_ints(x.dst, x.src.data(), x.src.size(), "boundary tables");
-    if (rc) {  // the next call starts over
-      for (auto &y : tables) cudaFree(*y.dst), *y.dst = nullptr;
-      return rc;
-    }
+  for (auto &x : tables)
+    if (!rc) rc = upload_ints(x.dst, x.src.data(), x.src.size(), "boundary tables");
+  if (!rc) rc = uploads_done("boundary tables");
+  if (rc) {  // the next call starts over
+    for (auto &x : tables) cudaFree(*x.dst), *x.dst = nullptr;
+    return rc;
   }
   fast.built = true;
   return ICA_OK;
