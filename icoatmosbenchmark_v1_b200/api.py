@@ -218,7 +218,7 @@ class IcoAdv:
         if self.h:
             lib().ica_finalize(self.h)
             self.h = C.c_void_p()
-    
+
     def __del__(self):
         try:
             self.close()

@@ -126,7 +126,7 @@ __global__ void k_adj_vrho(Dims D, double *a_rho, double *a_rho_pl, double *a_rh
 // ---------------------------------------------------------------------------
 // vertical sub-step of one tracer, one column per thread, levels streamed from the top.
 //
-// Forward (step.cu k_vertical, mod_src_tracer.f90:107-186 with d = 0):
+// Forward (step.cu k_plain_column, mod_src_tracer.f90:107-186 with d = 0):
 //   qc(k) = Qh(k) / rh(k), ghosts qc(1) = qc(kmin), qc(kall) = qc(kmax)
 //   ck1(k) = -w(k) dt rdgz(k) / rh(k), ck2(k) = w(k+1) dt rdgz(k) / rh(k), ck1(kall) likewise
 //   qh(k) = afact(k) qc(k) + bfact(k) qc(k-1), clamped to the Qout bounds of level k-1 or k

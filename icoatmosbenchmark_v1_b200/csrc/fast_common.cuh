@@ -110,10 +110,6 @@ __device__ __forceinline__ int find_inst(const MultiInst &M, long long &w, F cnt
 __device__ __forceinline__ double fsg(double a, double b) { return copysign(fabs(a), b); }
 __device__ __forceinline__ double mn64(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double mx64(double a, double b) { return (b > a) ? b : a; }
-// FP32 min / max: one FMNMX instruction each (the select form takes a compare and a select).
-// Operands here are never NaN; for them the two agree except for the sign of a zero result.
-__device__ __forceinline__ float mn32(float a, float b) { return fminf(a, b); }
-__device__ __forceinline__ float mx32(float a, float b) { return fmaxf(a, b); }
 
 // field readers at flat offset o: var 0..3 = rhogvx, rhogvy, rhogvz, rhogw (FP64 of either variant)
 __device__ __forceinline__ double fld(const FastInst &I, int var, size_t o) {
@@ -131,6 +127,8 @@ template <> struct Arith<float> {
   using V2 = float2;
   using V4 = float4;
   static constexpr float BIG = FLT_MAX, RR_EPS = FLT_EPSILON;
+  // one FMNMX instruction each (the select form takes a compare and a select); operands here are
+  // never NaN, and for them the two agree except for the sign of a zero result
   static __device__ __forceinline__ float mn(float a, float b) { return fminf(a, b); }
   static __device__ __forceinline__ float mx(float a, float b) { return fmaxf(a, b); }
   static __device__ __forceinline__ float sgn(float a, float b) { return copysignf(a, b); }
@@ -233,30 +231,6 @@ __device__ __forceinline__ double face_geo(const FastInst &I, int l, int i, int 
   xc[1] = gxr(I, l, i, j, a, 2) - vy * rr * I.dt * 0.5;
   xc[2] = gxr(I, l, i, j, a, 3) - vz * rr * I.dt * 0.5;
   return flux;
-}
-
-// 4-point bounds of face a of cell (i,j) incl. the clamps (:152-153) and the singular AIJ stencil (:192-214)
-template <class QAcc>
-__device__ __forceinline__ void bounds64(const FastInst &I, int i, int j, int a, bool sgp, const QAcc &q,
-                                         double &lo, double &hi) {
-  const int G = I.G;
-  const int ij = (j - 1) * G + i;
-  int im1j = ij - 1, ijm1 = ij - G;
-  if (im1j < 1) im1j = 1;
-  if (ijm1 < 1) ijm1 = 1;
-  auto Q = [&](int cell) { return q((cell - 1) % G + 1, (cell - 1) / G + 1); };
-  const double q0 = Q(ij);
-  double b, c, d;
-  if (a == AI) {
-    b = Q(ijm1), c = Q(ij + 1), d = Q(ij + G + 1);
-  } else if (a == AIJ) {
-    if (sgp && i == I.gmin - 1 && j == I.gmin - 1) b = Q(ij + G + 1), c = Q(ij + G + 2), d = Q(ij + G);
-    else b = Q(ij + 1), c = Q(ij + G + 1), d = Q(ij + G);
-  } else {
-    b = Q(ij + G + 1), c = Q(ij + G), d = Q(im1j);
-  }
-  lo = mn64(mn64(mn64(q0, b), c), d);
-  hi = mx64(mx64(mx64(q0, b), c), d);
 }
 
 // flx_h(c, m) of the reference from face fluxes (FP64), with halo zeros and the singular zero

@@ -220,7 +220,7 @@ __global__ void k_fast_boundary(const __grid_constant__ MultiInst M) {
   for (int x = 0; x < 3; ++x)
     for (int n = 0; n < 7; ++n) cgr[x][n] = I.cg[(((size_t)l * 3 + x) * 7 + n) * I.gall + c];
   const int di7[7] = {0, 1, 1, 0, -1, -1, 0}, dj7[7] = {0, 0, 1, 1, 0, -1, -1};
-  // The 4 points of each face's bounds (bounds64 for the face's owner), as offsets in the 3x3
+  // The 4 points of each face's bounds (mod_src_tracer.f90:152-214), as offsets in the 3x3
   // block: a region-boundary cell lies in [gmin, gmax]^2, so every point is in the block and
   // no index clamp applies.  Face 5's owner is the singular corner (gmin-1, gmin-1) when the
   // cell is (gmin, gmin) of a region with the singular point: then its points shift.
@@ -254,7 +254,7 @@ __global__ void k_fast_boundary(const __grid_constant__ MultiInst M) {
       for (int n = 1; n <= 6; ++n) s = s + cgr[x][n] * q9[1 + dj7[n]][1 + di7[n]];
       out[x] = s;
     }
-    // (q0, b, c, d) of bounds64, in its order
+    // a face's owner, then its other three points in the reference's order (mod_src_tracer.f90:152-214)
     double lo[7], hi[7];
     auto b4 = [&](int m, double q0, double b, double c, double d) {
       lo[m] = mn64(mn64(mn64(q0, b), c), d);
@@ -325,7 +325,8 @@ __global__ void k_fast_seam(const __grid_constant__ MultiInst M) {
   const int bu = I.bsrc[(size_t)l * I.gall + (uj - 1) * G + (ui - 1)];
   double dxu[3];
   for (int x = 0; x < 3; ++x) dxu[x] = xc[x] - gx(I, l, ui, uj, x);
-  // the 4 cells of the face's bounds (bounds64's selection) and 1/rho there; the owner is [0]
+  // the 4 cells of the face's bounds (mod_src_tracer.f90:152-214, with its index clamps and its singular
+  // stencil) and 1/rho there; the owner is [0]
   int pc[4];
   {
     const int ij = (j - 1) * G + i;

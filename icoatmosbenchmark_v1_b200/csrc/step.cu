@@ -5,7 +5,8 @@
 //
 // The composition (horizontal sub-step, then vertical sub-step, then the halo
 // fill of the state) and every formula match the CPU oracle's definition of
-// the step; compiled with --fmad=false the FP64 results equal it bit for bit.
+// the step; compiled with --fmad=false the FP64 results of a finite state equal
+// it bit for bit.
 //
 //   ch    = flx_h / rhog,  cmask = 0.5 - sign(0.5, ch - EPS)
 //   q     = rhogq / rhog
@@ -44,7 +45,9 @@ namespace icoadv {
 // (14 launches a tracer, a column's levels in local memory): 9.90 -> 3.17 ms for glevel 7, kall 61,
 // 5 tracers, 1.59 -> 0.30 ms for glevel 5, kall 42, 8 tracers.  Every value is the result of the
 // reference's operation sequence; where the reference blends two sides by a mask of 0 or 1
-// (c a + (1 - c) b), the chosen side is taken, which is the same number.
+// (c a + (1 - c) b), the chosen side is taken, which is the same number while both are finite.
+// A state that holds a NaN or an infinity keeps one there, but its faces' other cells get it only
+// where the face's flow or bounds bring it; the blend (0 * NaN) handed it upwind as well.
 constexpr int kTileCells = 256;  // threads of k_plain_cells: one per cell of a TX x (256 / TX) tile
 constexpr int kCellBlocks = 2;   // its blocks per SM: 128 registers a thread, which hold one tracer's values
 
